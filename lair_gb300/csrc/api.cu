@@ -526,6 +526,7 @@ int luhot_create(luhot_ctx** out, int device) {
   ok = ok && cudaMallocHost(&ctx->h_status, sizeof(DeviceStatus)) == cudaSuccess;
   ok = ok && cudaMallocHost(&ctx->h_scalars, kIrScalarSlots * sizeof(double)) == cudaSuccess;
   ok = ok && cudaMalloc(&ctx->panel_scratch, kPanelScratchBytes) == cudaSuccess;
+  if (ok) ctx->panel_cluster = panel_cluster_limit(ctx);
   if (!ok || ctx->num_sms > kMaxPanelCtas) {
     cudaGetLastError();
     luhot_destroy(ctx);

@@ -68,6 +68,7 @@ struct luhot_ctx {
   int device = 0;
   int num_sms = 0;
   int max_smem_optin = 0;
+  int panel_cluster = 0;  // largest cluster of panel CTAs (power of two) the device schedules; 0: none
   cudaStream_t own_stream = nullptr;
   cudaStream_t stream = nullptr;
   std::mutex mu;
@@ -125,6 +126,10 @@ int ensure_buf(luhot_ctx* ctx, DevBuf& b, size_t bytes);
 // are contiguous, a kernel for strided device-to-device, else cudaMemcpy2DAsync.
 int copy_2d(luhot_ctx* ctx, void* dst, size_t dpitch, const void* src, size_t spitch, size_t wbytes, size_t rows,
             cudaMemcpyKind kind);
+
+// Largest power-of-two cluster in which the cluster form of the panel
+// (panel_cluster.cu) can run with its full shared memory, 0 if none.
+int panel_cluster_limit(luhot_ctx* ctx);
 
 template <typename T>
 int getrf_device(luhot_ctx* ctx, int m, int n, T* a, int64_t lda, int* piv, int mode,
