@@ -357,18 +357,30 @@ __global__ void __launch_bounds__(kThreads) trsv_syncfree_kernel(const TA* __res
 size_t trsv_syncfree_smem(size_t elem) { return (2 * (size_t)kBS * kLds + 2 * (size_t)kBS * kMaxRhs) * elem; }
 int trsv_syncfree_blocks(int n) { return (n + kBS - 1) / kBS; }
 
-// Fast sweeps of more than four right-hand sides run as independent chains
-// of four (one launch): each chain step (the last off-diagonal tile and the
-// diagonal block of a 64-row block) is then a quarter of the FP64 work on
-// the critical path of one chain of sixteen.
-static int trsv_chains(bool exact, int nc) { return (!exact && nc > 4) ? (nc + 3) / 4 : 1; }
+// Right-hand sides of one chain.  Fast sweeps run every right-hand side as a
+// chain of its own while the sweep is bound by its chain (the last off-diagonal
+// tile and the diagonal inverse of a 64-row block on one SM: 2.4 us of FP64 work
+// a right-hand side), and in wider chains, which read the factor fewer times,
+// once the whole sweep's work is the bound.  Two sweeps with their inverses in
+// us, chains of 1 / 2 / 4: FP64 n = 2048, 8 rhs 354 / 430 / 669, n = 4097, 16 rhs
+// 1079 / 1170 / 1638, n = 16384, 4 rhs 4090 / 4407 / 6161, 8 rhs 6541 / 6226 /
+// 7614, 16 rhs 11777 / 10145 / 10879; FP32 n = 2048, 16 rhs 210 / 219 / 211,
+// n = 4097, 8 rhs 375 / 406 / 401, 16 rhs 512 / 447 / 427.  Exact sweeps stay one
+// chain (one order for all right-hand sides of the launch).
+static int trsv_width(bool exact, size_t elem, int n, int nc) {
+  const int one = nc > 4 ? kMaxRhs : nc > 2 ? 4 : nc;
+  if (exact) return one;
+  const int64_t work = (int64_t)n * nc;
+  const int w = elem == 8 ? (work > 100000 ? 2 : 1) : (work > 40000 ? 4 : 1);
+  return std::min(w, nc > 2 ? 4 : nc);
+}
 
 template <typename T, typename TA, bool EX, bool LO, bool UN, bool TR>
 static cudaError_t launch_case(cudaStream_t stream, const TA* a, int64_t lda, T* x, int64_t ldx, int n, int nc,
                                int* flags, int* ticket, DeviceStatus* st, const T* dinv) {
   const int nblk = trsv_syncfree_blocks(n);
   const size_t smem = trsv_syncfree_smem(sizeof(T));
-  const int nchain = trsv_chains(EX, nc);
+  const int width = trsv_width(EX, sizeof(T), n, nc), nchain = (nc + width - 1) / width;
   cudaError_t e;
 #define LUHOT_TRSV_NR(NR)                                                                                \
   {                                                                                                      \
@@ -378,9 +390,9 @@ static cudaError_t launch_case(cudaStream_t stream, const TA* a, int64_t lda, T*
     k<<<nblk * nchain, kThreads, smem, stream>>>(a, lda, x, ldx, n, nc, nchain, flags, ticket, st, dinv); \
     return cudaGetLastError();                                                                           \
   }
-  if (nc == 1) LUHOT_TRSV_NR(1)
-  if (nc == 2) LUHOT_TRSV_NR(2)
-  if (nc <= 4 || nchain > 1) LUHOT_TRSV_NR(4)
+  if (width == 1) LUHOT_TRSV_NR(1)
+  if (width == 2) LUHOT_TRSV_NR(2)
+  if (width == 4) LUHOT_TRSV_NR(4)
   LUHOT_TRSV_NR(16)
 #undef LUHOT_TRSV_NR
 }
@@ -394,7 +406,8 @@ cudaError_t launch_trsv_syncfree(cudaStream_t stream, const TA* a, int64_t lda, 
   if (exact) dinv = nullptr;  // inverses serve the fast sweeps only
   for (int c0 = 0; c0 < nrhs; c0 += kMaxRhs) {
     const int nc = std::min(kMaxRhs, nrhs - c0);
-    cudaError_t e = cudaMemsetAsync(flags, 0, (size_t)nblk * trsv_chains(exact, nc) * sizeof(int), stream);
+    const int width = trsv_width(exact, sizeof(T), n, nc);
+    cudaError_t e = cudaMemsetAsync(flags, 0, (size_t)nblk * ((nc + width - 1) / width) * sizeof(int), stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(ticket, 0, sizeof(int), stream);
     if (e != cudaSuccess) return e;
     T* xc = x + c0;
@@ -415,67 +428,93 @@ cudaError_t launch_trsv_syncfree(cudaStream_t stream, const TA* a, int64_t lda, 
   return cudaSuccess;
 }
 
-// Inverse of every 64 x 64 diagonal block of a triangular factor (lower unit
-// or upper non-unit), row-major 64 x 64 per block, zero-padded past n.  One
-// CTA per block, one thread per column of the inverse (substitution on the
-// unit vector), all in shared memory.
-template <typename T, typename TA, bool kLower, bool kUnit>
-__global__ void __launch_bounds__(kBS) trsv_invert_diag_kernel(const TA* __restrict__ a, int64_t lda, int n, T* dinv) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* S = reinterpret_cast<T*>(smem_raw);  // [64][65] diagonal block
-  T* Y = S + kBS * kLds;                   // [64][65] inverse, column c owned by thread c
+// Inverses of the 64 x 64 diagonal blocks of both triangles of an LU factor
+// (lower unit, upper non-unit), row-major 64 x 64 per block, zero past n.  A
+// CTA per (block, four columns, triangle), a warp per column: lane L holds rows
+// L and L + 32 of x and runs the column sweep x_i -= T(i,k) x_k with x_k by
+// shuffle.  A warp's FP64 instruction takes 64 cycles of its SM quarter's pipe
+// however few lanes it has, so the columns are spread over as many quarters as
+// there are: 4 warps a CTA, 16 CTAs a block.  (One CTA per block with a thread
+// per column and sums along the rows: 110 + 130 us for the two triangles at any
+// small n; this: 11 us for both, both in one launch.)
+constexpr int kInvCols = 4;
+
+// y / d for the warp's running quotient: by the reciprocal r = 1/d with one
+// correction step where r is a normal number (`good`), else by division.
+__device__ __forceinline__ double inv_quot(double y, double d, double r, bool good) {
+  if (!good) return y / d;
+  const double q = y * r;
+  return isfinite(q) ? fma(fma(-q, d, y), r, q) : q;
+}
+__device__ __forceinline__ float inv_quot(float y, float d, float, bool) { return y / d; }
+
+template <typename T, typename TA>
+__global__ void __launch_bounds__(32 * kInvCols) trsv_invert_diag_kernel(const TA* __restrict__ a, int64_t lda, int n,
+                                                                         T* dinv_l, T* dinv_u) {
+  __shared__ T S[kBS * kLds];
   const int i0 = blockIdx.x * kBS;
   const int rows = min(kBS, n - i0);
-  for (int idx = threadIdx.x; idx < kBS * kBS; idx += kBS) {
-    const int r = idx / kBS, c = idx - r * kBS;
-    S[r * kLds + c] = (r < rows && c < rows) ? static_cast<T>(a[(int64_t)(i0 + r) * lda + i0 + c]) : T(0);
+  const bool lower = blockIdx.z == 0;
+  const int cmin = blockIdx.y * kInvCols;
+  const int lane = threadIdx.x & 31, c = cmin + (threadIdx.x >> 5);
+  // The part the sweeps read: rows and columns from cmin on (lower), up to the
+  // last column (upper).
+  const int lo = lower ? cmin : 0, hi = lower ? rows : min(rows, cmin + kInvCols);
+  for (int idx = threadIdx.x; idx < kBS * kBS; idx += 32 * kInvCols) {
+    const int r = idx / kBS, q = idx - r * kBS;
+    const bool on = r >= lo && q >= lo && r < hi && q < hi && (lower ? q < r : q >= r);
+    S[r * kLds + q] = on ? static_cast<T>(a[(int64_t)(i0 + r) * lda + i0 + q]) : T(0);
   }
   __syncthreads();
-  const int c = threadIdx.x;
-  if (kLower) {
-    for (int i = 0; i < kBS; ++i) {
-      T v = T(0);
-      if (c < rows && i < rows && i >= c) {
-        v = (i == c) ? T(1) : T(0);
-        for (int k = c; k < i; ++k) v = fma(-S[i * kLds + k], Y[k * kLds + c], v);
-        if (!kUnit) v = v / S[i * kLds + i];
+  T x0 = lane == c ? T(1) : T(0), x1 = lane + 32 == c ? T(1) : T(0);
+  if (c < rows) {
+    if (lower) {
+      for (int k = c; k < rows - 1; ++k) {
+        const T xk = __shfl_sync(0xffffffffu, k < 32 ? x0 : x1, k & 31);
+        if (k < 31 && lane > k) x0 = fma(-S[lane * kLds + k], xk, x0);
+        if (lane + 32 > k) x1 = fma(-S[(lane + 32) * kLds + k], xk, x1);
       }
-      Y[i * kLds + c] = v;
-    }
-  } else {
-    for (int i = kBS - 1; i >= 0; --i) {
-      T v = T(0);
-      if (c < rows && i < rows && i <= c) {
-        v = (i == c) ? T(1) : T(0);
-        for (int k = i + 1; k <= c; ++k) v = fma(-S[i * kLds + k], Y[k * kLds + c], v);
-        if (!kUnit) v = v / S[i * kLds + i];
+    } else {
+      const bool on0 = lane < hi, on1 = lane + 32 < hi;
+      const T d0 = on0 ? S[lane * kLds + lane] : T(1), d1 = on1 ? S[(lane + 32) * kLds + lane + 32] : T(1);
+      const T r0 = T(1) / d0, r1 = T(1) / d1;
+      const bool good = __all_sync(0xffffffffu, isfinite(r0) && isfinite(r1) && isfinite(d0) && isfinite(d1) &&
+                                                    fabs(r0) > T(1e-30) && fabs(r1) > T(1e-30) &&
+                                                    fabs(d0) > T(1e-30) && fabs(d1) > T(1e-30));
+      for (int k = c; k >= 0; --k) {
+        if (k >= 32) {
+          if (lane + 32 == k) x1 = inv_quot(x1, d1, r1, good);
+          const T xk = __shfl_sync(0xffffffffu, x1, k & 31);
+          x0 = fma(-S[lane * kLds + k], xk, x0);
+          if (lane + 32 < k) x1 = fma(-S[(lane + 32) * kLds + k], xk, x1);
+        } else {
+          if (lane == k) x0 = inv_quot(x0, d0, r0, good);
+          const T xk = __shfl_sync(0xffffffffu, x0, k);
+          if (lane < k) x0 = fma(-S[lane * kLds + k], xk, x0);
+        }
       }
-      Y[i * kLds + c] = v;
     }
   }
-  __syncthreads();
-  T* out = dinv + (int64_t)blockIdx.x * kBS * kBS;
-  for (int idx = threadIdx.x; idx < kBS * kBS; idx += kBS) out[idx] = Y[(idx / kBS) * kLds + idx % kBS];
+  T* out = (lower ? dinv_l : dinv_u) + (int64_t)blockIdx.x * kBS * kBS;
+  const bool in = c < rows;
+  out[lane * kBS + c] = in && lane < rows && (lower ? lane >= c : lane <= c) ? x0 : T(0);
+  out[(lane + 32) * kBS + c] = in && lane + 32 < rows && (lower ? lane + 32 >= c : lane + 32 <= c) ? x1 : T(0);
 }
 
 size_t trsv_inverse_elems(int n) { return (size_t)trsv_syncfree_blocks(n) * kBS * kBS; }
 
 template <typename T, typename TA>
-cudaError_t launch_trsv_invert_diag(cudaStream_t stream, const TA* a, int64_t lda, int n, bool lower, T* dinv) {
+cudaError_t launch_trsv_invert_diag(cudaStream_t stream, const TA* a, int64_t lda, int n, T* dinv_l, T* dinv_u) {
   if (n <= 0) return cudaSuccess;
-  const size_t smem = 2 * (size_t)kBS * kLds * sizeof(T);
-  const int nblk = trsv_syncfree_blocks(n);
-  auto k = lower ? trsv_invert_diag_kernel<T, TA, true, true> : trsv_invert_diag_kernel<T, TA, false, false>;
-  cudaError_t e = allow_max_dynamic_smem(k);
-  if (e != cudaSuccess) return e;
-  k<<<nblk, kBS, smem, stream>>>(a, lda, n, dinv);
+  const dim3 grid(trsv_syncfree_blocks(n), kBS / kInvCols, 2);
+  trsv_invert_diag_kernel<T, TA><<<grid, 32 * kInvCols, 0, stream>>>(a, lda, n, dinv_l, dinv_u);
   return cudaGetLastError();
 }
 
 #define LUHOT_TRSV_INST(T, TA)                                                                                  \
   template cudaError_t launch_trsv_syncfree<T, TA>(cudaStream_t, const TA*, int64_t, T*, int64_t, int, int, bool, \
                                                    bool, bool, bool, int*, int*, DeviceStatus*, const T*);      \
-  template cudaError_t launch_trsv_invert_diag<T, TA>(cudaStream_t, const TA*, int64_t, int, bool, T*);
+  template cudaError_t launch_trsv_invert_diag<T, TA>(cudaStream_t, const TA*, int64_t, int, T*, T*);
 LUHOT_TRSV_INST(double, double)
 LUHOT_TRSV_INST(float, float)
 LUHOT_TRSV_INST(double, float)

@@ -12,8 +12,11 @@ struct DeviceStatus;
 size_t trsv_syncfree_smem(size_t elem_bytes);
 int trsv_syncfree_blocks(int n);
 
+// Chains of right-hand sides that one launch runs side by side, at most.
+constexpr int kTrsvMaxChains = 16;
+
 // op(A) x = b in place for nrhs columns of x (row-major, ldx); flags must hold
-// 4 * trsv_syncfree_blocks(n) ints and ticket one int of device scratch (both
+// kTrsvMaxChains * trsv_syncfree_blocks(n) ints and ticket one int of device scratch (both
 // cleared by this call); st supplies the wait limit and records a timeout.
 // TA is the storage type of the factor (it may be narrower than T).  dinv,
 // when not null, holds the inverses of the 64 x 64 diagonal blocks of the
@@ -44,10 +47,10 @@ cudaError_t launch_trsv_scaled(cudaStream_t stream, const TW* w, int64_t ldw, co
 
 // Elements of the diagonal-block inverses for order n.
 size_t trsv_inverse_elems(int n);
-// Inverses of the diagonal blocks of the unit lower (lower) or non-unit upper
-// triangle of a row-major LU factor.
+// Inverses of the diagonal blocks of the unit lower and the non-unit upper
+// triangle of a row-major LU factor (one launch).
 template <typename T, typename TA = T>
-cudaError_t launch_trsv_invert_diag(cudaStream_t stream, const TA* a, int64_t lda, int n, bool lower, T* dinv);
+cudaError_t launch_trsv_invert_diag(cudaStream_t stream, const TA* a, int64_t lda, int n, T* dinv_l, T* dinv_u);
 
 // Chained sweep for one right-hand side with FP32 factors (trsv_chain.cu):
 // 128-row blocks publishing x as epoch-tagged words.  dinv holds the inverses
