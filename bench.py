@@ -228,7 +228,7 @@ def workload_config(args):
     return {"workload": f"plain FP64 getrf+getrs drop-in, n={args.n}, nrhs={args.nrhs}, A,B iid N(0,1) seeded "
                         "(portable generator, lair_gb300.synthetic)",
             "n": args.n, "nrhs": args.nrhs, "mode": args.mode,
-            "fp64_update": {"auto": "FP16 tensor cores, exact integer slices (Ozaki), on trailing blocks >= 256 x 256; "
+            "fp64_update": {"auto": "FP16 tensor cores, exact integer slices (Ozaki), on trailing blocks > 200000 elements; "
                                     "DMMA below",
                             "dmma": "FP64 tensor cores (DMMA) only",
                             "ozaki": "FP16 tensor cores, exact integer slices, on every block >= 128 x 64"}[
@@ -445,7 +445,7 @@ def run_ours(args):
     total_prof_ms = sum(v["ms"] for v in prof.values())
     share = g["ms"] / total_prof_ms if total_prof_ms else None
     overall = flops_of(n, nrhs) * args.steps / (ms_max * 1e-3) / 1e12
-    sliced = args.fp64_update != "dmma" and prof.get("other", {}).get("launches", 0) > 0
+    sliced = args.fp64_update != "dmma" and mode == _lib.MODE_FAST
     if sliced:
         # Every large update is 28 FP16 slice GEMMs of the same shape (the
         # few small trailing blocks on DMMA are a negligible share).
@@ -466,7 +466,7 @@ def run_ours(args):
                             "bytes_are": "C read + written once per update, the slices read once"},
                     "per_launch_fp64_flops": g["flops"] / max(1, g["launches"]),
                     "launches": g["launches"], "share_of_step": share,
-                    "split_ms": prof["other"]["ms"] / args.steps,
+                    "swap_solve_split_ms": prof["trsm"]["ms"] / args.steps,
                     "overall_fp64_tflops": overall}
     else:
         traffic = read_traffic(os.path.join(ROOT, "profiles", "gemm_dmma_persistent_fp64_n16384.md"))

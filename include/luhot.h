@@ -72,16 +72,14 @@ int luhot_set_stream(luhot_ctx* ctx, void* cuda_stream);
 /* Panel width override (0 = default 64); for tuning and tests. */
 int luhot_set_block(luhot_ctx* ctx, int nb);
 /* Schur-update engine of fast-mode FP64 getrf (no lair counterpart).
- * LUHOT_UPDATE_AUTO (default): trailing blocks of at least 256 x 256 are
- * updated on the FP16 tensor cores by an exact integer-slice product (Ozaki
- * scheme: seven 8-bit slices per operand, 28 slice products, FP32 sums that
- * are exact, one FP64 rounding; error at or below an FP64 GEMM's), smaller
- * ones on the FP64 tensor cores (DMMA); the U12 solves of at least 256
- * columns run as the same product, U12 = A12 - (I - L11^-1) A12.
- * LUHOT_UPDATE_DMMA: DMMA updates and FMA substitutions only.
+ * LUHOT_UPDATE_AUTO (default): trailing blocks of more than 200 000 elements
+ * (at least 128 x 64) are updated on the FP16 tensor cores by an exact
+ * integer-slice product (Ozaki scheme: seven 8-bit slices per operand, 28 slice
+ * products, FP32 sums that are exact, one FP64 rounding; error at or below an
+ * FP64 GEMM's), smaller ones on the FP64 tensor cores (DMMA).
+ * LUHOT_UPDATE_DMMA: DMMA updates only.
  * LUHOT_UPDATE_OZAKI: the tensor-core product on every block of at least
- * 128 x 64 (U12 solves from 128 columns).  Exact mode and FP32 ignore the
- * setting. */
+ * 128 x 64.  Exact mode and FP32 ignore the setting. */
 #define LUHOT_UPDATE_AUTO 0
 #define LUHOT_UPDATE_DMMA 1
 #define LUHOT_UPDATE_OZAKI 2
@@ -101,9 +99,9 @@ int64_t luhot_launch_count(const luhot_ctx* ctx);
 int luhot_selftest_wait_timeout(luhot_ctx* ctx, int64_t timeout_ms);
 
 /* Per-kernel-class CUDA-event profile (no lair counterpart).  Classes:
- * 0 panel, 1 laswp, 2 trsm, 3 Schur GEMM, 4 triangular solve (getrs),
- * 5 permutation, 6 refinement (residual / update), 7 other (in getrf: the
- * operand splits of the tensor-core FP64 update).  flops and bytes are the
+ * 0 panel, 1 laswp, 2 trsm (in getrf with the panel's row interchanges and the
+ * operand splits of the tensor-core FP64 update), 3 Schur GEMM, 4 triangular
+ * solve (getrs), 5 permutation, 6 refinement (residual / update), 7 other.  flops and bytes are the
  * algorithmic work of the timed launches. */
 typedef struct luhot_profile {
   double ms[8];

@@ -5,7 +5,7 @@
 // (step i swapped row i with row piv[i]), the convention of lair's
 // src/lapack/getrf.rs:12-27.
 //
-// One block step k0 (panel width w) runs four kernels:
+// One block step k0 (panel width w) runs three kernels:
 //   1. panel_kernel   cooperative; factors rows [k0, m) x cols [k0, k0+w) held
 //                     in shared memory across all CTAs; per column one
 //                     exchange of step-tagged candidates through L2 (integer
@@ -15,11 +15,11 @@
 //                     update of the previous step overlapping the exchange.
 //                     Panels whose rows fit in one thread-block cluster run
 //                     there (panel_cluster.cu): 1.1 us a column instead of 2.5.
-//   2. laswp_moves_kernel  applies the panel's interchanges to the columns
-//                     left and right of it, as a gather of the (at most 2w)
-//                     rows that moved.
-//   3. trsm_kernel    U12 <- L11^-1 A12 (unit lower).
-//   4. gemm_*_kernel  A22 <- A22 - L21 U12 (the Schur complement).
+//   2. swap_solve_kernel (swap_solve.cu): the panel's interchanges on the
+//                     columns left and right of it (a gather of the at most 2w
+//                     rows that moved), U12 <- L11^-1 A12, and the operand slices
+//                     of a tensor-core update.
+//   3. gemm_*_kernel  A22 <- A22 - L21 U12 (the Schur complement).
 //
 // Two arithmetic modes:
 //   exact: every update is a separately rounded multiply then subtract, in
@@ -36,6 +36,7 @@
 #include "luhot_internal.h"
 #include "ozaki.cuh"
 #include "panel.cuh"
+#include "swap_solve.cuh"
 #include "tc_gemm.cuh"
 
 namespace luhot {
@@ -606,99 +607,7 @@ __global__ void __launch_bounds__(256) laswp_moves_kernel(T* a, int64_t lda, con
 
 
 // ---------------------------------------------------------------------------
-// 3. U12 <- L11^-1 A12 for rows [k0, k0+w), columns [c0, n).  One thread per
-//    column; each row i subtracts l[i][k]*u[k][c] for k = 0..i-1 in order,
-//    the order in which lair's elimination steps reach these entries.
-// ---------------------------------------------------------------------------
-constexpr int kTrsmCols = 64;
-
-template <typename T, bool kExact>
-__global__ void __launch_bounds__(kTrsmCols) trsm_kernel(T* a, int64_t lda, int k0, int w, int c0,
-                                                         int n) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* L = reinterpret_cast<T*>(smem_raw);  // [w][w]
-  T* X = L + w * w;                       // [w][kTrsmCols]
-  const int cb = c0 + blockIdx.x * kTrsmCols;
-  const int tid = threadIdx.x;
-  for (int idx = tid; idx < w * w; idx += blockDim.x) {
-    const int i = idx / w, k = idx - i * w;
-    L[idx] = a[(int64_t)(k0 + i) * lda + k0 + k];
-  }
-  const int c = cb + tid;
-  const bool active = c < n;
-  if (active)
-    for (int i = 0; i < w; ++i) X[i * kTrsmCols + tid] = a[(int64_t)(k0 + i) * lda + c];
-  __syncthreads();
-  if (!active) return;
-  for (int i = 1; i < w; ++i) {
-    T acc = X[i * kTrsmCols + tid];
-    for (int k = 0; k < i; ++k) acc = upd<kExact>(acc, L[i * w + k], X[k * kTrsmCols + tid]);
-    X[i * kTrsmCols + tid] = acc;
-  }
-  for (int i = 1; i < w; ++i) a[(int64_t)(k0 + i) * lda + c] = X[i * kTrsmCols + tid];
-}
-
-// Fast-mode U12 solve, left-looking in blocks of 16 rows: one thread per
-// column; for rows i0..i0+15 it accumulates x_i = b_i - sum_{k<i0} l_ik x_k
-// in 16 registers (16 independent FMA chains per loaded x_k, the l_ik
-// broadcast from shared memory with L11 stored transposed), then solves the
-// 16 x 16 diagonal block.  x lives in shared memory (one column per thread,
-// conflict-free).  W = 64 or 128 >= w; L11 is zero-padded to W x W.  The
-// CTA's 256 threads stage L11 and the 64 columns of A12 together (the
-// loads, not the solve, were most of the time with 64 threads); the first
-// 64 then solve and all of them write the rows back.  The exact mode keeps
-// trsm_kernel's order.
-constexpr int kTrsmFastThreads = 256;
-
-template <typename T, int W>
-__global__ void __launch_bounds__(kTrsmFastThreads) trsm_fast_kernel(T* a, int64_t lda, int k0, int w, int c0,
-                                                                      int n) {
-  constexpr int RB = 16;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* Lt = reinterpret_cast<T*>(smem_raw);  // [W][W]: Lt[k][i] = L11[i][k] for i > k, else 0
-  T* X = Lt + W * W;                       // [W][kTrsmCols]
-  const int tid = threadIdx.x;
-  const int cb = c0 + blockIdx.x * kTrsmCols;
-  for (int idx = tid; idx < W * W; idx += blockDim.x) {
-    const int k = idx / W, i = idx - k * W;
-    Lt[idx] = (i > k && i < w && k < w) ? a[(int64_t)(k0 + i) * lda + k0 + k] : T(0);
-  }
-  for (int idx = tid; idx < W * kTrsmCols; idx += blockDim.x) {
-    const int i = idx / kTrsmCols, cc = idx - i * kTrsmCols;
-    X[idx] = (cb + cc < n && i < w) ? a[(int64_t)(k0 + i) * lda + cb + cc] : T(0);
-  }
-  __syncthreads();
-  if (tid < kTrsmCols) {
-    for (int i0 = 0; i0 < w; i0 += RB) {
-      T acc[RB];
-#pragma unroll
-      for (int r = 0; r < RB; ++r) acc[r] = X[(i0 + r) * kTrsmCols + tid];
-      for (int k = 0; k < i0; ++k) {
-        const T xk = X[k * kTrsmCols + tid];
-        const T* lk = Lt + k * W + i0;
-#pragma unroll
-        for (int r = 0; r < RB; ++r) acc[r] = fma(-lk[r], xk, acc[r]);
-      }
-#pragma unroll
-      for (int kk = 0; kk < RB - 1; ++kk) {
-        const T* lk = Lt + (i0 + kk) * W + i0;
-#pragma unroll
-        for (int r = 0; r < RB; ++r)
-          if (r > kk) acc[r] = fma(-lk[r], acc[kk], acc[r]);
-      }
-#pragma unroll
-      for (int r = 0; r < RB; ++r) X[(i0 + r) * kTrsmCols + tid] = acc[r];
-    }
-  }
-  __syncthreads();
-  for (int idx = kTrsmCols + tid; idx < w * kTrsmCols; idx += blockDim.x) {
-    const int i = idx / kTrsmCols, cc = idx - i * kTrsmCols;
-    if (cb + cc < n) a[(int64_t)(k0 + i) * lda + cb + cc] = X[idx];
-  }
-}
-
-// ---------------------------------------------------------------------------
-// 4a. Schur update on the CUDA cores (exact mode and FP32): C -= A B with a
+// 3a. Schur update on the CUDA cores (exact mode and FP32): C -= A B with a
 //     64x64 tile per CTA, 4x4 per thread, K <= 64 staged in shared memory.
 //     Each C entry starts from its old value and takes the K updates one at a
 //     time in increasing k, which is lair's order.
@@ -759,7 +668,7 @@ __global__ void __launch_bounds__(256) gemm_cuda_kernel(T* a, int64_t lda, int r
 }
 
 // ---------------------------------------------------------------------------
-// 4b. Schur update on the FP64 tensor cores: mma.sync.m8n8k4 (DMMA).
+// 3b. Schur update on the FP64 tensor cores: mma.sync.m8n8k4 (DMMA).
 //     CTA tile 128x128, 8 warps as 4 (rows) x 2 (cols), warp tile 32x64 =
 //     4 x 8 MMA tiles.  L21/U12 slices (K <= 64) are staged in shared memory
 //     once; C is read, updated and written once.
@@ -968,6 +877,59 @@ __global__ void __launch_bounds__(256, 1) gemm_dmma_persistent_kernel(double* a,
   }
 }
 
+// The same product for small blocks: a 16 x 32 tile per CTA, four warps of 8 x 16
+// (two MMA tiles each).  One SM's FP64 pipes take 300 us for a 128 x 128 tile at
+// K = 64, so blocks of fewer such tiles than SMs are cut finer: a 200 x 200 block
+// 302 -> 12 us, 400 x 400 308 -> 24 us.  Any alignment.
+constexpr int kSmallBM = 16, kSmallBN = 32;
+
+__global__ void __launch_bounds__(128) gemm_dmma_small_kernel(double* a, int64_t lda, int r0, int c0, int kk0, int K,
+                                                              int M, int N) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int Kpad = (K + 3) & ~3;
+  const int Kp = Kpad + 4;
+  constexpr int ldb = kSmallBN + 4;
+  double* As = reinterpret_cast<double*>(smem_raw);  // [16][Kp]
+  double* Bs = As + kSmallBM * Kp;                   // [Kpad][ldb]
+  const int tile_r = r0 + blockIdx.y * kSmallBM, tile_c = c0 + blockIdx.x * kSmallBN;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int wr = (warp >> 1) * 8, wc = (warp & 1) * 16;
+  const int g = lane >> 2, t4 = lane & 3;
+  // C first: its loads overlap those of the operands.
+  double cv[2][2];
+  const int r = tile_r + wr + g;
+#pragma unroll
+  for (int ni = 0; ni < 2; ++ni)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int c = tile_c + wc + ni * 8 + t4 * 2 + e;
+      cv[ni][e] = (r < r0 + M && c < c0 + N) ? a[(int64_t)r * lda + c] : 0.0;
+    }
+  for (int idx = tid; idx < kSmallBM * Kpad; idx += 128) {
+    const int i = idx / Kpad, k = idx - i * Kpad;
+    As[i * Kp + k] = (tile_r + i < r0 + M && k < K) ? a[(int64_t)(tile_r + i) * lda + kk0 + k] : 0.0;
+  }
+  for (int idx = tid; idx < Kpad * kSmallBN; idx += 128) {
+    const int k = idx / kSmallBN, j = idx - k * kSmallBN;
+    Bs[k * ldb + j] = (tile_c + j < c0 + N && k < K) ? a[(int64_t)(kk0 + k) * lda + tile_c + j] : 0.0;
+  }
+  __syncthreads();
+  double acc[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+  for (int k = 0; k < Kpad; k += 4) {
+    const double af = As[(wr + g) * Kp + k + t4];
+#pragma unroll
+    for (int ni = 0; ni < 2; ++ni)
+      dmma_8x8x4(acc[ni][0], acc[ni][1], af, Bs[(k + t4) * ldb + wc + ni * 8 + g]);
+  }
+#pragma unroll
+  for (int ni = 0; ni < 2; ++ni)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int c = tile_c + wc + ni * 8 + t4 * 2 + e;
+      if (r < r0 + M && c < c0 + N) a[(int64_t)r * lda + c] = cv[ni][e] - acc[ni][e];
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Host driver.
 // ---------------------------------------------------------------------------
@@ -1055,6 +1017,17 @@ static int launch_gemm(luhot_ctx* ctx, T* a, int64_t lda, int r0, int c0, int kk
     const size_t smem = ((size_t)kDmmaBM * (Kpad + 4) + (size_t)Kpad * (kDmmaBN + 4)) * sizeof(double);
     const size_t smem_p = smem + (size_t)Kpad * (kDmmaBN + 4) * sizeof(double);
     const int tiles = ((N + kDmmaBN - 1) / kDmmaBN) * ((M + kDmmaBM - 1) / kDmmaBM);
+    if (tiles < ctx->num_sms) {
+      const int Kq = (K + 3) & ~3;
+      const size_t smem_s = ((size_t)kSmallBM * (Kq + 4) + (size_t)Kq * (kSmallBN + 4)) * sizeof(double);
+      LUHOT_CUDA_TRY(ctx, allow_max_dynamic_smem(gemm_dmma_small_kernel));
+      dim3 grid((N + kSmallBN - 1) / kSmallBN, (M + kSmallBM - 1) / kSmallBM);
+      prof_begin(ctx, kProfGemm);
+      gemm_dmma_small_kernel<<<grid, 128, smem_s, stream>>>(a, lda, r0, c0, kk0, K, M, N);
+      prof_end(ctx, kProfGemm, 2.0 * M * N * K, ((double)2 * M * N + (double)M * K + (double)K * N) * sizeof(T));
+      LUHOT_CUDA_TRY(ctx, cudaGetLastError());
+      return LUHOT_OK;
+    }
     const bool aligned = (lda % 2 == 0) && (kk0 % 2 == 0) && (c0 % 2 == 0) &&
                          (reinterpret_cast<uintptr_t>(a) % 16 == 0);
     if (aligned && smem_p <= (size_t)ctx->max_smem_optin) {
@@ -1098,75 +1071,13 @@ static int launch_laswp_cols(luhot_ctx* ctx, T* a, int64_t lda, const int* moves
   return LUHOT_OK;
 }
 
-// Row interchanges of the panel [k0, k0 + w) (the moves it reported) on every
-// column outside the panel: [0, k0) and [k0 + w, n).
-template <typename T>
-static int launch_laswp(luhot_ctx* ctx, T* a, int64_t lda, int k0, int w, int n, cudaStream_t stream) {
-  const int* moves = reinterpret_cast<const int*>(static_cast<char*>(ctx->panel_scratch) + kPanelSlotBytes);
-  return launch_laswp_cols<T>(ctx, a, lda, moves, w, 0, k0, k0 + w, n, stream);
-}
-
-// The tensor-core engine takes the U12 solve of fast-mode FP64 as well
-// (ozaki_trsm: U12 = A12 - (I - L11^-1) A12) for at least 256 columns (128
-// with LUHOT_UPDATE_OZAKI), when the trailing update runs on it.
-static bool trsm_on_slices(const void* oz_ws, int engine, int ncols) {
-  if (!oz_ws || engine == LUHOT_UPDATE_DMMA) return false;
-  return ncols >= (engine == LUHOT_UPDATE_OZAKI ? 128 : 256);
-}
-
-// U12 = L11^-1 A12 for the panel [k0, k0 + w): rows [k0, k0 + w) of the
-// columns [c_begin, c_end).
-template <typename T, bool kExact>
-static int launch_trsm(luhot_ctx* ctx, T* a, int64_t lda, int k0, int w, int c_begin, int c_end,
-                       cudaStream_t stream, void* oz_ws = nullptr, int engine = LUHOT_UPDATE_DMMA) {
-  if (c_begin >= c_end) return LUHOT_OK;
-  const int tgrid = (c_end - c_begin + kTrsmCols - 1) / kTrsmCols;
-  prof_begin(ctx, kProfTrsm);
-  if constexpr (std::is_same<T, double>::value && !kExact) {
-    if (w <= 64 && trsm_on_slices(oz_ws, engine, c_end - c_begin)) {
-      const int rc = ozaki_trsm(ctx, a, lda, k0, w, c_begin, c_end, oz_ws, stream);
-      prof_end(ctx, kProfTrsm, (double)w * (w - 1) * (c_end - c_begin),
-               ((double)w * w + 2.0 * w * (c_end - c_begin)) * sizeof(T));
-      return rc;
-    }
-  }
-  if (!kExact && w <= 64) {
-    const size_t smem = ((size_t)64 * 64 + (size_t)64 * kTrsmCols) * sizeof(T);
-    LUHOT_CUDA_TRY(ctx, allow_max_dynamic_smem(trsm_fast_kernel<T, 64>));
-    trsm_fast_kernel<T, 64><<<tgrid, kTrsmFastThreads, smem, stream>>>(a, lda, k0, w, c_begin, c_end);
-  } else if (!kExact && std::is_same<T, float>::value && w <= 128) {
-    if constexpr (std::is_same<T, float>::value) {
-      const size_t smem = ((size_t)128 * 128 + (size_t)128 * kTrsmCols) * sizeof(T);
-      LUHOT_CUDA_TRY(ctx, allow_max_dynamic_smem(trsm_fast_kernel<T, 128>));
-      trsm_fast_kernel<T, 128><<<tgrid, kTrsmFastThreads, smem, stream>>>(a, lda, k0, w, c_begin, c_end);
-    }
-  } else {
-    const size_t smem = ((size_t)w * w + (size_t)w * kTrsmCols) * sizeof(T);
-    auto kern = trsm_kernel<T, kExact>;
-    LUHOT_CUDA_TRY(ctx, allow_max_dynamic_smem(kern));
-    kern<<<tgrid, kTrsmCols, smem, stream>>>(a, lda, k0, w, c_begin, c_end);
-  }
-  prof_end(ctx, kProfTrsm, (double)w * (w - 1) * (c_end - c_begin),
-           ((double)w * w + 2.0 * w * (c_end - c_begin)) * sizeof(T));
-  LUHOT_CUDA_TRY(ctx, cudaGetLastError());
-  return LUHOT_OK;
-}
-
-// The trailing update of the panel [k0, k0 + w): a[r1.., r1..] -= L21 U12,
-// r1 = k0 + w.  Fast-mode FP64 runs it on the FP16 tensor cores (ozaki.cu)
-// when a workspace was given and the block is large enough for the engine
-// setting, else on the FP64 tensor cores.
-template <typename T, bool kExact>
-static int schur_update(luhot_ctx* ctx, T* a, int64_t lda, int k0, int w, int m, int n, void* oz_ws, int engine,
-                        cudaStream_t stream) {
-  const int r1 = k0 + w;
-  if constexpr (std::is_same<T, double>::value && !kExact) {
-    const int M = m - r1, N = n - r1;
-    const bool big = engine == LUHOT_UPDATE_OZAKI ? (M >= 128 && N >= 64) : (M >= 256 && N >= 256);
-    if (oz_ws && engine != LUHOT_UPDATE_DMMA && big)
-      return ozaki_update(ctx, a, lda, k0, w, r1, m, r1, n, oz_ws, stream);
-  }
-  return launch_gemm<T, kExact>(ctx, a, lda, r1, r1, k0, w, m - r1, n - r1, stream);
+// Whether the trailing update of M rows and N columns runs on the FP16 tensor
+// cores as a slice product (ozaki.cu).  A slice product takes 28 us for up to one
+// 128 x 128 tile per SM, FP64 arithmetic 8 us + 0.12 ns an element at K = 64:
+// they meet at 170 000 - 200 000 elements (512 x 400: 28 against 32 us).
+static bool update_on_slices(const void* oz_ws, int engine, int M, int N) {
+  if (!oz_ws || engine == LUHOT_UPDATE_DMMA || M < 128 || N < 64) return false;
+  return engine == LUHOT_UPDATE_OZAKI || (int64_t)M * N > 200000;
 }
 
 // Workspace of the tensor-core FP64 update for an m x n factorization
@@ -1184,7 +1095,12 @@ int fp64_schur_update(luhot_ctx* ctx, double* a, int64_t lda, int k, int m, int 
   void* ws = nullptr;
   int rc = ozaki_workspace(ctx, m, n, engine, &ws);
   if (rc) return rc;
-  return schur_update<double, false>(ctx, a, lda, 0, k, m, n, ws, engine, ctx->stream);
+  if (update_on_slices(ws, engine, m - k, n - k)) return ozaki_update(ctx, a, lda, 0, k, k, m, k, n, ws, ctx->stream);
+  return launch_gemm<double, false>(ctx, a, lda, k, k, 0, k, m - k, n - k, ctx->stream);
+}
+
+static const int* live_moves(luhot_ctx* ctx) {
+  return reinterpret_cast<const int*>(static_cast<char*>(ctx->panel_scratch) + kPanelSlotBytes);
 }
 
 template <typename T, bool kExact>
@@ -1197,14 +1113,27 @@ static int getrf_impl(luhot_ctx* ctx, int m, int n, T* a, int64_t lda, int* piv,
   for (int k0 = 0; k0 < dim_min; k0 += nb) {
     const int w = std::min(nb, dim_min - k0);
     int rc = launch_panel<T, kExact>(ctx, a, lda, m, k0, w, piv, stream);
-    if (!rc) rc = launch_laswp<T>(ctx, a, lda, k0, w, n, stream);
     if (rc) return rc;
-    const int c_right = k0 + w;
-    if (c_right < n) {
-      rc = launch_trsm<T, kExact>(ctx, a, lda, k0, w, c_right, n, stream, oz_ws, ctx->fp64_update);
-      if (!rc) rc = schur_update<T, kExact>(ctx, a, lda, k0, w, m, n, oz_ws, ctx->fp64_update, stream);
-      if (rc) return rc;
+    // Everything between the panel and the update in one launch, then the
+    // update: on the FP16 tensor cores (fast FP64, large blocks), whose operand
+    // slices that launch has written, else FP64 / FP32 arithmetic.
+    const int r1 = k0 + w, M = m - r1, N = n - r1;
+    const bool slices = !kExact && std::is_same<T, double>::value && w <= 64 &&
+                        update_on_slices(oz_ws, ctx->fp64_update, M, N);
+    SplitOut split;
+    if (slices) split = ozaki_split_out(oz_ws, r1, M, N);
+    rc = launch_swap_solve<T, kExact>(ctx, a, lda, live_moves(ctx), k0, w, 0, k0, r1, n, slices ? &split : nullptr,
+                                      stream);
+    if (rc) return rc;
+    if constexpr (std::is_same<T, double>::value && !kExact) {
+      if (slices) {
+        rc = ozaki_update_split(ctx, a, lda, w, r1, m, r1, n, oz_ws, stream);
+        if (rc) return rc;
+        continue;
+      }
     }
+    rc = launch_gemm<T, kExact>(ctx, a, lda, r1, r1, k0, w, M, N, stream);
+    if (rc) return rc;
   }
   return LUHOT_OK;
 }
@@ -1251,16 +1180,23 @@ static int la_setup(luhot_ctx* ctx) {
   return ensure_buf(ctx, ctx->la_moves, 4 * kPanelMovesBytes);
 }
 
-// Rows [s0, s1) of U on the columns [c0, c1) (two trsm steps with the K =
-// 128 update of panel B's rows between them), then the update of rows
-// [s1, m) x columns [c0, c1) on the tensor cores (K = s1 - s0).
-static int slab_columns(luhot_ctx* ctx, float* a, int64_t lda, int m, int s0, int h0, int h1, int c0, int c1,
-                        int tc_kind, void* tc_a, void* tc_b, float* tc_scal, cudaStream_t st) {
-  if (c0 >= c1) return LUHOT_OK;
-  int rc = launch_trsm<float, false>(ctx, a, lda, s0, h0, c0, c1, st);
+// The slab's interchanges (mv_a, mv_b: its panels' moved rows) on the columns
+// [cl0, cl1) and [c0, c1); rows [s0, s1) of U on the columns [c0, c1) (two
+// solves with the K = 128 update of panel B's rows between them), then the
+// update of rows [s1, m) x columns [c0, c1) on the tensor cores (K = s1 - s0).
+static int slab_columns(luhot_ctx* ctx, float* a, int64_t lda, int m, int s0, int h0, int h1, const int* mv_a,
+                        const int* mv_b, int cl0, int cl1, int c0, int c1, int tc_kind, void* tc_a, void* tc_b,
+                        float* tc_scal, cudaStream_t st) {
+  if (c0 >= c1) {  // no columns to the right: the interchanges on the left alone
+    int rc = launch_laswp_cols<float>(ctx, a, lda, mv_a, h0, cl0, cl1, 0, 0, st);
+    if (!rc && h1 > 0) rc = launch_laswp_cols<float>(ctx, a, lda, mv_b, h1, cl0, cl1, 0, 0, st);
+    return rc;
+  }
+  int rc = launch_swap_solve<float, false>(ctx, a, lda, mv_a, s0, h0, cl0, cl1, c0, c1, nullptr, st);
   if (!rc && h1 > 0) {
-    rc = launch_gemm<float, false>(ctx, a, lda, s0 + h0, c0, s0, h0, h1, c1 - c0, st);
-    if (!rc) rc = launch_trsm<float, false>(ctx, a, lda, s0 + h0, h1, c0, c1, st);
+    rc = launch_laswp_cols<float>(ctx, a, lda, mv_b, h1, cl0, cl1, c0, c1, st);
+    if (!rc) rc = launch_gemm<float, false>(ctx, a, lda, s0 + h0, c0, s0, h0, h1, c1 - c0, st);
+    if (!rc) rc = launch_swap_solve<float, false>(ctx, a, lda, nullptr, s0 + h0, h1, 0, 0, c0, c1, nullptr, st);
   }
   const int s1 = s0 + h0 + h1;
   if (!rc) rc = tc_gemm_update(ctx, tc_kind, a, lda, s0, h0 + h1, s1, m, c0, c1, tc_a, tc_b, tc_scal, st);
@@ -1272,7 +1208,6 @@ static int tc_slab_loop(luhot_ctx* ctx, int m, int n, float* a, int64_t lda, int
   const int dim_min = std::min(m, n);
   cudaStream_t hs = ctx->la_hi, ls = ctx->la_lo;
   cudaEvent_t ev_ready = ctx->la_ev[1];
-  const int* live_moves = reinterpret_cast<const int*>(static_cast<char*>(ctx->panel_scratch) + kPanelSlotBytes);
   constexpr int hw = kTcPanelWidth, sl = 2 * hw;
   const int cap_rest = std::max(1, ctx->num_sms - 64);
   int slab = 0;
@@ -1289,21 +1224,18 @@ static int tc_slab_loop(luhot_ctx* ctx, int m, int n, float* a, int64_t lda, int
       if (slab >= 2) LUHOT_CUDA_TRY(ctx, cudaStreamWaitEvent(hs, ctx->la_ev[2 + par], 0));
       int rc = launch_panel<float, false>(ctx, a, lda, m, s0, h0, piv, hs);
       if (rc) return rc;
-      LUHOT_CUDA_TRY(ctx, cudaMemcpyAsync(mv_a, live_moves, kPanelMovesBytes, cudaMemcpyDeviceToDevice, hs));
-      rc = launch_laswp_cols<float>(ctx, a, lda, mv_a, h0, 0, 0, s0 + h0, s1, hs);
-      if (!rc && h1 > 0) {
-        rc = launch_trsm<float, false>(ctx, a, lda, s0, h0, s0 + h0, s1, hs);
+      LUHOT_CUDA_TRY(ctx, cudaMemcpyAsync(mv_a, live_moves(ctx), kPanelMovesBytes, cudaMemcpyDeviceToDevice, hs));
+      if (h1 > 0) {
+        rc = launch_swap_solve<float, false>(ctx, a, lda, mv_a, s0, h0, 0, 0, s0 + h0, s1, nullptr, hs);
         if (!rc) rc = launch_gemm<float, false>(ctx, a, lda, s0 + h0, s0 + h0, s0, h0, m - (s0 + h0), h1, hs);
         if (!rc) rc = launch_panel<float, false>(ctx, a, lda, m, s0 + h0, h1, piv, hs);
         if (rc) return rc;
-        LUHOT_CUDA_TRY(ctx, cudaMemcpyAsync(mv_b, live_moves, kPanelMovesBytes, cudaMemcpyDeviceToDevice, hs));
+        LUHOT_CUDA_TRY(ctx, cudaMemcpyAsync(mv_b, live_moves(ctx), kPanelMovesBytes, cudaMemcpyDeviceToDevice, hs));
         rc = launch_laswp_cols<float>(ctx, a, lda, mv_b, h1, s0, s0 + h0, 0, 0, hs);
       }
       if (!rc && s1 < e1) {
         if (slab >= 1) LUHOT_CUDA_TRY(ctx, cudaStreamWaitEvent(hs, ctx->la_ev[2 + (par ^ 1)], 0));
-        rc = launch_laswp_cols<float>(ctx, a, lda, mv_a, h0, 0, 0, s1, e1, hs);
-        if (!rc && h1 > 0) rc = launch_laswp_cols<float>(ctx, a, lda, mv_b, h1, 0, 0, s1, e1, hs);
-        if (!rc) rc = slab_columns(ctx, a, lda, m, s0, h0, h1, s1, e1, tc_kind, tc_a, tc_b, tc_scal, hs);
+        rc = slab_columns(ctx, a, lda, m, s0, h0, h1, mv_a, mv_b, 0, 0, s1, e1, tc_kind, tc_a, tc_b, tc_scal, hs);
       }
       if (rc) return rc;
       LUHOT_CUDA_TRY(ctx, cudaEventRecord(ev_ready, hs));
@@ -1311,13 +1243,9 @@ static int tc_slab_loop(luhot_ctx* ctx, int m, int n, float* a, int64_t lda, int
     {
       OnStream on(ctx, ls);
       LUHOT_CUDA_TRY(ctx, cudaStreamWaitEvent(ls, ev_ready, 0));
-      int rc = launch_laswp_cols<float>(ctx, a, lda, mv_a, h0, 0, s0, e1, n, ls);
-      if (!rc && h1 > 0) rc = launch_laswp_cols<float>(ctx, a, lda, mv_b, h1, 0, s0, e1, n, ls);
-      if (!rc && e1 < n) {
-        ctx->tc_grid_cap = cap_rest;
-        rc = slab_columns(ctx, a, lda, m, s0, h0, h1, e1, n, tc_kind, tc_a, tc_b, tc_scal, ls);
-        ctx->tc_grid_cap = 0;
-      }
+      ctx->tc_grid_cap = cap_rest;
+      int rc = slab_columns(ctx, a, lda, m, s0, h0, h1, mv_a, mv_b, 0, s0, e1, n, tc_kind, tc_a, tc_b, tc_scal, ls);
+      ctx->tc_grid_cap = 0;
       if (rc) return rc;
       LUHOT_CUDA_TRY(ctx, cudaEventRecord(ctx->la_ev[2 + par], ls));
     }

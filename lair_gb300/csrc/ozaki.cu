@@ -70,13 +70,11 @@
 #include "common.cuh"
 #include "luhot_internal.h"
 #include "ozaki.cuh"
+#include "ozaki_split.cuh"
 #include "tcgen05.cuh"
 
 namespace luhot {
 
-constexpr int kOzSlices = 7;
-constexpr int kOzGroups = 7;   // G = p + q = 0 .. 6
-constexpr int kOzK = 64;       // K of one update (one 128-byte box row of FP16)
 constexpr int kOzBM = 128, kOzBN = 128;
 constexpr int kOzFrac = 38;    // fractional bits of the fixed-point combine
 constexpr int kOzEpiWarps = 16;
@@ -85,86 +83,11 @@ constexpr int kOzSliceBytes = 128 * 128;  // one slice box: 128 rows x 128 B
 constexpr int kOzAccBufs = 3;           // TMEM accumulators of 128 columns, used in turn by the groups
 constexpr unsigned kOzLoCol = 384;      // TMEM columns 384-511: low words of the fixed-point sums
 constexpr size_t kOzSmem = 1024 + 2 * (size_t)kOzSlices * kOzSliceBytes;
-constexpr int kOzNonFinite = 1 << 20;  // exponent of a row / column that holds Inf or NaN
-constexpr int kOzZero = -(1 << 20);    // exponent of a zero element
 static_assert(kOzAccBufs * kOzBM <= (int)kOzLoCol && kOzLoCol + kOzBM <= 512, "accumulators and sums fit in TMEM");
 
 // ---------------------------------------------------------------------------
-// Split.
+// Split (digits: ozaki_split.cuh).
 // ---------------------------------------------------------------------------
-
-// The e of frexp(x) (|x| < 2^e, |x| >= 2^(e-1)) from the bits; kOzZero for
-// zeros, kOzNonFinite for Inf and NaN.
-__device__ __forceinline__ int oz_exponent(double x) {
-  const unsigned long long u = (unsigned long long)__double_as_longlong(x);
-  const int E = (int)((u >> 52) & 0x7ff);
-  const unsigned long long m = u & 0xFFFFFFFFFFFFFull;
-  if (E == 0x7ff) return kOzNonFinite;
-  if (E != 0) return E - 1022;
-  if (m == 0) return kOzZero;
-  return (64 - __clzll((long long)m)) - 1074;
-}
-
-// Seven balanced base-256 digits of round(|x| 2^(56-e)), signed like x, most
-// significant first; |x| < 2^e.  Integer arithmetic only.
-__device__ __forceinline__ void oz_digits(double x, int e, int (&d)[kOzSlices]) {
-  const unsigned long long u = (unsigned long long)__double_as_longlong(x);
-  const int E = (int)((u >> 52) & 0x7ff);
-  unsigned long long m = u & 0xFFFFFFFFFFFFFull;
-  int ex = -1074;
-  if (E != 0) {
-    m |= 1ull << 52;
-    ex = E - 1075;
-  }
-  // |x| = m 2^ex < 2^e, so m 2^(ex - e + 56) < 2^56.
-  const int sh = ex - e + 56;
-  unsigned long long N;
-  if (m == 0 || sh <= -64)
-    N = 0;
-  else if (sh >= 0)
-    N = m << sh;
-  else
-    N = (m + (1ull << (-sh - 1))) >> (-sh);  // round half up; m < 2^53, so no overflow
-  int carry = 0;
-#pragma unroll
-  for (int p = kOzSlices - 1; p >= 1; --p) {
-    const int v = (int)(N & 255u) + carry;
-    N >>= 8;
-    carry = v >= 128 ? 1 : 0;
-    d[p] = v - (carry << 8);
-  }
-  d[0] = (int)N + carry;  // N < 2^8 here: d_0 <= 256
-  if (u >> 63) {
-#pragma unroll
-    for (int p = 0; p < kOzSlices; ++p) d[p] = -d[p];
-  }
-}
-
-// One warp writes the digits of a 64-element row (x0 = element lane, x1 =
-// element lane + 32) with the warp-reduced exponent e into slice rows
-// dst[p * slice + 0..63].
-__device__ __forceinline__ void oz_emit_row(double x0, double x1, int e, __half* __restrict__ dst, int64_t slice,
-                                            int lane) {
-  int d0[kOzSlices], d1[kOzSlices];
-  if (e == kOzZero || e >= kOzNonFinite) {
-#pragma unroll
-    for (int p = 0; p < kOzSlices; ++p) d0[p] = d1[p] = 0;
-  } else {
-    oz_digits(x0, e, d0);
-    oz_digits(x1, e, d1);
-  }
-#pragma unroll
-  for (int p = 0; p < kOzSlices; ++p) {
-    dst[p * slice + lane] = __int2half_rn(d0[p]);
-    dst[p * slice + lane + 32] = __int2half_rn(d1[p]);
-  }
-}
-
-__device__ __forceinline__ int oz_warp_max(int v) {
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, off));
-  return v;
-}
 
 // Rows r1 .. r1 + M - 1, columns k0 .. k0 + w - 1 of the row-major a (w <= 64):
 // As[p][i][k] (zero for k >= w), ea[i].  One warp per row.
@@ -204,42 +127,6 @@ __global__ void __launch_bounds__(256) oz_split_cols_kernel(const double* __rest
     oz_emit_row(x0, x1, e, bs + (int64_t)j * kOzK, (int64_t)N * kOzK, lane);
     if (lane == 0) eb[j] = e == kOzZero ? 0 : e;
   }
-}
-
-// U12 = L11^-1 A12 as a product: U12 = A12 - N A12 with N = I - L11^-1
-// (strictly lower).  oz_trsm_inverse_kernel forms N for the unit lower
-// triangular L11 = a[k0.., k0..] (w x w, w <= 64) into nb (128 x 64,
-// row-major; rows >= w and columns >= w zero), one CTA per column c: warp 0
-// holds x = L11^-1 e_c (rows lane and lane + 32) and runs the column sweep
-// x_i -= L(i,k) x_k for i > k, k = c, c + 1, ... (x_k by shuffle), so each
-// step costs one shuffle and two FMAs on this part's thin FP64 pipe; the
-// CTA's four warps first stage L11 in shared memory.  oz_split_rows_kernel
-// then writes N's digit slices like any L21.
-constexpr int kOzInvLds = 65;
-constexpr int kOzMapRows = 128;  // rows of the L-slice tensor map of the triangular solve
-
-__global__ void __launch_bounds__(128) oz_trsm_inverse_kernel(const double* __restrict__ a, int64_t lda, int k0, int w,
-                                                              double* __restrict__ nb) {
-  __shared__ double L[kOzK * kOzInvLds];  // L[i * kOzInvLds + k] = L11(i, k) for k < i < w, else 0
-  const int c = blockIdx.x, tid = threadIdx.x;
-  for (int idx = tid; idx < kOzK * kOzK; idx += blockDim.x) {
-    const int i = idx >> 6, k = idx & 63;
-    L[i * kOzInvLds + k] = (i < w && k < i && k >= c) ? a[(int64_t)(k0 + i) * lda + k0 + k] : 0.0;
-  }
-  __syncthreads();
-  if (tid >= 32) return;
-  const int lane = tid;
-  double x0 = lane == c ? 1.0 : 0.0, x1 = lane + 32 == c ? 1.0 : 0.0;
-  for (int k = c; k < w - 1; ++k) {
-    const double xk = __shfl_sync(0xffffffffu, k < 32 ? x0 : x1, k & 31);
-    if (lane > k) x0 = fma(-L[lane * kOzInvLds + k], xk, x0);
-    if (lane + 32 > k) x1 = fma(-L[(lane + 32) * kOzInvLds + k], xk, x1);
-  }
-  // N(i, c) = -x_i below the diagonal (the unit diagonal cancels), zero elsewhere
-  nb[lane * kOzK + c] = (lane > c && lane < w && c < w) ? -x0 : 0.0;
-  nb[(lane + 32) * kOzK + c] = (lane + 32 > c && lane + 32 < w && c < w) ? -x1 : 0.0;
-  nb[(lane + 64) * kOzK + c] = 0.0;
-  nb[(lane + 96) * kOzK + c] = 0.0;
 }
 
 // ---------------------------------------------------------------------------
@@ -678,36 +565,30 @@ __global__ void __launch_bounds__(kOzThreads, 1)
 // ---------------------------------------------------------------------------
 static size_t oz_round(size_t b) { return (b + 1023) / 1024 * 1024; }
 
-// Workspace layout for an M x N product: A slices [7][M'][64], B slices
-// [7][N][64], exponents ea[M'], eb[N], with M' = max(M, 128) (the triangular
-// solve's L slices always have 128 rows).
+// Workspace layout for an M x N product: A slices [7][M][64], B slices
+// [7][N][64], exponents ea[M], eb[N].
 struct OzWs {
   __half* as;
   __half* bs;
   int* ea;
   int* eb;
-  double* nb;  // N = I - L11^-1 of the triangular solve (128 x 64)
 };
 static OzWs oz_layout(void* ws, int M, int N) {
-  const size_t Mp = (size_t)std::max(M, kOzMapRows);
   char* p = static_cast<char*>(ws);
   OzWs w;
   w.as = reinterpret_cast<__half*>(p);
-  p += oz_round((size_t)kOzSlices * Mp * kOzK * 2);
+  p += oz_round((size_t)kOzSlices * M * kOzK * 2);
   w.bs = reinterpret_cast<__half*>(p);
   p += oz_round((size_t)kOzSlices * N * kOzK * 2);
   w.ea = reinterpret_cast<int*>(p);
-  p += oz_round(Mp * 4);
+  p += oz_round((size_t)M * 4);
   w.eb = reinterpret_cast<int*>(p);
-  p += oz_round((size_t)N * 4);
-  w.nb = reinterpret_cast<double*>(p);
   return w;
 }
 
 size_t ozaki_workspace_bytes(int m, int n) {
-  const size_t mp = (size_t)std::max(m, kOzMapRows);
-  return oz_round((size_t)kOzSlices * mp * kOzK * 2) + oz_round((size_t)kOzSlices * n * kOzK * 2) + oz_round(mp * 4) +
-         oz_round((size_t)n * 4) + oz_round((size_t)kOzMapRows * kOzK * sizeof(double));
+  return oz_round((size_t)kOzSlices * m * kOzK * 2) + oz_round((size_t)kOzSlices * n * kOzK * 2) +
+         oz_round((size_t)m * 4) + oz_round((size_t)n * 4);
 }
 
 bool ozaki_available(luhot_ctx* ctx) { return kOzSmem <= (size_t)ctx->max_smem_optin && encode_fn() != nullptr; }
@@ -729,12 +610,11 @@ static int make_slice_map(luhot_ctx* ctx, CUtensorMap* map, void* ptr, int rows,
   return LUHOT_OK;
 }
 
-// C (M x N, ldc) -= the product of the slices in `w` (L map of map_rows
-// rows); one persistent launch.
-static int oz_launch_gemm(luhot_ctx* ctx, const OzWs& w, int map_rows, double* c, int64_t ldc, int M, int N,
+// C (M x N, ldc) -= the product of the slices in `w`; one persistent launch.
+static int oz_launch_gemm(luhot_ctx* ctx, const OzWs& w, double* c, int64_t ldc, int M, int N,
                           cudaStream_t stream) {
   CUtensorMap tmL, tmU;
-  int rc = make_slice_map(ctx, &tmL, w.as, map_rows, kOzBM);
+  int rc = make_slice_map(ctx, &tmL, w.as, M, kOzBM);
   if (!rc) rc = make_slice_map(ctx, &tmU, w.bs, N, kOzBN);
   if (rc) return rc;
   const int tiles = ((M + kOzBM - 1) / kOzBM) * ((N + kOzBN - 1) / kOzBN);
@@ -743,6 +623,30 @@ static int oz_launch_gemm(luhot_ctx* ctx, const OzWs& w, int map_rows, double* c
                                                                                 ctx->d_status);
   LUHOT_CUDA_TRY(ctx, cudaGetLastError());
   return LUHOT_OK;
+}
+
+SplitOut ozaki_split_out(void* ws, int r1, int M, int N) {
+  const OzWs lay = oz_layout(ws, M, N);
+  SplitOut s;
+  s.as = lay.as;
+  s.ea = lay.ea;
+  s.r1 = r1;
+  s.M = M;
+  s.bs = lay.bs;
+  s.eb = lay.eb;
+  return s;
+}
+
+int ozaki_update_split(luhot_ctx* ctx, double* a, int64_t lda, int w, int r1, int m, int c1, int n, void* ws,
+                       cudaStream_t stream) {
+  const int M = m - r1, N = n - c1;
+  const OzWs lay = oz_layout(ws, M, N);
+  prof_begin(ctx, kProfGemm);
+  int rc = oz_launch_gemm(ctx, lay, a + (int64_t)r1 * lda + c1, lda, M, N, stream);
+  // algorithmic work: 2MNK FP64 flops; bytes: C read + written, the slices read once
+  prof_end(ctx, kProfGemm, 2.0 * M * N * w,
+           (double)M * N * 16 + (double)(M + N) * kOzK * kOzSlices * 2 + (double)(M + N) * 4);
+  return rc;
 }
 
 int ozaki_update(luhot_ctx* ctx, double* a, int64_t lda, int k0, int w, int r1, int m, int c1, int n, void* ws,
@@ -764,25 +668,7 @@ int ozaki_update(luhot_ctx* ctx, double* a, int64_t lda, int k0, int w, int r1, 
   prof_end(ctx, kProfOther, 0.0, (double)N * w * 8 + (double)N * kOzK * kOzSlices * 2);
   LUHOT_CUDA_TRY(ctx, cudaGetLastError());
 
-  prof_begin(ctx, kProfGemm);
-  int rc = oz_launch_gemm(ctx, lay, M, a + (int64_t)r1 * lda + c1, lda, M, N, stream);
-  // algorithmic work: 2MNK FP64 flops; bytes: C read + written, the slices read once
-  prof_end(ctx, kProfGemm, 2.0 * M * N * w,
-           (double)M * N * 16 + (double)(M + N) * kOzK * kOzSlices * 2 + (double)(M + N) * 4);
-  return rc;
-}
-
-int ozaki_trsm(luhot_ctx* ctx, double* a, int64_t lda, int k0, int w, int c1, int n, void* ws, cudaStream_t stream) {
-  const int N = n - c1;
-  if (N <= 0 || w <= 1) return LUHOT_OK;
-  if (w > kOzK || N < kOzBN) return set_error(ctx, LUHOT_ERR_INVALID_ARG, "ozaki_trsm: w > 64 or fewer than 128 columns");
-  const OzWs lay = oz_layout(ws, w, N);
-  oz_trsm_inverse_kernel<<<kOzK, 128, 0, stream>>>(a, lda, k0, w, lay.nb);
-  oz_split_rows_kernel<<<kOzMapRows / 8, 256, 0, stream>>>(lay.nb, kOzK, 0, kOzMapRows, 0, w, lay.as, lay.ea);
-  oz_split_cols_kernel<<<(N + 31) / 32, 256, 0, stream>>>(a, lda, k0, w, c1, N, lay.bs, lay.eb);
-  LUHOT_CUDA_TRY(ctx, cudaGetLastError());
-  // rows [k0, k0 + w) of columns [c1, n): A12 -= N A12 (its slices were taken first)
-  return oz_launch_gemm(ctx, lay, kOzMapRows, a + (int64_t)k0 * lda + c1, lda, w, N, stream);
+  return ozaki_update_split(ctx, a, lda, w, r1, m, c1, n, ws, stream);
 }
 
 }  // namespace luhot
