@@ -228,8 +228,8 @@ int luhot_dgesv_backward_ir_dev(luhot_ctx* ctx, int64_t n, int64_t nrhs, const d
 
 /* ---- Batched uneven solves ----------------------------------------------
  * No lair counterpart: lair factors one matrix per call; these factor and
- * solve `count` independent systems A_i x_i = b_i (1 <= n_i <= 256) in one
- * persistent kernel launch replayed from a CUDA graph, with lair's per-system
+ * solve `count` independent systems A_i x_i = b_i (1 <= n_i <= 256) with one
+ * persistent launch per size class, replayed from one CUDA graph, with lair's per-system
  * semantics (pivots, last-zero-pivot singular step; LUHOT_MODE_EXACT gives
  * lair's bits for every system).  Packed layout: A_i row-major at element
  * offset sum_{j<i} n_j^2, b_i (overwritten by x_i) and int32 pivots at
@@ -240,11 +240,13 @@ int luhot_batch_create(luhot_ctx* ctx, int64_t count, const int32_t* sizes, int 
 void luhot_batch_destroy(luhot_batch* plan);
 /* Total elements of the packed A and b arrays. */
 int luhot_batch_layout(const luhot_batch* plan, int64_t* a_elems, int64_t* b_elems);
-/* Choose, per size bucket, the shared-memory path or a panel width (8, 16,
- * 32) by timing each on sample systems copied from d_a / d_b (not modified). */
+/* Choose, per size bucket, shared memory or the scratch form (matrices in
+ * global memory, which holds more of them at once) by timing both on sample
+ * systems copied from d_a / d_b (not modified). */
 int luhot_batch_autotune(luhot_batch* plan, const void* d_a, const void* d_b);
-/* Chosen per-bucket settings (9 buckets: 0 = shared memory, else the panel
- * width) and the largest n of the shared-memory path. */
+/* Chosen per-bucket settings (9 buckets: 0 = shared memory where it fits, else
+ * the panel width of the scratch form) and the largest n that fits in shared
+ * memory. */
 int luhot_batch_tuning(const luhot_batch* plan, int32_t* nb_per_bucket, int32_t* smem_n);
 /* Factor and solve every system in place on the device (one graph launch). */
 int luhot_batch_solve(luhot_batch* plan, void* d_a, void* d_b, int32_t* d_piv, int32_t* d_info);

@@ -1,6 +1,6 @@
 """Batched uneven LU solves (no lair counterpart) and their multi-GPU sharding.
 
-``BatchSolver(sizes)`` plans one persistent, graph-captured launch that
+``BatchSolver(sizes)`` plans one graph of persistent launches (one per size class) that
 factors and solves ``len(sizes)`` independent systems of sizes 1..256 with
 lair's per-system semantics (pivots, singular step; ``mode="exact"`` gives
 lair's bits).  Arrays are packed: A_i row-major back to back, b_i back to

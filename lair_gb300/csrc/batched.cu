@@ -1,26 +1,37 @@
-// Batched LU + solve of thousands of small uneven systems in one persistent
-// launch (replayed from a CUDA graph).
+// Batched LU + solve of thousands of small uneven systems in one graph launch.
 //
 // Packed layout: system i is an n_i x n_i row-major matrix at element offset
 // a_off[i] = sum_{j<i} n_j^2 and a right-hand side (overwritten by x) and
 // int32 pivots at b_off[i] = sum_{j<i} n_j.  info[i] = last all-zero pivot
 // step of system i (lair's Option<usize>) or -1.
 //
-// One CTA (256 threads) per system at a time; CTAs draw systems from an
-// atomic counter in largest-first order (longest-processing-time first
-// keeps the tail short).  Two per-system algorithms:
-//   * shared-memory path (n <= smem_n): the whole matrix and x live in
-//     shared memory; unblocked right-looking elimination (warp-shuffle
-//     pivot search, row swap, reciprocal scale, rank-1 update), then the
-//     two triangular sweeps, all in shared memory;
-//   * blocked path: panels of nb columns are factored in shared memory, the
-//     interchanges, U12 and the Schur update run on the L2-resident matrix.
-// Which path and which nb each size bucket uses is chosen by the autotuner
-// (luhot_batch_autotune), which times the candidates on sample systems of
-// the batch.  In exact mode every update is lair's separately rounded
-// multiply and subtract in elimination order (src/lapack/getrf.rs:76-89),
-// and the solve follows src/lapack/getrs.rs:24-36, so each system's LU,
-// pivots and x are bit-identical to lair's.
+// One CTA per system at a time; the CTAs of a size class draw its systems from
+// an atomic counter, largest first, and the classes run side by side (branches
+// of the graph), so each has the shared memory, threads and registers it needs:
+// a class is a range of n whose matrices fit so many to an SM, and the systems
+// that do not fit (or that the autotuner moved) use a scratch matrix per CTA in
+// global memory, which stays in L2.
+//
+// Per system the matrix (and the right-hand side as column n) is copied in and
+// factored in panels of NB columns:
+//   panel   one warp, the active rows in registers (NI rows x NB columns a lane),
+//           no block barrier inside: pivot by one redux and a vote, pivot row by
+//           shuffle, rank-1 updates in registers.  Rows never move: a row's logical
+//           index is relabelled, and the copy-out writes rows in logical order.
+//   U12     a thread per column (the right-hand side among them, so the forward
+//           substitution needs no pass of its own);
+//   update  FP32: 8 rows x 4 columns a lane, vector loads of both operands; FP64,
+//           bound by its pipe, where a warp instruction takes 64 cycles however
+//           few lanes it has: (row, column) pairs flattened over the lanes.
+// The back substitution is one warp's column sweep with the solution in
+// registers.  Elements get their updates one at a time in elimination order
+// with lair's roundings in exact mode (src/lapack/getrf.rs:76-89, getrs.rs:24-36),
+// so each system's LU, pivots and x are bit-identical to lair's there.
+//
+// 10 000 FP32 systems of n ~ U{8..256} 15.0 -> 8.0 ms, 1500 FP64 7.3 -> 6.0 ms,
+// against one 256-thread CTA per system with a block-wide search and four barriers
+// per column.  FP64 is within 1.5 of its pipe's 4.1 ms; FP32 is bound by the
+// panel warp (about 1100 cycles a step, instruction fetches among them).
 #include <algorithm>
 #include <climits>
 #include <cstring>
@@ -29,13 +40,15 @@
 
 #include "common.cuh"
 #include "luhot_internal.h"
+#include "panel.cuh"
 
 namespace luhot {
 
-constexpr int kBatchThreads = 256;
 constexpr int kBatchMaxN = 256;
 constexpr int kBuckets = 9;         // n in (0,16], (16,32], (32,64], (64,96], ..., (224,256]
-constexpr size_t kBatchSmem = 76 * 1024;
+constexpr size_t kBatchSmem = 222 * 1024;
+constexpr int kScratchLd = 260;     // row stride of a scratch matrix (256 + the right-hand side, whole 16 bytes)
+constexpr size_t kScratchElems = (size_t)kBatchMaxN * kScratchLd;
 
 __host__ __device__ inline int batch_bucket(int n) {
   if (n <= 16) return 0;
@@ -44,266 +57,489 @@ __host__ __device__ inline int batch_bucket(int n) {
   return min(kBuckets - 1, 3 + (n - 65) / 32);
 }
 
+// Panel width: a lane's NI x NB panel values are registers; FP32 panels of more
+// than 128 rows are kept to 64 registers so that 16 warps share an SM.
+template <typename T>
+__host__ __device__ constexpr int batch_nb(int ni) {
+  return sizeof(T) == 8 || ni == 8 ? 8 : 16;
+}
+// Row stride in shared memory (n columns and the right-hand side): FP32 whole
+// 16-byte pieces, an odd number of them (conflict-free panel loads); FP64 odd.
+template <typename T>
+__host__ __device__ inline int batch_ld(int n) {
+  if (sizeof(T) == 8) return (n + 1) | 1;
+  const int q = (n + 4) / 4;
+  return 4 * (q | 1);
+}
+
 struct BatchMeta {
   const int* sizes;
   const int64_t* aoff;
   const int64_t* boff;
-  const int* order;
-  const int* tune;  // [kBuckets]: 0 = shared-memory path, else the panel width
+  const int* order;  // the class's systems, largest first
   int count;
-  int smem_n;
 };
 
-template <bool kExact>
-__device__ __forceinline__ double bupd(double c, double l, double u) {
-  if (kExact) return __dsub_rn(c, __dmul_rn(l, u));
-  return fma(-l, u, c);
+// A22 -= L21 U12 for the active rows act[0, na) and the columns [c1, c1 + nc),
+// panel columns [k0, k0 + w); steps in `mask` made no update.  FP32, kCV columns
+// a lane: 4 (16 lanes, two groups of 8 rows a warp) or 1.
+template <bool kExact, int kNB, int kCV, bool kMasked>
+__device__ __forceinline__ void batch_update_f32(float* S, int ld, const int* act, int na, const int* prow, int k0,
+                                                 int c1, int nc, unsigned mask) {
+  constexpr int kRows = 8, kLanes = kCV == 4 ? 16 : 32, kGroups = 32 / kLanes;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  const int cgs = (nc + kLanes * kCV - 1) / (kLanes * kCV);
+  const int rgs = (na + kRows * kGroups - 1) / (kRows * kGroups);
+  for (int unit = warp; unit < rgs * cgs; unit += warps) {
+    const int rg = unit / cgs, cg = unit - rg * cgs;
+    const int cc = (cg * kLanes + lane % kLanes) * kCV;
+    const bool on = cc < nc;
+    const int c = c1 + (on ? cc : 0);
+    const int q0 = (rg * kGroups + lane / kLanes) * kRows;
+    int row[kRows];
+    float acc[kRows][kCV];
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) {
+      row[r] = act[min(q0 + r, na - 1)] * ld;
+      if constexpr (kCV == 4) {
+        const float4 v = *reinterpret_cast<const float4*>(S + row[r] + c);
+        acc[r][0] = v.x, acc[r][1] = v.y, acc[r][2] = v.z, acc[r][3] = v.w;
+      } else {
+        acc[r][0] = S[row[r] + c];
+      }
+    }
+    // w is the whole panel width here: after a narrower (last) panel no row is left.
+#pragma unroll
+    for (int kb = 0; kb < kNB; kb += 4) {
+      float4 l[kRows];
+#pragma unroll
+      for (int r = 0; r < kRows; ++r) l[r] = *reinterpret_cast<const float4*>(S + row[r] + k0 + kb);
+#pragma unroll
+      for (int kk = 0; kk < 4; ++kk) {
+        if (kMasked && (mask >> (kb + kk)) & 1u) continue;
+        const float* up = S + prow[k0 + kb + kk] * ld + c;
+        float u[kCV];
+        if constexpr (kCV == 4) {
+          const float4 v = *reinterpret_cast<const float4*>(up);
+          u[0] = v.x, u[1] = v.y, u[2] = v.z, u[3] = v.w;
+        } else {
+          u[0] = *up;
+        }
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) {
+          const float lv = kk == 0 ? l[r].x : kk == 1 ? l[r].y : kk == 2 ? l[r].z : l[r].w;
+#pragma unroll
+          for (int e = 0; e < kCV; ++e) acc[r][e] = upd<kExact>(acc[r][e], lv, u[e]);
+        }
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) {
+      if (!on || q0 + r >= na) continue;
+      if constexpr (kCV == 4)
+        *reinterpret_cast<float4*>(S + row[r] + c) = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
+      else
+        S[row[r] + c] = acc[r][0];
+    }
+  }
 }
-template <bool kExact>
-__device__ __forceinline__ float bupd(float c, float l, float u) {
-  if (kExact) return __fsub_rn(c, __fmul_rn(l, u));
-  return fmaf(-l, u, c);
+template <bool kExact, int kNB>
+__device__ __forceinline__ void batch_update(float* S, int ld, const int* act, int na, const int* prow, int k0, int,
+                                             int c1, int nc, unsigned mask) {
+  if (mask)
+    batch_update_f32<kExact, kNB, 1, true>(S, ld, act, na, prow, k0, c1, nc, mask);
+  else if (nc > 32)
+    batch_update_f32<kExact, kNB, 4, false>(S, ld, act, na, prow, k0, c1, nc, mask);
+  else
+    batch_update_f32<kExact, kNB, 1, false>(S, ld, act, na, prow, k0, c1, nc, mask);
 }
-__device__ __forceinline__ double bmul(double a, double b) { return __dmul_rn(a, b); }
-__device__ __forceinline__ float bmul(float a, float b) { return __fmul_rn(a, b); }
+template <bool kExact, int kNB>
+__device__ __forceinline__ void batch_update(double* S, int ld, const int* act, int na, const int* prow, int k0,
+                                             int w, int c1, int nc, unsigned mask) {
+  constexpr int kE = 4;  // elements of a lane in flight
+  const int total = na * nc, step = blockDim.x * kE;
+  for (int base = threadIdx.x; base < total; base += step) {
+    int crow[kE], cc[kE];
+    double acc[kE];
+#pragma unroll
+    for (int e = 0; e < kE; ++e) {
+      const int idx = min(base + e * (int)blockDim.x, total - 1);
+      const int q = idx / nc;
+      cc[e] = c1 + idx - q * nc;
+      crow[e] = act[q] * ld;
+      acc[e] = S[crow[e] + cc[e]];
+    }
+    for (int k = 0; k < w; ++k) {
+      if ((mask >> k) & 1u) continue;
+      const int ur = prow[k0 + k] * ld;
+#pragma unroll
+      for (int e = 0; e < kE; ++e) acc[e] = upd<kExact>(acc[e], S[crow[e] + k0 + k], S[ur + cc[e]]);
+    }
+#pragma unroll
+    for (int e = 0; e < kE; ++e)
+      if (base + e * (int)blockDim.x < total) S[crow[e] + cc[e]] = acc[e];
+  }
+}
 
-// Block-wide pivot search over rows [r0, r1) of column c of S (stride ld):
-// strict '>' first-index semantics of src/blas/iamax.rs:6-21.  Returns the
-// pivot row (r0 when the column is all zero or NaN) and the max in *maxv.
+// y / d with the reciprocal r = 1/d and one correction where r and d are plain
+// numbers (`good`), else a division.
 template <typename T>
-__device__ __forceinline__ int block_iamax(const T* S, int ld, int c, int r0, int r1, T* maxv, T* red_v,
-                                           int* red_i) {
+__device__ __forceinline__ T batch_quot(T y, T d, T r, bool good) {
+  if (!good) return y / d;
+  const T q = y * r;
+  return isfinite(q) ? fma(fma(-q, d, y), r, q) : q;
+}
+
+// u[c] = P[ib][c] of lane src for c in [kC0, kCW) (ib and src uniform).
+template <typename T, int NI, int kC0, int kCW>
+__device__ __forceinline__ void batch_row(const T (&P)[NI][batch_nb<T>(NI)], int ib, int src, T (&u)[batch_nb<T>(NI)]) {
+#pragma unroll
+  for (int i = 0; i < NI; ++i)
+    if (i == ib) {
+#pragma unroll
+      for (int c = kC0; c < kCW; ++c) u[c] = __shfl_sync(0xffffffffu, P[i][c], src);
+    }
+}
+
+// Elimination step k = k0 + j of a panel, by one warp: P[i][kC0] is column k of
+// the lane's row pr[i] (logical row lid[i], alive[i] all ones while it is active),
+// P[i][kC0 + 1 ..) the panel's later columns.  kShift: the results move one
+// register to the left, so the loop over the steps needs no unrolling (FP32: 16
+// unrolled steps of 8 rows are over 100 KB of code, and the instruction fetches
+// took ten times the step); FP64 steps are unrolled, since every FMA on a column
+// past the panel would cost 64 cycles.  Finished multipliers go to S, the pivot
+// row to pv[j][0 ..).
+// The search looks at the top 32 bits of |a|; ties there, zeros, infinities and
+// NaN take the full comparison (strict > in logical row order, NaN never wins).
+template <typename T, bool kExact, int NI, int kC0, int kCW, bool kShift>
+__device__ __forceinline__ void batch_step(T (&P)[NI][batch_nb<T>(NI)], int (&lid)[NI], unsigned (&alive)[NI],
+                                           const int (&pr)[NI], int groups, T* S, int ld, int k, int j, int* piv,
+                                           int* prow, T* pv, int& sing, unsigned& mask) {
+  constexpr unsigned kFull = 0xffffffffu;
+  constexpr int NB = batch_nb<T>(NI);
+  constexpr unsigned kInfTop = sizeof(T) == 8 ? 0x7ff00000u : 0x7f800000u;
+  using K = typename PivotKey<T>::K;
+  const int lane = threadIdx.x & 31;
+  unsigned key[NI], m = 0;
+#pragma unroll
+  for (int i = 0; i < NI; ++i) {
+    key[i] = 0u;
+    if (i >= groups) continue;  // no row beyond (uniform)
+    unsigned top;
+    if constexpr (sizeof(T) == 8)
+      top = (unsigned)__double2hiint(P[i][kC0]);
+    else
+      top = __float_as_uint(P[i][kC0]);
+    key[i] = top & 0x7fffffffu & alive[i];
+    m = max(m, key[i]);
+  }
+  const unsigned best = __reduce_max_sync(kFull, m);
+  const unsigned vote = __ballot_sync(kFull, m == best);
+  int src = __ffs(vote) - 1, ib = 0, same = 0;
+#pragma unroll
+  for (int i = 0; i < NI; ++i)
+    if (i < groups && key[i] == best) {
+      ib = i;
+      ++same;
+    }
+  ib = __shfl_sync(kFull, ib | (same > 1 ? 256 : 0), src);
+  bool pivot = true;
+  if (best == 0 || best >= kInfTop || (vote & (vote - 1u)) || ib >= 256) {
+    K bk = 0;
+    int bid = INT_MAX, bi = 0, at = -1;
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+      const K full = PivotKey<T>::of(P[i][kC0]);
+      if (alive[i] && (full > bk || (full == bk && lid[i] < bid))) {
+        bk = full;
+        bid = lid[i];
+        bi = i;
+      }
+      if (alive[i] && lid[i] == k) at = i;
+    }
+    src = warp_best(bk, bid);
+    pivot = __shfl_sync(kFull, bk, src) > 0;
+    if (!pivot) {  // lair: no swap, no update; the row at k retires as it is
+      src = __ffs(__ballot_sync(kFull, at >= 0)) - 1;
+      bi = at;
+      sing = k;
+      mask |= 1u << j;
+    }
+    ib = __shfl_sync(kFull, bi, src);
+  }
+  T u[NB];
+  batch_row<T, NI, kC0, kCW>(P, ib, src, u);
+  // Relabel: the row at k takes the pivot's place, the pivot row retires as row k.
+  int mine = 0, prr = 0;
+#pragma unroll
+  for (int i = 0; i < NI; ++i)
+    if (i == ib) {
+      mine = lid[i];
+      prr = pr[i];
+    }
+  const int pl = __shfl_sync(kFull, mine, src);
+#pragma unroll
+  for (int i = 0; i < NI; ++i) {
+    if (i >= groups) continue;
+    if (lid[i] == k) lid[i] = pl;
+    if (i == ib && lane == src) {
+      lid[i] = k;
+      alive[i] = 0u;
+    }
+  }
+  if (lane == src) {
+    prow[k] = prr;
+    piv[k] = pl;
+  }
+  if (lane == 0) {
+#pragma unroll
+    for (int c = kC0; c < kCW; ++c) pv[j * NB + c - kC0] = u[c];
+  }
+  if (!pivot) {
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+      if (alive[i]) S[pr[i] * ld + k] = P[i][kC0];
+#pragma unroll
+      for (int c = kC0 + 1; c < kCW; ++c)
+        if (kShift) P[i][c - 1] = P[i][c];
+    }
+    return;
+  }
+  const T recip = T(1) / u[kC0];
+#pragma unroll
+  for (int i = 0; i < NI; ++i) {
+    if (i >= groups) continue;
+    const T l = mul_rn(P[i][kC0], recip);
+    if (alive[i]) S[pr[i] * ld + k] = l;
+#pragma unroll
+    for (int c = kC0 + 1; c < kCW; ++c) P[i][kShift ? c - 1 : c] = upd<kExact>(P[i][c], l, u[c]);
+  }
+}
+template <typename T, bool kExact, int NI, int J>
+__device__ __forceinline__ void batch_steps_unrolled(T (&P)[NI][batch_nb<T>(NI)], int (&lid)[NI], unsigned (&alive)[NI],
+                                                     const int (&pr)[NI], int groups, T* S, int ld, int k0, int w,
+                                                     int* piv, int* prow, T* pv, int& sing, unsigned& mask) {
+  if constexpr (J < batch_nb<T>(NI)) {
+    if (J >= w) return;
+    batch_step<T, kExact, NI, J, batch_nb<T>(NI), false>(P, lid, alive, pr, groups, S, ld, k0 + J, J, piv, prow, pv,
+                                                       sing, mask);
+    batch_steps_unrolled<T, kExact, NI, J + 1>(P, lid, alive, pr, groups, S, ld, k0, w, piv, prow, pv, sing, mask);
+  }
+}
+
+// Factor and solve one system held in S (n rows of stride ld, the right-hand
+// side in column n); prow: physical row of each logical row.  Returns (in warp
+// pw, which runs the panels) the last singular step or -1.
+template <typename T, bool kExact, int NI>
+__device__ __forceinline__ int batch_factor(T* S, int ld, int n, int* piv, int* prow, int* act, int* slid, T* pv,
+                                            int* s_na, unsigned* s_mask, int pw) {
+  constexpr int NB = batch_nb<T>(NI);
+  constexpr unsigned kFull = 0xffffffffu;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  T bv = T(0);
-  int bi = INT_MAX;
-  for (int r = r0 + tid; r < r1; r += kBatchThreads) {
-    const T v = fabs(S[r * ld + c]);
-    if (v > bv) {
-      bv = v;
-      bi = r;
+  int sing = -1;
+  for (int k0 = 0; k0 < n; k0 += NB) {
+    const int w = min(NB, n - k0);
+    if (warp == pw) {
+      // The active rows, in the order of act: lane's rows act[lane + 32 i].
+      const int rows = n - k0, groups = (rows + 31) / 32;
+      T P[NI][NB];
+      int lid[NI], pr[NI];
+      unsigned alive[NI];
+#pragma unroll
+      for (int i = 0; i < NI; ++i) {
+        const int q = lane + 32 * i;
+        const bool on = q < rows;
+        pr[i] = on ? act[q] : 0;
+        lid[i] = on ? slid[pr[i]] : -1;
+        alive[i] = on ? kFull : 0u;
+        const T* row = S + pr[i] * ld + k0;
+        if (sizeof(T) == 4 && w == NB) {
+#pragma unroll
+          for (int c = 0; c < NB; c += 4) {
+            const float4 v = on ? *reinterpret_cast<const float4*>(row + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+            P[i][c] = v.x, P[i][c + 1] = v.y, P[i][c + 2] = v.z, P[i][c + 3] = v.w;
+          }
+        } else {
+#pragma unroll
+          for (int c = 0; c < NB; ++c) P[i][c] = (on && c < w) ? row[c] : T(0);
+        }
+      }
+      unsigned mask = 0;
+      if constexpr (sizeof(T) == 8) {
+        batch_steps_unrolled<T, kExact, NI, 0>(P, lid, alive, pr, groups, S, ld, k0, w, piv, prow, pv, sing, mask);
+      } else {
+        const int half = min(w, NB / 2);
+        for (int j = 0; j < half; ++j)
+          batch_step<T, kExact, NI, 0, NB, true>(P, lid, alive, pr, groups, S, ld, k0 + j, j, piv, prow, pv, sing, mask);
+        for (int j = half; j < w; ++j)
+          batch_step<T, kExact, NI, 0, NB / 2, true>(P, lid, alive, pr, groups, S, ld, k0 + j, j, piv, prow, pv, sing,
+                                                     mask);
+      }
+      __syncwarp();  // act was read by every lane
+      int na = 0;
+#pragma unroll
+      for (int i = 0; i < NI; ++i) {
+        const bool rest = alive[i] != 0;
+        const unsigned vote = __ballot_sync(kFull, rest);
+        if (rest) {
+          act[na + __popc(vote & ((1u << lane) - 1u))] = pr[i];
+          slid[pr[i]] = lid[i];
+        }
+        na += __popc(vote);
+      }
+      if (lane == 0) {
+        *s_na = na;
+        *s_mask = mask;
+      }
+    }
+    __syncthreads();
+    // The pivot rows' panel part (columns k0 + j ..) from pv.
+    for (int idx = tid; idx < w * NB; idx += blockDim.x) {
+      const int j = idx / NB, c = idx - j * NB;
+      if (j + c < w) S[prow[k0 + j] * ld + k0 + j + c] = pv[idx];
+    }
+    const int c1 = k0 + w, nc = n + 1 - c1, na = *s_na;
+    const unsigned mask = *s_mask;
+    for (int c = c1 + tid; c <= n; c += blockDim.x) {
+      T t[NB];
+#pragma unroll
+      for (int i = 0; i < NB; ++i) t[i] = i < w ? S[prow[k0 + i] * ld + c] : T(0);
+#pragma unroll
+      for (int i = 1; i < NB; ++i) {
+        if (i >= w) break;
+        const T* l = S + prow[k0 + i] * ld + k0;
+#pragma unroll
+        for (int j = 0; j < NB; ++j)
+          if (j < i && !((mask >> j) & 1u)) t[i] = upd<kExact>(t[i], l[j], t[j]);
+        S[prow[k0 + i] * ld + c] = t[i];
+      }
+    }
+    if (na > 0) {
+      __syncthreads();
+      batch_update<kExact, NB>(S, ld, act, na, prow, k0, w, c1, nc, mask);
+    }
+    __syncthreads();
+  }
+  return sing;
+}
+
+// Back substitution of the factored system; x to global memory.
+template <typename T, bool kExact, int NI>
+__device__ __forceinline__ void batch_back(T* S, int ld, int n, const int* prow, T* xg, int pw) {
+  constexpr unsigned kFull = 0xffffffffu;
+  if (kExact) {
+    // lair's order: x[i] -= u[i][k] x[k] for k = i+1.. in increasing k.
+    if ((int)threadIdx.x == 32 * pw)
+      for (int i = n - 1; i >= 0; --i) {
+        const T* u = S + prow[i] * ld;
+        T acc = u[n];
+        for (int k = i + 1; k < n; ++k) acc = upd<true>(acc, u[k], S[prow[k] * ld + n]);
+        acc = acc / u[i];
+        S[prow[i] * ld + n] = acc;
+        xg[i] = acc;
+      }
+    return;
+  }
+  if ((int)(threadIdx.x >> 5) != pw) return;
+  const int lane = threadIdx.x & 31;
+  T x[NI], d[NI], rc[NI];
+  const T* row[NI];
+  bool good = true;
+#pragma unroll
+  for (int q = 0; q < NI; ++q) {
+    const int i = lane + 32 * q;
+    const bool on = i < n;
+    row[q] = S + (on ? prow[i] : 0) * ld;
+    x[q] = on ? row[q][n] : T(0);
+    d[q] = on ? row[q][i] : T(1);
+    rc[q] = T(1) / d[q];
+    good = good && isfinite(rc[q]) && isfinite(d[q]) && fabs(rc[q]) > T(1e-30) && fabs(d[q]) > T(1e-30);
+  }
+  good = __all_sync(kFull, good);
+#pragma unroll
+  for (int qb = NI - 1; qb >= 0; --qb) {
+    if (32 * qb >= n) continue;
+    for (int kk = min(31, n - 1 - 32 * qb); kk >= 0; --kk) {
+      const int k = 32 * qb + kk;
+      if (lane == kk) x[qb] = batch_quot(x[qb], d[qb], rc[qb], good);
+      const T xk = __shfl_sync(kFull, x[qb], kk);
+#pragma unroll
+      for (int q = 0; q < NI; ++q)
+        if (q < qb || (q == qb && lane < kk)) x[q] = upd<false>(x[q], row[q][k], xk);
     }
   }
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) {
-    const T v2 = __shfl_down_sync(0xffffffffu, bv, off);
-    const int i2 = __shfl_down_sync(0xffffffffu, bi, off);
-    if (v2 > bv || (v2 == bv && i2 < bi)) {
-      bv = v2;
-      bi = i2;
-    }
-  }
-  if (lane == 0) {
-    red_v[warp] = bv;
-    red_i[warp] = bi;
-  }
-  __syncthreads();
-  if (tid == 0) {
-    for (int q = 1; q < kBatchThreads / 32; ++q)
-      if (red_v[q] > bv || (red_v[q] == bv && red_i[q] < bi)) {
-        bv = red_v[q];
-        bi = red_i[q];
-      }
-    red_v[0] = bv;
-    red_i[0] = (bv > T(0)) ? bi : r0;
-  }
-  __syncthreads();
-  const int p = red_i[0];
-  *maxv = red_v[0];
-  __syncthreads();  // red_* reused by the next search
-  return p;
+  for (int q = 0; q < NI; ++q)
+    if (lane + 32 * q < n) xg[lane + 32 * q] = x[q];
 }
 
-// Unblocked elimination of columns [c0, c0 + w) of S (rows [c0, nrow) active),
-// row swaps across columns [0, ncol).  Pivots are recorded as absolute rows
-// (row offset `roff` added).  Returns the last singular step (+roff) or -1.
-template <typename T, bool kExact>
-__device__ int eliminate(T* S, int ld, int nrow, int ncol, int c0, int w, int roff, int* piv, T* red_v, int* red_i) {
-  const int tid = threadIdx.x;
-  int sing = -1;
-  for (int j = 0; j < w; ++j) {
-    const int k = c0 + j;
-    T maxv;
-    const int p = block_iamax<T>(S, ld, k, k, nrow, &maxv, red_v, red_i);
-    if (!(maxv > T(0))) {
-      sing = k + roff;
-      if (tid == 0) piv[k] = k + roff;
-      continue;
-    }
-    if (tid == 0) piv[k] = p + roff;
-    if (p != k)
-      for (int c = tid; c < ncol; c += kBatchThreads) {
-        const T t = S[k * ld + c];
-        S[k * ld + c] = S[p * ld + c];
-        S[p * ld + c] = t;
-      }
-    __syncthreads();
-    const T recip = T(1) / S[k * ld + k];
-    for (int r = k + 1 + tid; r < nrow; r += kBatchThreads) S[r * ld + k] = bmul(S[r * ld + k], recip);
-    __syncthreads();
-    const int cols = c0 + w - k - 1;  // update only the columns of this panel
-    if (cols > 0 && k + 1 < nrow) {
-      // Fixed column per thread, rows strided: one division per step.
-      const int rstep = kBatchThreads / cols;  // >= 1 since cols < 256
-      const int tr = tid / cols, tc = tid - tr * cols;
-      if (tr < rstep) {
-        const int c = k + 1 + tc;
-        const T u = S[k * ld + c];
-        for (int r = k + 1 + tr; r < nrow; r += rstep) S[r * ld + c] = bupd<kExact>(S[r * ld + c], S[r * ld + k], u);
-      }
-    }
-    __syncthreads();
-  }
-  return sing;
+// Threads of a CTA, and CTAs an SM's registers must hold.
+__host__ __device__ constexpr int batch_max_threads(size_t elem, int ni) { return elem == 4 && ni == 8 ? 256 : 128; }
+__host__ __device__ constexpr int batch_min_ctas(size_t elem, int ni) {
+  return ni <= 2 ? 5 : elem == 4 ? (ni == 4 ? 4 : 2) : (ni == 4 ? 3 : 2);
 }
 
-// x <- U^-1 L^-1 P^T x for factors in M (stride ld, may be shared or global).
-template <typename T, bool kExact>
-__device__ void solve_factored(const T* M, int ld, int n, const int* piv, int poff, T* x) {
-  const int tid = threadIdx.x;
-  if (tid == 0)
-    for (int i = 0; i < n; ++i) {
-      const int p = piv[i] - poff;
-      if (p != i) {
-        const T t = x[i];
-        x[i] = x[p];
-        x[p] = t;
-      }
-    }
-  __syncthreads();
-  // Forward (unit L), column-oriented: x[i] takes its updates in increasing k.
-  for (int k = 0; k < n - 1; ++k) {
-    const T xk = x[k];
-    for (int i = k + 1 + tid; i < n; i += kBatchThreads) x[i] = bupd<kExact>(x[i], M[i * ld + k], xk);
-    __syncthreads();
-  }
-  if (kExact) {
-    // lair's backward order: x[i] -= u[i][k] * x[k] for k = i+1.. in increasing k.
-    if (tid == 0)
-      for (int i = n - 1; i >= 0; --i) {
-        T acc = x[i];
-        for (int k = i + 1; k < n; ++k) acc = bupd<true>(acc, M[i * ld + k], x[k]);
-        x[i] = acc / M[i * ld + i];
-      }
-    __syncthreads();
-  } else {
-    for (int k = n - 1; k >= 0; --k) {
-      const T xk = x[k] / M[k * ld + k];
-      __syncthreads();
-      if (tid == 0) x[k] = xk;
-      for (int i = tid; i < k; i += kBatchThreads) x[i] = bupd<false>(x[i], M[i * ld + k], xk);
-      __syncthreads();
-    }
-  }
-}
-
-template <typename T, bool kExact>
-__device__ int lu_solve_smem(T* A, T* xg, int* piv, int n, T* sm, T* red_v, int* red_i) {
-  const int tid = threadIdx.x;
-  const int ld = n + 1;
-  T* S = sm;
-  T* xs = sm + n * ld;
-  for (int idx = tid; idx < n * n; idx += kBatchThreads) S[(idx / n) * ld + idx % n] = A[idx];
-  for (int i = tid; i < n; i += kBatchThreads) xs[i] = xg[i];
-  __syncthreads();
-  const int sing = eliminate<T, kExact>(S, ld, n, n, 0, n, 0, piv, red_v, red_i);
-  solve_factored<T, kExact>(S, ld, n, piv, 0, xs);
-  for (int idx = tid; idx < n * n; idx += kBatchThreads) A[idx] = S[(idx / n) * ld + idx % n];
-  for (int i = tid; i < n; i += kBatchThreads) xg[i] = xs[i];
-  __syncthreads();
-  return sing;
-}
-
-template <typename T, bool kExact>
-__device__ int lu_solve_blocked(T* A, T* xg, int* piv, int n, int nb, T* sm, T* red_v, int* red_i) {
-  const int tid = threadIdx.x;
-  int sing = -1;
-  for (int k0 = 0; k0 < n; k0 += nb) {
-    const int w = min(nb, n - k0);
-    const int prow = n - k0;
-    const int ld = w + 1;
-    T* P = sm;  // panel rows [k0, n), columns [k0, k0+w)
-    for (int idx = tid; idx < prow * w; idx += kBatchThreads) {
-      const int r = idx / w, c = idx - r * w;
-      P[r * ld + c] = A[(k0 + r) * n + k0 + c];
-    }
-    __syncthreads();
-    // piv entries k0.. are written relative to the panel, then made absolute.
-    const int s = eliminate<T, kExact>(P, ld, prow, w, 0, w, k0, piv + k0, red_v, red_i);
-    if (s >= 0) sing = s;
-    for (int idx = tid; idx < prow * w; idx += kBatchThreads) {
-      const int r = idx / w, c = idx - r * w;
-      A[(k0 + r) * n + k0 + c] = P[r * ld + c];
-    }
-    __syncthreads();
-    // Interchanges on the columns outside the panel, in order.
-    const int nout = n - w;
-    for (int c2 = tid; c2 < nout; c2 += kBatchThreads) {
-      const int c = (c2 < k0) ? c2 : c2 + w;
-      for (int j = 0; j < w; ++j) {
-        const int r = k0 + j, p = piv[k0 + j];
-        if (p != r) {
-          const T t = A[r * n + c];
-          A[r * n + c] = A[p * n + c];
-          A[p * n + c] = t;
-        }
-      }
-    }
-    __syncthreads();
-    const int c1 = k0 + w;
-    if (c1 < n) {
-      // U12 <- L11^-1 A12, one column per thread, increasing elimination step.
-      for (int c = c1 + tid; c < n; c += kBatchThreads)
-        for (int r = 1; r < w; ++r) {
-          T acc = A[(k0 + r) * n + c];
-          for (int q = 0; q < r; ++q) acc = bupd<kExact>(acc, P[r * ld + q], A[(k0 + q) * n + c]);
-          A[(k0 + r) * n + c] = acc;
-        }
-      __syncthreads();
-      // A22 <- A22 - L21 U12, each element's updates in increasing step.
-      const int rows = n - c1, cols = n - c1;
-      for (int idx = tid; idx < rows * cols; idx += kBatchThreads) {
-        const int r = idx / cols, c = idx - r * cols;
-        T acc = A[(c1 + r) * n + c1 + c];
-        for (int q = 0; q < w; ++q) acc = bupd<kExact>(acc, P[(w + r) * ld + q], A[(k0 + q) * n + c1 + c]);
-        A[(c1 + r) * n + c1 + c] = acc;
-      }
-      __syncthreads();
-    }
-  }
-  solve_factored<T, kExact>(A, n, n, piv, 0, xg);
-  return sing;
-}
-
-template <typename T, bool kExact>
-__global__ void __launch_bounds__(kBatchThreads) batched_lu_kernel(BatchMeta m, T* a, T* b, int* piv, int* info,
-                                                                   int* counter) {
+// kScratch: the matrix lives in this CTA's part of `scratch`.
+template <typename T, bool kExact, int NI, bool kScratch>
+__global__ void __launch_bounds__(batch_max_threads(sizeof(T), NI), batch_min_ctas(sizeof(T), NI)) batched_lu_kernel(BatchMeta m, T* a, T* b, int* piv, int* info, int* counter,
+                                                         T* scratch) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* sm = reinterpret_cast<T*>(smem_raw);
-  __shared__ T red_v[kBatchThreads / 32];
-  __shared__ int red_i[kBatchThreads / 32];
-  __shared__ int s_item;
+  __shared__ int prow[kBatchMaxN], act[kBatchMaxN], slid[kBatchMaxN];
+  __shared__ __align__(16) T pv[batch_nb<T>(NI) * batch_nb<T>(NI)];
+  __shared__ int s_item, s_na;
+  __shared__ unsigned s_mask;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5;
+  // The panel warps of an SM's CTAs (numbers 152 apart as they are first placed)
+  // on different quarters of it, whose FP64 pipes they occupy.
+  const int pw = (blockIdx.x / kNumSmsGB300) & 3;
   for (;;) {
-    if (threadIdx.x == 0) s_item = atomicAdd(counter, 1);
+    if (tid == 0) s_item = atomicAdd(counter, 1);
     __syncthreads();
     const int item = s_item;
-    __syncthreads();
     if (item >= m.count) break;
     const int sys = m.order[item];
     const int n = m.sizes[sys];
-    if (n <= 0 || n > kBatchMaxN) {
-      if (threadIdx.x == 0) info[sys] = -2;  // rejected on the host; never reached
-      continue;
-    }
     T* A = a + m.aoff[sys];
-    T* x = b + m.boff[sys];
-    int* p = piv + m.boff[sys];
-    const int nb = m.tune[batch_bucket(n)];
-    int sing;
-    if ((nb == 0 && n <= m.smem_n) || n <= 8)
-      sing = lu_solve_smem<T, kExact>(A, x, p, n, sm, red_v, red_i);
-    else
-      sing = lu_solve_blocked<T, kExact>(A, x, p, n, nb > 0 ? nb : 32, sm, red_v, red_i);
-    if (threadIdx.x == 0) info[sys] = sing;
+    T* xg = b + m.boff[sys];
+    T* S = kScratch ? scratch + (size_t)blockIdx.x * kScratchElems : reinterpret_cast<T*>(smem_raw);
+    const int ld = kScratch ? kScratchLd : batch_ld<T>(n);
+    if (n >= 32) {
+      // 32-column pieces of rows, four loads of a lane in flight.
+      const int pieces = (n + 31) / 32, items = n * pieces;
+      for (int it = warp; it < items; it += 4 * warps) {
+        T v[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int q = it + e * warps, r = q / pieces, c = (q - r * pieces) * 32 + lane;
+          v[e] = (q < items && c < n) ? A[r * n + c] : T(0);
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int q = it + e * warps, r = q / pieces, c = (q - r * pieces) * 32 + lane;
+          if (q < items && c < n) S[r * ld + c] = v[e];
+        }
+      }
+    } else {
+      for (int idx = tid; idx < n * n; idx += blockDim.x) S[(idx / n) * ld + idx % n] = A[idx];
+    }
+    for (int i = tid; i < n; i += blockDim.x) {
+      S[i * ld + n] = xg[i];
+      act[i] = slid[i] = i;
+    }
+    __syncthreads();
+    const int sing = batch_factor<T, kExact, NI>(S, ld, n, piv + m.boff[sys], prow, act, slid, pv, &s_na,
+                                                 &s_mask, pw);
+    batch_back<T, kExact, NI>(S, ld, n, prow, xg, pw);
+    if (n >= 32) {
+      for (int r = warp; r < n; r += warps) {
+        const T* src = S + prow[r] * ld;
+        for (int c = lane; c < n; c += 32) A[r * n + c] = src[c];
+      }
+    } else {
+      for (int idx = tid; idx < n * n; idx += blockDim.x) A[idx] = S[prow[idx / n] * ld + idx % n];
+    }
+    if (tid == 32 * pw) info[sys] = sing;
+    __syncthreads();
   }
 }
 
@@ -312,6 +548,21 @@ __global__ void __launch_bounds__(kBatchThreads) batched_lu_kernel(BatchMeta m, 
 // ---------------------------------------------------------------------------
 // Plan object (host).
 // ---------------------------------------------------------------------------
+namespace luhot {
+
+// A launch: the systems order[first .. first + count) on CTAs of one kernel.
+struct BatchClass {
+  int first = 0, count = 0;
+  int ni = 1;            // rows of a panel lane
+  bool scratch = false;
+  int threads = 0, grid = 0;
+  size_t smem = 0;
+};
+constexpr int kMaxBatchClasses = 16;
+constexpr int kBatchStreams = 4;  // the capturing stream and three branches
+
+}  // namespace luhot
+
 struct luhot_batch {
   luhot_ctx* ctx = nullptr;
   int dtype = 0;  // 0 f64, 1 f32
@@ -321,13 +572,18 @@ struct luhot_batch {
   std::vector<int> sizes;
   std::vector<int64_t> aoff, boff;
   std::vector<int> order;
-  int tune[luhot::kBuckets];
+  std::vector<luhot::BatchClass> classes;
+  int tune[luhot::kBuckets];  // 0: shared memory where it fits, else the panel width of the scratch form
   int smem_n = 0;
-  int grid = 0;
-  // device metadata: sizes, aoff, boff, order, tune, counter
+  // device metadata: sizes, aoff, boff, order, counters
   void* d_meta = nullptr;
   int* d_counter = nullptr;
   luhot::BatchMeta meta{};
+  // matrices of the CTAs of scratch classes (none without such systems)
+  void* d_scratch = nullptr;
+  size_t scratch_ctas = 0;
+  cudaStream_t branch[luhot::kBatchStreams - 1] = {nullptr, nullptr, nullptr};
+  cudaEvent_t fork = nullptr, joined[luhot::kBatchStreams - 1] = {nullptr, nullptr, nullptr};
   // cached graph
   cudaGraphExec_t exec = nullptr;
   cudaGraph_t graph = nullptr;
@@ -337,55 +593,137 @@ struct luhot_batch {
 namespace luhot {
 
 static size_t elem_size(int dtype) { return dtype == 0 ? sizeof(double) : sizeof(float); }
+static size_t smem_bytes(int dtype, int n) {
+  return dtype == 0 ? (size_t)n * batch_ld<double>(n) * sizeof(double) : (size_t)n * batch_ld<float>(n) * sizeof(float);
+}
+static int batch_width(int dtype) { return dtype == 0 ? batch_nb<double>(8) : batch_nb<float>(8); }
 
-static int smem_n_for(size_t budget, size_t es) {
+static int smem_n_for(int dtype, size_t budget) {
   int n = 8;
-  while ((size_t)((n + 1) * (n + 2) + (n + 1)) * es <= budget && n + 1 <= kBatchMaxN) ++n;
+  while (n + 1 <= kBatchMaxN && smem_bytes(dtype, n + 1) <= budget) ++n;
   return n;
 }
 
 template <typename T, bool kExact>
-static cudaError_t launch_batched(luhot_ctx* ctx, const BatchMeta& m, int grid, void* a, void* b, int* piv, int* info,
-                                  int* counter, cudaStream_t stream) {
-  // The shared-memory attribute was set when the plan was created (grid_for),
-  // outside any stream capture.
-  auto k = batched_lu_kernel<T, kExact>;
-  cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(int), stream);
-  if (e != cudaSuccess) return e;
-  k<<<grid, kBatchThreads, kBatchSmem, stream>>>(m, static_cast<T*>(a), static_cast<T*>(b), piv, info, counter);
-  (void)ctx;
-  return cudaGetLastError();
+static const void* batch_kernel_of(int ni, bool scratch) {
+  if (scratch)
+    return ni == 1   ? (const void*)batched_lu_kernel<T, kExact, 1, true>
+           : ni == 2 ? (const void*)batched_lu_kernel<T, kExact, 2, true>
+           : ni == 4 ? (const void*)batched_lu_kernel<T, kExact, 4, true>
+                     : (const void*)batched_lu_kernel<T, kExact, 8, true>;
+  return ni == 1   ? (const void*)batched_lu_kernel<T, kExact, 1, false>
+         : ni == 2 ? (const void*)batched_lu_kernel<T, kExact, 2, false>
+         : ni == 4 ? (const void*)batched_lu_kernel<T, kExact, 4, false>
+                   : (const void*)batched_lu_kernel<T, kExact, 8, false>;
 }
-
-static cudaError_t launch_plan(luhot_batch* p, const BatchMeta& m, int grid, void* a, void* b, int* piv, int* info,
-                               int* counter, cudaStream_t stream) {
-  const bool ex = p->mode == LUHOT_MODE_EXACT;
-  if (p->dtype == 0)
-    return ex ? launch_batched<double, true>(p->ctx, m, grid, a, b, piv, info, counter, stream)
-              : launch_batched<double, false>(p->ctx, m, grid, a, b, piv, info, counter, stream);
-  return ex ? launch_batched<float, true>(p->ctx, m, grid, a, b, piv, info, counter, stream)
-            : launch_batched<float, false>(p->ctx, m, grid, a, b, piv, info, counter, stream);
-}
-
-static int grid_for(luhot_ctx* ctx, int dtype, int mode) {
-  int per_sm = 0;
-  const void* k;
+static const void* batch_kernel(int dtype, int mode, int ni, bool scratch) {
+  const bool ex = mode == LUHOT_MODE_EXACT;
   if (dtype == 0)
-    k = mode == LUHOT_MODE_EXACT ? (const void*)batched_lu_kernel<double, true> : (const void*)batched_lu_kernel<double, false>;
-  else
-    k = mode == LUHOT_MODE_EXACT ? (const void*)batched_lu_kernel<float, true> : (const void*)batched_lu_kernel<float, false>;
-  allow_max_dynamic_smem(k);
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kBatchThreads, kBatchSmem) != cudaSuccess) {
-    cudaGetLastError();
-    per_sm = 1;
+    return ex ? batch_kernel_of<double, true>(ni, scratch) : batch_kernel_of<double, false>(ni, scratch);
+  return ex ? batch_kernel_of<float, true>(ni, scratch) : batch_kernel_of<float, false>(ni, scratch);
+}
+
+// Orders the systems (indices into sizes) by class, largest class and largest
+// system first.  A class is a panel form (NI) and the number of its largest
+// matrices that fit in an SM's shared memory (or the scratch form).
+static void build_classes(luhot_ctx* ctx, int dtype, int mode, const int* tune, int smem_n,
+                          const std::vector<int>& sizes, std::vector<int>& order, std::vector<BatchClass>& classes) {
+  auto key = [&](int n) {
+    const int ni = n <= 32 ? 1 : n <= 64 ? 2 : n <= 128 ? 4 : 8;
+    const bool scratch = n > smem_n || tune[batch_bucket(n)] != 0;
+    const size_t bytes = smem_bytes(dtype, n);
+    int fit = 8;  // CTAs to an SM
+    if (scratch)
+      fit = 0;
+    else
+      for (int f : {6, 4, 3, 2, 1})
+        if (bytes + 3 * 1024 > kBatchSmem / f) fit = f == 6 ? 4 : f == 4 ? 3 : f == 3 ? 2 : 1;
+    return (8 - ni) * 16 + fit;  // larger rows first, then fewer to an SM
+  };
+  order.resize(sizes.size());
+  std::iota(order.begin(), order.end(), 0);
+  std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
+    const int kx = key(sizes[x]), ky = key(sizes[y]);
+    return kx != ky ? kx < ky : sizes[x] > sizes[y];
+  });
+  classes.clear();
+  for (size_t i = 0; i < order.size();) {
+    const int n = sizes[order[i]], k = key(n);
+    size_t e = i;
+    while (e < order.size() && key(sizes[order[e]]) == k) ++e;
+    BatchClass c;
+    c.first = (int)i;
+    c.count = (int)(e - i);
+    c.ni = 8 - k / 16;
+    c.scratch = k % 16 == 0;
+    c.smem = c.scratch ? 0 : smem_bytes(dtype, n);  // the class's first system is its largest
+    // Few matrices of more than 128 rows fit in an SM's shared memory: 8 warps each.
+    c.threads = c.scratch ? 128 : batch_max_threads(elem_size(dtype), c.ni);
+    const void* kern = batch_kernel(dtype, mode, c.ni, c.scratch);
+    allow_max_dynamic_smem(kern);
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, c.threads, c.smem) != cudaSuccess) {
+      cudaGetLastError();
+      per_sm = 1;
+    }
+    c.grid = std::min(c.count, std::max(1, per_sm) * ctx->num_sms);
+    classes.push_back(c);
+    i = e;
   }
-  return std::max(1, per_sm) * ctx->num_sms;
+}
+
+// Clears the counters and launches every class, the branches' share on their
+// streams between a fork and a join (so a capture of `stream` holds them all).
+static cudaError_t launch_classes(luhot_batch* p, const std::vector<BatchClass>& classes, const BatchMeta& m,
+                                  void* scratch, void* a, void* b, int* piv, int* info, int* counters,
+                                  cudaStream_t stream) {
+  cudaError_t e = cudaMemsetAsync(counters, 0, kMaxBatchClasses * sizeof(int), stream);
+  const int nb = std::min((int)classes.size(), kBatchStreams) - 1;
+  if (e == cudaSuccess && nb > 0) e = cudaEventRecord(p->fork, stream);
+  for (int q = 0; q < nb && e == cudaSuccess; ++q) e = cudaStreamWaitEvent(p->branch[q], p->fork, 0);
+  char* sp = static_cast<char*>(scratch);
+  for (size_t i = 0; i < classes.size() && e == cudaSuccess; ++i) {
+    const BatchClass& c = classes[i];
+    BatchMeta cm = m;
+    cm.order = m.order + c.first;
+    cm.count = c.count;
+    int* counter = counters + i;
+    void* cs = c.scratch ? sp : nullptr;
+    if (c.scratch) sp += (size_t)c.grid * kScratchElems * elem_size(p->dtype);
+    void* args[] = {&cm, &a, &b, &piv, &info, &counter, &cs};
+    const int q = (int)(i % kBatchStreams);
+    e = cudaLaunchKernel(batch_kernel(p->dtype, p->mode, c.ni, c.scratch), dim3(c.grid), dim3(c.threads), args, c.smem,
+                         q == 0 ? stream : p->branch[q - 1]);
+  }
+  for (int q = 0; q < nb; ++q) {  // the join, also after an error
+    cudaError_t j = cudaEventRecord(p->joined[q], p->branch[q]);
+    if (j == cudaSuccess) j = cudaStreamWaitEvent(stream, p->joined[q], 0);
+    if (e == cudaSuccess) e = j;
+  }
+  return e;
+}
+
+static size_t scratch_ctas(const std::vector<BatchClass>& classes) {
+  size_t n = 0;
+  for (const auto& c : classes)
+    if (c.scratch) n += c.grid;
+  return n;
 }
 
 static int upload_meta(luhot_batch* p) {
   luhot_ctx* ctx = p->ctx;
   const size_t c = (size_t)p->count;
-  const size_t bytes = c * (sizeof(int) + 2 * sizeof(int64_t) + sizeof(int)) + kBuckets * sizeof(int) + 256;
+  build_classes(ctx, p->dtype, p->mode, p->tune, p->smem_n, p->sizes, p->order, p->classes);
+  if ((int)p->classes.size() > kMaxBatchClasses) return set_error(ctx, LUHOT_ERR_UNSUPPORTED, "batch: too many size classes");
+  const size_t need = scratch_ctas(p->classes);
+  if (need > p->scratch_ctas) {
+    if (p->d_scratch) cudaFree(p->d_scratch);
+    p->d_scratch = nullptr;
+    p->scratch_ctas = 0;
+    LUHOT_CUDA_TRY(ctx, cudaMalloc(&p->d_scratch, need * kScratchElems * elem_size(p->dtype)));
+    p->scratch_ctas = need;
+  }
+  const size_t bytes = c * (sizeof(int) + 2 * sizeof(int64_t) + sizeof(int)) + 256;
   if (!p->d_meta) {
     LUHOT_CUDA_TRY(ctx, cudaMalloc(&p->d_meta, bytes));
     LUHOT_CUDA_TRY(ctx, cudaMalloc(&p->d_counter, 256));
@@ -395,19 +733,15 @@ static int upload_meta(luhot_batch* p) {
   int64_t* boff = aoff + c;
   int* sizes = reinterpret_cast<int*>(boff + c);
   int* order = sizes + c;
-  int* tune = order + c;
   LUHOT_CUDA_TRY(ctx, cudaMemcpy(aoff, p->aoff.data(), c * sizeof(int64_t), cudaMemcpyHostToDevice));
   LUHOT_CUDA_TRY(ctx, cudaMemcpy(boff, p->boff.data(), c * sizeof(int64_t), cudaMemcpyHostToDevice));
   LUHOT_CUDA_TRY(ctx, cudaMemcpy(sizes, p->sizes.data(), c * sizeof(int), cudaMemcpyHostToDevice));
   LUHOT_CUDA_TRY(ctx, cudaMemcpy(order, p->order.data(), c * sizeof(int), cudaMemcpyHostToDevice));
-  LUHOT_CUDA_TRY(ctx, cudaMemcpy(tune, p->tune, kBuckets * sizeof(int), cudaMemcpyHostToDevice));
   p->meta.sizes = sizes;
   p->meta.aoff = aoff;
   p->meta.boff = boff;
   p->meta.order = order;
-  p->meta.tune = tune;
   p->meta.count = (int)p->count;
-  p->meta.smem_n = p->smem_n;
   return LUHOT_OK;
 }
 
@@ -454,16 +788,18 @@ int luhot_batch_create(luhot_ctx* ctx, int64_t count, const int32_t* sizes, int 
   }
   p->a_elems = ao;
   p->b_elems = bo;
-  p->order.resize(count);
-  std::iota(p->order.begin(), p->order.end(), 0);
-  std::stable_sort(p->order.begin(), p->order.end(), [&](int x, int y) { return p->sizes[x] > p->sizes[y]; });
-  p->smem_n = smem_n_for(kBatchSmem, elem_size(dtype));
-  // Untuned default: shared memory where it fits, else 32-wide panels.
-  for (int bk = 0; bk < kBuckets; ++bk) {
-    const int hi = bk == 0 ? 16 : bk == 1 ? 32 : bk == 2 ? 64 : 64 + 32 * (bk - 2);
-    p->tune[bk] = hi <= p->smem_n ? 0 : 32;
+  p->smem_n = smem_n_for(dtype, kBatchSmem);
+  // Untuned: shared memory where it fits for FP32; FP64 up to 96, where three
+  // CTAs or more share an SM (its pipe idles while one CTA's panel runs).
+  for (int bk = 0; bk < kBuckets; ++bk) p->tune[bk] = dtype == 0 && bk > 3 ? batch_width(dtype) : 0;
+  bool ok = cudaEventCreateWithFlags(&p->fork, cudaEventDisableTiming) == cudaSuccess;
+  for (int q = 0; q < kBatchStreams - 1; ++q)
+    ok = ok && cudaStreamCreateWithFlags(&p->branch[q], cudaStreamNonBlocking) == cudaSuccess &&
+         cudaEventCreateWithFlags(&p->joined[q], cudaEventDisableTiming) == cudaSuccess;
+  if (!ok) {
+    luhot_batch_destroy(p);
+    return set_error(ctx, LUHOT_ERR_CUDA, std::string("batch: ") + cudaGetErrorString(cudaGetLastError()));
   }
-  p->grid = grid_for(ctx, dtype, mode);
   int rc = count > 0 ? upload_meta(p) : LUHOT_OK;
   if (rc) {
     luhot_batch_destroy(p);
@@ -479,6 +815,12 @@ void luhot_batch_destroy(luhot_batch* p) {
   drop_graph(p);
   if (p->d_meta) cudaFree(p->d_meta);
   if (p->d_counter) cudaFree(p->d_counter);
+  if (p->d_scratch) cudaFree(p->d_scratch);
+  for (auto& s : p->branch)
+    if (s) cudaStreamDestroy(s);
+  for (auto& e : p->joined)
+    if (e) cudaEventDestroy(e);
+  if (p->fork) cudaEventDestroy(p->fork);
   delete p;
 }
 
@@ -507,9 +849,10 @@ int luhot_batch_solve(luhot_batch* p, void* d_a, void* d_b, int32_t* d_piv, int3
   void* ptrs[4] = {d_a, d_b, d_piv, d_info};
   if (!p->exec || memcmp(ptrs, p->g_ptrs, sizeof(ptrs)) != 0) {
     drop_graph(p);
-    // Capture [counter reset, persistent kernel] once for these buffers.
+    // Capture [counter reset, the classes' launches] once for these buffers.
     LUHOT_CUDA_TRY(ctx, cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-    cudaError_t e = launch_plan(p, p->meta, p->grid, d_a, d_b, d_piv, d_info, p->d_counter, ctx->stream);
+    cudaError_t e = launch_classes(p, p->classes, p->meta, p->d_scratch, d_a, d_b, d_piv, d_info, p->d_counter,
+                                   ctx->stream);
     cudaGraph_t graph = nullptr;
     cudaError_t e2 = cudaStreamEndCapture(ctx->stream, &graph);
     if (e != cudaSuccess || e2 != cudaSuccess) {
@@ -531,9 +874,11 @@ int luhot_batch_solve(luhot_batch* p, void* d_a, void* d_b, int32_t* d_piv, int3
   return LUHOT_OK;
 }
 
-// Time every candidate (shared-memory path where it fits, panels of 8, 16,
-// 32) per size bucket on up to 48 sample systems of that bucket, copied from
-// the caller's data into scratch before each run, and keep the fastest.
+// Time both forms (shared memory where it fits, scratch) per size bucket on up
+// to 304 sample systems of that bucket (two per SM, so that it is throughput and
+// not one system's latency that is compared), copied from the caller's data into
+// scratch before each run, and keep the faster.
+constexpr size_t kTuneSample = 2 * kNumSmsGB300;
 int luhot_batch_autotune(luhot_batch* p, const void* d_a, const void* d_b) {
   LUHOT_NVTX_FN();
   if (!p) return LUHOT_ERR_INVALID_ARG;
@@ -545,7 +890,7 @@ int luhot_batch_autotune(luhot_batch* p, const void* d_a, const void* d_b) {
   std::vector<std::vector<int>> members(kBuckets);
   for (int64_t i = 0; i < p->count; ++i) {
     auto& v = members[batch_bucket(p->sizes[i])];
-    if (v.size() < 48) v.push_back((int)i);
+    if (v.size() < kTuneSample) v.push_back((int)i);
   }
   // Scratch: sample matrices + rhs, and a pristine copy to restore from.
   int64_t sa = 0, sb = 0;
@@ -588,63 +933,70 @@ int luhot_batch_autotune(luhot_batch* p, const void* d_a, const void* d_b) {
   }
   bucket_first[kBuckets] = (int)s_sizes.size();
   const int ns = (int)s_sizes.size();
-  DevBuf meta_buf;
-  rc = ensure_buf(ctx, meta_buf, (size_t)ns * (2 * sizeof(int64_t) + 2 * sizeof(int)) + kBuckets * sizeof(int) + 512);
+  DevBuf meta_buf, mat_buf;
+  rc = ensure_buf(ctx, meta_buf, (size_t)ns * (2 * sizeof(int64_t) + 2 * sizeof(int)) + kMaxBatchClasses * sizeof(int) + 512);
   if (rc) return rc;
   int64_t* m_aoff = static_cast<int64_t*>(meta_buf.ptr);
   int64_t* m_boff = m_aoff + ns;
   int* m_sizes = reinterpret_cast<int*>(m_boff + ns);
   int* m_order = m_sizes + ns;
-  int* m_tune = m_order + ns;
-  int* m_counter = m_tune + kBuckets + 1;
+  int* m_counter = m_order + ns;
   cudaMemcpy(m_aoff, s_aoff.data(), ns * sizeof(int64_t), cudaMemcpyHostToDevice);
   cudaMemcpy(m_boff, s_boff.data(), ns * sizeof(int64_t), cudaMemcpyHostToDevice);
   cudaMemcpy(m_sizes, s_sizes.data(), ns * sizeof(int), cudaMemcpyHostToDevice);
-  cudaMemcpy(m_order, s_order.data(), ns * sizeof(int), cudaMemcpyHostToDevice);
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
-  const int cands[4] = {0, 8, 16, 32};
-  for (int bk = 0; bk < kBuckets; ++bk) {
+  cudaError_t err = cudaSuccess;
+  for (int bk = 0; bk < kBuckets && !rc; ++bk) {
     const int first = bucket_first[bk], cnt = bucket_first[bk + 1] - first;
     if (cnt == 0) continue;
-    int maxn = 0;
-    for (int q = first; q < first + cnt; ++q) maxn = std::max(maxn, s_sizes[q]);
+    const std::vector<int> b_sizes(s_sizes.begin() + first, s_sizes.begin() + first + cnt);
+    if (*std::min_element(b_sizes.begin(), b_sizes.end()) > p->smem_n) {
+      p->tune[bk] = batch_width(p->dtype);  // nothing of it fits in shared memory
+      continue;
+    }
     float best = 1e30f;
-    int best_nb = p->tune[bk];
-    for (int nb : cands) {
-      if (nb == 0 && maxn > p->smem_n) continue;
+    int best_form = p->tune[bk];
+    for (const int form : {0, batch_width(p->dtype)}) {
       int tune_all[kBuckets];
-      for (int q = 0; q < kBuckets; ++q) tune_all[q] = nb;
-      cudaMemcpy(m_tune, tune_all, sizeof(tune_all), cudaMemcpyHostToDevice);
-      BatchMeta m{m_sizes, m_aoff, m_boff, m_order + first, m_tune, cnt, p->smem_n};
+      for (int q = 0; q < kBuckets; ++q) tune_all[q] = form;
+      std::vector<int> order;
+      std::vector<BatchClass> classes;
+      build_classes(ctx, p->dtype, p->mode, tune_all, p->smem_n, b_sizes, order, classes);
+      for (auto& q : order) q += first;
+      rc = ensure_buf(ctx, mat_buf, scratch_ctas(classes) * kScratchElems * es);
+      if (rc) break;
+      cudaMemcpy(m_order, order.data(), cnt * sizeof(int), cudaMemcpyHostToDevice);
+      BatchMeta m{m_sizes, m_aoff, m_boff, m_order, cnt};
       float ms = 0.f;
-      for (int rep = 0; rep < 2; ++rep) {
-        cudaMemcpyAsync(wa, pa, sa * es, cudaMemcpyDeviceToDevice, ctx->stream);
+      for (int rep = 0; rep < 2 && err == cudaSuccess; ++rep) {
+        const int64_t a0 = s_aoff[first], a1 = first + cnt < ns ? s_aoff[first + cnt] : sa;
+        cudaMemcpyAsync(wa + a0 * es, pa + a0 * es, (a1 - a0) * es, cudaMemcpyDeviceToDevice, ctx->stream);
         cudaMemcpyAsync(wb, pb, sb * es, cudaMemcpyDeviceToDevice, ctx->stream);
         cudaEventRecord(e0, ctx->stream);
-        cudaError_t e = launch_plan(p, m, p->grid, wa, wb, spiv, sinfo, m_counter, ctx->stream);
+        err = launch_classes(p, classes, m, mat_buf.ptr, wa, wb, spiv, sinfo, m_counter, ctx->stream);
         cudaEventRecord(e1, ctx->stream);
-        if (e != cudaSuccess) {
-          cudaEventDestroy(e0);
-          cudaEventDestroy(e1);
-          cudaFree(meta_buf.ptr);
-          return set_error(ctx, LUHOT_ERR_CUDA, std::string("batch autotune: ") + cudaGetErrorString(e));
-        }
-        cudaEventSynchronize(e1);
+        if (err == cudaSuccess) err = cudaEventSynchronize(e1);
         cudaEventElapsedTime(&ms, e0, e1);
       }
-      count_launch(ctx, 2);
+      if (err != cudaSuccess) {
+        rc = set_error(ctx, LUHOT_ERR_CUDA, std::string("batch autotune: ") + cudaGetErrorString(err));
+        break;
+      }
+      count_launch(ctx, 2 * (int64_t)classes.size());
       if (ms < best) {
         best = ms;
-        best_nb = nb;
+        best_form = form;
       }
     }
-    p->tune[bk] = best_nb;
+    p->tune[bk] = best_form;
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   cudaFree(meta_buf.ptr);
+  if (mat_buf.ptr) cudaFree(mat_buf.ptr);
+  if (rc) return rc;
   drop_graph(p);
   return upload_meta(p);
 }

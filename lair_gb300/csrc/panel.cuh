@@ -107,6 +107,30 @@ __device__ __forceinline__ int key_reduce_redux(unsigned long long& k, int& i, i
   return src;
 }
 
+// Lane of a warp that holds the largest key (the smallest id among equal
+// keys).  One redux and one vote unless (the high words of) keys tie.
+__device__ __forceinline__ int warp_best(unsigned int k, int id) {
+  const unsigned m = __reduce_max_sync(0xffffffffu, k);
+  unsigned mask = __ballot_sync(0xffffffffu, k == m);
+  if (mask & (mask - 1u)) {
+    const int mi = __reduce_min_sync(0xffffffffu, k == m ? id : INT_MAX);
+    mask = __ballot_sync(0xffffffffu, k == m && id == mi);
+  }
+  return __ffs(mask) - 1;
+}
+__device__ __forceinline__ int warp_best(unsigned long long k, int id) {
+  const unsigned hi = (unsigned)(k >> 32);
+  const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+  unsigned mask = __ballot_sync(0xffffffffu, hi == mh);
+  if (mask & (mask - 1u)) {
+    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? (unsigned)k : 0u);
+    const unsigned long long m = ((unsigned long long)mh << 32) | ml;
+    const int mi = __reduce_min_sync(0xffffffffu, k == m ? id : INT_MAX);
+    mask = __ballot_sync(0xffffffffu, k == m && id == mi);
+  }
+  return __ffs(mask) - 1;
+}
+
 // Cooperative form over one thread-block cluster (panel_cluster.cu): whether
 // it takes a panel of `rows` rows and width w, and its launch.
 template <typename T>

@@ -165,30 +165,6 @@ __device__ __forceinline__ void cl_bar_arrive(int id, int threads) {
   asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
-// Lane of a warp that holds the largest key (the smallest id among equal
-// keys).  One redux and one vote unless (the high words of) keys tie.
-__device__ __forceinline__ int cl_best(unsigned int k, int id) {
-  const unsigned m = __reduce_max_sync(0xffffffffu, k);
-  unsigned mask = __ballot_sync(0xffffffffu, k == m);
-  if (mask & (mask - 1u)) {
-    const int mi = __reduce_min_sync(0xffffffffu, k == m ? id : INT_MAX);
-    mask = __ballot_sync(0xffffffffu, k == m && id == mi);
-  }
-  return __ffs(mask) - 1;
-}
-__device__ __forceinline__ int cl_best(unsigned long long k, int id) {
-  const unsigned hi = (unsigned)(k >> 32);
-  const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
-  unsigned mask = __ballot_sync(0xffffffffu, hi == mh);
-  if (mask & (mask - 1u)) {
-    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? (unsigned)k : 0u);
-    const unsigned long long m = ((unsigned long long)mh << 32) | ml;
-    const int mi = __reduce_min_sync(0xffffffffu, k == m ? id : INT_MAX);
-    mask = __ballot_sync(0xffffffffu, k == m && id == mi);
-  }
-  return __ffs(mask) - 1;
-}
-
 // The winner among the n headers of one step (the same answer in every warp):
 // its index, row id, signed key and column j+1 value.  key 0: no pivot.
 template <typename T>
@@ -220,7 +196,7 @@ __device__ __forceinline__ void cl_winner(const unsigned long long (*box)[4], in
       u1 = hu;
     }
   }
-  const int src = cl_best(k, pr);
+  const int src = warp_best(k, pr);
   win = __shfl_sync(0xffffffffu, win, src);
   pr = __shfl_sync(0xffffffffu, pr, src);
   kraw = __shfl_sync(0xffffffffu, kraw, src);
@@ -421,7 +397,7 @@ __global__ void __launch_bounds__(cl_threads<T>(), 1) panel_cluster_kernel(Panel
           bi = i;
         }
       }
-      src = cl_best(bk, bid);
+      src = warp_best(bk, bid);
       ck = __shfl_sync(kFull, bk | (bi >= 0 && signbit(pick(a)) ? H::kSign : K(0)), src);
       cid = __shfl_sync(kFull, bid, src);
       if (lane == src) {
