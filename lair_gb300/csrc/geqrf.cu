@@ -23,6 +23,7 @@
 #include <algorithm>
 #include <cmath>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "common.cuh"
@@ -407,6 +408,9 @@ int geqrf_device(luhot_ctx* ctx, int m, int n, T* d_a, int64_t lda, T* d_tau, in
   if (mode != LUHOT_MODE_FAST && mode != LUHOT_MODE_EXACT)
     return set_error(ctx, LUHOT_ERR_INVALID_ARG, "geqrf: unknown mode");
   if (m == 0 || n == 0) return LUHOT_OK;
+  if constexpr (std::is_same<T, double>::value) {
+    if (mode == LUHOT_MODE_FAST && geqrf_blocked_fits(ctx, m, n)) return geqrf_blocked(ctx, m, n, d_a, lda, d_tau);
+  }
   return mode == LUHOT_MODE_EXACT ? geqrf_impl<T, true>(ctx, m, n, d_a, lda, d_tau)
                                   : geqrf_impl<T, false>(ctx, m, n, d_a, lda, d_tau);
 }
@@ -427,6 +431,10 @@ int geqrf_host(luhot_ctx* ctx, int64_t m, int64_t n, T* a, int64_t rs, int64_t c
   if (rc) return rc;
   rc = geqrf_device<T>(ctx, (int)m, (int)n, d_a, lda, d_tau, mode);
   if (rc) return rc;
+  if (std::is_same<T, double>::value && mode == LUHOT_MODE_FAST && geqrf_blocked_fits(ctx, (int)m, (int)n)) {
+    rc = finish_status(ctx, nullptr);  // its panels wait on one another
+    if (rc) return rc;
+  }
   rc = stage_out<T>(ctx, d_a, lda, a, m, n, rs, cs, ctx->work[1]);
   if (rc) return rc;
   LUHOT_CUDA_TRY(ctx, cudaMemcpy(tau, d_tau, (size_t)k * sizeof(T), cudaMemcpyDeviceToHost));

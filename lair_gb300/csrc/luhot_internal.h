@@ -127,6 +127,11 @@ int ensure_buf(luhot_ctx* ctx, DevBuf& b, size_t bytes);
 int copy_2d(luhot_ctx* ctx, void* dst, size_t dpitch, const void* src, size_t spitch, size_t wbytes, size_t rows,
             cudaMemcpyKind kind);
 
+// Blocked Householder QR of fast-mode FP64 (geqrf_blocked.cu): whether it takes
+// an m x n matrix, and the factorization (asynchronous; A and tau in device memory).
+bool geqrf_blocked_fits(luhot_ctx* ctx, int m, int n);
+int geqrf_blocked(luhot_ctx* ctx, int m, int n, double* a, int64_t lda, double* tau);
+
 // Largest power-of-two cluster in which the cluster form of the panel
 // (panel_cluster.cu) can run with its full shared memory, 0 if none.
 int panel_cluster_limit(luhot_ctx* ctx);

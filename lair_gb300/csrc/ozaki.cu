@@ -649,6 +649,25 @@ int ozaki_update_split(luhot_ctx* ctx, double* a, int64_t lda, int w, int r1, in
   return rc;
 }
 
+int ozaki_product(luhot_ctx* ctx, const double* l, int64_t ldl, const double* u, int64_t ldu, int w, double* c,
+                  int64_t ldc, int M, int N, void* ws, cudaStream_t stream) {
+  if (M <= 0 || N <= 0 || w <= 0) return LUHOT_OK;
+  if (w > kOzK) return set_error(ctx, LUHOT_ERR_INVALID_ARG, "ozaki_product: more than 64 columns");
+  const OzWs lay = oz_layout(ws, M, N);
+  prof_begin(ctx, kProfOther);
+  oz_split_rows_kernel<<<(M + 7) / 8, 256, 0, stream>>>(l, ldl, 0, M, 0, w, lay.as, lay.ea);
+  prof_end(ctx, kProfOther, 0.0, (double)M * w * 8 + (double)M * kOzK * kOzSlices * 2);
+  prof_begin(ctx, kProfOther);
+  oz_split_cols_kernel<<<(N + 31) / 32, 256, 0, stream>>>(u, ldu, 0, w, 0, N, lay.bs, lay.eb);
+  prof_end(ctx, kProfOther, 0.0, (double)N * w * 8 + (double)N * kOzK * kOzSlices * 2);
+  LUHOT_CUDA_TRY(ctx, cudaGetLastError());
+  prof_begin(ctx, kProfGemm);
+  int rc = oz_launch_gemm(ctx, lay, c, ldc, M, N, stream);
+  prof_end(ctx, kProfGemm, 2.0 * M * N * w,
+           (double)M * N * 16 + (double)(M + N) * kOzK * kOzSlices * 2 + (double)(M + N) * 4);
+  return rc;
+}
+
 int ozaki_update(luhot_ctx* ctx, double* a, int64_t lda, int k0, int w, int r1, int m, int c1, int n, void* ws,
                  cudaStream_t stream) {
   const int M = m - r1, N = n - c1;

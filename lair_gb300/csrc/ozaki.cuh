@@ -20,7 +20,10 @@ bool ozaki_available(luhot_ctx* ctx);
 // ozaki_workspace_bytes(m - r1, n - c1) bytes.  Asynchronous on `stream`.
 int ozaki_update(luhot_ctx* ctx, double* a, int64_t lda, int k0, int w, int r1, int m, int c1, int n, void* ws,
                  cudaStream_t stream);
-// The same in two parts: where the digit slices of the operands go (for
+// c (M x N, ldc) -= l (M x w, ldl) u (w x N, ldu), w <= 64, separate operands.
+int ozaki_product(luhot_ctx* ctx, const double* l, int64_t ldl, const double* u, int64_t ldu, int w, double* c,
+                  int64_t ldc, int M, int N, void* ws, cudaStream_t stream);
+// ozaki_update in two parts: where the digit slices of the operands go (for
 // launch_swap_solve), and the product of the slices that are there (w <= 64).
 SplitOut ozaki_split_out(void* ws, int r1, int M, int N);
 int ozaki_update_split(luhot_ctx* ctx, double* a, int64_t lda, int w, int r1, int m, int c1, int n, void* ws,

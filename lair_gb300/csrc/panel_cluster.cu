@@ -41,10 +41,8 @@
 // Arithmetic and its order per element are those of panel_kernel, so exact
 // mode keeps lair's bits (src/lapack/getrf.rs:56-89).
 #include <algorithm>
-#include <mutex>
-#include <set>
-#include <utility>
 
+#include "cluster.cuh"
 #include "common.cuh"
 #include "luhot_internal.h"
 #include "panel.cuh"
@@ -72,57 +70,6 @@ template <typename T>
 static size_t cl_smem_bytes(int rows_per, int w) {
   return ((((size_t)rows_per * cl_lds<T>(w) + 3) & ~(size_t)3) + 2 * (kMaxPanelWidth + kClSegPad)) * sizeof(T) +
          2 * (size_t)rows_per * sizeof(int);
-}
-
-__device__ __forceinline__ unsigned cl_smem(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ unsigned cl_peer(unsigned addr, int cta) {
-  unsigned d;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(d) : "r"(addr), "r"(cta));
-  return d;
-}
-// 16 bytes into a peer's shared memory, counted on the peer's mbarrier.
-__device__ __forceinline__ void cl_push16(unsigned dst, unsigned bar, unsigned long long a, unsigned long long b) {
-  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%0], {%1, %2}, [%3];" ::"r"(dst),
-               "l"(a), "l"(b), "r"(bar)
-               : "memory");
-}
-__device__ __forceinline__ void cl_push8(unsigned dst, unsigned bar, unsigned long long a) {
-  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(dst), "l"(a),
-               "r"(bar)
-               : "memory");
-}
-__device__ __forceinline__ void cl_expect(unsigned bar, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-// Bounded wait of a whole warp; false (for all lanes) once it gave up.
-__device__ __forceinline__ bool cl_wait(unsigned bar, unsigned parity, DeviceStatus* st, int step) {
-  unsigned long long t0 = 0;
-  for (unsigned spins = 0;; ++spins) {
-    unsigned done;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, "
-        "0, p;\n}\n"
-        : "=r"(done)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    if (__all_sync(0xffffffffu, done != 0)) return true;
-    if ((spins & 15u) == 0) {
-      const unsigned long long now = global_timer_ns();
-      if (t0 == 0) t0 = now;
-      const bool late = now - t0 > st->timeout_ns;
-      if (__any_sync(0xffffffffu, late || ld_relaxed_i32(&st->abort) != 0)) {
-        if (late && (threadIdx.x & 31) == 0) {
-          atomicCAS(&st->error, kDevOk, kDevBarrierTimeout);
-          atomicExch(&st->timeout_where, (unsigned long long)step);
-          atomicExch(&st->abort, 1);
-        }
-        return false;
-      }
-    }
-  }
-}
-__device__ __forceinline__ void cl_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 // A CTA's header: 16 bytes (FP32: key | id, value) or 24 (FP64: key, id; value).
@@ -618,36 +565,6 @@ static void cl_split(luhot_ctx* ctx, int rows, int* P, int* rows_per) {
 
 // Static shared memory of the kernel and rounding, left out of the budget.
 constexpr size_t kClStaticSmem = 8192;
-
-// Lets `kernel` launch with clusters of more than 8 CTAs; once per kernel and
-// device, like allow_max_dynamic_smem.
-static cudaError_t allow_wide_clusters(const void* kernel) {
-  static std::mutex mu;
-  static std::set<std::pair<const void*, int>> allowed;
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  std::lock_guard<std::mutex> lock(mu);
-  if (allowed.count({kernel, dev})) return cudaSuccess;
-  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  if (e == cudaSuccess) allowed.insert({kernel, dev});
-  return e;
-}
-
-static cudaLaunchConfig_t cl_config(int P, int threads, size_t smem, cudaStream_t stream, cudaLaunchAttribute* attr) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(P);
-  cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  attr->id = cudaLaunchAttributeClusterDimension;
-  attr->val.clusterDim.x = P;
-  attr->val.clusterDim.y = 1;
-  attr->val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cfg;
-}
 
 int panel_cluster_limit(luhot_ctx* ctx) {
   auto kern = panel_cluster_kernel<double, false, 4>;
