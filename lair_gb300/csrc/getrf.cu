@@ -608,60 +608,63 @@ __global__ void __launch_bounds__(256) laswp_moves_kernel(T* a, int64_t lda, con
 
 // ---------------------------------------------------------------------------
 // 3a. Schur update on the CUDA cores (exact mode and FP32): C -= A B with a
-//     64x64 tile per CTA, 4x4 per thread, K <= 64 staged in shared memory.
-//     Each C entry starts from its old value and takes the K updates one at a
-//     time in increasing k, which is lair's order.
+//     kTile x kTile tile per CTA, a quarter of kTile / 4 squared elements a
+//     thread, K staged in shared memory.  Each C entry starts from its old value
+//     and takes the K updates one at a time in increasing k, which is lair's
+//     order.  The tile is 64 where that makes two CTAs per SM, else smaller: FP64
+//     arithmetic on one SM takes 150 us for a 64 x 64 tile (K = 64, a product and
+//     a subtraction), 10 us for a 16 x 16 one.
 // ---------------------------------------------------------------------------
-constexpr int kGemmTile = 64;
 constexpr int kGemmKC = 32;  // K chunk staged per pass (static smem stays < 48 KB)
 
-template <typename T, bool kExact>
+template <typename T, bool kExact, int kTile>
 __global__ void __launch_bounds__(256) gemm_cuda_kernel(T* a, int64_t lda, int r0, int c0, int kk0,
                                                         int K, int M, int N) {
-  __shared__ T As[kGemmKC][kGemmTile + 1];  // As[k][i] = L21[i][k]
-  __shared__ T Bs[kGemmKC][kGemmTile];      // Bs[k][j] = U12[k][j]
-  const int tile_r = r0 + blockIdx.y * kGemmTile;
-  const int tile_c = c0 + blockIdx.x * kGemmTile;
+  constexpr int kE = kTile / 16;  // elements of a thread in each direction
+  __shared__ T As[kGemmKC][kTile + 1];  // As[k][i] = L21[i][k]
+  __shared__ T Bs[kGemmKC][kTile];      // Bs[k][j] = U12[k][j]
+  const int tile_r = r0 + blockIdx.y * kTile;
+  const int tile_c = c0 + blockIdx.x * kTile;
   const int tid = threadIdx.x;
-  const int tr = (tid / 16) * 4, tc = (tid % 16);
-  T acc[4][4];
+  const int tr = (tid / 16) * kE, tc = (tid % 16);
+  T acc[kE][kE];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < kE; ++i)
 #pragma unroll
-    for (int jj = 0; jj < 4; ++jj) {
+    for (int jj = 0; jj < kE; ++jj) {
       const int r = tile_r + tr + i, c = tile_c + tc + 16 * jj;
       acc[i][jj] = (r < r0 + M && c < c0 + N) ? a[(int64_t)r * lda + c] : T(0);
     }
   for (int kb = 0; kb < K; kb += kGemmKC) {
     const int kc = min(kGemmKC, K - kb);
     __syncthreads();
-    for (int idx = tid; idx < kc * kGemmTile; idx += 256) {
+    for (int idx = tid; idx < kc * kTile; idx += 256) {
       const int i = idx / kc, k = idx - i * kc;
       const int r = tile_r + i;
       As[k][i] = (r < r0 + M) ? a[(int64_t)r * lda + kk0 + kb + k] : T(0);
     }
-    for (int idx = tid; idx < kc * kGemmTile; idx += 256) {
-      const int k = idx / kGemmTile, j = idx - k * kGemmTile;
+    for (int idx = tid; idx < kc * kTile; idx += 256) {
+      const int k = idx / kTile, j = idx - k * kTile;
       const int c = tile_c + j;
       Bs[k][j] = (c < c0 + N) ? a[(int64_t)(kk0 + kb + k) * lda + c] : T(0);
     }
     __syncthreads();
     for (int k = 0; k < kc; ++k) {
-      T av[4], bv[4];
+      T av[kE], bv[kE];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) av[i] = As[k][tr + i];
+      for (int i = 0; i < kE; ++i) av[i] = As[k][tr + i];
 #pragma unroll
-      for (int jj = 0; jj < 4; ++jj) bv[jj] = Bs[k][tc + 16 * jj];
+      for (int jj = 0; jj < kE; ++jj) bv[jj] = Bs[k][tc + 16 * jj];
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < kE; ++i)
 #pragma unroll
-        for (int jj = 0; jj < 4; ++jj) acc[i][jj] = upd<kExact>(acc[i][jj], av[i], bv[jj]);
+        for (int jj = 0; jj < kE; ++jj) acc[i][jj] = upd<kExact>(acc[i][jj], av[i], bv[jj]);
     }
   }
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < kE; ++i)
 #pragma unroll
-    for (int jj = 0; jj < 4; ++jj) {
+    for (int jj = 0; jj < kE; ++jj) {
       const int r = tile_r + tr + i, c = tile_c + tc + 16 * jj;
       if (r < r0 + M && c < c0 + N) a[(int64_t)r * lda + c] = acc[i][jj];
     }
@@ -1042,9 +1045,16 @@ static int launch_gemm(luhot_ctx* ctx, T* a, int64_t lda, int r0, int c0, int kk
       gemm_dmma_kernel<<<grid, 256, smem, stream>>>(a, lda, r0, c0, kk0, K, M, N);
     }
   } else {
-    dim3 grid((N + kGemmTile - 1) / kGemmTile, (M + kGemmTile - 1) / kGemmTile);
+    auto ctas = [&](int t) { return (int64_t)((N + t - 1) / t) * ((M + t - 1) / t); };
+    const int tile = ctas(64) >= 2 * ctx->num_sms ? 64 : (ctas(32) >= 2 * ctx->num_sms || sizeof(T) == 4) ? 32 : 16;
+    dim3 grid((N + tile - 1) / tile, (M + tile - 1) / tile);
     prof_begin(ctx, kProfGemm);
-    gemm_cuda_kernel<T, kExact><<<grid, 256, 0, stream>>>(a, lda, r0, c0, kk0, K, M, N);
+    if (tile == 64)
+      gemm_cuda_kernel<T, kExact, 64><<<grid, 256, 0, stream>>>(a, lda, r0, c0, kk0, K, M, N);
+    else if (tile == 32)
+      gemm_cuda_kernel<T, kExact, 32><<<grid, 256, 0, stream>>>(a, lda, r0, c0, kk0, K, M, N);
+    else
+      gemm_cuda_kernel<T, kExact, 16><<<grid, 256, 0, stream>>>(a, lda, r0, c0, kk0, K, M, N);
   }
   // algorithmic work: 2MNK flops; bytes: C read + written, L21 and U12 read once
   prof_end(ctx, kProfGemm, 2.0 * M * N * K,
