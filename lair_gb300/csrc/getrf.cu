@@ -1113,6 +1113,41 @@ static const int* live_moves(luhot_ctx* ctx) {
   return reinterpret_cast<const int*>(static_cast<char*>(ctx->panel_scratch) + kPanelSlotBytes);
 }
 
+// Two panels [k0, k0 + 64), [k0 + 64, k0 + 128) of fast-mode FP64 and one trailing
+// update with K = 128: a slice product's time is its epilogue's, which a pair pays
+// once.  In between, the second panel's columns and the second panel's rows of U
+// take K = 64 products of their own and the interchanges two launches, some 40 us
+// in all, so that the pair pays from about 4000 x 4000 on (kPairElems: the block
+// behind the pair).  n = 16384: updates 114 -> 75 ms, 193 -> 159 ms in all; n = 4097
+// (31 pairs smaller than the rule's limit): 15.65 ms without, 15.59 with pairs from
+// 3000 x 3000 on, 15.8 from 2000 x 2000 on.
+constexpr int64_t kPairElems = 16000000;
+
+static int fp64_panel_pair(luhot_ctx* ctx, double* a, int64_t lda, int m, int n, int k0, int* piv, void* oz_ws,
+                           cudaStream_t stream) {
+  constexpr int w = kDefaultPanelWidth;
+  const int k1 = k0 + w, r1 = k1 + w, N = n - r1;
+  int rc = ensure_buf(ctx, ctx->la_moves, 4 * kPanelMovesBytes);
+  if (rc) return rc;
+  int* mv = static_cast<int*>(ctx->la_moves.ptr);
+  double* const ab = a + (int64_t)k1 * lda;  // row k1
+  rc = launch_panel<double, false>(ctx, a, lda, m, k0, w, piv, stream);
+  if (rc) return rc;
+  // The first panel's interchanges on the other columns come after the second's
+  // columns are done: keep them.
+  LUHOT_CUDA_TRY(ctx, cudaMemcpyAsync(mv, live_moves(ctx), kPanelMovesBytes, cudaMemcpyDeviceToDevice, stream));
+  const SplitOut split = ozaki_split_out(oz_ws, k1, m - k1, w);
+  rc = launch_swap_solve<double, false>(ctx, a, lda, mv, k0, w, 0, 0, k1, r1, &split, stream);
+  if (!rc) rc = ozaki_update_split(ctx, a, lda, w, k1, m, k1, r1, oz_ws, stream);
+  if (!rc) rc = launch_panel<double, false>(ctx, a, lda, m, k1, w, piv, stream);
+  if (!rc) rc = launch_swap_solve<double, false>(ctx, a, lda, mv, k0, w, 0, k0, r1, n, nullptr, stream);
+  if (!rc) rc = launch_laswp_cols<double>(ctx, a, lda, live_moves(ctx), w, 0, k1, r1, n, stream);
+  if (!rc) rc = ozaki_product(ctx, ab + k0, lda, a + (int64_t)k0 * lda + r1, lda, w, ab + r1, lda, w, N, oz_ws, stream);
+  if (!rc) rc = launch_swap_solve<double, false>(ctx, a, lda, nullptr, k1, w, 0, 0, r1, n, nullptr, stream);
+  if (!rc) rc = ozaki_update(ctx, a, lda, k0, 2 * w, r1, m, r1, n, oz_ws, stream);
+  return rc;
+}
+
 template <typename T, bool kExact>
 static int getrf_impl(luhot_ctx* ctx, int m, int n, T* a, int64_t lda, int* piv, int nb, void* oz_ws,
                       cudaStream_t stream) {
@@ -1121,6 +1156,16 @@ static int getrf_impl(luhot_ctx* ctx, int m, int n, T* a, int64_t lda, int* piv,
   // factorization carries a live tag.
   LUHOT_CUDA_TRY(ctx, cudaMemsetAsync(ctx->panel_scratch, 0, kPanelScratchBytes, stream));
   for (int k0 = 0; k0 < dim_min; k0 += nb) {
+    if constexpr (std::is_same<T, double>::value && !kExact) {
+      const int64_t M2 = m - k0 - 2 * nb, N2 = n - k0 - 2 * nb;
+      if (nb == kDefaultPanelWidth && oz_ws && ctx->fp64_update != LUHOT_UPDATE_DMMA && dim_min - k0 >= 2 * nb &&
+          M2 > 0 && N2 > 0 && M2 * N2 >= kPairElems) {
+        int rc = fp64_panel_pair(ctx, a, lda, m, n, k0, piv, oz_ws, stream);
+        if (rc) return rc;
+        k0 += nb;  // and the loop's own step
+        continue;
+      }
+    }
     const int w = std::min(nb, dim_min - k0);
     int rc = launch_panel<T, kExact>(ctx, a, lda, m, k0, w, piv, stream);
     if (rc) return rc;

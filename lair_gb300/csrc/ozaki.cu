@@ -18,45 +18,45 @@
 // Products (oz_gemm_kernel).  With A_p, B_q the digit matrices,
 //       L U = 2^(ea+eb) sum_G T_G 2^(-8(G+2)),   T_G = sum_{p+q=G} A_p B_q^T,
 //   kept for G = 0..6 (28 slice products of the 49).  Every partial sum of
-//   T_G is an integer of magnitude below 9 * 2^20 for K <= 64, so the FP32
-//   accumulation in TMEM is exact.  The dropped groups (G >= 7) weigh at most
-//   2^-49.4 of 2^(ea+eb) (typically 2^-55), the element roundings 2^-57 of
-//   each operand's scale: the product error stays well inside FP64's own
-//   bound for a K-term dot product (measured on N(0,1) factors: 1.1e-16 of
-//   |C| + |L||U| against 4.7e-16 for the FP64 tensor cores).
-// Combine (epilogue).  R = sum_G T_G 2^(38-8G) in 64-bit fixed point, formed by
-//   Horner from G = 6 down (each step truncates below 2^-38 of T_0's unit;
-//   |R| < 2^62), then C = C - R 2^(ea+eb-54): one rounding of R to 53 bits
-//   (built with integer operations) and one of the subtraction.  Rows or columns holding Inf or NaN give
-//   NaN in the elements they touch.
+//   T_G is an integer of magnitude below 9 * 2^20 for K <= 64, and at most 2^24
+//   for K <= 128 but for group 6, whose two K halves have an accumulator each, so
+//   the FP32 accumulation in TMEM is exact.  The dropped groups (G >= 7) weigh at
+//   most 2^-49.4 of 2^(ea+eb) for K = 64, 2^-48.4 for K = 128 (typically 2^-55),
+//   the element roundings 2^-57 of each operand's scale: the product error stays
+//   well inside FP64's own bound for a K-term dot product (measured on N(0,1)
+//   factors: 1.1e-16 of |C| + |L||U| against 4.7e-16 for the FP64 tensor cores).
+// Combine (epilogue).  R = floor(sum_G T_G 2^(38-8G)), a 64-bit integer (|R| < 2^62),
+//   then C = C - R 2^(ea+eb-54): one rounding of R to 53 bits (built with integer
+//   operations) and one of the subtraction.  Rows or columns holding Inf or NaN
+//   give NaN in the elements they touch.
 //
-// oz_gemm_kernel: persistent, one CTA per SM, 128 x 128 output tiles, a
-// contiguous range per CTA in column-block order.  An M = 128 MMA costs the
-// tensor pipe about the same time for any N up to 256 (measured: ~128 cycles
-// at N = 64), so the tile is as wide as TMEM allows: three 128-column FP32
-// accumulators and the low words of the tile's 64-bit fixed-point sums
-// (512 columns).  The MMAs compute C^T: TMEM lanes are C's columns, so a
-// warp's accesses to one row of C are 32 consecutive doubles.  Eighteen warps:
-//   warp 0      TMA producer: the seven U slices of the CTA's current column
-//               block (112 KB, reloaded when the column block changes) and
-//               the seven L slices of each tile (112 KB), one barrier pair
-//               per slice: L slice p is last read by group G = p, so the
-//               slices free up in the order the next tile needs them (6 .. 0);
-//               3-D tensor maps (k, row, slice), 128-byte swizzle, rows past M
-//               or N zero-filled;
-//   warp 1      TMEM owner (512 columns) and MMA issuer: per tile, groups
-//               G = 6 .. 0, taking the three accumulators in turn over the
-//               launch: the group's slice products, 4 k-steps of M = 128,
-//               N = 128, K = 16 each, then a commit to that accumulator's full
-//               barrier;
-//   warps 2-17  epilogue: warp w reads TMEM lanes 32 (w % 4) .. + 31 (32
-//               columns of C) and 32 of the tile's 128 rows ((w - 2) / 4); its
-//               thread keeps the high words of its column's 32 sums in
-//               registers and the low words in TMEM; per group it folds the
-//               accumulator in (Horner on word pairs) and releases it, so the
-//               MMAs of the next group (and of the next tile) overlap the
-//               epilogue; after group 0 it applies the sums to C (C prefetched
-//               into L2 at the tile's start; one FP64 subtraction per element).
+// oz_gemm_kernel: persistent, one CTA per SM, tiles of 128 columns x 64 rows of C,
+// a contiguous range per CTA in row-block order.  What bounds it is the epilogue's
+// arithmetic, 64 cycles of an SM quarter's FP64 pipe a warp's subtraction and about
+// as many for the rest, so that a product is worth doing over K = 128 (two "halves"
+// of 64): one epilogue instead of two.  A 128 x 64 tile leaves TMEM room for all
+// eight accumulators at once, and the MMAs of a piece of U against stacked pieces
+// of L are then single products with N up to 256 on neighbouring accumulators:
+// 10 a k-step in place of 28, the tensor pipe's full rate (3700 cycles a half).  The
+// MMAs compute C^T: TMEM lanes are C's columns, so a warp's accesses to one row of C
+// are 32 consecutive doubles.  Cycles a tile, K = 64 / 128: MMAs 5300 / 10100 (U's
+// pieces come from L2 at 23 bytes a cycle and SM), folds 3500 / 4000, C and
+// subtraction 7200; together 11800 / 14400 (a 128 x 128 tile with three
+// accumulators, a fold per group on 64-bit words: 29000 for K = 64).  n = 16384's
+// updates: 142 ms before, 114 in steps of K = 64, 74 with K = 128.  Eighteen warps:
+//   warp 0      TMA producer: the L pieces (a slice's 64 rows x 64 k, 8 KB) of the
+//               CTA's row block, reloaded when the row block changes, and the
+//               seven U pieces (128 columns, 16 KB) of each tile and half, one
+//               barrier pair per piece, in the order the MMAs free them (6 .. 0);
+//               3-D tensor maps (k, row, slice), 128-byte swizzle, rows past M or
+//               N zero-filled;
+//   warp 1      TMEM owner (512 columns) and MMA issuer: per tile and half, U pieces
+//               6 .. 0 against L pieces 0 .. 6 - q, 4 k-steps of K = 16 each, then
+//               a commit to that piece's empty barrier; a commit to the tile's full
+//               barrier at its end;
+//   warps 2-17  epilogue: per group the accumulator is read and released, so that
+//               the next tile's first MMAs overlap the folds and the rest of them
+//               the work on C; C is prefetched into L2 at the tile's start.
 // All mbarrier waits are bounded by the context's wait limit; on expiry a role
 // records the error and raises the CTA's abort flag, the others stop at their
 // next wait, and before exit the CTA waits (bounded) for its copies and MMAs
@@ -75,46 +75,59 @@
 
 namespace luhot {
 
-constexpr int kOzBM = 128, kOzBN = 128;
+constexpr int kOzBN = 128;     // columns of C of a tile (TMEM lanes)
+constexpr int kOzBM = 64;      // rows of C of a tile (TMEM columns of an accumulator)
+constexpr int kOzMaxHalves = 2;  // K = 64 or 128
 constexpr int kOzFrac = 38;    // fractional bits of the fixed-point combine
 constexpr int kOzEpiWarps = 16;
 constexpr int kOzThreads = 64 + 32 * kOzEpiWarps;
-constexpr int kOzSliceBytes = 128 * 128;  // one slice box: 128 rows x 128 B
-constexpr int kOzAccBufs = 3;           // TMEM accumulators of 128 columns, used in turn by the groups
-constexpr unsigned kOzLoCol = 384;      // TMEM columns 384-511: low words of the fixed-point sums
-constexpr size_t kOzSmem = 1024 + 2 * (size_t)kOzSlices * kOzSliceBytes;
-static_assert(kOzAccBufs * kOzBM <= (int)kOzLoCol && kOzLoCol + kOzBM <= 512, "accumulators and sums fit in TMEM");
+constexpr int kOzRows = kOzBM / 4;              // rows of C of an epilogue thread
+constexpr int kOzUBytes = kOzBN * kOzK * 2;     // a U piece: one slice, one K half, 128 columns
+constexpr int kOzLBytes = kOzBM * kOzK * 2;     // an L piece: 64 rows
+constexpr size_t kOzSmem = 1024 + (size_t)kOzSlices * kOzUBytes + (size_t)kOzMaxHalves * kOzSlices * kOzLBytes;
+constexpr int kOzAccs = kOzGroups + 1;  // accumulators: groups 0 .. 6 and group 6 of the second K half
+static_assert(kOzAccs * kOzBM <= 512, "the accumulators fit in TMEM");
 
 // ---------------------------------------------------------------------------
 // Split (digits: ozaki_split.cuh).
 // ---------------------------------------------------------------------------
 
-// Rows r1 .. r1 + M - 1, columns k0 .. k0 + w - 1 of the row-major a (w <= 64):
-// As[p][i][k] (zero for k >= w), ea[i].  One warp per row.
+// Rows r1 .. r1 + M - 1, columns k0 .. k0 + w - 1 of the row-major a (w <= 64
+// kH): As[p][i][k] (zero for k >= w), ea[i].  One warp per row.
+template <int kH>
 __global__ void __launch_bounds__(256) oz_split_rows_kernel(const double* __restrict__ a, int64_t lda, int r1, int M,
                                                             int k0, int w, __half* __restrict__ as,
                                                             int* __restrict__ ea) {
   const int i = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (i >= M) return;
   const double* row = a + (int64_t)(r1 + i) * lda + k0;
-  const double x0 = lane < w ? row[lane] : 0.0;
-  const double x1 = lane + 32 < w ? row[lane + 32] : 0.0;
-  const int e = oz_warp_max(max(oz_exponent(x0), oz_exponent(x1)));
-  oz_emit_row(x0, x1, e, as + (int64_t)i * kOzK, (int64_t)M * kOzK, lane);
+  double x[2 * kH];
+  int e = kOzZero;
+#pragma unroll
+  for (int q = 0; q < 2 * kH; ++q) {
+    x[q] = lane + 32 * q < w ? row[lane + 32 * q] : 0.0;
+    e = max(e, oz_exponent(x[q]));
+  }
+  e = oz_warp_max(e);
+#pragma unroll
+  for (int h = 0; h < kH; ++h)
+    oz_emit_row(x[2 * h], x[2 * h + 1], e, as + ((int64_t)i * kH + h) * kOzK, (int64_t)M * kH * kOzK, lane);
   if (lane == 0) ea[i] = e == kOzZero ? 0 : e;
 }
 
-// Rows k0 .. k0 + w - 1 (w <= 64), columns c1 .. c1 + N - 1 of the row-major
-// a: Bs[p][j][k] (the transpose; zero for k >= w), eb[j].  A CTA stages 64 x 32
+// Rows k0 .. k0 + w - 1 (w <= 64 kH), columns c1 .. c1 + N - 1 of the row-major
+// a: Bs[p][j][k] (the transpose; zero for k >= w), eb[j].  A CTA stages 64 kH x 32
 // elements through shared memory (coalesced reads along the rows), then each
 // warp splits four columns.
+template <int kH>
 __global__ void __launch_bounds__(256) oz_split_cols_kernel(const double* __restrict__ a, int64_t lda, int k0, int w,
                                                             int c1, int N, __half* __restrict__ bs,
                                                             int* __restrict__ eb) {
-  __shared__ double tile[kOzK][33];
+  __shared__ double tile[kH * kOzK][33];
   const int j0 = blockIdx.x * 32;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int k = warp; k < kOzK; k += 8) {
+#pragma unroll 8
+  for (int k = warp; k < kH * kOzK; k += 8) {
     const int j = j0 + lane;
     tile[k][lane] = (k < w && j < N) ? a[(int64_t)(k0 + k) * lda + c1 + j] : 0.0;
   }
@@ -122,9 +135,17 @@ __global__ void __launch_bounds__(256) oz_split_cols_kernel(const double* __rest
   for (int jj = warp; jj < 32; jj += 8) {
     const int j = j0 + jj;
     if (j >= N) break;
-    const double x0 = tile[lane][jj], x1 = tile[lane + 32][jj];
-    const int e = oz_warp_max(max(oz_exponent(x0), oz_exponent(x1)));
-    oz_emit_row(x0, x1, e, bs + (int64_t)j * kOzK, (int64_t)N * kOzK, lane);
+    double x[2 * kH];
+    int e = kOzZero;
+#pragma unroll
+    for (int q = 0; q < 2 * kH; ++q) {
+      x[q] = tile[lane + 32 * q][jj];
+      e = max(e, oz_exponent(x[q]));
+    }
+    e = oz_warp_max(e);
+#pragma unroll
+    for (int h = 0; h < kH; ++h)
+      oz_emit_row(x[2 * h], x[2 * h + 1], e, bs + ((int64_t)j * kH + h) * kOzK, (int64_t)N * kH * kOzK, lane);
     if (lane == 0) eb[j] = e == kOzZero ? 0 : e;
   }
 }
@@ -139,35 +160,43 @@ __device__ __forceinline__ void oz_abort(DeviceStatus* st, int* s_abort) {
   atomicExch(s_abort, 1);
 }
 
-// Bounded mbarrier wait that also gives up once the CTA's abort flag is up.
-__device__ __forceinline__ bool oz_wait(unsigned bar, unsigned parity, unsigned long long limit_ns,
-                                        const int* s_abort) {
+// Bounded mbarrier wait that also gives up once the CTA's abort flag is up.  The
+// timer is read only when the first try fails: the read takes longer than the try.
+__device__ __forceinline__ bool oz_try(unsigned bar, unsigned parity) {
+  unsigned done;
+  asm volatile(
+      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(done)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return done != 0u;
+}
+__device__ __noinline__ bool oz_wait_long(unsigned bar, unsigned parity, unsigned long long limit_ns,
+                                          const int* s_abort) {
   const unsigned long long t0 = global_timer_ns();
   for (unsigned spins = 0;; ++spins) {
-    unsigned done;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(done)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    if (done) return true;
+    if (oz_try(bar, parity)) return true;
     if ((spins & 15u) == 15u) {
       if (*reinterpret_cast<const volatile int*>(s_abort)) return false;
       if (global_timer_ns() - t0 > limit_ns) return false;
     }
   }
 }
+__device__ __forceinline__ bool oz_wait(unsigned bar, unsigned parity, unsigned long long limit_ns,
+                                        const int* s_abort) {
+  return oz_try(bar, parity) || oz_wait_long(bar, parity, limit_ns, s_abort);
+}
 
-__device__ __forceinline__ void oz_tma3d(unsigned dst, const CUtensorMap* map, int y, int z, unsigned bar) {
+__device__ __forceinline__ void oz_tma3d(unsigned dst, const CUtensorMap* map, int x, int y, int z, unsigned bar) {
   asm volatile(
       "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
           dst),
-      "l"(map), "r"(0), "r"(y), "r"(z), "r"(bar)
+      "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar)
       : "memory");
 }
 
-// TMEM loads and stores of one warp: its 32 lanes, 4 or 16 consecutive
-// 32-bit columns from taddr (lane field in bits 16+).
+// TMEM load of one warp: its 32 lanes, 16 consecutive 32-bit columns from taddr
+// (lane field in bits 16+).
 __device__ __forceinline__ void tmem_ld16(unsigned taddr, unsigned (&r)[16]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
@@ -175,21 +204,81 @@ __device__ __forceinline__ void tmem_ld16(unsigned taddr, unsigned (&r)[16]) {
         "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(taddr));
 }
-__device__ __forceinline__ void tmem_ld4(unsigned taddr, unsigned (&r)[4]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"(taddr));
-}
-__device__ __forceinline__ void tmem_st16(unsigned taddr, const unsigned (&r)[16]) {
+// One M = 128, K = 16 MMA on K-major operands in 128-byte swizzled rows; the
+// descriptors' low words (address and leading offset) vary, the high word (8-row
+// groups 1024 bytes apart, version, swizzle) does not.
+__device__ __forceinline__ void oz_mma(unsigned acc, unsigned a_lo, unsigned b_lo, unsigned idesc, unsigned accumulate) {
+  constexpr unsigned hi = (1024u >> 4) | (1u << 14) | (2u << 29);
   asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
-      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
-        "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-      : "memory");
+      "{\n .reg .pred p;\n .reg .b64 da, db;\n mov.b64 da, {%1, %5};\n mov.b64 db, {%2, %5};\n setp.ne.b32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n}\n" ::"r"(acc),
+      "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(hi));
+}
+
+// Instruction descriptor: D FP32 (bit 4), A and B FP16 (format 0), both K-major,
+// M = 128, N = 64 per piece.
+__device__ __forceinline__ constexpr unsigned oz_idesc(int pieces) {
+  return (1u << 4) | ((unsigned)(pieces * kOzBM >> 3) << 17) | ((unsigned)(kOzBN >> 4) << 24);
+}
+// One k-step of a U piece against `pieces` stacked L pieces, added to as many
+// accumulators from `acc` on (N = 256 at most in one MMA).
+__device__ __forceinline__ void oz_mma_range(unsigned acc, unsigned a_lo, unsigned b_lo, int pieces) {
+  if (pieces > 4) {
+    oz_mma(acc, a_lo, b_lo, oz_idesc(4), 1u);
+    oz_mma(acc + 4 * kOzBM, a_lo, b_lo + 4 * (kOzLBytes >> 4), oz_idesc(pieces - 4), 1u);
+  } else {
+    oz_mma(acc, a_lo, b_lo, oz_idesc(pieces), 1u);
+  }
 }
 
 __device__ __forceinline__ void oz_commit(unsigned bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+
+// The products of one K half of a tile, q = 6 .. 0: piece q adds to the groups from
+// q up, so each step needs one more accumulator, in the order the epilogue frees
+// them.  Called by the whole MMA warp; one lane issues.  Unrolled: what a product
+// costs the warp besides the instruction itself has to stay below the tensor
+// pipe's 128 cycles, so that descriptors and addresses are constants off a base.
+template <int kHalf>
+__device__ __forceinline__ bool oz_mma_half(unsigned tmem, unsigned u_lo, unsigned l_lo, bool leader, unsigned acc_empty,
+                                            unsigned u_full, unsigned u_empty, unsigned acc_parity, unsigned u_parity,
+                                            unsigned long long limit, const int* s_abort) {
+  const unsigned db = l_lo + (unsigned)(kHalf * kOzSlices * (kOzLBytes >> 4));
+#pragma unroll
+  for (int q = kOzSlices - 1; q >= 0; --q) {
+    if (kHalf == 0 || q == kOzSlices - 1) {
+      if (!__all_sync(0xffffffffu, oz_wait(acc_empty + 8u * (unsigned)(kHalf == 0 ? q : kOzGroups), acc_parity, limit, s_abort)))
+        return false;
+    }
+    if (!__all_sync(0xffffffffu, oz_wait(u_full + 8u * (unsigned)q, u_parity, limit, s_abort))) return false;
+    asm volatile("tcgen05.fence::after_thread_sync;");
+    const unsigned da = u_lo + (unsigned)(q * (kOzUBytes >> 4));
+    const unsigned acc = tmem + (unsigned)(q * kOzBM);
+    if (leader) {
+#pragma unroll
+      for (int ks = 0; ks < kOzK / 16; ++ks) {
+        if (kHalf == 0) {
+          // Group q's accumulator starts here (its first k-step alone).
+          if (ks == 0) {
+            oz_mma(acc, da, db, oz_idesc(1), 0u);
+            if (q < kOzSlices - 1) oz_mma_range(acc + kOzBM, da, db + (kOzLBytes >> 4), kOzSlices - 1 - q);
+          } else {
+            oz_mma_range(acc, da + 2 * ks, db + 2 * ks, kOzSlices - q);
+          }
+        } else {
+          // Second half: group 6 has an accumulator of its own (its sum over both
+          // halves could pass 2^24).
+          if (q < kOzSlices - 1) oz_mma_range(acc, da + 2 * ks, db + 2 * ks, kOzSlices - 1 - q);
+          oz_mma(tmem + (unsigned)(kOzGroups * kOzBM), da + 2 * ks,
+                 db + 2 * ks + (unsigned)((kOzSlices - 1 - q) * (kOzLBytes >> 4)), oz_idesc(1),
+                 q == kOzSlices - 1 && ks == 0 ? 0u : 1u);
+        }
+      }
+      oz_commit(u_empty + 8u * (unsigned)q);
+    }
+  }
+  return true;
 }
 
 // C - R 2^s for the fixed-point R = hi 2^32 + lo (s = ea + eb - 54); NaN
@@ -228,29 +317,42 @@ __device__ __noinline__ double oz_combine_rare(long long R, int s, double c) {
   return __dsub_rn(c, __dmul_rn(mid, p2));
 }
 
-// The common case of oz_combine: |R| >= 2^32 and a normal product.  s
-// already holds ea + eb - 54 (huge when a row or column is non-finite).
+// The common case of oz_combine: |R| >= 2^32, and an s for which every such R gives
+// a normal number (kOzMinScale .. kOzMaxScale); s20 = s 2^20 (mod 2^32).  The
+// words of R 2^s are |R| normalised to 53 bits with the leading one left in
+// place: it adds one to the exponent field below it, and a rounding that carries
+// out of the 53 bits adds another, so the rounding is one addition with carry.
 // Returns false, leaving c alone, when the element needs oz_combine.
-__device__ __forceinline__ bool oz_combine_fast(unsigned hi, unsigned lo, int s, double& c) {
+constexpr int kOzMinScale = 1 - 1023 - 32, kOzMaxScale = 2046 - 1023 - 64;
+__device__ __forceinline__ bool oz_combine_fast(unsigned hi, unsigned lo, unsigned s20, double& c) {
   const unsigned sgn = (unsigned)((int)hi >> 31);  // 0 or ~0
-  // |R| = (hi, lo) negated when negative: one's complement plus one, with carry.
-  const unsigned xl = lo ^ sgn, xh = hi ^ sgn;
-  const unsigned ul = xl - sgn;
-  const unsigned uh = xh + ((sgn != 0u && ul == 0u) ? 1u : 0u);  // uh < 2^30
+  unsigned ul, uh;                                 // |R| < 2^62
+  asm("{\n sub.cc.u32 %0, %2, %4;\n subc.u32 %1, %3, %4;\n}\n" : "=&r"(ul), "=r"(uh) : "r"(lo ^ sgn), "r"(hi ^ sgn), "r"(sgn));
   const int lz = __clz((int)uh);
   const unsigned nh = __funnelshift_l(ul, uh, lz);  // leading one at bit 31 (when uh != 0)
   const unsigned nl = ul << lz;
-  unsigned mh = nh >> 11, ml = __funnelshift_r(nl, nh, 11);  // 53 bits: mh has 21
-  const unsigned rem = nl & 0x7FFu;
-  const unsigned inc = (rem > 0x400u || (rem == 0x400u && (ml & 1u))) ? 1u : 0u;
-  ml += inc;
-  mh += (inc != 0u && ml == 0u) ? 1u : 0u;
-  const int E = 63 - lz + (int)(mh >> 21) + s + 1023;
-  if (uh == 0u || (unsigned)(E - 1) >= 2046u) return false;
-  const unsigned dh = (sgn & 0x80000000u) | ((unsigned)E << 20) | (mh & 0xFFFFFu);
-  c = __dsub_rn(c, __hiloint2double((int)dh, (int)ml));
+  const unsigned ml = __funnelshift_r(nl, nh, 11);
+  // Round to nearest even: the 11 bits below, plus the last bit kept, above one half.
+  const unsigned x = (nl & 0x7FFu) + (ml & 1u);
+  const unsigned eh = s20 + ((unsigned)(62 + 1023) << 20) - ((unsigned)lz << 20) + (nh >> 11);
+  unsigned t, dl, dh;
+  asm("{\n add.cc.u32 %0, %3, 0xfffffbff;\n addc.cc.u32 %1, %4, 0;\n addc.u32 %2, %5, 0;\n}\n"
+      : "=&r"(t), "=&r"(dl), "=r"(dh)
+      : "r"(x), "r"(ml), "r"(eh));
+  if (uh == 0u) return false;
+  c = __dsub_rn(c, __hiloint2double((int)(dh | (sgn & 0x80000000u)), (int)dl));
   return true;
 }
+
+// Splitting an exact integer x, |x| < 2^30 in FP32, at its low 8 bits: returns the
+// multiple of 256 nearest to x; lo = the rest, -128 .. 128.
+__device__ __forceinline__ float oz_carry(float x, float& lo) {
+  const float q = __fsub_rn(__fadd_rn(x, 3221225472.0f), 3221225472.0f);  // 1.5 2^31: an ulp of 256
+  lo = __fsub_rn(x, q);
+  return q;
+}
+// x 2^0 as the low bits of an integer (0x4B400000 + x), |x| < 2^22.
+__device__ __forceinline__ unsigned oz_int_bits(float x) { return __float_as_uint(__fadd_rn(x, 12582912.0f)); }
 
 __device__ __forceinline__ double oz_combine(unsigned hi, unsigned lo, int ea_i, int eb_j, double c) {
   if (ea_i >= kOzNonFinite || eb_j >= kOzNonFinite) return __longlong_as_double(0x7ff8000000000000ll);
@@ -258,22 +360,22 @@ __device__ __forceinline__ double oz_combine(unsigned hi, unsigned lo, int ea_i,
 }
 
 __global__ void __launch_bounds__(kOzThreads, 1)
-    oz_gemm_kernel(const __grid_constant__ CUtensorMap tmL, const __grid_constant__ CUtensorMap tmU,
+    oz_gemm_kernel(const __grid_constant__ CUtensorMap tmL, const __grid_constant__ CUtensorMap tmU, int halves,
                    double* __restrict__ c, int64_t ldc, int M, int N, const int* __restrict__ ea,
                    const int* __restrict__ eb, DeviceStatus* st) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  unsigned char* sU = base;                                    // resident: U^T slices of the column block
-  unsigned char* sL = base + (size_t)kOzSlices * kOzSliceBytes;  // streamed: L slices of each tile's rows
-  __shared__ __align__(8) unsigned long long u_full, u_empty, l_full[kOzSlices], l_empty[kOzSlices],
-      acc_full[kOzAccBufs], acc_empty[kOzAccBufs], mma_done;
+  unsigned char* sU = base;                                  // streamed: the U pieces of each tile and K half
+  unsigned char* sL = base + (size_t)kOzSlices * kOzUBytes;  // resident: the L pieces of the row block
+  __shared__ __align__(8) unsigned long long l_full, l_empty, u_full[kOzSlices], u_empty[kOzSlices],
+      acc_full, acc_empty[kOzAccs], mma_done;
   __shared__ unsigned tmem_base;
-  __shared__ int s_abort, s_u_issued, s_u_consumed, s_l_issued;
+  __shared__ int s_abort, s_l_issued, s_l_consumed, s_u_issued;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const unsigned long long limit = st->timeout_ns;
-  const int tiles_i = (M + kOzBM - 1) / kOzBM;
-  const int tiles = tiles_i * ((N + kOzBN - 1) / kOzBN);
+  const int tiles_j = (N + kOzBN - 1) / kOzBN;
+  const int tiles = tiles_j * ((M + kOzBM - 1) / kOzBM);
   const int t_begin = (int)((int64_t)blockIdx.x * tiles / gridDim.x);
   const int t_end = (int)((int64_t)(blockIdx.x + 1) * tiles / gridDim.x);
 
@@ -282,19 +384,18 @@ __global__ void __launch_bounds__(kOzThreads, 1)
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   if (threadIdx.x == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&u_full)));
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&u_empty)));
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&l_full)));
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&l_empty)));
     for (int p = 0; p < kOzSlices; ++p) {
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&l_full[p])));
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&l_empty[p])));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&u_full[p])));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&u_empty[p])));
     }
-    for (int b = 0; b < kOzAccBufs; ++b) {
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&acc_full[b])));
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&acc_empty[b])), "r"(kOzEpiWarps));
-    }
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&acc_full)));
+    for (int g = 0; g < kOzAccs; ++g)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&acc_empty[g])), "r"(kOzEpiWarps));
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&mma_done)));
     s_abort = 0;
-    s_u_issued = s_u_consumed = s_l_issued = 0;
+    s_l_issued = s_l_consumed = s_u_issued = 0;
     asm volatile("fence.mbarrier_init.release.cluster;");
     asm volatile("fence.proxy.async.shared::cta;");
   }
@@ -305,240 +406,243 @@ __global__ void __launch_bounds__(kOzThreads, 1)
 
   if (warp == 0) {
     if (lane == 0) {
-      // Producer.  L slices go in the order the MMAs free them (6 .. 0).
-      int cur_jb = -1, nu = 0, tc = 0;
-      for (int t = t_begin; t < t_end; ++t, ++tc) {
+      // Producer.  U pieces go in the order the MMAs free them (6 .. 0).
+      int cur_ib = -1, nl = 0, use = 0;
+      bool ok = true;
+      for (int t = t_begin; t < t_end && ok; ++t) {
         if (*reinterpret_cast<volatile int*>(&s_abort)) break;
-        const int jb = t / tiles_i, ib = t - jb * tiles_i;
-        if (jb != cur_jb) {
-          // The previous column block's slices are free once its last MMAs end.
-          if (nu > 0 && !oz_wait(smem_u32(&u_empty), (unsigned)((nu - 1) & 1), limit, &s_abort)) {
-            oz_abort(st, &s_abort);
-            break;
-          }
-          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&u_full)),
-                       "r"((unsigned)(kOzSlices * kOzSliceBytes))
-                       : "memory");
-          for (int q = 0; q < kOzSlices; ++q)
-            oz_tma3d(smem_u32(sU + q * kOzSliceBytes), &tmU, jb * kOzBN, q, smem_u32(&u_full));
-          s_u_issued = ++nu;
-          cur_jb = jb;
-        }
-        bool ok = true;
-        for (int p = kOzSlices - 1; p >= 0; --p) {
-          if (!oz_wait(smem_u32(&l_empty[p]), (unsigned)(tc & 1) ^ 1u, limit, &s_abort)) {
+        const int ib = t / tiles_j, jb = t - ib * tiles_j;
+        if (ib != cur_ib) {
+          // The previous row block's pieces are free once its last MMAs end.
+          if (nl > 0 && !oz_wait(smem_u32(&l_empty), (unsigned)((nl - 1) & 1), limit, &s_abort)) {
             ok = false;
             break;
           }
-          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&l_full[p])),
-                       "r"((unsigned)kOzSliceBytes)
+          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&l_full)),
+                       "r"((unsigned)(halves * kOzSlices * kOzLBytes))
                        : "memory");
-          oz_tma3d(smem_u32(sL + p * kOzSliceBytes), &tmL, ib * kOzBM, p, smem_u32(&l_full[p]));
-          ++s_l_issued;
+          for (int h = 0; h < halves; ++h)
+            for (int p = kOzSlices - 1; p >= 0; --p)
+              oz_tma3d(smem_u32(sL + (h * kOzSlices + p) * kOzLBytes), &tmL, h * kOzK, ib * kOzBM, p,
+                       smem_u32(&l_full));
+          s_l_issued = ++nl;
+          cur_ib = ib;
         }
-        if (!ok) {
-          oz_abort(st, &s_abort);
-          break;
+        for (int h = 0; h < halves && ok; ++h, ++use) {
+          for (int q = kOzSlices - 1; q >= 0; --q) {
+            if (!oz_wait(smem_u32(&u_empty[q]), (unsigned)(use & 1) ^ 1u, limit, &s_abort)) {
+              ok = false;
+              break;
+            }
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&u_full[q])),
+                         "r"((unsigned)kOzUBytes)
+                         : "memory");
+            oz_tma3d(smem_u32(sU + q * kOzUBytes), &tmU, h * kOzK, jb * kOzBN, q, smem_u32(&u_full[q]));
+            ++s_u_issued;
+          }
         }
       }
+      if (!ok) oz_abort(st, &s_abort);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      // MMA issuer: D FP32 (bit 4), A and B FP16 (format 0), K-major, M = N = 128.
-      // D[j][i] += sum_k U^T_q[j][k] L_p[i][k]: TMEM lanes are columns of C.
-      constexpr unsigned idesc = (1u << 4) | ((unsigned)(kOzBM >> 3) << 17) | ((unsigned)(kOzBN >> 4) << 24);
-      int cur_jb = -1, nu = 0, tc = 0;
-      bool ok = true;
-      for (int t = t_begin; t < t_end && ok; ++t, ++tc) {
-        if (*reinterpret_cast<volatile int*>(&s_abort)) break;
-        const int jb = t / tiles_i;
-        if (jb != cur_jb) {
-          if (!oz_wait(smem_u32(&u_full), (unsigned)(nu & 1), limit, &s_abort)) {
-            ok = false;
-            break;
-          }
-          s_u_consumed = ++nu;
-          cur_jb = jb;
-        }
-        unsigned have = 0;  // L slices of this tile already waited for
-        for (int G = kOzGroups - 1; G >= 0 && ok; --G) {
-          // The groups take the accumulators in turn over the whole launch:
-          // group number i = 8 tc + 7 - G uses accumulator i % 3 for its use
-          // i / 3; wait for the epilogue's release of the previous use.
-          const int gi = kOzGroups * tc + kOzGroups - 1 - G;
-          const int buf = gi % kOzAccBufs;
-          const unsigned use_parity = (unsigned)((gi / kOzAccBufs) & 1);
-          if (!oz_wait(smem_u32(&acc_empty[buf]), use_parity ^ 1u, limit, &s_abort)) {
-            ok = false;
-            break;
-          }
-          asm volatile("tcgen05.fence::after_thread_sync;");
-          const unsigned acc_addr = tmem + (unsigned)(buf * kOzBM);
-          unsigned accf = 0;
-          for (int p = max(0, G - (kOzSlices - 1)); p <= min(G, kOzSlices - 1); ++p) {
-            const int q = G - p;
-            if (!(have & (1u << p))) {
-              if (!oz_wait(smem_u32(&l_full[p]), (unsigned)(tc & 1), limit, &s_abort)) {
-                ok = false;
-                break;
-              }
-              asm volatile("tcgen05.fence::after_thread_sync;");
-              have |= 1u << p;
-            }
-#pragma unroll
-            for (int ks = 0; ks < kOzK / 16; ++ks) {
-              const unsigned long long da = sw128_desc(smem_u32(sU + q * kOzSliceBytes + ks * 32));
-              const unsigned long long db = sw128_desc(smem_u32(sL + p * kOzSliceBytes + ks * 32));
-              asm volatile(
-                  "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, "
-                  "p;\n}\n" ::"r"(acc_addr),
-                  "l"(da), "l"(db), "r"(idesc), "r"(accf));
-              accf = 1;
-            }
-          }
-          if (!ok) break;
-          oz_commit(smem_u32(&acc_full[buf]));
-          // L slice G is last used by group G.
-          if (G < kOzSlices) oz_commit(smem_u32(&l_empty[G]));
-        }
+    // MMA issuer: D[j][i] += sum_k U^T_q[j][k] L_p[i][k]: TMEM lanes are columns of C.
+    // The whole warp runs the loop, so its addresses and descriptors stay in
+    // uniform registers, which the MMAs take them from; one lane issues.
+    // U piece q against the stacked L pieces 0, 1, .. is one product with N = 64 a
+    // piece whose columns are the accumulators of groups q, q + 1, ..: 10 MMAs a
+    // k-step instead of 28, each of them long enough for the pipe (an MMA of N = 64
+    // takes as long as one of N = 128: 128 cycles with its operands from shared
+    // memory).
+    const bool leader = lane == 0;
+    const unsigned u_lo = (smem_u32(sU) >> 4) | (1u << 16), l_lo = (smem_u32(sL) >> 4) | (1u << 16);
+    int cur_ib = -1, nl = 0, tc = 0, use = 0;
+    bool ok = true;
+    for (int t = t_begin; t < t_end && ok; ++t, ++tc) {
+      const int ib = t / tiles_j;
+      if (ib != cur_ib) {
+        ok = __all_sync(0xffffffffu, oz_wait(smem_u32(&l_full), (unsigned)(nl & 1), limit, &s_abort));
         if (!ok) break;
-        const bool block_ends = (t + 1 >= t_end) || ((t + 1) / tiles_i != jb);
-        if (block_ends) oz_commit(smem_u32(&u_empty));
+        ++nl;
+        if (leader) s_l_consumed = nl;
+        cur_ib = ib;
       }
+      ok = oz_mma_half<0>(tmem, u_lo, l_lo, leader, smem_u32(acc_empty), smem_u32(u_full), smem_u32(u_empty),
+                          (unsigned)(tc & 1) ^ 1u, (unsigned)(use & 1), limit, &s_abort);
+      ++use;
+      if (ok && halves == 2) {
+        ok = oz_mma_half<1>(tmem, u_lo, l_lo, leader, smem_u32(acc_empty), smem_u32(u_full), smem_u32(u_empty),
+                            (unsigned)(tc & 1) ^ 1u, (unsigned)(use & 1), limit, &s_abort);
+        ++use;
+      }
+      if (!ok) break;
+      if (leader) {
+        oz_commit(smem_u32(&acc_full));
+        const bool block_ends = (t + 1 >= t_end) || ((t + 1) / tiles_j != ib);
+        if (block_ends) oz_commit(smem_u32(&l_empty));
+      }
+      __syncwarp();
+    }
+    if (leader) {
       if (!ok) oz_abort(st, &s_abort);
       // Arrives once every MMA issued above has completed.
       oz_commit(smem_u32(&mma_done));
       mbar_wait(smem_u32(&mma_done), 0u, limit);
     }
+    __syncwarp();
   } else {
     // Epilogue: warp w owns TMEM lanes 32 (w % 4) .. + 31 (32 columns of the
-    // tile) and 32 of its 128 rows, g = (w - 2) / 4.  Its thread keeps the
-    // high words of its column's 32 fixed-point sums in registers and the low
-    // words in TMEM (tile row r: column kOzLoCol + r); 16 rows of an
-    // accumulator at a time pass through registers.
+    // tile) and 16 of its 64 rows, (w - 2) / 4.  Its thread keeps its column's
+    // 16 sums in two registers each.
+    // Fold.  R = floor(sum_G T_G 2^(38-8G)), exactly.  Converting each T_G and
+    // shifting 64-bit sums costs a conversion (8 cycles of a quarter's unit) and
+    // three integer instructions (2 cycles each) a group; FP32 additions run at full
+    // rate and are exact here, so the groups' low 8 bits are split off in FP32 and
+    // the rest carried to the next group: with q_G the carry out of group G, and
+    // lo_G its digit (-128 .. 128),
+    //   x_G = T_G + q_(G+1) / 256 = q_G + lo_G,
+    //   R = T_0 2^38 + x_1 2^30 + lo_2 2^22 + lo_3 2^14 + floor((lo_4 2^16 + lo_5 2^8 + lo_6) / 2^10),
+    // three conversions in all.  |T_G| < 2^24 - 2^20 for G <= 4, so that x_G is
+    // exact; T_5 can come within 2^15 of 2^24 (K = 128) and is split before it
+    // takes the carry, as are the two sums of group 6.
     const int quarter = warp & 3, rq = (warp - 2) >> 2;
-    const unsigned lane_base = tmem + ((unsigned)(quarter * 32) << 16);
-    const unsigned lo_base = lane_base + kOzLoCol + (unsigned)(rq * 32);
+    const unsigned lane_base = tmem + ((unsigned)(quarter * 32) << 16) + (unsigned)(rq * kOzRows);
     int tc = 0;
     for (int t = t_begin; t < t_end; ++t, ++tc) {
-      const int jb = t / tiles_i, ib = t - jb * tiles_i;
+      const int ib = t / tiles_j, jb = t - ib * tiles_j;
       const int col = jb * kOzBN + quarter * 32 + lane;
-      const int row0 = ib * kOzBM + rq * 32;
+      const int row0 = ib * kOzBM + rq * kOzRows;
       const bool col_ok = col < N;
       {
-        // Bring this warp's 32 rows x 32 columns of C into L2 while the
-        // tile's products run (lane r: row r, 256 bytes).
-        const int c0 = jb * kOzBN + quarter * 32;
-        if (c0 < N && row0 + lane < M) {
-          const double* pr = c + (int64_t)(row0 + lane) * ldc + c0;
-          asm volatile("prefetch.global.L2 [%0];" ::"l"(pr));
-          if (c0 + 16 < N) asm volatile("prefetch.global.L2 [%0];" ::"l"(pr + 16));
-        }
+        // Bring this warp's 16 rows x 32 columns of C into L2 while the tile's
+        // products run (lane r: half of row r % 16, 128 bytes).
+        const int c0 = jb * kOzBN + quarter * 32 + (lane >> 4) * 16, rr = row0 + (lane & 15);
+        if (c0 < N && rr < M) asm volatile("prefetch.global.L2 [%0];" ::"l"(c + (int64_t)rr * ldc + c0));
       }
-      unsigned rh[32];
-      bool ok = true;
-      for (int G = kOzGroups - 1; G >= 0; --G) {
-        const int gi = kOzGroups * tc + kOzGroups - 1 - G;
-        const int buf = gi % kOzAccBufs;
-        const unsigned use_parity = (unsigned)((gi / kOzAccBufs) & 1);
-        const bool got = oz_wait(smem_u32(&acc_full[buf]), use_parity, limit, &s_abort);
-        if (!__all_sync(0xffffffffu, got)) {
-          ok = false;
-          break;
-        }
-        asm volatile("tcgen05.fence::after_thread_sync;");
-        const unsigned acc = lane_base + (unsigned)(buf * kOzBM + rq * 32);
-        if (G == kOzGroups - 1) {
-          // First group: R = T 2^38.
-#pragma unroll
-          for (int cc = 0; cc < 2; ++cc) {
-            unsigned tv[16], lv[16];
-            tmem_ld16(acc + (unsigned)(cc * 16), tv);
-            asm volatile("tcgen05.wait::ld.sync.aligned;");
-#pragma unroll
-            for (int r = 0; r < 16; ++r) {
-              rh[cc * 16 + r] = (unsigned)(__float2int_rn(__uint_as_float(tv[r])) << (kOzFrac - 32));
-              lv[r] = 0u;
-            }
-            tmem_st16(lo_base + (unsigned)(cc * 16), lv);
-          }
-        } else {
-          // R = T 2^38 + floor(R / 2^8) on (hi, lo) words: T 2^38 only
-          // touches hi (|R| < 2^62), so no carry crosses the words.
-#pragma unroll
-          for (int cc = 0; cc < 2; ++cc) {
-            unsigned tv[16], lv[16];
-            tmem_ld16(acc + (unsigned)(cc * 16), tv);
-            tmem_ld16(lo_base + (unsigned)(cc * 16), lv);
-            asm volatile("tcgen05.wait::ld.sync.aligned;");
-#pragma unroll
-            for (int r = 0; r < 16; ++r) {
-              const unsigned hi = rh[cc * 16 + r];
-              lv[r] = __funnelshift_r(lv[r], hi, 8);
-              rh[cc * 16 + r] =
-                  (unsigned)(((int)hi >> 8) + (__float2int_rn(__uint_as_float(tv[r])) << (kOzFrac - 32)));
-            }
-            tmem_st16(lo_base + (unsigned)(cc * 16), lv);
-          }
-        }
-        // This warp has read the accumulator: the MMA warp may reuse it.
-        asm volatile("tcgen05.wait::st.sync.aligned;");
-        asm volatile("tcgen05.fence::before_thread_sync;");
-        __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&acc_empty[buf]));
-      }
-      if (!ok) {
+      const bool got = oz_wait(smem_u32(&acc_full), (unsigned)(tc & 1), limit, &s_abort);
+      if (!__all_sync(0xffffffffu, got)) {
         if (lane == 0) oz_abort(st, &s_abort);
         break;
       }
-      // C -= the sums: thread = one column of C, its 32 rows in chunks of 4;
+      asm volatile("tcgen05.fence::after_thread_sync;");
+      float xq[kOzRows], lo[kOzRows];
+      unsigned rh[kOzRows], rl[kOzRows];
+      auto load = [&](int acc, unsigned (&tv)[kOzRows]) {
+        tmem_ld16(lane_base + (unsigned)(acc * kOzBM), tv);
+        asm volatile("tcgen05.wait::ld.sync.aligned;");
+        // This warp has read the accumulator: the MMA warp may reuse it.
+        asm volatile("tcgen05.fence::before_thread_sync;");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&acc_empty[acc]));
+      };
+      {
+        unsigned tv[kOzRows];
+        load(6, tv);
+#pragma unroll
+        for (int r = 0; r < kOzRows; ++r) xq[r] = oz_carry(__uint_as_float(tv[r]), lo[r]);
+      }
+      if (halves == 2) {
+        unsigned tv[kOzRows];
+        load(kOzGroups, tv);
+#pragma unroll
+        for (int r = 0; r < kOzRows; ++r) {
+          float lo2;
+          xq[r] = __fadd_rn(xq[r], oz_carry(__uint_as_float(tv[r]), lo2));
+          lo[r] = __fadd_rn(lo[r], lo2);
+        }
+      }
+      {
+        unsigned tv[kOzRows];
+        load(5, tv);
+#pragma unroll
+        for (int r = 0; r < kOzRows; ++r) {
+          float d, e;
+          const float qa = oz_carry(__uint_as_float(tv[r]), d);
+          const float qb = oz_carry(__fmaf_rn(xq[r], 0.00390625f, d), e);
+          xq[r] = __fadd_rn(qa, qb);
+          lo[r] = __fmaf_rn(e, 256.0f, lo[r]);
+        }
+      }
+      {
+        unsigned tv[kOzRows];
+        load(4, tv);
+#pragma unroll
+        for (int r = 0; r < kOzRows; ++r) {
+          float d;
+          xq[r] = oz_carry(__fmaf_rn(xq[r], 0.00390625f, __uint_as_float(tv[r])), d);
+          rl[r] = (unsigned)(__float2int_rn(__fmaf_rn(d, 65536.0f, lo[r])) >> 10);
+        }
+      }
+#pragma unroll
+      for (int g = 3; g >= 2; --g) {
+        unsigned tv[kOzRows];
+        load(g, tv);
+#pragma unroll
+        for (int r = 0; r < kOzRows; ++r) {
+          float d;
+          xq[r] = oz_carry(__fmaf_rn(xq[r], 0.00390625f, __uint_as_float(tv[r])), d);
+          rl[r] += oz_int_bits(d) << (kOzFrac - 8 * g);  // the bias is shifted out
+        }
+      }
+      {
+        unsigned tv[kOzRows];
+        load(1, tv);
+#pragma unroll
+        for (int r = 0; r < kOzRows; ++r) {
+          const int x1 = __float2int_rn(__fmaf_rn(xq[r], 0.00390625f, __uint_as_float(tv[r])));
+          const unsigned h = (unsigned)((x1 >> 2) + ((int)rl[r] >> 31));
+          asm("{\n add.cc.u32 %0, %2, %3;\n addc.u32 %1, %4, 0;\n}\n"
+              : "=&r"(rl[r]), "=r"(rh[r])
+              : "r"(rl[r]), "r"((unsigned)x1 << 30), "r"(h));
+        }
+      }
+      {
+        unsigned tv[kOzRows];
+        load(0, tv);
+#pragma unroll
+        for (int r = 0; r < kOzRows; ++r)
+          rh[r] += (unsigned)__float2int_rn(__uint_as_float(tv[r])) << (kOzFrac - 32);
+      }
+      // C -= the sums: thread = one column of C, its rows in chunks of 4;
       // a warp's loads and stores of one row are 32 consecutive doubles.
       // Lane r holds the exponent of row r.  Elements the fast path declines
       // (rare) are redone, warp-uniformly, by the general path.
       const int eb_j = col_ok ? eb[col] : 0;
-      const int my_ea = row0 + lane < M ? ea[row0 + lane] : 0;
+      const int my_ea = lane < kOzRows && row0 + lane < M ? ea[row0 + lane] : 0;
       const int s_col = eb_j >= kOzNonFinite ? (1 << 24) : eb_j - (kOzFrac + 16);
       const int s_row = my_ea >= kOzNonFinite ? (1 << 24) : my_ea;
-      const bool whole = (jb * kOzBN + quarter * 32 + 32 <= N) && (row0 + 32 <= M);  // warp-uniform
+      const bool in_range =
+          __reduce_min_sync(0xffffffffu, s_col) + __reduce_min_sync(0xffffffffu, s_row) >= kOzMinScale &&
+          __reduce_max_sync(0xffffffffu, s_col) + __reduce_max_sync(0xffffffffu, s_row) <= kOzMaxScale;
+      const bool whole = (jb * kOzBN + quarter * 32 + 32 <= N) && (row0 + kOzRows <= M);  // warp-uniform
       double* cptr = c + (int64_t)row0 * ldc + (col_ok ? col : 0);
+      constexpr int kC = 4;
 #pragma unroll
-      for (int cc = 0; cc < 8; ++cc) {
-        unsigned lv[4];
-        tmem_ld4(lo_base + (unsigned)(cc * 4), lv);
-        double cv[4];
-        if (whole) {
+      for (int cc = 0; cc < kOzRows / kC; ++cc) {
+        double cv[kC];
 #pragma unroll
-          for (int r = 0; r < 4; ++r) cv[r] = __ldcs(cptr + (int64_t)r * ldc);
-        } else {
+        for (int r = 0; r < kC; ++r)
+          cv[r] = (whole || (col_ok && row0 + kC * cc + r < M)) ? __ldcs(cptr + (int64_t)r * ldc) : 0.0;
+        unsigned declined = in_range ? 0u : (1u << kC) - 1u;
+        if (in_range) {
 #pragma unroll
-          for (int r = 0; r < 4; ++r)
-            cv[r] = (col_ok && row0 + 4 * cc + r < M) ? __ldcs(cptr + (int64_t)r * ldc) : 0.0;
-        }
-        asm volatile("tcgen05.wait::ld.sync.aligned;");
-        unsigned declined = 0;
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-          const int k = 4 * cc + r;
-          const int s = s_col + __shfl_sync(0xffffffffu, s_row, k);
-          if (!oz_combine_fast(rh[k], lv[r], s, cv[r])) declined |= 1u << r;
+          for (int r = 0; r < kC; ++r) {
+            const int k = kC * cc + r;
+            const unsigned s20 = (unsigned)(s_col + __shfl_sync(0xffffffffu, s_row, k)) << 20;
+            if (!oz_combine_fast(rh[k], rl[k], s20, cv[r])) declined |= 1u << r;
+          }
         }
         if (__any_sync(0xffffffffu, declined != 0u)) {
 #pragma unroll
-          for (int r = 0; r < 4; ++r) {
-            const int k = 4 * cc + r;
+          for (int r = 0; r < kC; ++r) {
+            const int k = kC * cc + r;
             const int ea_i = __shfl_sync(0xffffffffu, my_ea, k);
-            if (declined & (1u << r)) cv[r] = oz_combine(rh[k], lv[r], ea_i, eb_j, cv[r]);
+            if (declined & (1u << r)) cv[r] = oz_combine(rh[k], rl[k], ea_i, eb_j, cv[r]);
           }
         }
-        if (whole) {
 #pragma unroll
-          for (int r = 0; r < 4; ++r) __stcs(cptr + (int64_t)r * ldc, cv[r]);
-        } else {
-#pragma unroll
-          for (int r = 0; r < 4; ++r)
-            if (col_ok && row0 + 4 * cc + r < M) __stcs(cptr + (int64_t)r * ldc, cv[r]);
-        }
-        cptr += 4 * ldc;
+        for (int r = 0; r < kC; ++r)
+          if (whole || (col_ok && row0 + kC * cc + r < M)) __stcs(cptr + (int64_t)r * ldc, cv[r]);
+        cptr += kC * ldc;
         asm volatile("" ::: "memory");  // keep the chunks' loads from being hoisted together
       }
     }
@@ -546,12 +650,12 @@ __global__ void __launch_bounds__(kOzThreads, 1)
   __syncthreads();
   if (threadIdx.x == 0 && s_abort) {
     // Copies issued but never consumed must land before the CTA exits.
-    if (s_u_issued > s_u_consumed) mbar_wait(smem_u32(&u_full), (unsigned)((s_u_issued - 1) & 1), limit);
-    // L slices: every issued slice's barrier completes once its bytes land
-    // (issue order 6 .. 0 per tile).
+    if (s_l_issued > s_l_consumed) mbar_wait(smem_u32(&l_full), (unsigned)((s_l_issued - 1) & 1), limit);
+    // U pieces: every issued piece's barrier completes once its bytes land
+    // (issue order 6 .. 0 per tile and half).
     for (int p = 0; p < kOzSlices; ++p) {
-      const int uses = s_l_issued / kOzSlices + (kOzSlices - 1 - p < s_l_issued % kOzSlices ? 1 : 0);
-      if (uses > 0) mbar_wait(smem_u32(&l_full[p]), (unsigned)((uses - 1) & 1), limit);
+      const int uses = s_u_issued / kOzSlices + (kOzSlices - 1 - p < s_u_issued % kOzSlices ? 1 : 0);
+      if (uses > 0) mbar_wait(smem_u32(&u_full[p]), (unsigned)((uses - 1) & 1), limit);
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
@@ -565,21 +669,22 @@ __global__ void __launch_bounds__(kOzThreads, 1)
 // ---------------------------------------------------------------------------
 static size_t oz_round(size_t b) { return (b + 1023) / 1024 * 1024; }
 
-// Workspace layout for an M x N product: A slices [7][M][64], B slices
-// [7][N][64], exponents ea[M], eb[N].
+// Workspace layout for an M x N product over K = 64 * halves: A slices
+// [7][M][K], B slices [7][N][K], exponents ea[M], eb[N].
 struct OzWs {
   __half* as;
   __half* bs;
   int* ea;
   int* eb;
 };
-static OzWs oz_layout(void* ws, int M, int N) {
+static OzWs oz_layout(void* ws, int M, int N, int halves = 1) {
+  const size_t kb = (size_t)kOzSlices * kOzK * 2 * halves;
   char* p = static_cast<char*>(ws);
   OzWs w;
   w.as = reinterpret_cast<__half*>(p);
-  p += oz_round((size_t)kOzSlices * M * kOzK * 2);
+  p += oz_round(kb * M);
   w.bs = reinterpret_cast<__half*>(p);
-  p += oz_round((size_t)kOzSlices * N * kOzK * 2);
+  p += oz_round(kb * N);
   w.ea = reinterpret_cast<int*>(p);
   p += oz_round((size_t)M * 4);
   w.eb = reinterpret_cast<int*>(p);
@@ -587,20 +692,21 @@ static OzWs oz_layout(void* ws, int M, int N) {
 }
 
 size_t ozaki_workspace_bytes(int m, int n) {
-  return oz_round((size_t)kOzSlices * m * kOzK * 2) + oz_round((size_t)kOzSlices * n * kOzK * 2) +
-         oz_round((size_t)m * 4) + oz_round((size_t)n * 4);
+  const size_t kb = (size_t)kOzSlices * kOzK * 2 * kOzMaxHalves;
+  return oz_round(kb * m) + oz_round(kb * n) + oz_round((size_t)m * 4) + oz_round((size_t)n * 4);
 }
 
 bool ozaki_available(luhot_ctx* ctx) { return kOzSmem <= (size_t)ctx->max_smem_optin && encode_fn() != nullptr; }
 
-// Slices [7][rows][64] FP16 as a 3-D tensor map (k, row, slice) with boxes of
-// 64 x box_rows x 1 (128-byte rows, 128-byte swizzle); rows past `rows` read
-// as zero.
-static int make_slice_map(luhot_ctx* ctx, CUtensorMap* map, void* ptr, int rows, int box_rows) {
+// Slices [7][rows][K] FP16, K = 64 * halves, as a 3-D tensor map (k, row, slice)
+// with boxes of 64 x box_rows x 1 (128-byte rows, 128-byte swizzle); rows past
+// `rows` read as zero.
+static int make_slice_map(luhot_ctx* ctx, CUtensorMap* map, void* ptr, int rows, int box_rows, int halves) {
   EncodeTiledFn enc = encode_fn();
   if (!enc) return set_error(ctx, LUHOT_ERR_UNSUPPORTED, "cuTensorMapEncodeTiled is unavailable");
-  cuuint64_t dims[3] = {(cuuint64_t)kOzK, (cuuint64_t)rows, (cuuint64_t)kOzSlices};
-  cuuint64_t strides[2] = {(cuuint64_t)kOzK * 2, (cuuint64_t)rows * kOzK * 2};
+  const cuuint64_t kk = (cuuint64_t)kOzK * halves;
+  cuuint64_t dims[3] = {kk, (cuuint64_t)rows, (cuuint64_t)kOzSlices};
+  cuuint64_t strides[2] = {kk * 2, (cuuint64_t)rows * kk * 2};
   cuuint32_t box[3] = {(cuuint32_t)kOzK, (cuuint32_t)box_rows, 1};
   cuuint32_t estr[3] = {1, 1, 1};
   const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, ptr, dims, strides, box, estr,
@@ -611,15 +717,15 @@ static int make_slice_map(luhot_ctx* ctx, CUtensorMap* map, void* ptr, int rows,
 }
 
 // C (M x N, ldc) -= the product of the slices in `w`; one persistent launch.
-static int oz_launch_gemm(luhot_ctx* ctx, const OzWs& w, double* c, int64_t ldc, int M, int N,
+static int oz_launch_gemm(luhot_ctx* ctx, const OzWs& w, int halves, double* c, int64_t ldc, int M, int N,
                           cudaStream_t stream) {
   CUtensorMap tmL, tmU;
-  int rc = make_slice_map(ctx, &tmL, w.as, M, kOzBM);
-  if (!rc) rc = make_slice_map(ctx, &tmU, w.bs, N, kOzBN);
+  int rc = make_slice_map(ctx, &tmL, w.as, M, kOzBM, halves);
+  if (!rc) rc = make_slice_map(ctx, &tmU, w.bs, N, kOzBN, halves);
   if (rc) return rc;
   const int tiles = ((M + kOzBM - 1) / kOzBM) * ((N + kOzBN - 1) / kOzBN);
   LUHOT_CUDA_TRY(ctx, allow_max_dynamic_smem(oz_gemm_kernel));
-  oz_gemm_kernel<<<std::min(tiles, ctx->num_sms), kOzThreads, kOzSmem, stream>>>(tmL, tmU, c, ldc, M, N, w.ea, w.eb,
+  oz_gemm_kernel<<<std::min(tiles, ctx->num_sms), kOzThreads, kOzSmem, stream>>>(tmL, tmU, halves, c, ldc, M, N, w.ea, w.eb,
                                                                                 ctx->d_status);
   LUHOT_CUDA_TRY(ctx, cudaGetLastError());
   return LUHOT_OK;
@@ -642,7 +748,7 @@ int ozaki_update_split(luhot_ctx* ctx, double* a, int64_t lda, int w, int r1, in
   const int M = m - r1, N = n - c1;
   const OzWs lay = oz_layout(ws, M, N);
   prof_begin(ctx, kProfGemm);
-  int rc = oz_launch_gemm(ctx, lay, a + (int64_t)r1 * lda + c1, lda, M, N, stream);
+  int rc = oz_launch_gemm(ctx, lay, 1, a + (int64_t)r1 * lda + c1, lda, M, N, stream);
   // algorithmic work: 2MNK FP64 flops; bytes: C read + written, the slices read once
   prof_end(ctx, kProfGemm, 2.0 * M * N * w,
            (double)M * N * 16 + (double)(M + N) * kOzK * kOzSlices * 2 + (double)(M + N) * 4);
@@ -652,42 +758,34 @@ int ozaki_update_split(luhot_ctx* ctx, double* a, int64_t lda, int w, int r1, in
 int ozaki_product(luhot_ctx* ctx, const double* l, int64_t ldl, const double* u, int64_t ldu, int w, double* c,
                   int64_t ldc, int M, int N, void* ws, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || w <= 0) return LUHOT_OK;
-  if (w > kOzK) return set_error(ctx, LUHOT_ERR_INVALID_ARG, "ozaki_product: more than 64 columns");
-  const OzWs lay = oz_layout(ws, M, N);
+  if (w > kOzMaxHalves * kOzK) return set_error(ctx, LUHOT_ERR_INVALID_ARG, "ozaki_product: more than 128 columns");
+  const int halves = w > kOzK ? 2 : 1;
+  const OzWs lay = oz_layout(ws, M, N, halves);
+  const double slice_bytes = (double)halves * kOzK * kOzSlices * 2;
   prof_begin(ctx, kProfOther);
-  oz_split_rows_kernel<<<(M + 7) / 8, 256, 0, stream>>>(l, ldl, 0, M, 0, w, lay.as, lay.ea);
-  prof_end(ctx, kProfOther, 0.0, (double)M * w * 8 + (double)M * kOzK * kOzSlices * 2);
+  if (halves == 2)
+    oz_split_rows_kernel<2><<<(M + 7) / 8, 256, 0, stream>>>(l, ldl, 0, M, 0, w, lay.as, lay.ea);
+  else
+    oz_split_rows_kernel<1><<<(M + 7) / 8, 256, 0, stream>>>(l, ldl, 0, M, 0, w, lay.as, lay.ea);
+  prof_end(ctx, kProfOther, 0.0, M * (w * 8.0 + slice_bytes));
   prof_begin(ctx, kProfOther);
-  oz_split_cols_kernel<<<(N + 31) / 32, 256, 0, stream>>>(u, ldu, 0, w, 0, N, lay.bs, lay.eb);
-  prof_end(ctx, kProfOther, 0.0, (double)N * w * 8 + (double)N * kOzK * kOzSlices * 2);
+  if (halves == 2)
+    oz_split_cols_kernel<2><<<(N + 31) / 32, 256, 0, stream>>>(u, ldu, 0, w, 0, N, lay.bs, lay.eb);
+  else
+    oz_split_cols_kernel<1><<<(N + 31) / 32, 256, 0, stream>>>(u, ldu, 0, w, 0, N, lay.bs, lay.eb);
+  prof_end(ctx, kProfOther, 0.0, N * (w * 8.0 + slice_bytes));
   LUHOT_CUDA_TRY(ctx, cudaGetLastError());
   prof_begin(ctx, kProfGemm);
-  int rc = oz_launch_gemm(ctx, lay, c, ldc, M, N, stream);
-  prof_end(ctx, kProfGemm, 2.0 * M * N * w,
-           (double)M * N * 16 + (double)(M + N) * kOzK * kOzSlices * 2 + (double)(M + N) * 4);
+  int rc = oz_launch_gemm(ctx, lay, halves, c, ldc, M, N, stream);
+  // algorithmic work: 2MNK FP64 flops; bytes: C read + written, the slices read once
+  prof_end(ctx, kProfGemm, 2.0 * M * N * w, (double)M * N * 16 + (M + N) * (slice_bytes + 4.0));
   return rc;
 }
 
 int ozaki_update(luhot_ctx* ctx, double* a, int64_t lda, int k0, int w, int r1, int m, int c1, int n, void* ws,
                  cudaStream_t stream) {
-  const int M = m - r1, N = n - c1;
-  if (M <= 0 || N <= 0 || w <= 0) return LUHOT_OK;
-  if (w > kOzK) {
-    int rc = ozaki_update(ctx, a, lda, k0, kOzK, r1, m, c1, n, ws, stream);
-    if (rc) return rc;
-    return ozaki_update(ctx, a, lda, k0 + kOzK, w - kOzK, r1, m, c1, n, ws, stream);
-  }
-  const OzWs lay = oz_layout(ws, M, N);
-
-  prof_begin(ctx, kProfOther);
-  oz_split_rows_kernel<<<(M + 7) / 8, 256, 0, stream>>>(a, lda, r1, M, k0, w, lay.as, lay.ea);
-  prof_end(ctx, kProfOther, 0.0, (double)M * w * 8 + (double)M * kOzK * kOzSlices * 2);
-  prof_begin(ctx, kProfOther);
-  oz_split_cols_kernel<<<(N + 31) / 32, 256, 0, stream>>>(a, lda, k0, w, c1, N, lay.bs, lay.eb);
-  prof_end(ctx, kProfOther, 0.0, (double)N * w * 8 + (double)N * kOzK * kOzSlices * 2);
-  LUHOT_CUDA_TRY(ctx, cudaGetLastError());
-
-  return ozaki_update_split(ctx, a, lda, w, r1, m, c1, n, ws, stream);
+  return ozaki_product(ctx, a + (int64_t)r1 * lda + k0, lda, a + (int64_t)k0 * lda + c1, lda, w,
+                       a + (int64_t)r1 * lda + c1, lda, m - r1, n - c1, ws, stream);
 }
 
 }  // namespace luhot

@@ -16,11 +16,11 @@ size_t ozaki_workspace_bytes(int m, int n);
 // The device has the shared memory and the driver the tensor-map encoder.
 bool ozaki_available(luhot_ctx* ctx);
 // a[r1..m, c1..n] -= a[r1..m, k0..k0+w] a[k0..k0+w, c1..n] for the row-major
-// FP64 matrix a (lda), K = w in steps of 64; ws holds
+// FP64 matrix a (lda), w <= 128; ws holds
 // ozaki_workspace_bytes(m - r1, n - c1) bytes.  Asynchronous on `stream`.
 int ozaki_update(luhot_ctx* ctx, double* a, int64_t lda, int k0, int w, int r1, int m, int c1, int n, void* ws,
                  cudaStream_t stream);
-// c (M x N, ldc) -= l (M x w, ldl) u (w x N, ldu), w <= 64, separate operands.
+// c (M x N, ldc) -= l (M x w, ldl) u (w x N, ldu), w <= 128, separate operands.
 int ozaki_product(luhot_ctx* ctx, const double* l, int64_t ldl, const double* u, int64_t ldu, int w, double* c,
                   int64_t ldc, int M, int N, void* ws, cudaStream_t stream);
 // ozaki_update in two parts: where the digit slices of the operands go (for
