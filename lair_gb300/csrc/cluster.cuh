@@ -32,18 +32,23 @@ __device__ __forceinline__ void cl_push8(unsigned dst, unsigned bar, unsigned lo
 __device__ __forceinline__ void cl_expect(unsigned bar, unsigned bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
-// Bounded wait of a whole warp; false (for all lanes) once it gave up.
-__device__ __forceinline__ bool cl_wait(unsigned bar, unsigned parity, DeviceStatus* st, int step) {
+__device__ __forceinline__ unsigned cl_try(unsigned bar, unsigned parity) {
+  unsigned done;
+  asm volatile(
+      "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, "
+      "0, p;\n}\n"
+      : "=r"(done)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return done;
+}
+// Bounded wait of a whole warp; false (for all lanes) once it gave up.  The loop is
+// kept out of line: a column's chain runs through its code once a column on one
+// warp, so that the length of that code is itself part of the chain.
+static __device__ __noinline__ bool cl_wait_long(unsigned bar, unsigned parity, DeviceStatus* st, int step) {
   unsigned long long t0 = 0;
-  for (unsigned spins = 0;; ++spins) {
-    unsigned done;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, "
-        "0, p;\n}\n"
-        : "=r"(done)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    if (__all_sync(0xffffffffu, done != 0)) return true;
+  for (unsigned spins = 1;; ++spins) {
+    if (__all_sync(0xffffffffu, cl_try(bar, parity) != 0)) return true;
     if ((spins & 15u) == 0) {
       const unsigned long long now = global_timer_ns();
       if (t0 == 0) t0 = now;
@@ -58,6 +63,10 @@ __device__ __forceinline__ bool cl_wait(unsigned bar, unsigned parity, DeviceSta
       }
     }
   }
+}
+__device__ __forceinline__ bool cl_wait(unsigned bar, unsigned parity, DeviceStatus* st, int step) {
+  if (__all_sync(0xffffffffu, cl_try(bar, parity) != 0)) return true;
+  return cl_wait_long(bar, parity, st, step);
 }
 __device__ __forceinline__ void cl_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");

@@ -1340,8 +1340,13 @@ int getrf_device(luhot_ctx* ctx, int m, int n, T* a, int64_t lda, int* piv, int 
   int nb = ctx->nb_override > 0 ? std::min(ctx->nb_override, kDefaultPanelWidth) : kDefaultPanelWidth;
   // A matrix of at most 128 columns (and at least as many rows) is one panel
   // when the cluster holds it: one launch, no interchanges, solves or updates
-  // outside it (n = 100: 0.10 ms, as two panels of 64 and 36 columns 0.63).
-  if (ctx->nb_override <= 0 && n <= kMaxPanelWidth && m >= n && panel_cluster_fits<T>(ctx, m, n)) nb = kMaxPanelWidth;
+  // outside it (n = 100: 0.10 ms, as two panels of 64 and 36 columns 0.63).  Up to 512
+  // (FP64) or 2048 rows: from there on the bulk of a wide panel's updates is slower
+  // in one cluster than outside (2048 x 128: FP64 0.48 ms as one panel, 0.32 as two;
+  // FP32 0.20 either way).
+  if (ctx->nb_override <= 0 && n <= kMaxPanelWidth && m >= n && m <= (sizeof(T) == 8 ? 512 : 2048) &&
+      panel_cluster_fits<T>(ctx, m, n))
+    nb = kMaxPanelWidth;
   void* oz_ws = nullptr;
   if (std::is_same<T, double>::value && mode != LUHOT_MODE_EXACT) {
     rc = ozaki_workspace(ctx, m, n, ctx->fp64_update, &oz_ws);

@@ -13,23 +13,35 @@
 // pushes its row segment the same way; it is needed only by the next column's
 // updates.
 //
-// Warps.  Warps 0 .. W-1 (W = 1 .. 4) own the rows: thread t keeps for its
+// Warps.  W owner warps (1 .. 4) own the rows: owner thread t keeps for its
 // rows t, t + 128, .. the value in column j (its candidate), the value in
 // column j+1 and the row id in registers, and every owner warp takes part in
 // the exchange by itself, so no block barrier lies on the column's chain:
 //   push of the warp's candidate (lanes = peers); wait; winner (every warp
-//   reduces all P W headers alike); reciprocal (an FP64 division is 366 cycles,
-//   the longest link); column j scaled and column j+1 updated in registers; the
-//   warp's next candidate; then, with the winner's segment, column j+2.
-// Warp W (helper) brings the candidates' rows up to date while their headers
-//   travel, arms the barriers, pushes the segment if this CTA won and records
-//   the pivot.
-// The other warps apply step j's update to columns j+3.. of the active rows
+//   reduces all P W headers alike); column j scaled and column j+1 updated in
+//   registers; the warp's next candidate; with the first piece of the winner's
+//   segment, the candidate's column j+2, then the push; the other rows' column
+//   j+2 while that is under way.
+// The divider (FP64) forms the candidates' reciprocals as soon as they are known
+// and adds them to their headers: a division is 340 cycles of dependent operations,
+// which on the winner's side of the exchange would be the longest link.
+// The helper brings the candidates' rows up to date while their headers
+//   travel, arms the barriers, pushes the segment if this CTA won (its first 16
+//   bytes, which hold column j+2, to all peers at once and on a barrier of its
+//   own) and records the pivot.
+// The bulk warps apply step j's update to columns j+3.. of the active rows
 // (all but the next candidates) one column behind: "column j scaled" and
 // "update of step j done" are named barriers, the second of which the owners
 // pass a column later.  FP64: the pipe of each quarter of an SM takes 64 cycles
 // a warp instruction, so the bulk update, not the exchange, bounds a panel of
 // many rows per CTA, and such panels are kept narrow.
+// What bounds a small panel is the length of that chain, some 1700 cycles a column
+// at one instruction every four cycles or so: no array of it is indexed by a
+// variable (such arrays live in local memory, whose lines the waits' acquire
+// discards), nor is there an integer division, and the waits' loops are out of line.
+// us a 64-column panel, before / now: FP64 75.6 / 61 at 64 rows, 77 / 64 at 256,
+// 82 / 71 at 512, 100 / 96 at 1024, 156 / 143 at 2048; FP32 61.4 / 59 at 64, 69 / 63
+// at 512, 73 / 68 at 1024, 91 / 92 at 2048.
 //
 // Reuse of the exchange buffers (two, by step parity): a warp pushes step j+2
 // only after it has every header of step j+1, and a warp sends that header only
@@ -53,12 +65,14 @@ constexpr int kClMaxCtas = 16;
 constexpr int kClSegPad = 4;
 constexpr int kClOwners = 4;  // owner warps at most
 constexpr int kClOwnRows = 32 * kClOwners;
-constexpr int kClMaxRows = 4 * kClOwnRows;  // rows of a CTA
-// 13 warps (FP64: two bulk warps or more for each FP64 pipe) or 20 (FP32,
-// bound by shared-memory latency).
+// FP64: 17 warps.  The owners (warps 0, 4, 8, 12) and the divider (4 W) have one
+// quarter of the SM to themselves, the helper (1) and eleven bulk warps the other
+// three: a bulk warp on the same FP64 pipe would make each of the dependent
+// operations of a column's chain wait for one or two of its own, 64 cycles each.
+// FP32: 20 warps (bound by shared-memory latency), owners 0 .. W-1, helper W.
 template <typename T>
 __host__ __device__ constexpr int cl_threads() {
-  return sizeof(T) == 8 ? 416 : 640;
+  return sizeof(T) == 8 ? 544 : 640;
 }
 // Odd row stride for FP64 (conflict-free column and row access); 16-byte rows
 // for FP32's float4 updates.
@@ -72,7 +86,8 @@ static size_t cl_smem_bytes(int rows_per, int w) {
          2 * (size_t)rows_per * sizeof(int);
 }
 
-// A CTA's header: 16 bytes (FP32: key | id, value) or 24 (FP64: key, id; value).
+// A warp's header: 16 bytes (FP32: key | id, value) or 32 (FP64: key, id; value;
+// reciprocal, pushed by the divider).
 template <typename T>
 struct ClHeader;
 template <>
@@ -83,25 +98,33 @@ struct ClHeader<float> {
   __device__ static void push(unsigned dst, unsigned bar, K key, int id, float u1) {
     cl_push16(dst, bar, key, ((unsigned long long)__float_as_uint(u1) << 32) | (unsigned)id);
   }
-  __device__ static void read(const unsigned long long* h, K& key, int& id, float& u1) {
-    key = (unsigned)h[0];
-    id = (int)(unsigned)h[1];
+  __device__ static void read_key(const unsigned long long* h, K& key, int& id) {
+    const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(h);
+    key = (unsigned)v.x;
+    id = (int)(unsigned)v.y;
+  }
+  __device__ static void read_value(const unsigned long long* h, float& u1, float&) {
     u1 = __uint_as_float((unsigned)(h[1] >> 32));
   }
 };
 template <>
 struct ClHeader<double> {
   using K = unsigned long long;
-  static constexpr unsigned kBytes = 24;
+  static constexpr unsigned kBytes = 32;
   static constexpr K kSign = 0x8000000000000000ull;
   __device__ static void push(unsigned dst, unsigned bar, K key, int id, double u1) {
     cl_push16(dst, bar, key, (unsigned)id);
     cl_push8(dst + 16, bar, (unsigned long long)__double_as_longlong(u1));
   }
-  __device__ static void read(const unsigned long long* h, K& key, int& id, double& u1) {
-    key = h[0];
-    id = (int)(unsigned)h[1];
-    u1 = __longlong_as_double((long long)h[2]);
+  __device__ static void read_key(const unsigned long long* h, K& key, int& id) {
+    const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(h);
+    key = v.x;
+    id = (int)(unsigned)v.y;
+  }
+  __device__ static void read_value(const unsigned long long* h, double& u1, double& recip) {
+    const double2 v = *reinterpret_cast<const double2*>(h + 2);
+    u1 = v.x;
+    recip = v.y;
   }
 };
 
@@ -112,42 +135,39 @@ __device__ __forceinline__ void cl_bar_arrive(int id, int threads) {
   asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
-// The winner among the n headers of one step (the same answer in every warp):
-// its index, row id, signed key and column j+1 value.  key 0: no pivot.
+// The winner among the n headers of one step (the same answer in every warp): its
+// index, row id, signed key (0: no pivot), column j+1 value and (FP64) reciprocal,
+// read from its header.
 template <typename T>
 __device__ __forceinline__ void cl_winner(const unsigned long long (*box)[4], int n, int lane, int& win, int& pr,
-                                          typename ClHeader<T>::K& kraw, T& u1) {
+                                          typename ClHeader<T>::K& kraw, T& u1, T& recip) {
   using H = ClHeader<T>;
   using K = typename H::K;
   K k = 0;
-  kraw = 0;
   pr = INT_MAX;
-  win = 0;
-  u1 = T(0);
+  win = lane;
   if (lane < n) {
-    H::read(box[lane], kraw, pr, u1);
-    k = kraw & ~H::kSign;
-    win = lane;
+    H::read_key(box[lane], k, pr);
+    k &= ~H::kSign;
   }
   if (lane + 32 < n) {
-    K hraw;
+    K hk;
     int hid;
-    T hu;
-    H::read(box[lane + 32], hraw, hid, hu);
-    const K hk = hraw & ~H::kSign;
+    H::read_key(box[lane + 32], hk, hid);
+    hk &= ~H::kSign;
     if (hk > k || (hk == k && hid < pr)) {
       k = hk;
-      kraw = hraw;
       pr = hid;
       win = lane + 32;
-      u1 = hu;
     }
   }
   const int src = warp_best(k, pr);
-  win = __shfl_sync(0xffffffffu, win, src);
-  pr = __shfl_sync(0xffffffffu, pr, src);
-  kraw = __shfl_sync(0xffffffffu, kraw, src);
-  u1 = __shfl_sync(0xffffffffu, u1, src);
+  if (n > 32)
+    win = __shfl_sync(0xffffffffu, win, src);
+  else
+    win = src;
+  H::read_key(box[win], kraw, pr);
+  H::read_value(box[win], u1, recip);
 }
 
 // S[r][c] -= S[r][jj] u[c] for the rows r of [0, n) that are active after step
@@ -258,7 +278,8 @@ __global__ void __launch_bounds__(cl_threads<T>(), 1) panel_cluster_kernel(Panel
   using H = ClHeader<T>;
   using K = typename H::K;
   constexpr unsigned kFull = 0xffffffffu;
-  constexpr int kThreads = cl_threads<T>();
+  constexpr int kThreads = cl_threads<T>(), kOwnRows = kClOwnRows;
+  constexpr bool kDivider = sizeof(T) == 8;
   constexpr int kWarps = kThreads / 32;
   constexpr int kVec = 16 / (int)sizeof(T);  // elements of one pushed piece
   constexpr int kSeg = kMaxPanelWidth + kClSegPad;
@@ -269,10 +290,12 @@ __global__ void __launch_bounds__(cl_threads<T>(), 1) panel_cluster_kernel(Panel
   int* ids = reinterpret_cast<int*>(segb + 2 * kSeg);     // final global row of each slot
   int* ret = ids + p.rows_per;                            // step in which a slot's row retired
   __shared__ __align__(16) unsigned long long box[2][kClMaxCtas * kClOwners][4];  // every warp's header
-  __shared__ __align__(8) unsigned long long hbar[2], sbar[2];
-  // The owner warps' next candidates: slot and the multiplier of the last step.
+  // Headers; the winner's segment, its first 16 bytes apart: column j+2 is on the
+  // next column's chain.
+  __shared__ __align__(8) unsigned long long hbar[2], ebar[2], sbar[2];
+  // The owner warps' next candidates.
   __shared__ __align__(16) int s_cand[2][kClOwners];
-  __shared__ T s_mult[2][kClOwners];
+  __shared__ T s_mult[2][kClOwners], s_val[2][kClOwners];  // its multiplier in the last step; its pivot
   __shared__ int s_pivoted[2], s_ok;
 
   const int P = gridDim.x, b = blockIdx.x;
@@ -280,19 +303,35 @@ __global__ void __launch_bounds__(cl_threads<T>(), 1) panel_cluster_kernel(Panel
   const int r_begin = p.k0 + b * p.rows_per;
   const int nloc = max(0, min(p.m, r_begin + p.rows_per) - r_begin);
   const int w = p.w, lds = p.lds;
-  const int W = (min(p.rows_per, kClOwnRows) + 31) / 32;  // owner warps, the same in every CTA
+  const int W = (min(p.rows_per, kOwnRows) + 31) / 32;  // owner warps, the same in every CTA
+  // Roles.  The barriers "scaled" (all of them) and "done" (but the divider).
+  enum { kOwner, kHelper, kDivide, kBulk, kIdle };
+  int role, index = 0;  // of an owner or bulk warp
+  if (kDivider) {
+    index = (warp & 3) == 0 ? warp >> 2 : (warp >> 2) * 3 + (warp & 3) - 2;
+    role = warp == 1 ? kHelper : (warp & 3) != 0 ? kBulk : index < W ? kOwner : index == W ? kDivide : kIdle;
+  } else {
+    index = warp < W ? warp : warp - W - 1;
+    role = warp < W ? kOwner : warp == W ? kHelper : kBulk;
+  }
+  const int bulk_threads = kDivider ? 11 * 32 : kThreads - 32 * (W + 1);
+  const int n_done = 32 * (W + 1) + bulk_threads, n_scaled = n_done + (kDivider ? 32 : 0);
 
   if (tid == 0) {
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(cl_smem(&hbar[i])));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(cl_smem(&ebar[i])));
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(cl_smem(&sbar[i])));
     }
     asm volatile("fence.mbarrier_init.release.cluster;");
     s_ok = 1;
     if (b == 0) *p.move_count = 0;
   }
-  if (tid < 2 * kClOwners) s_cand[tid / kClOwners][tid % kClOwners] = -1;
+  if (tid < 2 * kClOwners) {
+    s_cand[tid / kClOwners][tid % kClOwners] = -1;
+    s_val[tid / kClOwners][tid % kClOwners] = T(1);
+  }
   for (int r = warp; r < nloc; r += kWarps) {
     const T* src = p.a + (int64_t)(r_begin + r) * p.lda + p.k0;
     for (int c = lane; c < w; c += 32) S[r * lds + c] = src[c];
@@ -300,82 +339,90 @@ __global__ void __launch_bounds__(cl_threads<T>(), 1) panel_cluster_kernel(Panel
   for (int r = tid; r < nloc; r += kThreads) ret[r] = INT_MAX;
   cl_sync();  // barriers initialised everywhere, move_count cleared, this CTA's rows loaded
 
-  if (warp < W) {
+  if (role == kOwner) {
     // ------------------------------------------------------------- owners
+    const int ot = 32 * index + lane;
     T a[kNR], c1[kNR], lv[kNR];  // column j, column j+1, multiplier of the last step
     int id[kNR];                 // global row, -1: none or retired
 #pragma unroll
     for (int i = 0; i < kNR; ++i) {
-      const int r = tid + kClOwnRows * i;
+      const int r = ot + kOwnRows * i;
       const bool on = r < nloc;
       id[i] = on ? r_begin + r : -1;
       a[i] = on ? S[r * lds] : T(0);
       c1[i] = on && w > 1 ? S[r * lds + 1] : T(0);
       lv[i] = T(0);
     }
-    // This lane's places in the peer of its number (lanes below P).
-    unsigned peer_box[2], peer_bar[2];
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      peer_box[q] = cl_peer(cl_smem(&box[q][b * W + warp][0]), min(lane, P - 1));
-      peer_bar[q] = cl_peer(cl_smem(&hbar[q]), min(lane, P - 1));
-    }
+    // This lane's places in the peer of its number (lanes below P), step parity 0.
+    const unsigned peer_box = cl_peer(cl_smem(&box[0][b * W + index][0]), min(lane, P - 1));
+    const unsigned peer_bar = cl_peer(cl_smem(&hbar[0]), min(lane, P - 1));
     K ck = 0;          // the warp's candidate: key with the pivot's sign,
     int cid = 0;       // row id,
+    int cslot = -1;    // slot,
+    T cl = T(0);       // multiplier of the last step,
     T cu = T(0);       // column j+1 value
-    int bi = 0, src = 0;  // this lane's best row; the candidate's lane
-    auto pick = [&](const T(&v)[kNR]) {
-      T x = v[0];
-#pragma unroll
-      for (int i = 1; i < kNR; ++i)
-        if (bi == i) x = v[i];
-      return x;
-    };
     auto candidate = [&](int par) {
       K bk = 0;
-      int bid = INT_MAX;
-      bi = -1;
+      int bid = INT_MAX, bslot = -1;
+      T bv = T(1), bl = T(0);
 #pragma unroll
       for (int i = 0; i < kNR; ++i) {
         const K k = PivotKey<T>::of(a[i]);
-        if (id[i] >= 0 && (bi < 0 || k > bk || (k == bk && id[i] < bid))) {
+        if (id[i] >= 0 && (bslot < 0 || k > bk || (k == bk && id[i] < bid))) {
           bk = k;
           bid = id[i];
-          bi = i;
+          bslot = ot + kOwnRows * i;
+          bv = a[i];
+          bl = lv[i];
         }
       }
-      src = warp_best(bk, bid);
-      ck = __shfl_sync(kFull, bk | (bi >= 0 && signbit(pick(a)) ? H::kSign : K(0)), src);
+      const int src = warp_best(bk, bid);
+      ck = __shfl_sync(kFull, bslot >= 0 && signbit(bv) ? bk | H::kSign : bk, src);
       cid = __shfl_sync(kFull, bid, src);
+      cslot = __shfl_sync(kFull, bslot, src);
+      cl = __shfl_sync(kFull, bl, src);
       if (lane == src) {
-        s_cand[par][warp] = bi >= 0 ? tid + kClOwnRows * bi : -1;
-        s_mult[par][warp] = pick(lv);
+        s_cand[par][index] = bslot;
+        s_mult[par][index] = bl;
+        s_val[par][index] = bv;
       }
     };
     candidate(1);
-    cu = __shfl_sync(kFull, pick(c1), src);
+    cu = cslot >= 0 && w > 1 ? S[cslot * lds + 1] : T(0);
     __syncwarp();
-    cl_bar_sync(kBarScaled, kThreads);
-    unsigned seg_phase[2] = {0u, 0u};  // phase of each segment barrier's next use
+    cl_bar_sync(kBarScaled, n_scaled);
+    unsigned seg_phase = 0u;  // bit q: phase of segment barrier q's next use (an array would live in local memory)
     bool ok = true;
+    bool was_pivot = false;  // the last step had a pivot; un: its row's next element
+    T un = T(0);
     for (int j = 0; j < w; ++j) {
       const int ul = p.k0 + j;
       const int par = j & 1;
-      if (ok && lane < P) H::push(peer_box[par], peer_bar[par], ck, cid, cu);
+      if (ok && lane < P) H::push(peer_box + (unsigned)par * (unsigned)sizeof(box[0]), peer_bar + 8u * (unsigned)par, ck, cid, cu);
+      if (j > 0 && j + 1 < w) {
+        // While the headers travel: column j+1 of this thread's rows (the
+        // candidate's went with the header).
+#pragma unroll
+        for (int i = 0; i < kNR; ++i) {
+          if (id[i] < 0) continue;
+          const T x = S[(ot + kOwnRows * i) * lds + j + 1];
+          c1[i] = was_pivot ? upd<kExact>(x, lv[i], un) : x;
+        }
+      }
       ok = ok && cl_wait(cl_smem(&hbar[par]), (unsigned)((j >> 1) & 1), p.st, ul);
       int win, pr;
       K kraw;
-      T u1;
-      cl_winner<T>(box[par], P * W, lane, win, pr, kraw, u1);
+      T u1, recip;
+      cl_winner<T>(box[par], P * W, lane, win, pr, kraw, u1, recip);
       const bool pivot = ok && (kraw & ~H::kSign) > 0;
       if (!pivot) pr = ul;
-      const T recip = T(1) / PivotKey<T>::value(kraw);
+      if constexpr (!kDivider) recip = T(1) / PivotKey<T>::value(kraw);
       // The row with id pr takes id ul and retires, the row with id ul takes
       // id pr; the other rows' column j is scaled and column j+1 updated.
 #pragma unroll
       for (int i = 0; i < kNR; ++i) {
         if (id[i] < 0) continue;
-        const int r = tid + kClOwnRows * i;
+        const int r = ot + kOwnRows * i;
         T* row = S + r * lds + j;
         if (id[i] == pr) {
           row[0] = a[i];
@@ -401,39 +448,37 @@ __global__ void __launch_bounds__(cl_threads<T>(), 1) panel_cluster_kernel(Panel
       // The helper passes "done" of step j-1 after "scaled" of step j, so the
       // owners never arrive twice at one "scaled"; the first one they wait for.
       if (j > 0) {
-        cl_bar_arrive(kBarScaled, kThreads);
-        cl_bar_sync(kBarDone + ((j - 1) & 1), kThreads);
+        cl_bar_arrive(kBarScaled, n_scaled);
+        cl_bar_sync(kBarDone + ((j - 1) & 1), n_done);
       } else {
-        cl_bar_sync(kBarScaled, kThreads);
+        cl_bar_sync(kBarScaled, n_scaled);
       }
       if (j + 2 < w) {
         // Column j+2 of this thread's rows: step j-1's update is in (the
         // barrier), step j's with the winner's segment.
         if (pivot) {
-          ok = ok && cl_wait(cl_smem(&sbar[par]), seg_phase[par], p.st, ul);
-          seg_phase[par] ^= 1u;
+          ok = ok && cl_wait(cl_smem(&ebar[par]), (seg_phase >> par) & 1u, p.st, ul);
+          seg_phase ^= 1u << par;
         }
-        const T u2 = segb[par * kSeg + j + 2];
-#pragma unroll
-        for (int i = 0; i < kNR; ++i) {
-          if (id[i] < 0) continue;
-          const T x = S[(tid + kClOwnRows * i) * lds + j + 2];
-          c1[i] = pivot ? upd<kExact>(x, lv[i], u2) : x;
+        un = segb[par * kSeg + j + 2];
+        if (cslot >= 0) {
+          const T x = S[cslot * lds + j + 2];
+          cu = pivot ? upd<kExact>(x, cl, un) : x;
         }
-        cu = __shfl_sync(kFull, pick(c1), src);
       }
+      was_pivot = pivot;
     }
 #pragma unroll
     for (int i = 0; i < kNR; ++i)
-      if (id[i] >= 0) ids[tid + kClOwnRows * i] = id[i];
+      if (id[i] >= 0) ids[ot + kOwnRows * i] = id[i];
     if (!ok && lane == 0) s_ok = 0;
-  } else if (warp == W) {
+  } else if (role == kHelper) {
     // ------------------------------------------------------------- helper
-    unsigned seg_phase[2] = {0u, 0u};
+    unsigned seg_phase = 0u;
     bool ok = true;
     int dj = -1;  // step whose update of the candidates' rows is pending
     if (lane == 0) cl_expect(cl_smem(&hbar[0]), (unsigned)(P * W) * H::kBytes);
-    cl_bar_sync(kBarScaled, kThreads);
+    cl_bar_sync(kBarScaled, n_scaled);
     for (int j = 0; j < w; ++j) {
       const int ul = p.k0 + j;
       const int par = j & 1;
@@ -442,8 +487,9 @@ __global__ void __launch_bounds__(cl_threads<T>(), 1) panel_cluster_kernel(Panel
         // Columns j+2.. of the candidates' rows (the owners hold j and j+1):
         // step j-1's update, once step j-2's is in (barrier of the last pass).
         const int sp = dj & 1;
-        ok = ok && cl_wait(cl_smem(&sbar[sp]), seg_phase[sp], p.st, ul);
-        seg_phase[sp] ^= 1u;
+        ok = ok && cl_wait(cl_smem(&ebar[sp]), (seg_phase >> sp) & 1u, p.st, ul) &&
+             cl_wait(cl_smem(&sbar[sp]), (seg_phase >> sp) & 1u, p.st, ul);
+        seg_phase ^= 1u << sp;
         const T* up = segb + sp * kSeg;
         for (int q = 0; q < W; ++q) {
           const int cs = cand[q];
@@ -457,20 +503,19 @@ __global__ void __launch_bounds__(cl_threads<T>(), 1) panel_cluster_kernel(Panel
       ok = ok && cl_wait(cl_smem(&hbar[par]), (unsigned)((j >> 1) & 1), p.st, ul);
       int win, pr;
       K kraw;
-      T u1;
-      cl_winner<T>(box[par], P * W, lane, win, pr, kraw, u1);
+      T u1, recip;
+      cl_winner<T>(box[par], P * W, lane, win, pr, kraw, u1, recip);
       const bool pivot = ok && (kraw & ~H::kSign) > 0;
       if (pivot && j + 2 < w) {
-        // The winner's segment j+2.. in 16-byte pieces, from an aligned column on.
-        const unsigned sb = cl_smem(&sbar[par]);
+        // The winner's segment j+2.. in 16-byte pieces, from an aligned column on;
+        // the first one to all peers at once.
+        const unsigned sb = cl_smem(&sbar[par]), eb = cl_smem(&ebar[par]);
         const int c0 = (j + 2) & ~(kVec - 1);
         const int pieces = (w - c0 + kVec - 1) / kVec;
-        if (win / W == b) {
+        if ((unsigned)(win - b * W) < (unsigned)W) {
           const T* row = S + cand[win - b * W] * lds;
           const unsigned dst = cl_smem(segb + par * kSeg);
-          for (int q = lane; q < pieces; q += 32) {
-            unsigned long long v[2];
-            const int c = c0 + q * kVec;
+          auto piece = [&](int c, unsigned long long(&v)[2]) {
             if constexpr (sizeof(T) == 8) {
               v[0] = (unsigned long long)__double_as_longlong(row[c]);
               v[1] = (unsigned long long)__double_as_longlong(row[c + 1]);
@@ -479,11 +524,23 @@ __global__ void __launch_bounds__(cl_threads<T>(), 1) panel_cluster_kernel(Panel
               v[0] = ((unsigned long long)x.y << 32) | x.x;
               v[1] = ((unsigned long long)x.w << 32) | x.z;
             }
+          };
+          unsigned long long v[2];
+          if (lane < P) {
+            piece(c0, v);
+            cl_push16(cl_peer(dst + (unsigned)c0 * (unsigned)sizeof(T), lane), cl_peer(eb, lane), v[0], v[1]);
+          }
+          for (int q = 1 + lane; q < pieces; q += 32) {
+            const int c = c0 + q * kVec;
+            piece(c, v);
             for (int cta = 0; cta < P; ++cta)
               cl_push16(cl_peer(dst + (unsigned)c * (unsigned)sizeof(T), cta), cl_peer(sb, cta), v[0], v[1]);
           }
         }
-        if (lane == 0) cl_expect(sb, (unsigned)pieces * 16u);
+        if (lane == 0) {
+          cl_expect(eb, 16u);
+          cl_expect(sb, (unsigned)(pieces - 1) * 16u);
+        }
       }
       if (lane == 0) {
         // Every header of step j is here, so the other barrier's phase of step
@@ -499,28 +556,50 @@ __global__ void __launch_bounds__(cl_threads<T>(), 1) panel_cluster_kernel(Panel
       }
       dj = pivot ? j : -1;
       __syncwarp();
-      cl_bar_sync(kBarScaled, kThreads);
-      if (j > 0) cl_bar_sync(kBarDone + ((j - 1) & 1), kThreads);
+      cl_bar_sync(kBarScaled, n_scaled);
+      if (j > 0) cl_bar_sync(kBarDone + ((j - 1) & 1), n_done);
     }
     if (!ok && lane == 0) s_ok = 0;
-  } else {
+  } else if (role == kDivide) {
+    // ------------------------------------------------------------ divider
+    // The candidates' reciprocals, while their headers are still being prepared.
+    // A division is some 430 cycles of dependent operations: on the winner's
+    // side of the exchange it would be the longest link of the chain.
+    if constexpr (kDivider) {
+      // Lane (q, cta) pushes candidate q's (and q + 2's) to peer cta.
+      const int cta = lane & (kClMaxCtas - 1), q0 = lane / kClMaxCtas;
+      const unsigned dst = cl_peer(cl_smem(&box[0][b * W + min(q0, W - 1)][3]), min(cta, P - 1));
+      const unsigned bar = cl_peer(cl_smem(&hbar[0]), min(cta, P - 1));
+      for (int j = -1; j < w; ++j) {
+        cl_bar_sync(kBarScaled, n_scaled);  // the candidates for step j+1 are known
+        if (j + 1 >= w) break;
+        const int par = j & 1, nxt = par ^ 1;
+        const unsigned to = dst + (unsigned)nxt * (unsigned)sizeof(box[0]), on = bar + 8u * (unsigned)nxt;
+        if (cta < P && q0 < W)
+          cl_push8(to, on, (unsigned long long)__double_as_longlong(1.0 / (double)s_val[par][q0]));
+        if (cta < P && q0 + 2 < W)
+          cl_push8(to + 2u * (unsigned)sizeof(box[0][0]), on,
+                   (unsigned long long)__double_as_longlong(1.0 / (double)s_val[par][q0 + 2]));
+      }
+    }
+  } else if (role == kBulk) {
     // ------------------------------------------------------------- bulk
-    unsigned seg_phase[2] = {0u, 0u};
+    unsigned seg_phase = 0u;
     bool ok = true;
-    cl_bar_sync(kBarScaled, kThreads);
+    cl_bar_sync(kBarScaled, n_scaled);
     for (int j = 0; j < w; ++j) {
       const int par = j & 1;
-      cl_bar_sync(kBarScaled, kThreads);
+      cl_bar_sync(kBarScaled, n_scaled);
       if (s_pivoted[par] && j + 3 < w) {
         const int4 cand = *reinterpret_cast<const int4*>(s_cand[par]);
-        ok = ok && cl_wait(cl_smem(&sbar[par]), seg_phase[par], p.st, p.k0 + j);
-        seg_phase[par] ^= 1u;
+        ok = ok && cl_wait(cl_smem(&ebar[par]), (seg_phase >> par) & 1u, p.st, p.k0 + j) &&
+             cl_wait(cl_smem(&sbar[par]), (seg_phase >> par) & 1u, p.st, p.k0 + j);
+        seg_phase ^= 1u << par;
         if (ok)
-          cl_update<kExact>(S, lds, ret, nloc, cand, j, j + 3, w, segb + par * kSeg, tid - 32 * (W + 1),
-                            kThreads - 32 * (W + 1));
+          cl_update<kExact>(S, lds, ret, nloc, cand, j, j + 3, w, segb + par * kSeg, index * 32 + lane, bulk_threads);
       }
       __syncwarp();
-      if (j + 1 < w) cl_bar_arrive(kBarDone + par, kThreads);
+      if (j + 1 < w) cl_bar_arrive(kBarDone + par, n_done);
     }
     if (!ok && lane == 0) s_ok = 0;
   }
@@ -586,12 +665,12 @@ int panel_cluster_limit(luhot_ctx* ctx) {
 
 // Rows of a CTA up to which the cluster is the faster form.  us per column of a
 // 64-column panel, cluster of 16 against the exchange through L2 on up to 96
-// (FP64) or 64 (FP32) CTAs: FP64 1.2 / 2.5 at 512 rows, 1.6 / 2.5 at 1024, 2.4 /
-// 2.6 at 2048, 3.9 / 2.8 at 4096 (the rank-1 updates of 256 rows fill one SM's
-// FP64 pipes); FP32 1.1 / 2.3 at 1024, 1.4 / 2.3 at 2048, 1.6 / 2.4 at 4096,
-// 2.5 / 2.4 at 8192.
-constexpr int kClRowsF64 = 128, kClRowsF32 = 384;
-static_assert(kClRowsF64 <= kClMaxRows && kClRowsF32 <= kClMaxRows, "an owner thread holds at most four rows");
+// (FP64) or 64 (FP32) CTAs: FP64 1.1 / 2.5 at 512 rows, 1.5 / 2.5 at 1024, 2.2 /
+// 2.6 at 2048, 2.7 / 2.9 at 2560, 3.0 / 3.0 at 3072, 3.6 / 3.0 at 4096 (the rank-1
+// updates of 256 rows fill one SM's FP64 pipes); FP32 1.1 / 2.3 at 1024, 1.4 / 2.3
+// at 2048, 1.7 / 2.4 at 4096, 2.5 / 2.4 at 8192.
+constexpr int kClRowsF64 = 160, kClRowsF32 = 384;
+static_assert(kClRowsF64 <= 4 * kClOwnRows && kClRowsF32 <= 4 * kClOwnRows, "an owner thread holds at most four rows");
 
 template <typename T>
 bool panel_cluster_fits(luhot_ctx* ctx, int rows, int w) {
