@@ -44,7 +44,8 @@ namespace luhot {
 // ---------------------------------------------------------------------------
 // 1. Panel factorization.
 // ---------------------------------------------------------------------------
-// Exchange words: payload in the low 32 bits, the step tag in the high 32.
+// Exchange words: payload in the low 32 bits, the step tag in the high 32 (headers:
+// 48 bits and 16).
 // A reader accepts a word only when its tag is the step it waits for, so no
 // fence or counter orders the writers and readers: each 8-byte word is
 // written and read whole.  Tags are step + 1 and the slots are zeroed before
@@ -68,13 +69,23 @@ __device__ __forceinline__ void st_word(unsigned long long* p, unsigned int bits
 __device__ __forceinline__ bool word_ok(unsigned long long v, unsigned int tag) {
   return (unsigned int)(v >> 32) == tag;
 }
-// Four words (one 32-byte L2 sector) in one load; each 8-byte element is
-// read whole.  p 32-byte aligned.
-__device__ __forceinline__ void ld_quad(const unsigned long long* p, unsigned long long* v) {
+// A whole header (FP64 32 bytes, FP32 16) in one load or store; each 8-byte
+// element is read and written whole.  p aligned to the header.
+__device__ __forceinline__ void ld_head(const unsigned long long* p, unsigned long long (&v)[4]) {
   asm volatile("ld.relaxed.gpu.global.v4.u64 {%0, %1, %2, %3}, [%4];"
                : "=l"(v[0]), "=l"(v[1]), "=l"(v[2]), "=l"(v[3])
                : "l"(p)
                : "memory");
+}
+__device__ __forceinline__ void ld_head(const unsigned long long* p, unsigned long long (&v)[2]) {
+  asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(v[0]), "=l"(v[1]) : "l"(p) : "memory");
+}
+__device__ __forceinline__ void st_head(unsigned long long* p, const unsigned long long (&v)[4]) {
+  asm volatile("st.relaxed.gpu.global.v4.u64 [%0], {%1, %2, %3, %4};" ::"l"(p), "l"(v[0]), "l"(v[1]), "l"(v[2]), "l"(v[3])
+               : "memory");
+}
+__device__ __forceinline__ void st_head(unsigned long long* p, const unsigned long long (&v)[2]) {
+  asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(v[0]), "l"(v[1]) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
@@ -85,44 +96,68 @@ __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src)
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(gmem_src) : "memory");
 }
 
-// Values and keys as one (FP32) or two (FP64) tagged words.  The header of
-// a CTA's slot holds its candidate's key with the pivot's sign in the top
-// bit (so the key word also gives the pivot value), the row id, and the
-// candidate's column j+1 value: words [0, 4 * kHdrQuads), whole 32-byte
-// sectors of the slot (slots are 32-byte aligned).
+// Segment values as one (FP32) or two (FP64) tagged words.  The header of a
+// CTA holds its candidate's key with the pivot's sign in the top bit (so the key
+// also gives the pivot value), the row id and the candidate's column j+1 value,
+// 96 (FP32) or 160 bits, in kHead words of 48 bits over a 16-bit tag (the step's
+// low bits; a header is rewritten at every second step, so that an old tag is
+// never 65536 steps old).  The headers of all CTAs are contiguous: a warp's poll of
+// 64 CTAs reads 16 lines of 128 bytes (FP32: 8) and has every load in flight
+// at once, an L2 latency (some 850 cycles across the dies) a poll.
 template <typename T>
 struct Tagged;
 template <>
 struct Tagged<float> {
   using K = unsigned int;
-  static constexpr int kWords = 1;
-  static constexpr int kIdW = 1, kU1W = 2, kHdrQuads = 1;
+  static constexpr int kWords = 1, kHead = 2;
   static constexpr K kSign = 0x80000000u;
   __device__ static void put(unsigned long long* p, float v, unsigned int tag) { st_word(p, __float_as_uint(v), tag); }
-  __device__ static void put_key(unsigned long long* p, K k, unsigned int tag) { st_word(p, k, tag); }
-  __device__ static K bits(const unsigned long long* w) { return (unsigned int)w[0]; }
   __device__ static float value(const unsigned long long* w) { return __uint_as_float((unsigned int)w[0]); }
   __device__ static bool ok(const unsigned long long* w, unsigned int tag) { return word_ok(w[0], tag); }
+  __device__ static void pack(K key, int id, float u1, unsigned int tag, unsigned long long (&h)[2]) {
+    const unsigned int u = __float_as_uint(u1), t = tag & 0xffffu;
+    h[0] = ((unsigned long long)key << 32) | (u & 0xffff0000u) | t;
+    h[1] = ((unsigned long long)(unsigned int)id << 32) | (u << 16) | t;
+  }
+  __device__ static bool head_ok(const unsigned long long (&h)[2], unsigned int tag) {
+    return (((h[0] ^ tag) | (h[1] ^ tag)) & 0xffffu) == 0;
+  }
+  __device__ static K key(const unsigned long long (&h)[2]) { return (K)(h[0] >> 32); }
+  __device__ static int id(const unsigned long long (&h)[2]) { return (int)(h[1] >> 32); }
+  __device__ static float u1(const unsigned long long (&h)[2]) {
+    return __uint_as_float(((unsigned int)h[0] & 0xffff0000u) | ((unsigned int)h[1] >> 16));
+  }
 };
 template <>
 struct Tagged<double> {
   using K = unsigned long long;
-  static constexpr int kWords = 2;
-  static constexpr int kIdW = 2, kU1W = 3, kHdrQuads = 2;
+  static constexpr int kWords = 2, kHead = 4;
   static constexpr K kSign = 0x8000000000000000ull;
-  __device__ static void put_key(unsigned long long* p, K k, unsigned int tag) {
+  __device__ static void put(unsigned long long* p, double v, unsigned int tag) {
+    const K k = (K)__double_as_longlong(v);
     st_word(p, (unsigned int)(k >> 32), tag);
     st_word(p + 1, (unsigned int)k, tag);
   }
-  __device__ static void put(unsigned long long* p, double v, unsigned int tag) {
-    put_key(p, (unsigned long long)__double_as_longlong(v), tag);
+  __device__ static double value(const unsigned long long* w) {
+    return __longlong_as_double((long long)(((K)(unsigned int)w[0] << 32) | (unsigned int)w[1]));
   }
-  __device__ static K bits(const unsigned long long* w) {
-    return ((unsigned long long)(unsigned int)w[0] << 32) | (unsigned int)w[1];
-  }
-  __device__ static double value(const unsigned long long* w) { return __longlong_as_double((long long)bits(w)); }
   __device__ static bool ok(const unsigned long long* w, unsigned int tag) {
     return word_ok(w[0], tag) && word_ok(w[1], tag);
+  }
+  __device__ static void pack(K key, int id, double u1, unsigned int tag, unsigned long long (&h)[4]) {
+    const K u = (K)__double_as_longlong(u1), t = tag & 0xffffu;
+    h[0] = (key & ~(K)0xffff) | t;
+    h[1] = (key << 48) | ((K)(unsigned int)id << 16) | t;
+    h[2] = (u & ~(K)0xffff) | t;
+    h[3] = (u << 48) | t;
+  }
+  __device__ static bool head_ok(const unsigned long long (&h)[4], unsigned int tag) {
+    return (((h[0] ^ tag) | (h[1] ^ tag) | (h[2] ^ tag) | (h[3] ^ tag)) & 0xffffu) == 0;
+  }
+  __device__ static K key(const unsigned long long (&h)[4]) { return (h[0] & ~(K)0xffff) | (h[1] >> 48); }
+  __device__ static int id(const unsigned long long (&h)[4]) { return (int)(unsigned int)(h[1] >> 16); }
+  __device__ static double u1(const unsigned long long (&h)[4]) {
+    return __longlong_as_double((long long)((h[2] & ~(K)0xffff) | (h[3] >> 48)));
   }
 };
 
@@ -244,19 +279,25 @@ __device__ __forceinline__ void panel_update(T* S, int lds, int r0, int nloc, in
 // to columns j+1.. still pending for all rows but this CTA's candidate row:
 //   warp 0:     publish the candidate's header (key = |pivot| bits with the
 //               pivot's sign on top, row id, column j+1 value after the
-//               pending update) as tagged words; poll the P headers until all
+//               pending update) in one store; poll the P headers until all
 //               carry this step's tag, folding them into the winner (the
-//               pivot and its column j+1 value come with its header); start
-//               the copy of the winner's segment into shared memory
-//               (cp.async); relabel the ids of rows ul and pr.
+//               pivot and its column j+1 value come with its header); pass the
+//               winner to warp 1 and form the reciprocal;
 //   warp 1:     meanwhile, the candidate row's pending update (columns
-//               j+2..) and the publication of its segment j+2..;
+//               j+2..) and the publication of its segment j+2..; once the winner
+//               is known, start the copy of its segment into shared memory
+//               (cp.async) and relabel the ids of rows ul and pr;
 //   warps 1-:   the pending update of step j-1 of the other rows (columns
 //               j+1..), which thus overlaps the exchange.
-//   barrier;    the pivot row's CTA retires it; warps 1- scale column j,
-//               update column j+1 only and find its candidates while warp 0
+//   barrier;    the pivot row's CTA retires it; the warps but 1 scale column j,
+//               update column j+1 only and find its candidates while warp 1
 //               checks the copied segment's tags and keeps it for the next
 //               step's updates; barrier.
+// What bounds it is that chain: some 2200 of a column's 5000 cycles are the header's
+// way through L2 and its polls, 500 an FP64 division, 800 the scaling and search.
+// us a 64-column panel, with 40- or 64-byte slots polled one after the other / now:
+// FP64 191 / 196 at 4096 rows, 212 / 195 at 6144, 217 / 200 at 8192, 256 / 229 at 16384;
+// FP32 170 / 160 at 8192, 177 / 170 at 16384.
 // The arithmetic and its order per element are those of lair's
 // getrf_row_major (src/lapack/getrf.rs:56-89): 1/p rounded, l = a*(1/p)
 // rounded, a - l*u (separately rounded in exact mode), steps in order.
@@ -274,11 +315,11 @@ __global__ void __launch_bounds__(512, 1) panel_kernel(PanelArgs<T> p) {
   __shared__ __align__(16) unsigned long long stage[2 * kMaxPanelWidth];  // the winner's segment words
   __shared__ int s_ok, s_r0, s_pivoted, s_ret;
   __shared__ T s_recip, s_u1;
+  __shared__ int s_pr, s_win;  // the step's pivot row and its CTA (-1: no pivot)
 
   constexpr unsigned kFull = 0xffffffffu;
-  const int kWarps = blockDim.x >> 5;  // 8 or 16
+  const int kWarps = blockDim.x >> 5;
   constexpr int kW = Tagged<T>::kWords;
-  constexpr int kHdr = kPanelHeaderWords;
   const int P = gridDim.x;
   const int b = blockIdx.x;
   const int tid = threadIdx.x;
@@ -328,120 +369,102 @@ __global__ void __launch_bounds__(512, 1) panel_kernel(PanelArgs<T> p) {
     K ck = lane < kWarps ? red_k[lane] : K(0);
     int ci = lane < kWarps ? red_i[lane] : INT_MAX;
     int cs = lane < kWarps ? red_s[lane] : -1;
-    key_reduce_redux(ck, ci, cs);
-    bool seg_live = false;  // the winner's segment j+2.. is being copied into stage
+    const int csrc = warp_best(ck, ci);
+    ck = PivotKey<T>::shfl(ck, csrc);
+    ci = __shfl_sync(kFull, ci, csrc);
+    cs = __shfl_sync(kFull, cs, csrc);
+    bool seg_live = false;  // warp 1: the winner's segment j+2.. is being copied into stage
     const unsigned long long* wseg = nullptr;
-    unsigned long long t0 = 0;
     if (warp == 0) {
-      unsigned long long* mine = slots + (size_t)b * kPanelSlotWords;
+      const unsigned long long* heads = p.heads + (size_t)(j & 1) * kMaxPanelCtas * kPanelHeaderWords;
       const T* up = segb + (dj & 1) * kMaxPanelWidth;  // step dj's pivot row
       // The header only (warp 1 publishes the segment): the column j+1 value
-      // after the pending update (kept in the row), the row id, then the key
+      // after the pending update (kept in the row), the row id and the key
       // with the pivot's sign.
-      if (lane == 0) {
+      {
         K sgn = 0;
+        T u1 = T(0);
         if (cs >= 0) {
+          const T* row = S + cs * lds;
           if (j + 1 < w) {
-            T u1 = S[cs * lds + j + 1];
-            if (dj >= 0) {
-              u1 = upd<kExact>(u1, S[cs * lds + dj], up[j + 1]);
-              S[cs * lds + j + 1] = u1;
-            }
-            Tagged<T>::put(mine + Tagged<T>::kU1W, u1, tag);
+            u1 = row[j + 1];
+            if (dj >= 0) u1 = upd<kExact>(u1, row[dj], up[j + 1]);
           }
-          if (signbit(S[cs * lds + j])) sgn = Tagged<T>::kSign;
+          if (signbit(row[j])) sgn = Tagged<T>::kSign;
         }
-        st_word(mine + Tagged<T>::kIdW, (unsigned int)ci, tag);
-        Tagged<T>::put_key(mine, ck | sgn, tag);
+        __syncwarp();
+        if (lane == 0) {
+          unsigned long long h[Tagged<T>::kHead];
+          Tagged<T>::pack(ck | sgn, ci, u1, tag, h);
+          st_head(const_cast<unsigned long long*>(heads) + b * Tagged<T>::kHead, h);
+          if (cs >= 0 && j + 1 < w && dj >= 0) S[cs * lds + j + 1] = u1;
+        }
       }
-      // Poll every CTA's header (32-byte loads); fold each one in as soon as
-      // it is current.  A positive key comes with its column j+1 value.
+      // Poll every CTA's header; fold each one in as soon as it is current.
       K k = 0, kraw = 0;
       int i = INT_MAX, win = -1;
       T u1b = T(0);
       unsigned pending = 0;
       for (int q = 0; q < nq; ++q)
         if (lane + 32 * q < P) pending |= 1u << q;
-      t0 = global_timer_ns();
+      unsigned long long t0 = 0;
       unsigned int spins = 0;
       int ok = 1;
       while (true) {
-        for (int q = 0; q < nq; ++q) {
-          if (!(pending & (1u << q))) continue;
-          const int cta = lane + 32 * q;
-          const unsigned long long* h = slots + (size_t)cta * kPanelSlotWords;
-          unsigned long long hw[4 * Tagged<T>::kHdrQuads];
+        constexpr int kB = 3;  // loads in flight (96 CTAs)
+        for (int q0 = 0; q0 < nq; q0 += kB) {
+          unsigned long long h[kB][Tagged<T>::kHead];
 #pragma unroll
-          for (int v = 0; v < Tagged<T>::kHdrQuads; ++v) ld_quad(h + 4 * v, hw + 4 * v);
-          const K hraw = Tagged<T>::bits(hw);
-          const K hk = hraw & ~Tagged<T>::kSign;
-          if (Tagged<T>::ok(hw, tag) && word_ok(hw[Tagged<T>::kIdW], tag) &&
-              (hk == 0 || j + 1 >= w || Tagged<T>::ok(hw + Tagged<T>::kU1W, tag))) {
-            const int hid = (int)(unsigned int)hw[Tagged<T>::kIdW];
+          for (int e = 0; e < kB; ++e)
+            if (pending & (1u << (q0 + e))) ld_head(heads + (lane + 32 * (q0 + e)) * Tagged<T>::kHead, h[e]);
+#pragma unroll
+          for (int e = 0; e < kB; ++e) {
+            if (!(pending & (1u << (q0 + e))) || !Tagged<T>::head_ok(h[e], tag)) continue;
+            const K hraw = Tagged<T>::key(h[e]);
+            const K hk = hraw & ~Tagged<T>::kSign;
+            const int hid = Tagged<T>::id(h[e]);
             if (hk > k || (hk == k && hid < i)) {
               k = hk;
               i = hid;
-              win = cta;
+              win = lane + 32 * (q0 + e);
               kraw = hraw;
-              u1b = Tagged<T>::value(hw + Tagged<T>::kU1W);
+              u1b = Tagged<T>::u1(h[e]);
             }
-            pending &= ~(1u << q);
+            pending &= ~(1u << (q0 + e));
           }
         }
         if (__all_sync(kFull, pending == 0)) break;
-        if ((++spins & 15u) == 0 && panel_wait_over(p.st, t0)) {
-          if (lane == 0 && !ld_relaxed_i32(&p.st->abort)) panel_give_up(p.st, ul);
-          ok = 0;
-          break;
+        if ((++spins & 15u) == 0) {
+          if (spins == 16u) t0 = global_timer_ns();
+          if (panel_wait_over(p.st, t0)) {
+            if (lane == 0 && !ld_relaxed_i32(&p.st->abort)) panel_give_up(p.st, ul);
+            ok = 0;
+            break;
+          }
         }
       }
-      int ret = -1;
-      if (ok) {
-        const int src = key_reduce_redux(k, i, win);
-        const K praw = PivotKey<T>::shfl(kraw, src);
-        const T u1 = __shfl_sync(kFull, u1b, src);
-        const int pr = (k > 0) ? i : ul;
-        if (k > 0) {
-          // Start the copy of the winner's segment j+2.. (whole 16-byte
-          // pairs of its slot's words) into stage; it completes while the
-          // step goes on.
-          wseg = slots + (size_t)win * kPanelSlotWords + kHdr;
-          const int o0 = ((j + 2) * kW) & ~1, o1 = (w * kW + 1) & ~1;
-          seg_live = o1 > o0;
-          for (int o = o0 + 2 * lane; o < o1; o += 64) cp_async16(stage + o, wseg + o);
-          cp_async_commit();
-          if (lane == 0) {
-            s_recip = T(1) / PivotKey<T>::value(praw);
-            s_u1 = u1;
-          }
-        } else if (b == 0 && lane == 0) {
+      const int src = warp_best(k, i);
+      const K praw = PivotKey<T>::shfl(kraw, src);
+      const bool pos = (praw & ~Tagged<T>::kSign) != 0;
+      if (lane == src) {
+        s_win = ok && pos ? win : -1;
+        s_pr = pos ? i : ul;
+        s_u1 = u1b;
+        s_pivoted = pos ? 1 : 0;
+        s_ok = ok;
+      }
+      __syncwarp();
+      asm volatile("bar.arrive 1, 64;" ::: "memory");
+      if (lane == 0 && ok) {
+        if (pos)
+          s_recip = T(1) / PivotKey<T>::value(praw);
+        else if (b == 0)
           // lair: max == 0 -> the step is singular, no swap, no update
           // (src/lapack/getrf.rs:72-73).  The last such step wins.
           atomicMax(&p.st->singular, ul);
-        }
-        // Relabel: the row with id ul takes id pr and the row with id pr
-        // takes id ul; the latter (the pivot row) retires after the barrier.
-        // Row pr is the winning CTA's candidate (slot cs); row ul's slot
-        // comes from the map of the panel's pending row ids.
-        const int s_ul = ulslot[j];
-        ret = s_ul;
-        if (pr != ul) {
-          const int s_pr = (win == b) ? cs : -1;
-          if (lane == 0) {
-            if (s_ul >= 0) ids[s_ul] = pr;
-            if (s_pr >= 0) ids[s_pr] = ul;
-            if (pr < p.k0 + w) ulslot[pr - p.k0] = s_ul;
-          }
-          ret = s_pr;
-        }
-        if (b == 0 && lane == 0) p.piv[ul] = pr;
-        if (lane == 0) s_pivoted = k > 0 ? 1 : 0;
-      }
-      if (lane == 0) {
-        s_ok = ok;
-        s_ret = ret;
       }
     } else {
+      unsigned long long* slots = p.slots + (size_t)(j & 1) * kMaxPanelCtas * kPanelSlotWords;
       if (warp == 1 && cs >= 0) {
         // The candidate row's pending update of columns j+2.. (warp 0 did
         // column j+1), then its segment j+2.., while warp 0 polls.
@@ -452,11 +475,41 @@ __global__ void __launch_bounds__(512, 1) panel_kernel(PanelArgs<T> p) {
           for (int c = dj + 3 + lane; c < w; c += 32) S[cs * lds + c] = upd<kExact>(S[cs * lds + c], l, up[c]);
           __syncwarp();
         }
-        for (int c = j + 2 + lane; c < w; c += 32) Tagged<T>::put(mine + kHdr + c * kW, S[cs * lds + c], tag);
+        for (int c = j + 2 + lane; c < w; c += 32) Tagged<T>::put(mine + c * kW, S[cs * lds + c], tag);
       }
       if (dj >= 0)
         panel_update<T, kExact>(S, lds, dr0, nloc, cs, dj, dj + 2, w, segb + (dj & 1) * kMaxPanelWidth, tid - 32,
                                 blockDim.x - 32);
+      if (warp == 1) {
+        asm volatile("bar.sync 1, 64;" ::: "memory");  // warp 0 has the winner
+        const int win = s_win, pr = s_pr;
+        if (win >= 0) {
+          // Start the copy of the winner's segment j+2.. (whole 16-byte pairs of
+          // its slot's words) into stage; it completes while the step goes on.
+          wseg = slots + (size_t)win * kPanelSlotWords;
+          const int o0 = ((j + 2) * kW) & ~1, o1 = (w * kW + 1) & ~1;
+          seg_live = o1 > o0;
+          for (int o = o0 + 2 * lane; o < o1; o += 64) cp_async16(stage + o, wseg + o);
+          cp_async_commit();
+        }
+        // Relabel: the row with id ul takes id pr and the row with id pr
+        // takes id ul; the latter (the pivot row) retires after the barrier.
+        // Row pr is the winning CTA's candidate (slot cs); row ul's slot
+        // comes from the map of the panel's pending row ids.
+        if (s_ok && lane == 0) {
+          const int s_ul = ulslot[j];
+          int ret = s_ul;
+          if (pr != ul) {
+            const int s_pr_slot = (win == b) ? cs : -1;
+            if (s_ul >= 0) ids[s_ul] = pr;
+            if (s_pr_slot >= 0) ids[s_pr_slot] = ul;
+            if (pr < p.k0 + w) ulslot[pr - p.k0] = s_ul;
+            ret = s_pr_slot;
+          }
+          if (b == 0) p.piv[ul] = pr;
+          s_ret = ret;
+        }
+      }
     }
     __syncthreads();
     if (!s_ok) return;
@@ -486,21 +539,23 @@ __global__ void __launch_bounds__(512, 1) panel_kernel(PanelArgs<T> p) {
       if (tid == 0) s_r0 = r0;
     }
 
-    // Warps 1-: scale column j, update column j+1 only, find its candidates.
-    // Warp 0 meanwhile keeps the winner's segment for the next step.
+    // Warps 0, 2-: scale column j, update column j+1 only, find its candidates.
+    // Warp 1 meanwhile keeps the winner's segment for the next step.
     K bk = 0;
     int bi = INT_MAX, bs = -1;
     const int pivoted = s_pivoted;
-    if (warp != 0) {
-      const int t1 = tid - 32, n1 = blockDim.x - 32;
+    if (warp != 1) {
+      const int t1 = warp == 0 ? tid : tid - 32, n1 = blockDim.x - 32;
       if (pivoted) {
-        const T recip = s_recip;
-        for (int r = r0 + t1; r < nloc; r += n1) S[r * lds + j] = mul_rn(S[r * lds + j], recip);
-        if (j + 1 < w) {
-          const T u1 = s_u1;
-          for (int r = r0 + t1; r < nloc; r += n1) {
-            const T v = upd<kExact>(S[r * lds + j + 1], S[r * lds + j], u1);
-            S[r * lds + j + 1] = v;
+        const T recip = s_recip, u1 = s_u1;
+        const bool more = j + 1 < w;
+        for (int r = r0 + t1; r < nloc; r += n1) {
+          T* row = S + r * lds;
+          const T l = mul_rn(row[j], recip);
+          row[j] = l;
+          if (more) {
+            const T v = upd<kExact>(row[j + 1], l, u1);
+            row[j + 1] = v;
             key_combine(bk, bi, bs, PivotKey<T>::of(v), ids[r], r);
           }
         }
@@ -508,7 +563,10 @@ __global__ void __launch_bounds__(512, 1) panel_kernel(PanelArgs<T> p) {
         for (int r = r0 + t1; r < nloc; r += n1)
           key_combine(bk, bi, bs, PivotKey<T>::of(S[r * lds + j + 1]), ids[r], r);
       }
-      key_reduce_redux(bk, bi, bs);
+      const int bsrc = warp_best(bk, bi);
+      bk = PivotKey<T>::shfl(bk, bsrc);
+      bi = __shfl_sync(kFull, bi, bsrc);
+      bs = __shfl_sync(kFull, bs, bsrc);
     } else if (seg_live) {
       // The winner's segment from stage into the pivot-row buffer; a word
       // whose tag is not yet this step's (relaxed stores land in any order)
@@ -516,6 +574,7 @@ __global__ void __launch_bounds__(512, 1) panel_kernel(PanelArgs<T> p) {
       cp_async_wait_all();
       __syncwarp();
       bool got = true;
+      unsigned long long t0 = 0;
       while (got) {
         for (int c = j + 2 + lane; c < w; c += 32) {
           unsigned long long* sw = stage + c * kW;
@@ -529,6 +588,7 @@ __global__ void __launch_bounds__(512, 1) panel_kernel(PanelArgs<T> p) {
         }
         if (__all_sync(kFull, got)) break;
         got = true;
+        if (t0 == 0) t0 = global_timer_ns();
         if (panel_wait_over(p.st, t0)) got = false;
       }
       if (!got && lane == 0) {
@@ -944,12 +1004,9 @@ template <typename T>
 static int panel_lds(int w) {
   return sizeof(T) == 4 ? ((w + 3) & ~3) + 4 : w + 1;
 }
-// Threads of a panel CTA: FP32 uses 16 warps so the look-ahead's shared-memory
-// latency is hidden; FP64's look-ahead is bound by the FP64 pipe.
-template <typename T>
-static int panel_threads() {
-  return sizeof(T) == 4 ? 512 : 256;
-}
+// Threads of a panel CTA: 16 warps hide the look-ahead's shared-memory latency
+// (FP64, 8 warps against 16: 207 / 200 us at 8192 rows, 270 / 229 at 16384).
+constexpr int kPanelThreads = 512;
 template <typename T>
 static size_t panel_smem_bytes(int rows_per, int w) {
   return ((size_t)rows_per * panel_lds<T>(w) + 2 * kMaxPanelWidth) * sizeof(T) + 2 * (size_t)rows_per * sizeof(int);
@@ -983,7 +1040,7 @@ static int launch_panel(luhot_ctx* ctx, T* a, int64_t lda, int m, int k0, int w,
   const size_t smem = panel_smem_bytes<T>(rows_per, w);
   LUHOT_CUDA_TRY(ctx, allow_max_dynamic_smem(kern));
   int per_sm = 0;
-  LUHOT_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, panel_threads<T>(), smem));
+  LUHOT_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kPanelThreads, smem));
   if (per_sm * ctx->num_sms < P)
     return set_error(ctx, LUHOT_ERR_UNSUPPORTED, "panel grid cannot be co-resident");
   PanelArgs<T> args;
@@ -995,14 +1052,15 @@ static int launch_panel(luhot_ctx* ctx, T* a, int64_t lda, int m, int k0, int w,
   args.rows_per = rows_per;
   args.lds = panel_lds<T>(w);
   args.piv = piv;
-  args.slots = static_cast<unsigned long long*>(ctx->panel_scratch);
+  args.heads = static_cast<unsigned long long*>(ctx->panel_scratch);
+  args.slots = args.heads + 2 * (size_t)kMaxPanelCtas * kPanelHeaderWords;
   args.moves = reinterpret_cast<int*>(static_cast<char*>(ctx->panel_scratch) + kPanelSlotBytes);
   args.move_count = args.moves + 4 * kMaxPanelWidth;
   args.st = ctx->d_status;
   LUHOT_CUDA_TRY(ctx, cudaMemsetAsync(args.move_count, 0, sizeof(int), stream));
   void* kargs[] = {&args};
   prof_begin(ctx, kProfPanel);
-  LUHOT_CUDA_TRY(ctx, cudaLaunchCooperativeKernel((void*)kern, dim3(P), dim3(panel_threads<T>()), kargs, smem,
+  LUHOT_CUDA_TRY(ctx, cudaLaunchCooperativeKernel((void*)kern, dim3(P), dim3(kPanelThreads), kargs, smem,
                                                   stream));
   // panel flops: sum over steps of (rows below) * (1 + 2 * cols right)
   double fl = 0.0;

@@ -36,6 +36,7 @@ struct PanelArgs {
   int rows_per;   // panel rows owned by each CTA
   int lds;        // shared-memory row stride (elements)
   int* piv;       // device pivots (global row index per step)
+  unsigned long long* heads;  // [2][kMaxPanelCtas][kPanelHeaderWords] exchange headers
   unsigned long long* slots;  // [2][kMaxPanelCtas][kPanelSlotWords] exchange words
   int* moves;                 // (destination, source) rows of the panel's rows that moved
   int* move_count;            // zeroed before the launch
