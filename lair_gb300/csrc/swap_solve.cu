@@ -20,6 +20,10 @@
 // 936 columns took 15 + 3 + 9 + 28 us as diagonal inverse, two splits and a slice
 // product (and 84 us as one thread per column), the interchanges 7 and the
 // update's own splits 4 + 9; this launch does all of it.
+// Few columns (a CTA a group, one pass): memory latency and the 64-step chain bound
+// it, so the list of moves, its count and 16 elements of L11 a thread are in
+// flight at once (2500-column FP32 factorization: 14 -> 11 us a launch; 936 FP64
+// columns 18.5 -> 17.4).
 #include <algorithm>
 #include <type_traits>
 
@@ -52,6 +56,8 @@ __host__ __device__ constexpr int ss_threads() {
   return 16 * ss_cols<T>();  // a warp per two columns
 }
 constexpr int kSsLeftCols = 32;
+static_assert(64 * 64 % (16 * ss_threads<float>()) == 0 && 64 * 64 % (16 * ss_threads<double>()) == 0,
+              "L11 is staged in whole batches");
 
 template <typename T, bool kExact, int W>
 __global__ void __launch_bounds__(ss_threads<T>()) swap_solve_kernel(SwapSolveArgs<T> p) {
@@ -83,8 +89,10 @@ __global__ void __launch_bounds__(ss_threads<T>()) swap_solve_kernel(SwapSolveAr
     return;
   }
 
-  const int count = p.moves ? min(*p.move_count, 2 * min(p.w, kMaxPanelWidth)) : 0;
-  for (int i = tid; i < 2 * count; i += kTh) mv[i] = p.moves[i];
+  // The list is read whole, beside its count: one trip to memory instead of two.
+  const int capacity = p.moves ? 2 * min(p.w, kMaxPanelWidth) : 0;
+  for (int i = tid; i < 2 * capacity; i += kTh) mv[i] = p.moves[i];
+  const int count = p.moves ? min(*p.move_count, capacity) : 0;
 
   if (bid >= p.right_ctas) {
     // Interchanges alone: 32 columns, every load of a group before its stores.
@@ -120,9 +128,19 @@ __global__ void __launch_bounds__(ss_threads<T>()) swap_solve_kernel(SwapSolveAr
   T* Lt = reinterpret_cast<T*>(smem_raw);  // [W][W + 1]: Lt[k][i] = L11(i, k) for i > k, else 0
   T* X = Lt + W * kWp;                     // [W][kCols + 1]
   __half* D = reinterpret_cast<__half*>(X + W * kXp);  // [7][kCols][64] (with a split)
-  for (int idx = tid; idx < W * W; idx += kTh) {
-    const int i = idx / W, k = idx - i * W;
-    Lt[k * kWp + i] = (i < p.w && k < i) ? p.a[(int64_t)(p.k0 + i) * p.lda + p.k0 + k] : T(0);
+  constexpr int kLoads = 16;  // in flight
+  for (int base = tid; base < W * W; base += kLoads * kTh) {
+    T l[kLoads];
+#pragma unroll
+    for (int q = 0; q < kLoads; ++q) {
+      const int idx = base + q * kTh, i = idx / W, k = idx - i * W;
+      l[q] = (i < p.w && k < i) ? p.a[(int64_t)(p.k0 + i) * p.lda + p.k0 + k] : T(0);
+    }
+#pragma unroll
+    for (int q = 0; q < kLoads; ++q) {
+      const int idx = base + q * kTh, i = idx / W, k = idx - i * W;
+      Lt[k * kWp + i] = l[q];
+    }
   }
   if (tid < W) srcrow[tid] = p.k0 + tid;
   if (tid == 0) s_below = 0;
