@@ -72,7 +72,7 @@ int luhot_set_stream(luhot_ctx* ctx, void* cuda_stream);
 /* Panel width override (0 = default 64); for tuning and tests. */
 int luhot_set_block(luhot_ctx* ctx, int nb);
 /* Schur-update engine of fast-mode FP64 getrf (no lair counterpart).
- * LUHOT_UPDATE_AUTO (default): trailing blocks of more than 200 000 elements
+ * LUHOT_UPDATE_AUTO (default): trailing blocks of more than 50 000 elements
  * (at least 128 x 64) are updated on the FP16 tensor cores by an exact
  * integer-slice product (Ozaki scheme: seven 8-bit slices per operand, 28 slice
  * products, FP32 sums that are exact, one FP64 rounding; error at or below an

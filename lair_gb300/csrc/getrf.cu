@@ -1012,11 +1012,25 @@ static size_t panel_smem_bytes(int rows_per, int w) {
   return ((size_t)rows_per * panel_lds<T>(w) + 2 * kMaxPanelWidth) * sizeof(T) + 2 * (size_t)rows_per * sizeof(int);
 }
 
+template <typename T>
+static int panel_ctas(luhot_ctx* ctx, int rows) {
+  const int pmax = std::min(ctx->num_sms, sizeof(T) == 4 ? 64 : 96);
+  const int min_rows = sizeof(T) == 4 ? 32 : 64;
+  return std::min(pmax, std::max(1, (rows + min_rows - 1) / min_rows));
+}
+
+// Where a panel reports its moved rows unless told otherwise.
+static int* live_moves(luhot_ctx* ctx) {
+  return reinterpret_cast<int*>(static_cast<char*>(ctx->panel_scratch) + kPanelSlotBytes);
+}
+
 template <typename T, bool kExact>
-static int launch_panel(luhot_ctx* ctx, T* a, int64_t lda, int m, int k0, int w, int* piv,
-                        cudaStream_t stream) {
+static int launch_panel(luhot_ctx* ctx, T* a, int64_t lda, int m, int k0, int w, int* piv, cudaStream_t stream,
+                        int* moves = nullptr) {
   const int rows = m - k0;
-  if (panel_cluster_fits<T>(ctx, rows, w)) return launch_panel_cluster<T, kExact>(ctx, a, lda, m, k0, w, piv, stream);
+  if (!moves) moves = live_moves(ctx);
+  if (panel_cluster_fits<T>(ctx, rows, w))
+    return launch_panel_cluster<T, kExact>(ctx, a, lda, m, k0, w, piv, moves, stream);
   auto kern = panel_kernel<T, kExact>;
   cudaFuncAttributes fa;
   LUHOT_CUDA_TRY(ctx, cudaFuncGetAttributes(&fa, kern));
@@ -1027,9 +1041,7 @@ static int launch_panel(luhot_ctx* ctx, T* a, int64_t lda, int m, int k0, int w,
   // fewer CTAs shorten the per-column exchange, more share the update).  The
   // count is raised, up to the SM count, when the rows of one CTA would not
   // fit in shared memory.
-  const int pmax = std::min(ctx->num_sms, sizeof(T) == 4 ? 64 : 96);
-  const int min_rows = sizeof(T) == 4 ? 32 : 64;
-  int P = std::min(pmax, std::max(1, (rows + min_rows - 1) / min_rows));
+  int P = panel_ctas<T>(ctx, rows);
   int rows_per = (rows + P - 1) / P;
   while (panel_smem_bytes<T>(rows_per, w) > (size_t)max_smem && P < ctx->num_sms) {
     P = std::min(ctx->num_sms, P * 2);
@@ -1054,7 +1066,7 @@ static int launch_panel(luhot_ctx* ctx, T* a, int64_t lda, int m, int k0, int w,
   args.piv = piv;
   args.heads = static_cast<unsigned long long*>(ctx->panel_scratch);
   args.slots = args.heads + 2 * (size_t)kMaxPanelCtas * kPanelHeaderWords;
-  args.moves = reinterpret_cast<int*>(static_cast<char*>(ctx->panel_scratch) + kPanelSlotBytes);
+  args.moves = moves;
   args.move_count = args.moves + 4 * kMaxPanelWidth;
   args.st = ctx->d_status;
   LUHOT_CUDA_TRY(ctx, cudaMemsetAsync(args.move_count, 0, sizeof(int), stream));
@@ -1094,7 +1106,7 @@ static int launch_gemm(luhot_ctx* ctx, T* a, int64_t lda, int r0, int c0, int kk
     if (aligned && smem_p <= (size_t)ctx->max_smem_optin) {
       LUHOT_CUDA_TRY(ctx, allow_max_dynamic_smem(gemm_dmma_persistent_kernel));
       prof_begin(ctx, kProfGemm);
-      gemm_dmma_persistent_kernel<<<std::min(tiles, ctx->num_sms), 256, smem_p, stream>>>(a, lda, r0, c0, kk0, K,
+      gemm_dmma_persistent_kernel<<<std::min(tiles, ctx->tc_grid_cap > 0 ? ctx->tc_grid_cap : ctx->num_sms), 256, smem_p, stream>>>(a, lda, r0, c0, kk0, K,
                                                                                           M, N);
     } else {
       LUHOT_CUDA_TRY(ctx, allow_max_dynamic_smem(gemm_dmma_kernel));
@@ -1140,22 +1152,27 @@ static int launch_laswp_cols(luhot_ctx* ctx, T* a, int64_t lda, const int* moves
 }
 
 // Whether the trailing update of M rows and N columns runs on the FP16 tensor
-// cores as a slice product (ozaki.cu).  A slice product takes 28 us for up to one
-// 128 x 128 tile per SM, FP64 arithmetic 8 us + 0.12 ns an element at K = 64:
-// they meet at 170 000 - 200 000 elements (512 x 400: 28 against 32 us).
+// cores as a slice product (ozaki.cu).  One takes some 8 us for up to a tile of 64 x
+// 128 per SM; FP64 arithmetic 14 us for 8 million multiply-adds (K = 64: 128 000
+// elements) on all SMs, and 9 us for the tile of 16 x 32 that one takes.  ms a
+// factorization with the line at 200 000 / 50 000 / 25 000 elements: n = 500 0.780 /
+// 0.746 / 0.745, 700 1.126 / 1.095 / 1.093, 1000 1.715 / 1.684 / 1.685; n = 4097 (whose
+// panels wait for updates of 64 columns) 13.56 / 13.14 / 13.13 with the solve.
 static bool update_on_slices(const void* oz_ws, int engine, int M, int N) {
   if (!oz_ws || engine == LUHOT_UPDATE_DMMA || M < 128 || N < 64) return false;
-  return engine == LUHOT_UPDATE_OZAKI || (int64_t)M * N > 200000;
+  return engine == LUHOT_UPDATE_OZAKI || (int64_t)M * N > 50000;
 }
 
 // Workspace of the tensor-core FP64 update for an m x n factorization
 // (nullptr: the engine setting or the device rules it out).
-static int ozaki_workspace(luhot_ctx* ctx, int m, int n, int engine, void** ws) {
+static int ozaki_workspace(luhot_ctx* ctx, int m, int n, int engine, void** ws, int n2 = 0, void** ws2 = nullptr) {
   *ws = nullptr;
   if (engine == LUHOT_UPDATE_DMMA || !ozaki_available(ctx)) return LUHOT_OK;
-  int rc = ensure_buf(ctx, ctx->oz_buf, ozaki_workspace_bytes(m, n));
+  const size_t bytes = (ozaki_workspace_bytes(m, n) + 1023) / 1024 * 1024;
+  int rc = ensure_buf(ctx, ctx->oz_buf, bytes + (n2 > 0 ? ozaki_workspace_bytes(m, n2) : 0));
   if (rc != LUHOT_OK) return rc;
   *ws = ctx->oz_buf.ptr;
+  if (ws2) *ws2 = static_cast<char*>(ctx->oz_buf.ptr) + bytes;
   return LUHOT_OK;
 }
 
@@ -1165,10 +1182,6 @@ int fp64_schur_update(luhot_ctx* ctx, double* a, int64_t lda, int k, int m, int 
   if (rc) return rc;
   if (update_on_slices(ws, engine, m - k, n - k)) return ozaki_update(ctx, a, lda, 0, k, k, m, k, n, ws, ctx->stream);
   return launch_gemm<double, false>(ctx, a, lda, k, k, 0, k, m - k, n - k, ctx->stream);
-}
-
-static const int* live_moves(luhot_ctx* ctx) {
-  return reinterpret_cast<const int*>(static_cast<char*>(ctx->panel_scratch) + kPanelSlotBytes);
 }
 
 // Two panels [k0, k0 + 64), [k0 + 64, k0 + 128) of fast-mode FP64 and one trailing
@@ -1189,11 +1202,10 @@ static int fp64_panel_pair(luhot_ctx* ctx, double* a, int64_t lda, int m, int n,
   if (rc) return rc;
   int* mv = static_cast<int*>(ctx->la_moves.ptr);
   double* const ab = a + (int64_t)k1 * lda;  // row k1
-  rc = launch_panel<double, false>(ctx, a, lda, m, k0, w, piv, stream);
-  if (rc) return rc;
   // The first panel's interchanges on the other columns come after the second's
-  // columns are done: keep them.
-  LUHOT_CUDA_TRY(ctx, cudaMemcpyAsync(mv, live_moves(ctx), kPanelMovesBytes, cudaMemcpyDeviceToDevice, stream));
+  // columns are done: its list is kept apart.
+  rc = launch_panel<double, false>(ctx, a, lda, m, k0, w, piv, stream, mv);
+  if (rc) return rc;
   const SplitOut split = ozaki_split_out(oz_ws, k1, m - k1, w);
   rc = launch_swap_solve<double, false>(ctx, a, lda, mv, k0, w, 0, 0, k1, r1, &split, stream);
   if (!rc) rc = ozaki_update_split(ctx, a, lda, w, k1, m, k1, r1, oz_ws, stream);
@@ -1206,8 +1218,115 @@ static int fp64_panel_pair(luhot_ctx* ctx, double* a, int64_t lda, int m, int n,
   return rc;
 }
 
+static int* la_saved_moves(luhot_ctx* ctx, int parity, int half) {
+  return reinterpret_cast<int*>(static_cast<char*>(ctx->la_moves.ptr) + (size_t)(2 * parity + half) * kPanelMovesBytes);
+}
+
+// Launches between its construction and destruction go to `s` (the
+// profile's events are recorded on the context's stream).
+struct OnStream {
+  luhot_ctx* ctx;
+  cudaStream_t old;
+  OnStream(luhot_ctx* c, cudaStream_t s) : ctx(c), old(c->stream) { c->stream = s; }
+  ~OnStream() { ctx->stream = old; }
+};
+
+static int la_setup(luhot_ctx* ctx) {
+  if (!ctx->la_hi) {
+    int least = 0, greatest = 0;
+    LUHOT_CUDA_TRY(ctx, cudaDeviceGetStreamPriorityRange(&least, &greatest));
+    LUHOT_CUDA_TRY(ctx, cudaStreamCreateWithPriority(&ctx->la_lo, cudaStreamNonBlocking, least));
+    LUHOT_CUDA_TRY(ctx, cudaStreamCreateWithPriority(&ctx->la_hi, cudaStreamNonBlocking, greatest));
+  }
+  for (auto& e : ctx->la_ev)
+    if (!e) LUHOT_CUDA_TRY(ctx, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  return ensure_buf(ctx, ctx->la_moves, 4 * kPanelMovesBytes);
+}
+
+// Look-ahead: panel k + 1 beside the rest of step k.  A high-priority stream (hs)
+// factors the panels and brings each next panel's columns up to date; a
+// low-priority one (ls) does the rest of the step (interchanges, rows of U, update
+// of the columns behind the next panel) on the SMs that the next panel leaves.
+// hs waits for the rest of step k - 1 before it touches step k + 1's columns,
+// so that at most two steps are under way; their lists of moved rows alternate.
+// Takes the steps from k0 on while la_pays; returns the first one it left in k0.
+// The price is two launches more a step on the panels' way, some 40 us, so that it
+// pays while the block behind the next panel is large.  ms, FP64 / FP32, step by
+// step against with look-ahead: n = 1000 1.69 -> 1.69 (1.71 with a limit of 500000) /
+// 1.25 -> 1.25, 2000 4.29 -> 4.17 / 3.07 -> 2.86, 3000 8.07 -> 7.41 / 5.36 -> 4.56.
+template <typename T>
+static bool la_pays(int m, int n, int k0, int nb) {
+  const int64_t M = m - k0 - 2 * nb, N = n - k0 - 2 * nb;
+  return M > 0 && N > 0 && M * N >= (sizeof(T) == 8 ? 1000000 : 500000);
+}
+
+template <typename T>
+static int la_loop(luhot_ctx* ctx, int m, int n, T* a, int64_t lda, int* piv, int nb, void* oz_ws, void* oz_hi,
+                   int* k0_io) {
+  cudaStream_t hs = ctx->la_hi, ls = ctx->la_lo;
+  // Columns [c0, c1) of step k0: interchanges (also on [0, cl1)), rows of U, update.
+  auto columns = [&](const int* mv, int k0, int cl1, int c0, int c1, void* ws, cudaStream_t st) -> int {
+    const int r1 = k0 + nb, M = m - r1, N = c1 - c0;
+    const bool slices = std::is_same<T, double>::value && update_on_slices(ws, ctx->fp64_update, M, N);
+    SplitOut split;
+    if (slices) split = ozaki_split_out(ws, r1, M, N);
+    int rc = launch_swap_solve<T, false>(ctx, a, lda, mv, k0, nb, 0, cl1, c0, c1, slices ? &split : nullptr, st);
+    if (rc) return rc;
+    if constexpr (std::is_same<T, double>::value) {
+      if (slices) return ozaki_update_split(ctx, a, lda, nb, r1, m, c0, c1, ws, st);
+    }
+    return launch_gemm<T, false>(ctx, a, lda, r1, c0, k0, nb, M, N, st);
+  };
+  int k0 = *k0_io;
+  for (int step = 0; la_pays<T>(m, n, k0, nb); ++step, k0 += nb) {
+    const int par = step & 1, k1 = k0 + nb, e1 = k1 + nb;
+    int* mv = la_saved_moves(ctx, par, 0);
+    {
+      OnStream on(ctx, hs);
+      int rc = launch_panel<T, false>(ctx, a, lda, m, k0, nb, piv, hs, mv);
+      if (rc) return rc;
+      if (step > 0) LUHOT_CUDA_TRY(ctx, cudaStreamWaitEvent(hs, ctx->la_ev[2 + (par ^ 1)], 0));
+      rc = columns(mv, k0, 0, k1, e1, oz_hi, hs);
+      if (rc) return rc;
+      LUHOT_CUDA_TRY(ctx, cudaEventRecord(ctx->la_ev[1], hs));
+    }
+    {
+      OnStream on(ctx, ls);
+      LUHOT_CUDA_TRY(ctx, cudaStreamWaitEvent(ls, ctx->la_ev[1], 0));
+      ctx->tc_grid_cap =
+          std::max(1, ctx->num_sms - (panel_cluster_fits<T>(ctx, m - k1, nb) ? ctx->panel_cluster : panel_ctas<T>(ctx, m - k1)));
+      const int rc = columns(mv, k0, k0, e1, n, oz_ws, ls);
+      ctx->tc_grid_cap = 0;
+      if (rc) return rc;
+      LUHOT_CUDA_TRY(ctx, cudaEventRecord(ctx->la_ev[2 + par], ls));
+    }
+  }
+  *k0_io = k0;
+  return LUHOT_OK;
+}
+
+// `run` on the look-ahead streams, behind what is on `stream` and before what
+// comes on it next (also after an error).
+template <typename F>
+static int la_fork_join(luhot_ctx* ctx, cudaStream_t stream, F run) {
+  int rc = la_setup(ctx);
+  if (rc) return rc;
+  LUHOT_CUDA_TRY(ctx, cudaEventRecord(ctx->la_ev[0], stream));
+  LUHOT_CUDA_TRY(ctx, cudaStreamWaitEvent(ctx->la_hi, ctx->la_ev[0], 0));
+  LUHOT_CUDA_TRY(ctx, cudaStreamWaitEvent(ctx->la_lo, ctx->la_ev[0], 0));
+  rc = run();
+  ctx->tc_grid_cap = 0;
+  cudaError_t e = cudaEventRecord(ctx->la_ev[0], ctx->la_hi);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(stream, ctx->la_ev[0], 0);
+  if (e == cudaSuccess) e = cudaEventRecord(ctx->la_ev[1], ctx->la_lo);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(stream, ctx->la_ev[1], 0);
+  if (rc) return rc;
+  if (e != cudaSuccess) return set_error(ctx, LUHOT_ERR_CUDA, std::string("look-ahead join: ") + cudaGetErrorString(e));
+  return LUHOT_OK;
+}
+
 template <typename T, bool kExact>
-static int getrf_impl(luhot_ctx* ctx, int m, int n, T* a, int64_t lda, int* piv, int nb, void* oz_ws,
+static int getrf_impl(luhot_ctx* ctx, int m, int n, T* a, int64_t lda, int* piv, int nb, void* oz_ws, void* oz_hi,
                       cudaStream_t stream) {
   const int dim_min = std::min(m, n);
   // Exchange words carry step tags; clear them so no word of an earlier
@@ -1222,6 +1341,12 @@ static int getrf_impl(luhot_ctx* ctx, int m, int n, T* a, int64_t lda, int* piv,
         if (rc) return rc;
         k0 += nb;  // and the loop's own step
         continue;
+      }
+    }
+    if constexpr (!kExact) {
+      if (la_pays<T>(m, n, k0, nb)) {
+        int rc = la_fork_join(ctx, stream, [&] { return la_loop<T>(ctx, m, n, a, lda, piv, nb, oz_ws, oz_hi, &k0); });
+        if (rc) return rc;
       }
     }
     const int w = std::min(nb, dim_min - k0);
@@ -1268,31 +1393,6 @@ static int getrf_impl(luhot_ctx* ctx, int m, int n, T* a, int64_t lda, int* piv,
 // for the rest of slab s - 2 before slab s's panels (it covered slab s's
 // columns) and for the rest of slab s - 1 before the next slab's columns.
 // Each panel's list of moved rows is saved per slab parity for ls.
-static int* la_saved_moves(luhot_ctx* ctx, int parity, int half) {
-  return reinterpret_cast<int*>(static_cast<char*>(ctx->la_moves.ptr) + (size_t)(2 * parity + half) * kPanelMovesBytes);
-}
-
-// Launches between its construction and destruction go to `s` (the
-// profile's events are recorded on the context's stream).
-struct OnStream {
-  luhot_ctx* ctx;
-  cudaStream_t old;
-  OnStream(luhot_ctx* c, cudaStream_t s) : ctx(c), old(c->stream) { c->stream = s; }
-  ~OnStream() { ctx->stream = old; }
-};
-
-static int la_setup(luhot_ctx* ctx) {
-  if (!ctx->la_hi) {
-    int least = 0, greatest = 0;
-    LUHOT_CUDA_TRY(ctx, cudaDeviceGetStreamPriorityRange(&least, &greatest));
-    LUHOT_CUDA_TRY(ctx, cudaStreamCreateWithPriority(&ctx->la_lo, cudaStreamNonBlocking, least));
-    LUHOT_CUDA_TRY(ctx, cudaStreamCreateWithPriority(&ctx->la_hi, cudaStreamNonBlocking, greatest));
-  }
-  for (auto& e : ctx->la_ev)
-    if (!e) LUHOT_CUDA_TRY(ctx, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-  return ensure_buf(ctx, ctx->la_moves, 4 * kPanelMovesBytes);
-}
-
 // The slab's interchanges (mv_a, mv_b: its panels' moved rows) on the columns
 // [cl0, cl1) and [c0, c1); rows [s0, s1) of U on the columns [c0, c1) (two
 // solves with the K = 128 update of panel B's rows between them), then the
@@ -1335,16 +1435,13 @@ static int tc_slab_loop(luhot_ctx* ctx, int m, int n, float* a, int64_t lda, int
     {
       OnStream on(ctx, hs);
       if (slab >= 2) LUHOT_CUDA_TRY(ctx, cudaStreamWaitEvent(hs, ctx->la_ev[2 + par], 0));
-      int rc = launch_panel<float, false>(ctx, a, lda, m, s0, h0, piv, hs);
+      int rc = launch_panel<float, false>(ctx, a, lda, m, s0, h0, piv, hs, mv_a);
       if (rc) return rc;
-      LUHOT_CUDA_TRY(ctx, cudaMemcpyAsync(mv_a, live_moves(ctx), kPanelMovesBytes, cudaMemcpyDeviceToDevice, hs));
       if (h1 > 0) {
         rc = launch_swap_solve<float, false>(ctx, a, lda, mv_a, s0, h0, 0, 0, s0 + h0, s1, nullptr, hs);
         if (!rc) rc = launch_gemm<float, false>(ctx, a, lda, s0 + h0, s0 + h0, s0, h0, m - (s0 + h0), h1, hs);
-        if (!rc) rc = launch_panel<float, false>(ctx, a, lda, m, s0 + h0, h1, piv, hs);
-        if (rc) return rc;
-        LUHOT_CUDA_TRY(ctx, cudaMemcpyAsync(mv_b, live_moves(ctx), kPanelMovesBytes, cudaMemcpyDeviceToDevice, hs));
-        rc = launch_laswp_cols<float>(ctx, a, lda, mv_b, h1, s0, s0 + h0, 0, 0, hs);
+        if (!rc) rc = launch_panel<float, false>(ctx, a, lda, m, s0 + h0, h1, piv, hs, mv_b);
+        if (!rc) rc = launch_laswp_cols<float>(ctx, a, lda, mv_b, h1, s0, s0 + h0, 0, 0, hs);
       }
       if (!rc && s1 < e1) {
         if (slab >= 1) LUHOT_CUDA_TRY(ctx, cudaStreamWaitEvent(hs, ctx->la_ev[2 + (par ^ 1)], 0));
@@ -1369,21 +1466,8 @@ static int tc_slab_loop(luhot_ctx* ctx, int m, int n, float* a, int64_t lda, int
 static int getrf_tc_slabs(luhot_ctx* ctx, int m, int n, float* a, int64_t lda, int* piv, int tc_kind, void* tc_a,
                           void* tc_b, float* tc_scal, cudaStream_t stream) {
   LUHOT_CUDA_TRY(ctx, cudaMemsetAsync(ctx->panel_scratch, 0, kPanelScratchBytes, stream));
-  int rc = la_setup(ctx);
-  if (rc) return rc;
-  LUHOT_CUDA_TRY(ctx, cudaEventRecord(ctx->la_ev[0], stream));
-  LUHOT_CUDA_TRY(ctx, cudaStreamWaitEvent(ctx->la_hi, ctx->la_ev[0], 0));
-  LUHOT_CUDA_TRY(ctx, cudaStreamWaitEvent(ctx->la_lo, ctx->la_ev[0], 0));
-  rc = tc_slab_loop(ctx, m, n, a, lda, piv, tc_kind, tc_a, tc_b, tc_scal);
-  ctx->tc_grid_cap = 0;
-  // The caller's stream waits for both streams, also after an error.
-  cudaError_t e = cudaEventRecord(ctx->la_ev[0], ctx->la_hi);
-  if (e == cudaSuccess) e = cudaStreamWaitEvent(stream, ctx->la_ev[0], 0);
-  if (e == cudaSuccess) e = cudaEventRecord(ctx->la_ev[1], ctx->la_lo);
-  if (e == cudaSuccess) e = cudaStreamWaitEvent(stream, ctx->la_ev[1], 0);
-  if (rc) return rc;
-  if (e != cudaSuccess) return set_error(ctx, LUHOT_ERR_CUDA, std::string("look-ahead join: ") + cudaGetErrorString(e));
-  return LUHOT_OK;
+  return la_fork_join(ctx, stream,
+                      [&] { return tc_slab_loop(ctx, m, n, a, lda, piv, tc_kind, tc_a, tc_b, tc_scal); });
 }
 
 template <typename T>
@@ -1405,15 +1489,15 @@ int getrf_device(luhot_ctx* ctx, int m, int n, T* a, int64_t lda, int* piv, int 
   if (ctx->nb_override <= 0 && n <= kMaxPanelWidth && m >= n && m <= (sizeof(T) == 8 ? 512 : 2048) &&
       panel_cluster_fits<T>(ctx, m, n))
     nb = kMaxPanelWidth;
-  void* oz_ws = nullptr;
+  void *oz_ws = nullptr, *oz_hi = nullptr;
   if (std::is_same<T, double>::value && mode != LUHOT_MODE_EXACT) {
-    rc = ozaki_workspace(ctx, m, n, ctx->fp64_update, &oz_ws);
+    rc = ozaki_workspace(ctx, m, n, ctx->fp64_update, &oz_ws, kDefaultPanelWidth, &oz_hi);
     if (rc != LUHOT_OK) return rc;
   }
   if (mode == LUHOT_MODE_EXACT)
-    rc = getrf_impl<T, true>(ctx, m, n, a, lda, piv, nb, nullptr, stream);
+    rc = getrf_impl<T, true>(ctx, m, n, a, lda, piv, nb, nullptr, nullptr, stream);
   else
-    rc = getrf_impl<T, false>(ctx, m, n, a, lda, piv, nb, oz_ws, stream);
+    rc = getrf_impl<T, false>(ctx, m, n, a, lda, piv, nb, oz_ws, oz_hi, stream);
   if (rc != LUHOT_OK) return rc;
   return finish_status(ctx, singular);
 }

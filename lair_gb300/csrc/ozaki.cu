@@ -725,7 +725,8 @@ static int oz_launch_gemm(luhot_ctx* ctx, const OzWs& w, int halves, double* c, 
   if (rc) return rc;
   const int tiles = ((M + kOzBM - 1) / kOzBM) * ((N + kOzBN - 1) / kOzBN);
   LUHOT_CUDA_TRY(ctx, allow_max_dynamic_smem(oz_gemm_kernel));
-  oz_gemm_kernel<<<std::min(tiles, ctx->num_sms), kOzThreads, kOzSmem, stream>>>(tmL, tmU, halves, c, ldc, M, N, w.ea, w.eb,
+  const int cap = ctx->tc_grid_cap > 0 ? ctx->tc_grid_cap : ctx->num_sms;
+  oz_gemm_kernel<<<std::min(tiles, cap), kOzThreads, kOzSmem, stream>>>(tmL, tmU, halves, c, ldc, M, N, w.ea, w.eb,
                                                                                 ctx->d_status);
   LUHOT_CUDA_TRY(ctx, cudaGetLastError());
   return LUHOT_OK;

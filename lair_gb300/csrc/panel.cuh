@@ -137,6 +137,7 @@ __device__ __forceinline__ int warp_best(unsigned long long k, int id) {
 template <typename T>
 bool panel_cluster_fits(luhot_ctx* ctx, int rows, int w);
 template <typename T, bool kExact>
-int launch_panel_cluster(luhot_ctx* ctx, T* a, int64_t lda, int m, int k0, int w, int* piv, cudaStream_t stream);
+int launch_panel_cluster(luhot_ctx* ctx, T* a, int64_t lda, int m, int k0, int w, int* piv, int* moves,
+                         cudaStream_t stream);
 
 }  // namespace luhot

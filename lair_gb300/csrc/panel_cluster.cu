@@ -681,7 +681,8 @@ bool panel_cluster_fits(luhot_ctx* ctx, int rows, int w) {
 }
 
 template <typename T, bool kExact>
-int launch_panel_cluster(luhot_ctx* ctx, T* a, int64_t lda, int m, int k0, int w, int* piv, cudaStream_t stream) {
+int launch_panel_cluster(luhot_ctx* ctx, T* a, int64_t lda, int m, int k0, int w, int* piv, int* moves,
+                         cudaStream_t stream) {
   const int rows = m - k0;
   int P, rows_per;
   cl_split<T>(ctx, rows, &P, &rows_per);
@@ -699,7 +700,7 @@ int launch_panel_cluster(luhot_ctx* ctx, T* a, int64_t lda, int m, int k0, int w
   args.rows_per = rows_per;
   args.lds = cl_lds<T>(w);
   args.piv = piv;
-  args.moves = reinterpret_cast<int*>(static_cast<char*>(ctx->panel_scratch) + kPanelSlotBytes);
+  args.moves = moves;
   args.move_count = args.moves + 4 * kMaxPanelWidth;
   args.st = ctx->d_status;
   cudaLaunchAttribute attr;
@@ -714,9 +715,9 @@ int launch_panel_cluster(luhot_ctx* ctx, T* a, int64_t lda, int m, int k0, int w
 
 template bool panel_cluster_fits<double>(luhot_ctx*, int, int);
 template bool panel_cluster_fits<float>(luhot_ctx*, int, int);
-template int launch_panel_cluster<double, false>(luhot_ctx*, double*, int64_t, int, int, int, int*, cudaStream_t);
-template int launch_panel_cluster<double, true>(luhot_ctx*, double*, int64_t, int, int, int, int*, cudaStream_t);
-template int launch_panel_cluster<float, false>(luhot_ctx*, float*, int64_t, int, int, int, int*, cudaStream_t);
-template int launch_panel_cluster<float, true>(luhot_ctx*, float*, int64_t, int, int, int, int*, cudaStream_t);
+template int launch_panel_cluster<double, false>(luhot_ctx*, double*, int64_t, int, int, int, int*, int*, cudaStream_t);
+template int launch_panel_cluster<double, true>(luhot_ctx*, double*, int64_t, int, int, int, int*, int*, cudaStream_t);
+template int launch_panel_cluster<float, false>(luhot_ctx*, float*, int64_t, int, int, int, int*, int*, cudaStream_t);
+template int launch_panel_cluster<float, true>(luhot_ctx*, float*, int64_t, int, int, int, int*, int*, cudaStream_t);
 
 }  // namespace luhot
