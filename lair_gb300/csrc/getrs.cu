@@ -319,6 +319,28 @@ static int sweep_tags(luhot_ctx* ctx, size_t words, unsigned long long** xt, int
   return LUHOT_OK;
 }
 
+template <typename T, typename TA>
+int cluster_sweep(luhot_ctx* ctx, const TA* lu, int64_t lda, T* x, int64_t ldx, int n, int nrhs, bool lower, bool trans,
+                  const T* dinv) {
+  if (n <= 0 || nrhs <= 0) return LUHOT_OK;
+  for (int c0 = 0; c0 < nrhs; c0 += kTrsvMaxChains) {
+    const int nc = std::min(kTrsvMaxChains, nrhs - c0);
+    unsigned long long* xt = nullptr;
+    int* ticket = nullptr;
+    unsigned int epoch = 0;
+    int rc = sweep_tags(ctx, trsv_cluster_tag_words(n, nc, sizeof(T)), &xt, &ticket, &epoch);
+    if (rc) return rc;
+    cudaError_t e = launch_trsv_cluster<T, TA>(ctx->stream, lu, lda, x + c0, ldx, n, nc, lower, trans, dinv, xt, epoch,
+                                               ticket, ctx->d_status);
+    if (e != cudaSuccess) return set_error(ctx, LUHOT_ERR_CUDA, std::string("sweep: ") + cudaGetErrorString(e));
+  }
+  return LUHOT_OK;
+}
+template int cluster_sweep<double, float>(luhot_ctx*, const float*, int64_t, double*, int64_t, int, int, bool, bool,
+                                          const double*);
+template int cluster_sweep<double, double>(luhot_ctx*, const double*, int64_t, double*, int64_t, int, int, bool, bool,
+                                           const double*);
+
 template <typename T>
 int trsv_chain_sweep(luhot_ctx* ctx, const float* lu, int64_t lda, T* x, int n, bool lower, const T* dinv) {
   unsigned long long* xt = nullptr;
@@ -417,8 +439,13 @@ int getrs_apply(luhot_ctx* ctx, int n, int nrhs, const T* lu, int64_t lda, const
     // op(A) lower: L, or U^T whose diagonal blocks invert to (D_U^-1)^T;
     // op(A) upper: U, or L^T (the kernel reads a given inverse transposed).
     const T* dinv = ex ? nullptr : ((lower != tr) ? dinv_l : dinv_u);
-    cudaError_t e = launch_trsv_syncfree<T>(stream, lu, lda, w, ldw, n, nrhs, lower, unit, tr, ex, flags, ticket,
-                                            ctx->d_status, dinv);
+    cudaError_t e = cudaSuccess;
+    if (dinv) {
+      const int rc_ = cluster_sweep<T, T>(ctx, lu, lda, w, ldw, n, nrhs, lower, tr, dinv);
+      if (rc_) return rc_;
+    } else {
+      e = launch_trsv_syncfree<T>(stream, lu, lda, w, ldw, n, nrhs, lower, unit, tr, ex, flags, ticket, ctx->d_status);
+    }
     prof_end(ctx, kProfTrsv, (double)n * n * nrhs, ((double)n * n / 2 + 2.0 * total) * sizeof(T));
     if (e != cudaSuccess) return set_error(ctx, LUHOT_ERR_CUDA, std::string("getrs sweep: ") + cudaGetErrorString(e));
     return LUHOT_OK;

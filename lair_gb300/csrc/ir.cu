@@ -307,22 +307,14 @@ struct IrRun {
       if (!rc) rc = scaled_sweep<double>(ctx, w64, ldlo, du64, u, out, 1, n, false);
       return rc;
     }
-    int* flags = nullptr;
-    int* ticket = nullptr;
-    int rc = trsv_scratch(ctx, n, &flags, &ticket);
-    if (rc) return rc;
     prof_begin(ctx, kProfRefine);
     ir_gather_kernel<double><<<grid_vec, 256, 0, ctx->stream>>>(v, perm, out, n);
     prof_end(ctx, kProfRefine, 0.0, 20.0 * n);
     prof_begin(ctx, kProfTrsv);
-    cudaError_t e = launch_trsv_syncfree<double, Tlo>(ctx->stream, lu, ldlo, out, 1, n, 1, true, true, false, false,
-                                                      flags, ticket, ctx->d_status, dl64);
-    if (e == cudaSuccess)
-      e = launch_trsv_syncfree<double, Tlo>(ctx->stream, lu, ldlo, out, 1, n, 1, false, false, false, false, flags,
-                                            ticket, ctx->d_status, du64);
+    int rc = cluster_sweep<double, Tlo>(ctx, lu, ldlo, out, 1, n, 1, true, false, dl64);
+    if (!rc) rc = cluster_sweep<double, Tlo>(ctx, lu, ldlo, out, 1, n, 1, false, false, du64);
     prof_end(ctx, kProfTrsv, 2.0 * n * (double)n, (double)n * n * sizeof(Tlo) + 32.0 * n);
-    if (e != cudaSuccess) return set_error(ctx, LUHOT_ERR_CUDA, std::string("ir sweep: ") + cudaGetErrorString(e));
-    return LUHOT_OK;
+    return rc;
   }
 
   // out (FP64) = (LU)^-1 v through the low precision with infinity-norm

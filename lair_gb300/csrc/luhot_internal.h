@@ -174,6 +174,11 @@ int getrs_device(luhot_ctx* ctx, int n, int nrhs, const T* lu, int64_t lda, cons
 // (getrs_perm), then apply any number of solves with it (getrs_apply, async;
 // w is n x nrhs scratch that must not alias b or x).
 int getrs_perm(luhot_ctx* ctx, const int* piv, int n, int* perm);
+// One sweep with given diagonal inverses over nrhs columns of x (trsv_cluster.cu),
+// 16 a launch.
+template <typename T, typename TA>
+int cluster_sweep(luhot_ctx* ctx, const TA* lu, int64_t lda, T* x, int64_t ldx, int n, int nrhs, bool lower, bool trans,
+                  const T* dinv);
 // Ready flags and ticket of the sync-free triangular sweeps for order n.
 int trsv_scratch(luhot_ctx* ctx, int n, int** flags, int** ticket);
 // One chained sweep (launch_trsv_chain) on the context's stream with a fresh

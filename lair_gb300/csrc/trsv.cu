@@ -1,4 +1,5 @@
-// Sync-free blocked triangular solve: one launch per sweep.
+// Sync-free blocked triangular solve without diagonal inverses: one launch per sweep
+// (exact mode; sweeps with inverses: trsv_cluster.cu).
 //
 // op(A) x = b with op(A) triangular (lower/upper, unit/non-unit, A or A^T of
 // a row-major LU factor), nrhs <= 16 columns of x (row-major, ldx), in place.
@@ -15,7 +16,7 @@
 // Latency hiding: the next tile of op(A) is loaded into registers while the
 // current one is used (A is read-only, so prefetching never waits on a
 // flag); every thread carries up to four independent (row, rhs) chains.  In
-// fast mode with fewer than four right-hand sides the 64 columns of a tile are
+// transposed sweeps with fewer than four right-hand sides the 64 columns of a tile are
 // also split among 256/(64*nrhs) threads per row and the partial sums are
 // added once, before the diagonal block.
 //
@@ -134,9 +135,8 @@ __device__ __forceinline__ bool wait_ready(const int* flags, int j, DeviceStatus
 template <typename T, typename TA, bool kExact, bool kLower, bool kUnit, bool kTrans, int kNR>
 __global__ void __launch_bounds__(kThreads) trsv_syncfree_kernel(const TA* __restrict__ a, int64_t lda, T* x,
                                                                  int64_t ldx, int n, int nrhs, int nchain,
-                                                                 int* flags, int* ticket, DeviceStatus* st,
-                                                                 const T* __restrict__ dinv) {
-  // Threads per (row, rhs) pair: k split only in fast mode.
+                                                                 int* flags, int* ticket, DeviceStatus* st) {
+  // Threads per (row, rhs) pair: no k split where lair's order is kept.
   constexpr int kKS = kExact ? 1 : (kNR >= 4 ? 1 : 4 / kNR);
   constexpr int kKLen = kBS / kKS;                      // k columns per thread and tile
   constexpr int kPairs = kBS * kNR;                      // (row, rhs) pairs
@@ -182,11 +182,6 @@ __global__ void __launch_bounds__(kThreads) trsv_syncfree_kernel(const TA* __res
   }
 
   const int nupd = kLower ? I : (nblk - 1 - I);  // blocks before I in sweep order
-  // Inverse of this block's diagonal tile (when given): fetched now, used last.
-  T ireg[kPrefetch];
-  // For op(A) = A^T the diagonal block of op(A) is the transpose of A's, and
-  // so is its inverse: the tile is read transposed.
-  if (!kExact && dinv != nullptr) tile_load<T, T, kTrans>(ireg, dinv + (int64_t)I * kBS * kBS, kBS, 0, 0, kBS, kBS);
   T reg[kPrefetch];
   if (nupd > 0) {
     const int J0 = kLower ? 0 : nblk - 1;
@@ -228,44 +223,6 @@ __global__ void __launch_bounds__(kThreads) trsv_syncfree_kernel(const TA* __res
       }
     }
     __syncthreads();
-  }
-
-  if (!kExact && dinv != nullptr) {
-    // Diagonal block by its precomputed inverse: x(I) = D^-1 xacc, a 64 x 64
-    // matvec split like the updates (no sequential chain on the critical path).
-    __syncthreads();
-    tile_store<T, kTrans>(tile0, ireg);
-#pragma unroll
-    for (int q = 0; q < kPP; ++q) {
-      T v = acc[q];
-      if (kKS > 1) {
-#pragma unroll
-        for (int off = 1; off < kKS; off <<= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-      }
-      if (pon[q] && pk0[q] == 0) xacc[prow[q] * kNR + pc[q]] = v;
-      if (!pon[q] && pk0[q] == 0 && (threadIdx.x + q * kThreads) / kKS < kPairs)
-        xacc[prow[q] * kNR + pc[q]] = T(0);
-    }
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < kPP; ++q) {
-      T v = T(0);
-      for (int kk = 0; kk < kKLen; ++kk) {
-        const int k = pk0[q] + kk;
-        v = fma(tile0[prow[q] * kLds + k], xacc[k * kNR + pc[q]], v);
-      }
-      if (kKS > 1) {
-#pragma unroll
-        for (int off = 1; off < kKS; off <<= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-      }
-      if (pon[q] && pk0[q] == 0) x[(int64_t)(i0 + prow[q]) * ldx + pc[q]] = v;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      __threadfence();
-      st_release_i32(flags + I, 1);
-    }
-    return;
   }
 
   // Sum the k parts of each pair into xacc.
@@ -357,16 +314,10 @@ __global__ void __launch_bounds__(kThreads) trsv_syncfree_kernel(const TA* __res
 size_t trsv_syncfree_smem(size_t elem) { return (2 * (size_t)kBS * kLds + 2 * (size_t)kBS * kMaxRhs) * elem; }
 int trsv_syncfree_blocks(int n) { return (n + kBS - 1) / kBS; }
 
-// Right-hand sides of one chain.  Fast sweeps run every right-hand side as a
-// chain of its own while the sweep is bound by its chain (the last off-diagonal
-// tile and the diagonal inverse of a 64-row block on one SM: 2.4 us of FP64 work
-// a right-hand side), and in wider chains, which read the factor fewer times,
-// once the whole sweep's work is the bound.  Two sweeps with their inverses in
-// us, chains of 1 / 2 / 4: FP64 n = 2048, 8 rhs 354 / 430 / 669, n = 4097, 16 rhs
-// 1079 / 1170 / 1638, n = 16384, 4 rhs 4090 / 4407 / 6161, 8 rhs 6541 / 6226 /
-// 7614, 16 rhs 11777 / 10145 / 10879; FP32 n = 2048, 16 rhs 210 / 219 / 211,
-// n = 4097, 8 rhs 375 / 406 / 401, 16 rhs 512 / 447 / 427.  Exact sweeps stay one
-// chain (one order for all right-hand sides of the launch).
+// Right-hand sides of one chain.  Exact sweeps are one chain (one order for all
+// right-hand sides of the launch); the transposed sweeps of exact mode, which have
+// no lair counterpart, run one a chain while the sweep is bound by its chain and
+// wider ones, which read the factor fewer times, once its work is the bound.
 static int trsv_width(bool exact, size_t elem, int n, int nc) {
   const int one = nc > 4 ? kMaxRhs : nc > 2 ? 4 : nc;
   if (exact) return one;
@@ -377,7 +328,7 @@ static int trsv_width(bool exact, size_t elem, int n, int nc) {
 
 template <typename T, typename TA, bool EX, bool LO, bool UN, bool TR>
 static cudaError_t launch_case(cudaStream_t stream, const TA* a, int64_t lda, T* x, int64_t ldx, int n, int nc,
-                               int* flags, int* ticket, DeviceStatus* st, const T* dinv) {
+                               int* flags, int* ticket, DeviceStatus* st) {
   const int nblk = trsv_syncfree_blocks(n);
   const size_t smem = trsv_syncfree_smem(sizeof(T));
   const int width = trsv_width(EX, sizeof(T), n, nc), nchain = (nc + width - 1) / width;
@@ -387,7 +338,7 @@ static cudaError_t launch_case(cudaStream_t stream, const TA* a, int64_t lda, T*
     auto k = trsv_syncfree_kernel<T, TA, EX, LO, UN, TR, NR>;                                            \
     e = allow_max_dynamic_smem(k);                                                                       \
     if (e != cudaSuccess) return e;                                                                      \
-    k<<<nblk * nchain, kThreads, smem, stream>>>(a, lda, x, ldx, n, nc, nchain, flags, ticket, st, dinv); \
+    k<<<nblk * nchain, kThreads, smem, stream>>>(a, lda, x, ldx, n, nc, nchain, flags, ticket, st);       \
     return cudaGetLastError();                                                                           \
   }
   if (width == 1) LUHOT_TRSV_NR(1)
@@ -400,10 +351,9 @@ static cudaError_t launch_case(cudaStream_t stream, const TA* a, int64_t lda, T*
 template <typename T, typename TA>
 cudaError_t launch_trsv_syncfree(cudaStream_t stream, const TA* a, int64_t lda, T* x, int64_t ldx, int n, int nrhs,
                                  bool lower, bool unit, bool trans, bool exact, int* flags, int* ticket,
-                                 DeviceStatus* st, const T* dinv) {
+                                 DeviceStatus* st) {
   if (n <= 0 || nrhs <= 0) return cudaSuccess;
   const int nblk = trsv_syncfree_blocks(n);
-  if (exact) dinv = nullptr;  // inverses serve the fast sweeps only
   for (int c0 = 0; c0 < nrhs; c0 += kMaxRhs) {
     const int nc = std::min(kMaxRhs, nrhs - c0);
     const int width = trsv_width(exact, sizeof(T), n, nc);
@@ -412,15 +362,11 @@ cudaError_t launch_trsv_syncfree(cudaStream_t stream, const TA* a, int64_t lda, 
     if (e != cudaSuccess) return e;
     T* xc = x + c0;
     if (exact && lower && unit && !trans)
-      e = launch_case<T, TA, true, true, true, false>(stream, a, lda, xc, ldx, n, nc, flags, ticket, st, nullptr);
-    else if (!exact && lower && unit && !trans)
-      e = launch_case<T, TA, false, true, true, false>(stream, a, lda, xc, ldx, n, nc, flags, ticket, st, dinv);
-    else if (!exact && !lower && !unit && !trans)
-      e = launch_case<T, TA, false, false, false, false>(stream, a, lda, xc, ldx, n, nc, flags, ticket, st, dinv);
+      e = launch_case<T, TA, true, true, true, false>(stream, a, lda, xc, ldx, n, nc, flags, ticket, st);
     else if (!exact && lower && !unit && trans)
-      e = launch_case<T, TA, false, true, false, true>(stream, a, lda, xc, ldx, n, nc, flags, ticket, st, dinv);
+      e = launch_case<T, TA, false, true, false, true>(stream, a, lda, xc, ldx, n, nc, flags, ticket, st);
     else if (!exact && !lower && unit && trans)
-      e = launch_case<T, TA, false, false, true, true>(stream, a, lda, xc, ldx, n, nc, flags, ticket, st, dinv);
+      e = launch_case<T, TA, false, false, true, true>(stream, a, lda, xc, ldx, n, nc, flags, ticket, st);
     else
       return cudaErrorNotSupported;
     if (e != cudaSuccess) return e;
@@ -511,9 +457,14 @@ cudaError_t launch_trsv_invert_diag(cudaStream_t stream, const TA* a, int64_t ld
   return cudaGetLastError();
 }
 
+#define LUHOT_TRSV_SYNCFREE(T)                                                                                   \
+  template cudaError_t launch_trsv_syncfree<T, T>(cudaStream_t, const T*, int64_t, T*, int64_t, int, int, bool, bool, \
+                                                  bool, bool, int*, int*, DeviceStatus*);
+LUHOT_TRSV_SYNCFREE(double)
+LUHOT_TRSV_SYNCFREE(float)
+#undef LUHOT_TRSV_SYNCFREE
+
 #define LUHOT_TRSV_INST(T, TA)                                                                                  \
-  template cudaError_t launch_trsv_syncfree<T, TA>(cudaStream_t, const TA*, int64_t, T*, int64_t, int, int, bool, \
-                                                   bool, bool, bool, int*, int*, DeviceStatus*, const T*);      \
   template cudaError_t launch_trsv_invert_diag<T, TA>(cudaStream_t, const TA*, int64_t, int, T*, T*);
 LUHOT_TRSV_INST(double, double)
 LUHOT_TRSV_INST(float, float)

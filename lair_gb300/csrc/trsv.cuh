@@ -18,15 +18,23 @@ constexpr int kTrsvMaxChains = 16;
 // op(A) x = b in place for nrhs columns of x (row-major, ldx); flags must hold
 // kTrsvMaxChains * trsv_syncfree_blocks(n) ints and ticket one int of device scratch (both
 // cleared by this call); st supplies the wait limit and records a timeout.
-// TA is the storage type of the factor (it may be narrower than T).  dinv,
-// when not null, holds the inverses of the 64 x 64 diagonal blocks of the
-// triangle of A that the sweep reads (launch_trsv_invert_diag; for a
-// transposed sweep the inverses of A's blocks, read transposed) and replaces
-// the sequential diagonal solve by a matvec; it is ignored in exact mode.
+// Combinations: lower unit in lair's order (exact), and the two transposed ones.
 template <typename T, typename TA = T>
 cudaError_t launch_trsv_syncfree(cudaStream_t stream, const TA* a, int64_t lda, T* x, int64_t ldx, int n, int nrhs,
                                  bool lower, bool unit, bool trans, bool exact, int* flags, int* ticket,
-                                 DeviceStatus* st, const T* dinv = nullptr);
+                                 DeviceStatus* st);
+
+// op(A) x = b in place for at most kTrsvMaxChains columns of x, any triangle, with
+// the inverses of the 64 x 64 diagonal blocks of the triangle of A that the sweep
+// reads (launch_trsv_invert_diag; a transposed sweep reads them transposed), by
+// clusters of four CTAs (trsv_cluster.cu).  TA is the storage type of the factor (it
+// may be narrower than T).  xt is tagged-word scratch of trsv_cluster_tag_words words, epoch a tag no word of xt holds yet, ticket one
+// int (cleared by the call).
+size_t trsv_cluster_tag_words(int n, int nrhs, size_t elem_bytes);
+template <typename T, typename TA = T>
+cudaError_t launch_trsv_cluster(cudaStream_t stream, const TA* a, int64_t lda, T* x, int64_t ldx, int n, int nc,
+                                bool lower, bool trans, const T* dinv, unsigned long long* xt, unsigned epoch,
+                                int* ticket, DeviceStatus* st);
 
 // Block-scaled single-right-hand-side sweeps (trsv_scaled.cu).  W holds,
 // for every off-diagonal 64 x 64 tile of L (below) and U (above) of an n x n
