@@ -72,6 +72,13 @@ __device__ __forceinline__ void cl_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
+// For a CTA that gave up a wait, behind the last cl_sync: pushes to it may still be
+// under way, which have to land before it leaves.
+static __device__ __noinline__ void cl_drain() {
+  const unsigned long long t0 = global_timer_ns();
+  while (global_timer_ns() - t0 < 200000ull) __nanosleep(1000);
+}
+
 // Lets `kernel` launch with clusters of more than 8 CTAs; once per kernel and
 // device, like allow_max_dynamic_smem.
 inline cudaError_t allow_wide_clusters(const void* kernel) {

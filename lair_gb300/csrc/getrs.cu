@@ -397,7 +397,7 @@ int scaled_sweep(luhot_ctx* ctx, const TW* w, int64_t ldw, const double* dinv, c
   if (rc) return rc;
   prof_begin(ctx, kProfTrsv);
   cudaError_t e = launch_trsv_scaled<TW>(ctx->stream, w, ldw, dinv, b, y, ldy, n, lower, xt, epoch, ticket,
-                                         ctx->d_status);
+                                         ctx->panel_cluster, ctx->d_status);
   prof_end(ctx, kProfTrsv, (double)n * n, (double)n * n / 2 * sizeof(TW) + 32.0 * n);
   count_launch(ctx);
   if (e != cudaSuccess) return set_error(ctx, LUHOT_ERR_CUDA, std::string("scaled sweep: ") + cudaGetErrorString(e));

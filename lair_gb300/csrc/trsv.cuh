@@ -43,7 +43,8 @@ cudaError_t launch_trsv_cluster(cudaStream_t stream, const TA* a, int64_t lda, T
 // L and U.  launch_trsv_scaled then runs y = T^-1 b for the lower (L) or upper
 // (U) triangle with b contiguous and y strided (y must not alias b); xt is
 // tagged-word scratch of trsv_scaled_tag_words(n) words, epoch a tag no word
-// of xt holds yet, ticket one int (cleared by the call).
+// of xt holds yet, ticket one int (cleared by the call), max_cluster the largest
+// cluster that the device schedules.
 size_t trsv_scaled_tag_words(int n);
 template <typename TA, typename TW>
 cudaError_t launch_scale_blocks(cudaStream_t stream, const TA* a, int64_t lda, const double* dinv_l,
@@ -51,7 +52,7 @@ cudaError_t launch_scale_blocks(cudaStream_t stream, const TA* a, int64_t lda, c
 template <typename TW>
 cudaError_t launch_trsv_scaled(cudaStream_t stream, const TW* w, int64_t ldw, const double* dinv, const double* b,
                                double* y, int64_t ldy, int n, bool lower, unsigned long long* xt, unsigned int epoch,
-                               int* ticket, DeviceStatus* st);
+                               int* ticket, int max_cluster, DeviceStatus* st);
 
 // Elements of the diagonal-block inverses for order n.
 size_t trsv_inverse_elems(int n);

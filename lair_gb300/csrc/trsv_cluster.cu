@@ -30,6 +30,7 @@ namespace luhot {
 constexpr int kTB = 64;         // block rows (the diagonal-inverse blocks)
 constexpr int kTCtas = 4;       // CTAs of a cluster
 constexpr int kTRows = 16;      // rows of a CTA
+constexpr int kTAhead = 3;      // tiles from memory to L2 ahead of their use
 
 template <int kNR>
 __host__ __device__ constexpr int tc_parts() {
@@ -177,6 +178,18 @@ __global__ void __launch_bounds__(tc_threads<kNR>())
       load_tile(block(s + 1), nv);
       if (polls) Word::load(word(block(s + 1)), w);
     }
+    if (kNR == 1 && s + kTAhead < nupd) {
+      // A later tile's lines from memory to L2 (n = 16384, 1 rhs 1725 -> 1544 us; chains
+      // of four, whose steps are longer, lose by it: 2206 -> 2277).
+      const int Jp = block(s + kTAhead) * kTB;
+      if (kTrans) {
+        const int k = Jp + tid / 2;
+        if (tid % 2 == 0 && k < n && i0 + rank * kTRows < n)
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(a + (int64_t)k * lda + i0 + rank * kTRows));
+      } else if (part < kTB * (int)sizeof(TA) / 128 && row < n && Jp + part * (128 / (int)sizeof(TA)) < n) {
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(a + (int64_t)row * lda + Jp + part * (128 / (int)sizeof(TA))));
+      }
+    }
     ok = __syncthreads_or(!ok) == 0;
     if (!ok) break;
 #pragma unroll
@@ -192,7 +205,8 @@ __global__ void __launch_bounds__(tc_threads<kNR>())
     for (int off = 1; off < kParts; off <<= 1) acc += __shfl_xor_sync(kFull, acc, off);
     if (part < kTCtas)
       cl_push8(cl_peer(cl_smem(&sums[r * kNR + c]), part), cl_peer(cl_smem(&bar), part), Word::bits(on ? acc : T(0)));
-    if (cl_wait(cl_smem(&bar), 0u, st, I)) {
+    ok = cl_wait(cl_smem(&bar), 0u, st, I);
+    if (ok) {
       T y = T(0);
 #pragma unroll
       for (int e = 0; e < kLen; ++e) y = fma(d[e], Word::from(sums[(part + kParts * e) * kNR + c]), y);
@@ -204,7 +218,8 @@ __global__ void __launch_bounds__(tc_threads<kNR>())
       }
     }
   }
-  cl_sync();  // no CTA leaves before the pushes to it have landed or its peers gave up
+  cl_sync();  // every push has been issued; those to this CTA have landed if it waited for them
+  if (!ok) cl_drain();
 }
 
 // Right-hand sides of one chain (at most 16 chains run in a launch).  FP64 sweeps
@@ -214,8 +229,8 @@ __global__ void __launch_bounds__(tc_threads<kNR>())
 // chains of 1 / 4: FP64 n = 2048, 8 rhs 212 / 288, n = 4097, 16 rhs 737 / 900, n =
 // 16384, 16 rhs 8098 / 9863; FP32 n = 2048, 16 rhs 110 / 101, n = 4097, 8 rhs 227 / 181,
 // 16 rhs 323 / 227, n = 16384, 4 rhs 1217 / 920.  (One CTA a block, flags and fences:
-// FP64 n = 1000, 1 rhs 174, now 98; 2048, 8 rhs 354; 4097, 16 rhs 1079; 16384, 16 rhs
-// 10145; FP32 n = 2048, 16 rhs 210, 4097, 8 rhs 375.)
+// FP64 n = 1000, 1 rhs 174, now 98; 2048, 8 rhs 354, now 208; 4097, 16 rhs 1079, now
+// 712; 16384, 16 rhs 10145, now 8003; FP32 n = 2048, 16 rhs 210, 4097, 8 rhs 375.)
 template <typename T>
 static int tc_width(int n, int nc) {
   return sizeof(T) == 4 && nc > 2 && (int64_t)n * nc > 30000 ? 4 : 1;

@@ -14,17 +14,23 @@
 // at this part's FP64 rate (about 1.6 FMA per clock per SM) those FMAs, not
 // the memory, bounded each step of the block chain.
 //
-// Order and publication follow the chained FP32 sweep (trsv_chain.cu): CTAs
-// take (block, quarter) tickets in sweep order and wait only for blocks of
-// earlier tickets, i.e. of CTAs already running; x(I) is published as
-// epoch-tagged words (two per FP64 value, each carrying the launch's epoch in
+// A thread-block cluster takes up to four consecutive blocks (a ticket per cluster,
+// in sweep order, so that it only waits for clusters already running): three of
+// four steps of the chain then go through distributed shared memory (cluster.cuh),
+// a one-way latency of some 300 cycles, in place of a store to L2 and a poll of it,
+// some 1700.  For the other clusters x(I) is published as in the chained FP32 sweep
+// (trsv_chain.cu), as epoch-tagged words (two per FP64 value, each carrying the launch's epoch in
 // its top half), which each warp polls with one 32-byte load per lane and a
 // vote, so the loop has no flags, fences or block barriers.
+// A step is now about as short as a load from memory, so tiles are requested into
+// L2 three steps ahead.  n = 6000, both sweeps: 297 us, with clusters 258 - 264, with
+// the requests 248.
 // Thread layout: 128 threads = 16 rows x 8 groups of 8 columns; each thread
 // keeps one partial sum, reduced over the 8 lanes of its row once at the end.
 // Every wait is bounded by the context's wait limit (LUHOT_ERR_TIMEOUT).
 #include <algorithm>
 
+#include "cluster.cuh"
 #include "common.cuh"
 #include "luhot_internal.h"
 #include "trsv.cuh"
@@ -35,6 +41,8 @@ constexpr int kSB = 64;         // block rows (the diagonal-inverse blocks)
 constexpr int kSParts = 4;      // CTAs per block
 constexpr int kSRows = 16;      // rows per CTA
 constexpr int kSThreads = 128;  // 16 rows x 8 column groups
+constexpr int kSBlocks = 4;     // blocks per cluster at most
+constexpr int kSAhead = 3;      // tiles from memory to L2 ahead of their use
 constexpr int kSLd = kSB + 1;
 
 // W(I, J) = D_I^-1 T(I, J) for every off-diagonal tile of one triangle, in
@@ -134,17 +142,33 @@ template <typename TW, bool kLower>
 __global__ void __launch_bounds__(kSThreads) trsv_scaled_kernel(const TW* __restrict__ w, int64_t ldw,
                                                                 const double* __restrict__ dinv,
                                                                 const double* __restrict__ b, double* y, int64_t ldy,
-                                                                int n, unsigned long long* xt, unsigned int epoch,
-                                                                int* ticket, DeviceStatus* st) {
+                                                                int n, int csize, unsigned long long* xt,
+                                                                unsigned int epoch, int* ticket, DeviceStatus* st) {
   __shared__ int s_ticket;
   __shared__ double s_x[kSThreads / 32][2][kSB];
-  if (threadIdx.x == 0) s_ticket = atomicAdd(ticket, 1);
-  __syncthreads();
+  __shared__ double s_in[kSBlocks][kSB];  // x of the cluster's earlier blocks
+  __shared__ __align__(8) unsigned long long s_bar[kSBlocks];
+  const int rank = blockIdx.x % csize, local = rank / kSParts, part = rank % kSParts, blocks = csize / kSParts;
+  if (threadIdx.x == 0) {
+    for (int q = 0; q < kSBlocks; ++q)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(cl_smem(&s_bar[q])));
+    asm volatile("fence.mbarrier_init.release.cluster;");
+    for (int q = 0; q < local; ++q) cl_expect(cl_smem(&s_bar[q]), kSB * 8u);
+    if (rank == 0) {
+      const int t = atomicAdd(ticket, 1);
+      for (int q = 0; q < csize; ++q)
+        asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cl_peer(cl_smem(&s_ticket), q)), "r"(t) : "memory");
+    }
+  }
+  cl_sync();
   const int nblk = (n + kSB - 1) / kSB;
-  const int t = s_ticket;
-  if (t >= nblk * kSParts) return;
-  const int I = kLower ? t / kSParts : nblk - 1 - t / kSParts;
-  const int part = t % kSParts;
+  const int first = s_ticket * blocks;  // the cluster's first block in sweep order
+  const int t = first + local;
+  if (t >= nblk) {  // past the last block: nothing is sent here
+    cl_sync();
+    return;
+  }
+  const int I = kLower ? t : nblk - 1 - t;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int r = threadIdx.x >> 3, kp = threadIdx.x & 7;
   const int rb = part * kSRows + r;  // row within the block
@@ -167,7 +191,7 @@ __global__ void __launch_bounds__(kSThreads) trsv_scaled_kernel(const TW* __rest
   if (nupd > 0) {
     const int J0 = kLower ? 0 : nblk - 1;
     scaled_load_row8(nxt, w, ldw, i, J0 * kSB + c8, n);
-    scaled_ld_quad(xt + 2 * (size_t)J0 * kSB + 4 * lane, q);
+    if (first > 0) scaled_ld_quad(xt + 2 * (size_t)J0 * kSB + 4 * lane, q);
   }
   const unsigned long long limit = st->timeout_ns;
   // Every branch below is warp-uniform (votes and shuffles), so a wait that
@@ -181,6 +205,17 @@ __global__ void __launch_bounds__(kSThreads) trsv_scaled_kernel(const TW* __rest
 #pragma unroll
     for (int e = 0; e < 8; ++e) cur[e] = nxt[e];
     if (s + 1 < nupd) scaled_load_row8(nxt, w, ldw, i, (kLower ? s + 1 : nblk - 2 - s) * kSB + c8, n);
+    if (s + kSAhead < nupd && i < n && (kp & 1) == 0) {
+      const int jp = (kLower ? s + kSAhead : nblk - 1 - s - kSAhead) * kSB + c8;
+      if (jp < n) asm volatile("prefetch.global.L2 [%0];" ::"l"(w + (int64_t)i * ldw + jp));
+    }
+    if (s >= first) {  // a block of this cluster
+      alive = cl_wait(cl_smem(&s_bar[s - first]), 0u, st, J);
+      if (!alive) break;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) acc = fma(-cur[e], s_in[s - first][c8 + e], acc);
+      continue;
+    }
     unsigned long long t0 = 0;
     unsigned int spins = 0;
     while (!__all_sync(0xffffffffu, scaled_quad_ok(q, lane, count, epoch))) {
@@ -208,7 +243,7 @@ __global__ void __launch_bounds__(kSThreads) trsv_scaled_kernel(const TW* __rest
     double* xb = s_x[warp][s & 1];
     xb[2 * lane] = 2 * lane < count ? scaled_decode(q[0], q[1]) : 0.0;
     xb[2 * lane + 1] = 2 * lane + 1 < count ? scaled_decode(q[2], q[3]) : 0.0;
-    if (s + 1 < nupd) scaled_ld_quad(xt + 2 * (size_t)(kLower ? s + 1 : nblk - 2 - s) * kSB + 4 * lane, q);
+    if (s + 1 < first) scaled_ld_quad(xt + 2 * (size_t)(kLower ? s + 1 : nblk - 2 - s) * kSB + 4 * lane, q);
     __syncwarp();
 #pragma unroll
     for (int e = 0; e < 8; ++e) acc = fma(-cur[e], xb[c8 + e], acc);
@@ -217,12 +252,21 @@ __global__ void __launch_bounds__(kSThreads) trsv_scaled_kernel(const TW* __rest
   acc += __shfl_xor_sync(0xffffffffu, acc, 1);
   acc += __shfl_xor_sync(0xffffffffu, acc, 2);
   acc += __shfl_xor_sync(0xffffffffu, acc, 4);
+  if (alive) {
+    // To the CTAs of the cluster's later blocks, a lane each (rows past n: zero).
+    const int last = min(blocks, nblk - first);  // of the cluster's blocks
+    for (int q = (local + 1) * kSParts + kp; q < last * kSParts; q += 8)
+      cl_push8(cl_peer(cl_smem(&s_in[local][rb]), q), cl_peer(cl_smem(&s_bar[local]), q),
+               (unsigned long long)__double_as_longlong(i < n ? acc : 0.0));
+  }
   if (alive && kp == 0 && i < n) {
     y[(int64_t)i * ldy] = acc;
     const unsigned long long bits = (unsigned long long)__double_as_longlong(acc);
     scaled_st_word(xt + 2 * (size_t)i, (unsigned int)(bits >> 32), epoch);
     scaled_st_word(xt + 2 * (size_t)i + 1, (unsigned int)bits, epoch);
   }
+  cl_sync();
+  if (!alive) cl_drain();
 }
 
 size_t trsv_scaled_tag_words(int n) { return (size_t)((n + kSB - 1) / kSB) * kSB * 2; }
@@ -245,16 +289,19 @@ cudaError_t launch_scale_blocks(cudaStream_t stream, const TA* a, int64_t lda, c
 template <typename TW>
 cudaError_t launch_trsv_scaled(cudaStream_t stream, const TW* w, int64_t ldw, const double* dinv, const double* b,
                                double* y, int64_t ldy, int n, bool lower, unsigned long long* xt, unsigned int epoch,
-                               int* ticket, DeviceStatus* st) {
+                               int* ticket, int max_cluster, DeviceStatus* st) {
   if (n <= 0) return cudaSuccess;
   cudaError_t e = cudaMemsetAsync(ticket, 0, sizeof(int), stream);
   if (e != cudaSuccess) return e;
-  const int grid = ((n + kSB - 1) / kSB) * kSParts;
-  if (lower)
-    trsv_scaled_kernel<TW, true><<<grid, kSThreads, 0, stream>>>(w, ldw, dinv, b, y, ldy, n, xt, epoch, ticket, st);
-  else
-    trsv_scaled_kernel<TW, false><<<grid, kSThreads, 0, stream>>>(w, ldw, dinv, b, y, ldy, n, xt, epoch, ticket, st);
-  return cudaGetLastError();
+  const int nblk = (n + kSB - 1) / kSB;
+  const int blocks = std::max(1, std::min(kSBlocks, max_cluster / kSParts)), csize = blocks * kSParts;
+  auto k = lower ? trsv_scaled_kernel<TW, true> : trsv_scaled_kernel<TW, false>;
+  e = allow_wide_clusters(reinterpret_cast<const void*>(k));
+  if (e != cudaSuccess) return e;
+  cudaLaunchAttribute attr;
+  cudaLaunchConfig_t cfg = cl_config(csize, kSThreads, 0, stream, &attr);
+  cfg.gridDim = dim3((nblk + blocks - 1) / blocks * csize);
+  return cudaLaunchKernelEx(&cfg, k, w, ldw, dinv, b, y, ldy, n, csize, xt, epoch, ticket, st);
 }
 
 template cudaError_t launch_scale_blocks<double, double>(cudaStream_t, const double*, int64_t, const double*,
@@ -262,7 +309,7 @@ template cudaError_t launch_scale_blocks<double, double>(cudaStream_t, const dou
 template cudaError_t launch_scale_blocks<float, double>(cudaStream_t, const float*, int64_t, const double*,
                                                         const double*, double*, int64_t, int);
 template cudaError_t launch_trsv_scaled<double>(cudaStream_t, const double*, int64_t, const double*, const double*,
-                                                double*, int64_t, int, bool, unsigned long long*, unsigned int, int*,
+                                                double*, int64_t, int, bool, unsigned long long*, unsigned int, int*, int,
                                                 DeviceStatus*);
 
 }  // namespace luhot

@@ -11,7 +11,7 @@ import ctypes
 import numpy as np
 import pytest
 
-from lair_gb300 import _lib, lapack
+from lair_gb300 import _lib, lapack, lu
 
 pytestmark = pytest.mark.gpu
 
@@ -22,12 +22,12 @@ def system(n, nrhs, dtype, seed):
     return a, rng.standard_normal((n, nrhs)).astype(dtype)
 
 
-def solve_dev(torch, lu, piv, b, ldb, trans, mode):
+def solve_dev(torch, fac, piv, b, ldb, trans, mode):
     lib, ctx = _lib.load(), _lib.context()
     n, nrhs = b.shape
     wide = np.full((n, ldb), 7.0, b.dtype)
     wide[:, :nrhs] = b
-    d_lu, d_b = torch.from_numpy(lu).cuda(), torch.from_numpy(wide).cuda()
+    d_lu, d_b = torch.from_numpy(fac).cuda(), torch.from_numpy(wide).cuda()
     d_p = torch.tensor(piv, dtype=torch.int32, device="cuda")
     torch.cuda.synchronize()
     fn = lib.luhot_dgetrs_dev if b.dtype == np.float64 else lib.luhot_sgetrs_dev
@@ -45,15 +45,15 @@ def solve_dev(torch, lu, piv, b, ldb, trans, mode):
 def test_sweeps(n, nrhs, pad, dtype):
     torch = pytest.importorskip("torch")
     a, b = system(n, nrhs, dtype, 3 * n + nrhs)
-    lu = a.copy()
-    piv, _ = lapack.getrf(lu, mode="fast")
+    fac = a.copy()
+    piv, _ = lapack.getrf(fac, mode="fast")
     eps = np.finfo(dtype).eps
     for trans in (0, 1):
         want = np.linalg.solve((a.T if trans else a).astype(np.float64), b.astype(np.float64))
         tol = 8 * n * eps * np.abs(want).max()
-        got = solve_dev(torch, lu, piv, b, nrhs + pad, trans, 0)
+        got = solve_dev(torch, fac, piv, b, nrhs + pad, trans, 0)
         assert np.abs(got - want).max() <= tol
-        exact = solve_dev(torch, lu, piv, b, nrhs + pad, trans, 1)
+        exact = solve_dev(torch, fac, piv, b, nrhs + pad, trans, 1)
         assert np.abs(got - exact).max() <= 2 * tol
 
 
@@ -62,9 +62,21 @@ def test_sweeps_many_blocks():
     torch = pytest.importorskip("torch")
     n, nrhs = 9001, 5
     a, b = system(n, nrhs, np.float64, 1)
-    lu = a.copy()
-    piv, _ = lapack.getrf(lu, mode="fast")
+    fac = a.copy()
+    piv, _ = lapack.getrf(fac, mode="fast")
     for trans in (0, 1):
-        got = solve_dev(torch, lu, piv, b, nrhs, trans, 0)
+        got = solve_dev(torch, fac, piv, b, nrhs, trans, 0)
         res = np.abs((a.T if trans else a) @ got - b).max()
         assert res <= 8 * n * np.finfo(float).eps * np.abs(b).max()
+
+
+@pytest.mark.parametrize("n", [1, 63, 64, 65, 128, 129, 255, 256, 257, 320, 321, 1000, 2049])
+def test_resident_sweeps_in_clusters(n):
+    """One right-hand side on resident factors (trsv_scaled.cu): fewer blocks than
+    a cluster takes, whole clusters, one block and one row more; solved twice."""
+    a, b = system(n, 1, np.float64, 11 * n)
+    f = lu.Factorized(a.copy(), device_resident=True)
+    want = np.linalg.solve(a, b[:, 0])
+    for _ in range(2):
+        got = np.asarray(f.solve(b[:, 0]))
+        assert np.abs(got - want).max() <= 8 * n * np.finfo(float).eps * np.abs(want).max()
