@@ -1330,8 +1330,10 @@ static int getrf_impl(luhot_ctx* ctx, int m, int n, T* a, int64_t lda, int* piv,
                       cudaStream_t stream) {
   const int dim_min = std::min(m, n);
   // Exchange words carry step tags; clear them so no word of an earlier
-  // factorization carries a live tag.
-  LUHOT_CUDA_TRY(ctx, cudaMemsetAsync(ctx->panel_scratch, 0, kPanelScratchBytes, stream));
+  // factorization carries a live tag.  Cluster panels exchange none, and once a panel
+  // fits a cluster all that follow do.
+  if (!panel_cluster_fits<T>(ctx, m, nb))
+    LUHOT_CUDA_TRY(ctx, cudaMemsetAsync(ctx->panel_scratch, 0, kPanelScratchBytes, stream));
   for (int k0 = 0; k0 < dim_min; k0 += nb) {
     if constexpr (std::is_same<T, double>::value && !kExact) {
       const int64_t M2 = m - k0 - 2 * nb, N2 = n - k0 - 2 * nb;
