@@ -1251,13 +1251,25 @@ static int la_setup(luhot_ctx* ctx) {
 // so that at most two steps are under way; their lists of moved rows alternate.
 // Takes the steps from k0 on while la_pays; returns the first one it left in k0.
 // The price is two launches more a step on the panels' way, some 40 us, so that it
-// pays while the block behind the next panel is large.  ms, FP64 / FP32, step by
-// step against with look-ahead: n = 1000 1.69 -> 1.69 (1.71 with a limit of 500000) /
-// 1.25 -> 1.25, 2000 4.29 -> 4.17 / 3.07 -> 2.86, 3000 8.07 -> 7.41 / 5.36 -> 4.56.
+// pays while the block behind the next panel is large; and the rest of the step has
+// only the SMs that the panel leaves, so that it pays while rest + panel in turn take
+// longer than the rest on those alone (rest P <= panel (SMs - P)): not beside a
+// panel on many SMs when the update is long (n = 16384, DMMA updates: 2.9 s in turn,
+// 7.5 s beside 96-CTA panels).  us: a panel as measured; an element of an update by
+// slices 5.0e-6, by DMMA 1.16e-4, FP32 2.5e-6.  ms, FP64 / FP32, step by step against
+// with look-ahead: n = 1000 1.69 -> 1.69 (1.71 with a limit of 500000) / 1.25 -> 1.25,
+// 2000 4.29 -> 4.17 / 3.07 -> 2.86, 3000 8.07 -> 7.41 / 5.36 -> 4.56.
 template <typename T>
-static bool la_pays(int m, int n, int k0, int nb) {
+static bool la_pays(luhot_ctx* ctx, const void* oz_ws, int m, int n, int k0, int nb) {
   const int64_t M = m - k0 - 2 * nb, N = n - k0 - 2 * nb;
-  return M > 0 && N > 0 && M * N >= (sizeof(T) == 8 ? 1000000 : 500000);
+  if (M <= 0 || N <= 0 || M * N < (sizeof(T) == 8 ? 1000000 : 500000)) return false;
+  const int rows = m - k0 - nb;
+  const bool cluster = panel_cluster_fits<T>(ctx, rows, nb);
+  const int P = cluster ? ctx->panel_cluster : panel_ctas<T>(ctx, rows);
+  const double panel = sizeof(T) == 8 ? (cluster ? 100.0 : 200.0) : (cluster ? 70.0 : 150.0);
+  const bool slices = sizeof(T) == 8 && update_on_slices(oz_ws, ctx->fp64_update, (int)M, (int)N);
+  const double rest = (double)M * N * (sizeof(T) == 4 ? 2.5e-6 : slices ? 5.0e-6 : 1.16e-4) * nb / 64;
+  return rest * P <= panel * (ctx->num_sms - P);
 }
 
 template <typename T>
@@ -1278,7 +1290,7 @@ static int la_loop(luhot_ctx* ctx, int m, int n, T* a, int64_t lda, int* piv, in
     return launch_gemm<T, false>(ctx, a, lda, r1, c0, k0, nb, M, N, st);
   };
   int k0 = *k0_io;
-  for (int step = 0; la_pays<T>(m, n, k0, nb); ++step, k0 += nb) {
+  for (int step = 0; la_pays<T>(ctx, oz_ws, m, n, k0, nb); ++step, k0 += nb) {
     const int par = step & 1, k1 = k0 + nb, e1 = k1 + nb;
     int* mv = la_saved_moves(ctx, par, 0);
     {
@@ -1346,7 +1358,7 @@ static int getrf_impl(luhot_ctx* ctx, int m, int n, T* a, int64_t lda, int* piv,
       }
     }
     if constexpr (!kExact) {
-      if (la_pays<T>(m, n, k0, nb)) {
+      if (la_pays<T>(ctx, oz_ws, m, n, k0, nb)) {
         int rc = la_fork_join(ctx, stream, [&] { return la_loop<T>(ctx, m, n, a, lda, piv, nb, oz_ws, oz_hi, &k0); });
         if (rc) return rc;
       }
