@@ -1251,25 +1251,28 @@ static int la_setup(luhot_ctx* ctx) {
 // so that at most two steps are under way; their lists of moved rows alternate.
 // Takes the steps from k0 on while la_pays; returns the first one it left in k0.
 // The price is two launches more a step on the panels' way, some 40 us, so that it
-// pays while the block behind the next panel is large; and the rest of the step has
-// only the SMs that the panel leaves, so that it pays while rest + panel in turn take
-// longer than the rest on those alone (rest P <= panel (SMs - P)): not beside a
-// panel on many SMs when the update is long (n = 16384, DMMA updates: 2.9 s in turn,
-// 7.5 s beside 96-CTA panels).  us: a panel as measured; an element of an update by
-// slices 5.0e-6, by DMMA 1.16e-4, FP32 2.5e-6.  ms, FP64 / FP32, step by step against
-// with look-ahead: n = 1000 1.69 -> 1.69 (1.71 with a limit of 500000) / 1.25 -> 1.25,
-// 2000 4.29 -> 4.17 / 3.07 -> 2.86, 3000 8.07 -> 7.41 / 5.36 -> 4.56.
+// pays while the block behind the next panel is large.  FP64 updates are persistent
+// kernels on the SMs that the panel leaves, so that it pays, besides, while rest +
+// panel in turn take longer than the rest on those alone (rest P <= panel (SMs - P)):
+// not beside a panel on many SMs when the update is long (n = 16384, DMMA updates:
+// 2.9 s in turn, 7.5 s beside 96-CTA panels).  us: a panel as measured; an element of
+// an update by slices 5.0e-6, by DMMA 1.16e-4.  FP32 updates are many short CTAs, which
+// take what is free (n = 16384: 171 ms in turn until panels are a cluster's, 162 beside).
+// ms, FP64 / FP32, step by step against with look-ahead: n = 1000 1.69 -> 1.69 (1.71 with
+// a limit of 500000) / 1.25 -> 1.25, 2000 4.29 -> 4.17 / 3.07 -> 2.86, 3000 8.07 -> 7.41 /
+// 5.36 -> 4.56.
 template <typename T>
 static bool la_pays(luhot_ctx* ctx, const void* oz_ws, int m, int n, int k0, int nb) {
   const int64_t M = m - k0 - 2 * nb, N = n - k0 - 2 * nb;
-  if (M <= 0 || N <= 0 || M * N < (sizeof(T) == 8 ? 1000000 : 500000)) return false;
+  if (M <= 0 || N <= 0) return false;
+  if (sizeof(T) == 4) return M * N >= 500000;
+  if (M * N < 1000000) return false;
   const int rows = m - k0 - nb;
   const bool cluster = panel_cluster_fits<T>(ctx, rows, nb);
   const int P = cluster ? ctx->panel_cluster : panel_ctas<T>(ctx, rows);
-  const double panel = sizeof(T) == 8 ? (cluster ? 100.0 : 200.0) : (cluster ? 70.0 : 150.0);
-  const bool slices = sizeof(T) == 8 && update_on_slices(oz_ws, ctx->fp64_update, (int)M, (int)N);
-  const double rest = (double)M * N * (sizeof(T) == 4 ? 2.5e-6 : slices ? 5.0e-6 : 1.16e-4) * nb / 64;
-  return rest * P <= panel * (ctx->num_sms - P);
+  const bool slices = update_on_slices(oz_ws, ctx->fp64_update, (int)M, (int)N);
+  const double rest = (double)M * N * (slices ? 5.0e-6 : 1.16e-4) * nb / 64;
+  return rest * P <= (cluster ? 100.0 : 200.0) * (ctx->num_sms - P);
 }
 
 template <typename T>
