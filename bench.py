@@ -850,7 +850,7 @@ def run_qr(args, lib, ctx, torch):
     return {"workload": f"Householder QR (geqrf, fast mode) of an n x n N(0,1) matrix, n={n}", "n": n,
             "ms": ms, "gflops": 4.0 / 3.0 * n ** 3 / (ms * 1e-3) / 1e9,
             "residual_max_rel": resid, "orthogonality_max": orth,
-            "bound": "FP64 pipe and HBM at the ridge (level-2 Householder, 4/3 n^3 flops over ~8 n^3 bytes)"}
+            "bound": "FP64 pipe (panels and W = V^T A of the blocked form; the updates run on the FP16 slices)"}
 
 
 def run_batched(args, lib, ctx, torch):
