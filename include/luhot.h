@@ -67,7 +67,9 @@ int luhot_create(luhot_ctx** out, int device);
 void luhot_destroy(luhot_ctx* ctx);
 /* Message of the last failed call on this context ("" if none). */
 const char* luhot_last_error(const luhot_ctx* ctx);
-/* Run subsequent calls on a caller-owned cudaStream_t (NULL: own stream). */
+/* Run subsequent calls on a caller-owned cudaStream_t (NULL: own stream).  The
+ * calls of a context share its workspace and this call orders no streams: before
+ * it, wait for a call on the old stream that was asynchronous. */
 int luhot_set_stream(luhot_ctx* ctx, void* cuda_stream);
 /* Panel width override (0 = default 64); for tuning and tests. */
 int luhot_set_block(luhot_ctx* ctx, int nb);
@@ -312,7 +314,10 @@ void luhot_factor_destroy(luhot_factor* f);
  * separately rounded products and sums) bit for bit. */
 int luhot_dgeqrf(luhot_ctx* ctx, int64_t m, int64_t n, double* a, int64_t rs, int64_t cs, double* tau, int mode);
 int luhot_sgeqrf(luhot_ctx* ctx, int64_t m, int64_t n, float* a, int64_t rs, int64_t cs, float* tau, int mode);
-/* Same on a row-major device matrix (leading dimension lda) and device tau. */
+/* Same on a row-major device matrix (leading dimension lda) and device tau.
+ * LUHOT_MODE_FAST with min(m, n) >= 32 waits for its result and reports a device
+ * wait that ran out (LUHOT_ERR_TIMEOUT), as luhot_dgetrf_dev does; other calls, and
+ * calls on a stream under capture, are asynchronous on the context's stream. */
 int luhot_dgeqrf_dev(luhot_ctx* ctx, int64_t m, int64_t n, double* d_a, int64_t lda, double* d_tau, int mode);
 /* Q (m x m, written with element strides q_rs, q_cs) from a factored array
  * and tau: lair's qr::Factorized::q (src/decomposition/qr.rs:26-60). */

@@ -409,7 +409,13 @@ int geqrf_device(luhot_ctx* ctx, int m, int n, T* d_a, int64_t lda, T* d_tau, in
     return set_error(ctx, LUHOT_ERR_INVALID_ARG, "geqrf: unknown mode");
   if (m == 0 || n == 0) return LUHOT_OK;
   if constexpr (std::is_same<T, double>::value) {
-    if (mode == LUHOT_MODE_FAST && geqrf_blocked_fits(ctx, m, n)) return geqrf_blocked(ctx, m, n, d_a, lda, d_tau);
+    if (mode == LUHOT_MODE_FAST && geqrf_blocked_fits(ctx, m, n)) {
+      // The blocked form ends with a look at the device status, which a stream
+      // under capture does not allow: there the level-2 form, which has no waits.
+      cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+      LUHOT_CUDA_TRY(ctx, cudaStreamIsCapturing(ctx->stream, &capture));
+      if (capture == cudaStreamCaptureStatusNone) return geqrf_blocked(ctx, m, n, d_a, lda, d_tau);
+    }
   }
   return mode == LUHOT_MODE_EXACT ? geqrf_impl<T, true>(ctx, m, n, d_a, lda, d_tau)
                                   : geqrf_impl<T, false>(ctx, m, n, d_a, lda, d_tau);
@@ -431,10 +437,6 @@ int geqrf_host(luhot_ctx* ctx, int64_t m, int64_t n, T* a, int64_t rs, int64_t c
   if (rc) return rc;
   rc = geqrf_device<T>(ctx, (int)m, (int)n, d_a, lda, d_tau, mode);
   if (rc) return rc;
-  if (std::is_same<T, double>::value && mode == LUHOT_MODE_FAST && geqrf_blocked_fits(ctx, (int)m, (int)n)) {
-    rc = finish_status(ctx, nullptr);  // its panels wait on one another
-    if (rc) return rc;
-  }
   rc = stage_out<T>(ctx, d_a, lda, a, m, n, rs, cs, ctx->work[1]);
   if (rc) return rc;
   LUHOT_CUDA_TRY(ctx, cudaMemcpy(tau, d_tau, (size_t)k * sizeof(T), cudaMemcpyDeviceToHost));

@@ -444,7 +444,9 @@ int geqrf_blocked(luhot_ctx* ctx, int m, int n, double* a, int64_t lda, double* 
       LUHOT_CUDA_TRY(ctx, cudaGetLastError());
     }
   }
-  return LUHOT_OK;
+  // Its panels wait on one another: a wait that gave up is reported by this call, and
+  // the status and workspace are free when it returns.
+  return finish_status(ctx, nullptr);
 }
 
 }  // namespace luhot

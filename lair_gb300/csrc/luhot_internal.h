@@ -127,7 +127,8 @@ int copy_2d(luhot_ctx* ctx, void* dst, size_t dpitch, const void* src, size_t sp
             cudaMemcpyKind kind);
 
 // Blocked Householder QR of fast-mode FP64 (geqrf_blocked.cu): whether it takes
-// an m x n matrix, and the factorization (asynchronous; A and tau in device memory).
+// an m x n matrix, and the factorization (A and tau in device memory), which waits
+// for its result and reads the device status.
 bool geqrf_blocked_fits(luhot_ctx* ctx, int m, int n);
 int geqrf_blocked(luhot_ctx* ctx, int m, int n, double* a, int64_t lda, double* tau);
 
