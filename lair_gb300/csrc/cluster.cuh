@@ -44,7 +44,8 @@ __device__ __forceinline__ unsigned cl_try(unsigned bar, unsigned parity) {
 }
 // Bounded wait of a whole warp; false (for all lanes) once it gave up.  The loop is
 // kept out of line: a column's chain runs through its code once a column on one
-// warp, so that the length of that code is itself part of the chain.
+// warp, so that the length of that code is itself part of the chain.  The lanes read
+// clocks of their own: whichever passes the limit first, lane 0 records it.
 static __device__ __noinline__ bool cl_wait_long(unsigned bar, unsigned parity, DeviceStatus* st, int step) {
   unsigned long long t0 = 0;
   for (unsigned spins = 1;; ++spins) {
@@ -52,8 +53,8 @@ static __device__ __noinline__ bool cl_wait_long(unsigned bar, unsigned parity, 
     if ((spins & 15u) == 0) {
       const unsigned long long now = global_timer_ns();
       if (t0 == 0) t0 = now;
-      const bool late = now - t0 > st->timeout_ns;
-      if (__any_sync(0xffffffffu, late || ld_relaxed_i32(&st->abort) != 0)) {
+      const bool late = __any_sync(0xffffffffu, now - t0 > st->timeout_ns);
+      if (late || __any_sync(0xffffffffu, ld_relaxed_i32(&st->abort) != 0)) {
         if (late && (threadIdx.x & 31) == 0) {
           atomicCAS(&st->error, kDevOk, kDevBarrierTimeout);
           atomicExch(&st->timeout_where, (unsigned long long)step);
