@@ -272,6 +272,7 @@ __global__ void back_exact_kernel(const T* u, int64_t lda, T* x, int64_t ldx, in
     T p[32];
 #pragma unroll
     for (int q = 0; q < 32; ++q) p[q] = buf[0][q];
+    __syncwarp();  // the first pass below writes buf[0] again
     int k0 = i + 1;
     for (int par = 1; k0 + 32 <= n; k0 += 32, par ^= 1) {
       const int kn = k0 + 64 + lane;  // two blocks on

@@ -29,8 +29,8 @@ static int ld_relaxed_i32(const int* p) { return __atomic_load_n(p, __ATOMIC_REL
 
 
 @pytest.mark.parametrize("first", [0, 1, 31, -1])
-def test_a_wait_that_gives_up_records_it(tmp_path, first):
+def test_a_wait_that_gives_up_records_it(first):
     body = BODY + warp.extract("cluster.cuh", "static __device__ __noinline__ bool cl_wait_long")
-    gave_up, error, abort, where = map(int, warp.run(tmp_path, body, MAIN, [first]).split())
+    gave_up, error, abort, where = map(int, warp.run(body, MAIN, [first]).split())
     assert gave_up == 32
     assert (error, abort, where) == ((1, 1, 7) if first >= 0 else (0, 1, 0))

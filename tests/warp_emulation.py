@@ -7,9 +7,11 @@ that lanes drift apart as far as the function's own barriers let them.
 prints.  It is test infrastructure: it shows what depends on the lanes of a warp
 running in step, which a GPU run does not.
 """
+import functools
 import os
 import re
 import subprocess
+import tempfile
 
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "lair_gb300", "csrc")
 
@@ -27,7 +29,7 @@ SHIM = r"""
 #define __forceinline__ inline
 #define __noinline__ __attribute__((noinline))
 #define __shared__ static
-#define __align__(n) alignas(n)
+#define __align__(n) __attribute__((aligned(n)))
 struct Index { int x = 0; };
 static thread_local Index threadIdx, blockIdx;
 static std::barrier<> warp_barrier(32);
@@ -61,12 +63,19 @@ def extract(source: str, start: str) -> str:
     return text[at:re.compile(r"^\};?$", re.M).search(text, at).end()]
 
 
-def run(tmp_path, body: str, main: str, args=()) -> str:
-    src, exe = tmp_path / "warp.cpp", tmp_path / "warp"
-    src.write_text(SHIM + body + main)
-    cmd = ["g++", "-std=c++20", "-O1", "-ffp-contract=off", "-pthread", "-w", str(src), "-o", str(exe)]
+@functools.lru_cache(maxsize=None)
+def _program(code: str):
+    where = tempfile.TemporaryDirectory()
+    src, exe = os.path.join(where.name, "warp.cpp"), os.path.join(where.name, "warp")
+    with open(src, "w") as f:
+        f.write(code)
+    cmd = ["g++", "-std=c++20", "-O1", "-ffp-contract=off", "-pthread", "-w", src, "-o", exe]
     r = subprocess.run(cmd, capture_output=True, text=True)
     assert r.returncode == 0, r.stderr
-    r = subprocess.run([str(exe), *map(str, args)], capture_output=True, text=True, timeout=300)
+    return where, exe  # the folder lives as long as the program is kept
+
+
+def run(body: str, main: str, args=()) -> str:
+    r = subprocess.run([_program(SHIM + body + main)[1], *map(str, args)], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr
     return r.stdout
