@@ -228,7 +228,7 @@ def workload_config(args):
     return {"workload": f"plain FP64 getrf+getrs drop-in, n={args.n}, nrhs={args.nrhs}, A,B iid N(0,1) seeded "
                         "(portable generator, lair_gb300.synthetic)",
             "n": args.n, "nrhs": args.nrhs, "mode": args.mode,
-            "fp64_update": {"auto": "FP16 tensor cores, exact integer slices (Ozaki), on trailing blocks > 50000 elements; "
+            "fp64_update": {"auto": "FP16 tensor cores, exact integer slices (Ozaki), on trailing blocks >= 256 x 256; "
                                     "DMMA below",
                             "dmma": "FP64 tensor cores (DMMA) only",
                             "ozaki": "FP16 tensor cores, exact integer slices, on every block >= 128 x 64"}[

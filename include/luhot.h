@@ -74,11 +74,15 @@ int luhot_set_stream(luhot_ctx* ctx, void* cuda_stream);
 /* Panel width override (0 = default 64); for tuning and tests. */
 int luhot_set_block(luhot_ctx* ctx, int nb);
 /* Schur-update engine of fast-mode FP64 getrf (no lair counterpart).
- * LUHOT_UPDATE_AUTO (default): trailing blocks of more than 50 000 elements
- * (at least 128 x 64) are updated on the FP16 tensor cores by an exact
- * integer-slice product (Ozaki scheme: seven 8-bit slices per operand, 28 slice
- * products, FP32 sums that are exact, one FP64 rounding; error at or below an
- * FP64 GEMM's), smaller ones on the FP64 tensor cores (DMMA).
+ * LUHOT_UPDATE_AUTO (default): trailing blocks of at least 256 x 256 are
+ * updated on the FP16 tensor cores by an exact integer-slice product (Ozaki
+ * scheme: seven 8-bit slices per operand, 28 slice products, FP32 sums that are
+ * exact, one FP64 rounding), smaller ones on the FP64 tensor cores (DMMA).  The
+ * slices hold each operand to 2^-57 of the largest element of its row of L21
+ * (column of U12), and the dropped products are below 2^-49 of the product of
+ * those two largest: at or below an FP64 GEMM's error where rows and columns are
+ * of one scale, but not relative to |L21| |U12| where a row's large elements meet
+ * only a column's small ones.
  * LUHOT_UPDATE_DMMA: DMMA updates only.
  * LUHOT_UPDATE_OZAKI: the tensor-core product on every block of at least
  * 128 x 64.  Exact mode and FP32 ignore the setting. */

@@ -1151,16 +1151,19 @@ static int launch_laswp_cols(luhot_ctx* ctx, T* a, int64_t lda, const int* moves
   return LUHOT_OK;
 }
 
-// Whether the trailing update of M rows and N columns runs on the FP16 tensor
-// cores as a slice product (ozaki.cu).  One takes some 8 us for up to a tile of 64 x
-// 128 per SM; FP64 arithmetic 14 us for 8 million multiply-adds (K = 64: 128 000
-// elements) on all SMs, and 9 us for the tile of 16 x 32 that one takes.  ms a
-// factorization with the line at 200 000 / 50 000 / 25 000 elements: n = 500 0.780 /
-// 0.746 / 0.745, 700 1.126 / 1.095 / 1.093, 1000 1.715 / 1.684 / 1.685; n = 4097 (whose
-// panels wait for updates of 64 columns) 13.56 / 13.14 / 13.13 with the solve.
+// Whether the update of a trailing block of M rows and N columns runs on the FP16
+// tensor cores as slice products (ozaki.cu).  M and N are those of the whole block
+// behind a panel, whatever part of it a launch takes: an element's digits come from
+// its row of L21 and its column of U12 alone, so that every part gives the same bits.
+// AUTO takes blocks of at least 256 x 256.  Smaller ones would gain a little (one
+// product takes some 8 us for up to a tile of 64 x 128 per SM, FP64 arithmetic 9 us
+// for the tile of 16 x 32 that each SM takes at 128 000 elements; factorizations of
+// n = 500 0.745 against 0.780 ms with the line at 25 000 / 200 000 elements, 1000
+// 1.685 / 1.715), but slices hold the elements relative to the largest of their row or
+// column, where FP64 arithmetic holds each to its own 53 bits.
 static bool update_on_slices(const void* oz_ws, int engine, int M, int N) {
-  if (!oz_ws || engine == LUHOT_UPDATE_DMMA || M < 128 || N < 64) return false;
-  return engine == LUHOT_UPDATE_OZAKI || (int64_t)M * N > 50000;
+  if (!oz_ws || engine == LUHOT_UPDATE_DMMA) return false;
+  return engine == LUHOT_UPDATE_OZAKI ? M >= 128 && N >= 64 : M >= 256 && N >= 256;
 }
 
 // Workspace of the tensor-core FP64 update for an m x n factorization
@@ -1270,7 +1273,7 @@ static bool la_pays(luhot_ctx* ctx, const void* oz_ws, int m, int n, int k0, int
   const int rows = m - k0 - nb;
   const bool cluster = panel_cluster_fits<T>(ctx, rows, nb);
   const int P = cluster ? ctx->panel_cluster : panel_ctas<T>(ctx, rows);
-  const bool slices = update_on_slices(oz_ws, ctx->fp64_update, (int)M, (int)N);
+  const bool slices = update_on_slices(oz_ws, ctx->fp64_update, rows, n - k0 - nb);
   const double rest = (double)M * N * (slices ? 5.0e-6 : 1.16e-4) * nb / 64;
   return rest * P <= (cluster ? 100.0 : 200.0) * (ctx->num_sms - P);
 }
@@ -1282,7 +1285,7 @@ static int la_loop(luhot_ctx* ctx, int m, int n, T* a, int64_t lda, int* piv, in
   // Columns [c0, c1) of step k0: interchanges (also on [0, cl1)), rows of U, update.
   auto columns = [&](const int* mv, int k0, int cl1, int c0, int c1, void* ws, cudaStream_t st) -> int {
     const int r1 = k0 + nb, M = m - r1, N = c1 - c0;
-    const bool slices = std::is_same<T, double>::value && update_on_slices(ws, ctx->fp64_update, M, N);
+    const bool slices = std::is_same<T, double>::value && update_on_slices(ws, ctx->fp64_update, M, n - r1);
     SplitOut split;
     if (slices) split = ozaki_split_out(ws, r1, M, N);
     int rc = launch_swap_solve<T, false>(ctx, a, lda, mv, k0, nb, 0, cl1, c0, c1, slices ? &split : nullptr, st);
