@@ -1,6 +1,6 @@
 // FP64 Schur update on the FP16 tensor cores (Ozaki scheme).
 //
-//   C (M x N, FP64, row-major, ldc)  -=  L (M x K) U (K x N),   K <= 64
+//   C (M x N, FP64, row-major, ldc)  -=  L (M x K) U (K x N),   K <= 128
 //
 // This part runs FP64 at about 2 FMA per clock per SM and FP16 tensor-core
 // products at 4096 per clock, so fast-mode FP64 trailing updates are computed
@@ -8,7 +8,8 @@
 //
 // Split (oz_split_rows_kernel for L, oz_split_cols_kernel for U).  Row i of L
 //   gets the exponent ea[i] with max_k |L(i,k)| < 2^ea[i], column j of U the
-//   exponent eb[j].  Each element x of a row (column) with exponent e is
+//   exponent eb[j] (K > 64: one for both halves of 64, unless they lie apart, see
+//   kOzApart).  Each element x of a row (column) with exponent e is
 //   rounded to the 56-bit integer N = round(|x| 2^(56-e)) and written as seven
 //   balanced base-256 digits, most significant first:
 //       x = sign(x) 2^e sum_{p=0..6} d_p 2^(-8(p+1))    (error <= 2^(e-57)),
@@ -22,9 +23,11 @@
 //   for K <= 128 but for group 6, whose two K halves have an accumulator each, so
 //   the FP32 accumulation in TMEM is exact.  The dropped groups (G >= 7) weigh at
 //   most 2^-49.4 of 2^(ea+eb) for K = 64, 2^-48.4 for K = 128 (typically 2^-55),
-//   the element roundings 2^-57 of each operand's scale: the product error stays
-//   well inside FP64's own bound for a K-term dot product (measured on N(0,1)
-//   factors: 1.1e-16 of |C| + |L||U| against 4.7e-16 for the FP64 tensor cores).
+//   the element roundings 2^-57 of each operand's scale.  That is relative to the
+//   largest elements of the row and the column, not to |L||U|: on rows and columns of
+//   one scale well inside FP64's own bound for a K-term dot product (measured on
+//   N(0,1) factors: 1.1e-16 of |C| + |L||U| against 4.7e-16 for the FP64 tensor
+//   cores), but more where a row's large elements meet a column's small ones.
 // Combine (epilogue).  R = floor(sum_G T_G 2^(38-8G)), a 64-bit integer (|R| < 2^62),
 //   then C = C - R 2^(ea+eb-54): one rounding of R to 53 bits (built with integer
 //   operations) and one of the subtraction.  Rows or columns holding Inf or NaN
@@ -66,6 +69,7 @@
 
 #include <algorithm>
 #include <string>
+#include <type_traits>
 
 #include "common.cuh"
 #include "luhot_internal.h"
@@ -92,61 +96,108 @@ static_assert(kOzAccs * kOzBM <= 512, "the accumulators fit in TMEM");
 // Split (digits: ozaki_split.cuh).
 // ---------------------------------------------------------------------------
 
-// Rows r1 .. r1 + M - 1, columns k0 .. k0 + w - 1 of the row-major a (w <= 64
-// kH): As[p][i][k] (zero for k >= w), ea[i].  One warp per row.
+// Two K halves share their exponents unless the halves of some row of L and those of
+// some column of U lie more than kOzApart bits apart (a zero half lies apart from
+// any other).  A shared exponent costs an element of C the smaller of its row's and
+// its column's distance at most, where the larger half of one meets the smaller half
+// of the other: without such a row, or without such a column, kOzApart bits.  With
+// both the operands are split again (oz_resplit_kernel), an exponent a half, and the
+// product is bit for bit that of two products of K = 64.  Halves of 64 normally
+// distributed elements hardly ever lie more than two bits apart; the columns of U do
+// while its rows grow (in the first pairs of an N(0,1) matrix), the rows of L do not.
+constexpr int kOzApart = 2;
+enum { kOzRowsApart = 0, kOzColsApart = 1 };  // flags
+
+// Exponents of the halves; true if they lie apart.  !own: the larger one for both.
 template <int kH>
-__global__ void __launch_bounds__(256) oz_split_rows_kernel(const double* __restrict__ a, int64_t lda, int r1, int M,
-                                                            int k0, int w, __half* __restrict__ as,
-                                                            int* __restrict__ ea) {
-  const int i = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (i >= M) return;
-  const double* row = a + (int64_t)(r1 + i) * lda + k0;
-  double x[2 * kH];
-  int e = kOzZero;
+__device__ __forceinline__ bool oz_half_exponents(const double (&x)[2 * kH], bool own, int (&e)[kH]) {
 #pragma unroll
-  for (int q = 0; q < 2 * kH; ++q) {
-    x[q] = lane + 32 * q < w ? row[lane + 32 * q] : 0.0;
-    e = max(e, oz_exponent(x[q]));
-  }
-  e = oz_warp_max(e);
-#pragma unroll
-  for (int h = 0; h < kH; ++h)
-    oz_emit_row(x[2 * h], x[2 * h + 1], e, as + ((int64_t)i * kH + h) * kOzK, (int64_t)M * kH * kOzK, lane);
-  if (lane == 0) ea[i] = e == kOzZero ? 0 : e;
+  for (int h = 0; h < kH; ++h) e[h] = oz_warp_max(max(oz_exponent(x[2 * h]), oz_exponent(x[2 * h + 1])));
+  const bool apart = kH == 2 && abs(e[0] - e[kH - 1]) > kOzApart;
+  if (kH == 2 && !own) e[0] = e[kH - 1] = max(e[0], e[kH - 1]);
+  return apart;
 }
 
-// Rows k0 .. k0 + w - 1 (w <= 64 kH), columns c1 .. c1 + N - 1 of the row-major
-// a: Bs[p][j][k] (the transpose; zero for k >= w), eb[j].  A CTA stages 64 kH x 32
-// elements through shared memory (coalesced reads along the rows), then each
-// warp splits four columns.
+// Row i of M rows of L (row: its w <= 64 kH elements): As[p][i][k] (zero for k >= w),
+// ea[h M + i].  One warp.
 template <int kH>
-__global__ void __launch_bounds__(256) oz_split_cols_kernel(const double* __restrict__ a, int64_t lda, int k0, int w,
-                                                            int c1, int N, __half* __restrict__ bs,
-                                                            int* __restrict__ eb) {
-  __shared__ double tile[kH * kOzK][33];
-  const int j0 = blockIdx.x * 32;
+__device__ __forceinline__ bool oz_split_row(const double* __restrict__ row, int i, int M, int w, bool own,
+                                             __half* __restrict__ as, int* __restrict__ ea, int lane) {
+  double x[2 * kH];
+  int e[kH];
+#pragma unroll
+  for (int q = 0; q < 2 * kH; ++q) x[q] = lane + 32 * q < w ? row[lane + 32 * q] : 0.0;
+  const bool apart = oz_half_exponents<kH>(x, own, e);
+#pragma unroll
+  for (int h = 0; h < kH; ++h) {
+    oz_emit_row(x[2 * h], x[2 * h + 1], e[h], as + ((int64_t)i * kH + h) * kOzK, (int64_t)M * kH * kOzK, lane);
+    if (lane == 0) ea[(int64_t)h * M + i] = e[h] == kOzZero ? 0 : e[h];
+  }
+  return apart;
+}
+// Columns j0 .. j0 + 31 of N columns of U (w <= 64 kH rows of a): Bs[p][j][k] (the
+// transpose; zero for k >= w), eb[h N + j].  A CTA of 256 threads stages 64 kH x 32
+// elements through shared memory (coalesced reads along the rows), then each warp
+// splits four columns.
+template <int kH>
+__device__ __forceinline__ bool oz_split_cols(double (&tile)[kH * kOzK][33], const double* __restrict__ a, int64_t lda,
+                                              int w, int j0, int N, bool own, __half* __restrict__ bs,
+                                              int* __restrict__ eb) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll 8
   for (int k = warp; k < kH * kOzK; k += 8) {
     const int j = j0 + lane;
-    tile[k][lane] = (k < w && j < N) ? a[(int64_t)(k0 + k) * lda + c1 + j] : 0.0;
+    tile[k][lane] = (k < w && j < N) ? a[(int64_t)k * lda + j] : 0.0;
   }
   __syncthreads();
+  bool apart = false;
   for (int jj = warp; jj < 32; jj += 8) {
     const int j = j0 + jj;
     if (j >= N) break;
     double x[2 * kH];
-    int e = kOzZero;
+    int e[kH];
 #pragma unroll
-    for (int q = 0; q < 2 * kH; ++q) {
-      x[q] = tile[lane + 32 * q][jj];
-      e = max(e, oz_exponent(x[q]));
+    for (int q = 0; q < 2 * kH; ++q) x[q] = tile[lane + 32 * q][jj];
+    apart |= oz_half_exponents<kH>(x, own, e);
+#pragma unroll
+    for (int h = 0; h < kH; ++h) {
+      oz_emit_row(x[2 * h], x[2 * h + 1], e[h], bs + ((int64_t)j * kH + h) * kOzK, (int64_t)N * kH * kOzK, lane);
+      if (lane == 0) eb[(int64_t)h * N + j] = e[h] == kOzZero ? 0 : e[h];
     }
-    e = oz_warp_max(e);
-#pragma unroll
-    for (int h = 0; h < kH; ++h)
-      oz_emit_row(x[2 * h], x[2 * h + 1], e, bs + ((int64_t)j * kH + h) * kOzK, (int64_t)N * kH * kOzK, lane);
-    if (lane == 0) eb[j] = e == kOzZero ? 0 : e;
+  }
+  return apart;
+}
+
+// kH = 2: raise the flags (cleared before).
+template <int kH>
+__global__ void __launch_bounds__(256) oz_split_rows_kernel(const double* __restrict__ l, int64_t ldl, int M, int w,
+                                                            __half* __restrict__ as, int* __restrict__ ea,
+                                                            int* flags) {
+  const int i = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (i >= M) return;
+  if (oz_split_row<kH>(l + (int64_t)i * ldl, i, M, w, false, as, ea, lane) && lane == 0) flags[kOzRowsApart] = 1;
+}
+template <int kH>
+__global__ void __launch_bounds__(256) oz_split_cols_kernel(const double* __restrict__ u, int64_t ldu, int w, int N,
+                                                            __half* __restrict__ bs, int* __restrict__ eb,
+                                                            int* flags) {
+  __shared__ double tile[kH * kOzK][33];
+  if (oz_split_cols<kH>(tile, u, ldu, w, blockIdx.x * 32, N, false, bs, eb) && (threadIdx.x & 31) == 0)
+    flags[kOzColsApart] = 1;
+}
+// Both operands of K = 128 again, an exponent a half, if both flags are up.
+__global__ void __launch_bounds__(256) oz_resplit_kernel(const double* __restrict__ l, int64_t ldl, int M,
+                                                         const double* __restrict__ u, int64_t ldu, int N, int w,
+                                                         __half* __restrict__ as, int* __restrict__ ea,
+                                                         __half* __restrict__ bs, int* __restrict__ eb,
+                                                         const int* __restrict__ flags) {
+  __shared__ double tile[2 * kOzK][33];
+  if (flags[kOzRowsApart] == 0 || flags[kOzColsApart] == 0) return;
+  for (int i = blockIdx.x * 8 + (threadIdx.x >> 5); i < M; i += gridDim.x * 8)
+    oz_split_row<2>(l + (int64_t)i * ldl, i, M, w, true, as, ea, threadIdx.x & 31);
+  for (int j0 = blockIdx.x * 32; j0 < N; j0 += gridDim.x * 32) {
+    __syncthreads();  // the tile's last readers
+    oz_split_cols<2>(tile, u, ldu, w, j0, N, true, bs, eb);
   }
 }
 
@@ -362,7 +413,7 @@ __device__ __forceinline__ double oz_combine(unsigned hi, unsigned lo, int ea_i,
 __global__ void __launch_bounds__(kOzThreads, 1)
     oz_gemm_kernel(const __grid_constant__ CUtensorMap tmL, const __grid_constant__ CUtensorMap tmU, int halves,
                    double* __restrict__ c, int64_t ldc, int M, int N, const int* __restrict__ ea,
-                   const int* __restrict__ eb, DeviceStatus* st) {
+                   const int* __restrict__ eb, const int* __restrict__ flags, DeviceStatus* st) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   unsigned char* sU = base;                                  // streamed: the U pieces of each tile and K half
@@ -374,6 +425,9 @@ __global__ void __launch_bounds__(kOzThreads, 1)
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const unsigned long long limit = st->timeout_ns;
+  // Two halves on exponents of their own: each tile in two passes of K = 64.
+  const int passes = halves == 2 && flags[kOzRowsApart] != 0 && flags[kOzColsApart] != 0 ? 2 : 1;
+  const bool joint = halves == 2 && passes == 1;
   const int tiles_j = (N + kOzBN - 1) / kOzBN;
   const int tiles = tiles_j * ((M + kOzBM - 1) / kOzBM);
   const int t_begin = (int)((int64_t)blockIdx.x * tiles / gridDim.x);
@@ -457,31 +511,43 @@ __global__ void __launch_bounds__(kOzThreads, 1)
     const unsigned u_lo = (smem_u32(sU) >> 4) | (1u << 16), l_lo = (smem_u32(sL) >> 4) | (1u << 16);
     int cur_ib = -1, nl = 0, tc = 0, use = 0;
     bool ok = true;
-    for (int t = t_begin; t < t_end && ok; ++t, ++tc) {
-      const int ib = t / tiles_j;
-      if (ib != cur_ib) {
-        ok = __all_sync(0xffffffffu, oz_wait(smem_u32(&l_full), (unsigned)(nl & 1), limit, &s_abort));
-        if (!ok) break;
-        ++nl;
-        if (leader) s_l_consumed = nl;
-        cur_ib = ib;
+    // The passes as a constant: with a count read from memory a factorization of n =
+    // 16384 takes 145.2 ms instead of 141.6.
+    auto tiles_of = [&](auto passes_constant) {
+      constexpr int kPasses = decltype(passes_constant)::value;
+      for (int t = t_begin; t < t_end && ok; ++t) {
+        const int ib = t / tiles_j;
+        if (ib != cur_ib) {
+          ok = __all_sync(0xffffffffu, oz_wait(smem_u32(&l_full), (unsigned)(nl & 1), limit, &s_abort));
+          if (!ok) break;
+          ++nl;
+          if (leader) s_l_consumed = nl;
+          cur_ib = ib;
+        }
+        for (int h = 0; h < kPasses; ++h, ++tc) {
+          ok = oz_mma_half<0>(tmem, u_lo, l_lo + (unsigned)(h * kOzSlices * (kOzLBytes >> 4)), leader,
+                              smem_u32(acc_empty), smem_u32(u_full), smem_u32(u_empty), (unsigned)(tc & 1) ^ 1u,
+                              (unsigned)(use & 1), limit, &s_abort);
+          ++use;
+          if (ok && kPasses == 1 && halves == 2) {
+            ok = oz_mma_half<1>(tmem, u_lo, l_lo, leader, smem_u32(acc_empty), smem_u32(u_full), smem_u32(u_empty),
+                                (unsigned)(tc & 1) ^ 1u, (unsigned)(use & 1), limit, &s_abort);
+            ++use;
+          }
+          if (!ok) break;
+          if (leader) {
+            oz_commit(smem_u32(&acc_full));
+            const bool block_ends = (t + 1 >= t_end) || ((t + 1) / tiles_j != ib);
+            if (block_ends && h + 1 == kPasses) oz_commit(smem_u32(&l_empty));
+          }
+          __syncwarp();
+        }
       }
-      ok = oz_mma_half<0>(tmem, u_lo, l_lo, leader, smem_u32(acc_empty), smem_u32(u_full), smem_u32(u_empty),
-                          (unsigned)(tc & 1) ^ 1u, (unsigned)(use & 1), limit, &s_abort);
-      ++use;
-      if (ok && halves == 2) {
-        ok = oz_mma_half<1>(tmem, u_lo, l_lo, leader, smem_u32(acc_empty), smem_u32(u_full), smem_u32(u_empty),
-                            (unsigned)(tc & 1) ^ 1u, (unsigned)(use & 1), limit, &s_abort);
-        ++use;
-      }
-      if (!ok) break;
-      if (leader) {
-        oz_commit(smem_u32(&acc_full));
-        const bool block_ends = (t + 1 >= t_end) || ((t + 1) / tiles_j != ib);
-        if (block_ends) oz_commit(smem_u32(&l_empty));
-      }
-      __syncwarp();
-    }
+    };
+    if (passes == 1)
+      tiles_of(std::integral_constant<int, 1>());
+    else
+      tiles_of(std::integral_constant<int, 2>());
     if (leader) {
       if (!ok) oz_abort(st, &s_abort);
       // Arrives once every MMA issued above has completed.
@@ -506,8 +572,8 @@ __global__ void __launch_bounds__(kOzThreads, 1)
     // takes the carry, as are the two sums of group 6.
     const int quarter = warp & 3, rq = (warp - 2) >> 2;
     const unsigned lane_base = tmem + ((unsigned)(quarter * 32) << 16) + (unsigned)(rq * kOzRows);
-    int tc = 0;
-    for (int t = t_begin; t < t_end; ++t, ++tc) {
+    for (int tc = 0; tc < (t_end - t_begin) * passes; ++tc) {
+      const int t = t_begin + (tc >> (passes - 1)), h = tc & (passes - 1);
       const int ib = t / tiles_j, jb = t - ib * tiles_j;
       const int col = jb * kOzBN + quarter * 32 + lane;
       const int row0 = ib * kOzBM + rq * kOzRows;
@@ -540,7 +606,7 @@ __global__ void __launch_bounds__(kOzThreads, 1)
 #pragma unroll
         for (int r = 0; r < kOzRows; ++r) xq[r] = oz_carry(__uint_as_float(tv[r]), lo[r]);
       }
-      if (halves == 2) {
+      if (joint) {
         unsigned tv[kOzRows];
         load(kOzGroups, tv);
 #pragma unroll
@@ -606,8 +672,8 @@ __global__ void __launch_bounds__(kOzThreads, 1)
       // a warp's loads and stores of one row are 32 consecutive doubles.
       // Lane r holds the exponent of row r.  Elements the fast path declines
       // (rare) are redone, warp-uniformly, by the general path.
-      const int eb_j = col_ok ? eb[col] : 0;
-      const int my_ea = lane < kOzRows && row0 + lane < M ? ea[row0 + lane] : 0;
+      const int eb_j = col_ok ? eb[(int64_t)h * N + col] : 0;
+      const int my_ea = lane < kOzRows && row0 + lane < M ? ea[(int64_t)h * M + row0 + lane] : 0;
       const int s_col = eb_j >= kOzNonFinite ? (1 << 24) : eb_j - (kOzFrac + 16);
       const int s_row = my_ea >= kOzNonFinite ? (1 << 24) : my_ea;
       const bool in_range =
@@ -670,12 +736,13 @@ __global__ void __launch_bounds__(kOzThreads, 1)
 static size_t oz_round(size_t b) { return (b + 1023) / 1024 * 1024; }
 
 // Workspace layout for an M x N product over K = 64 * halves: A slices
-// [7][M][K], B slices [7][N][K], exponents ea[M], eb[N].
+// [7][M][K], B slices [7][N][K], exponents ea[halves][M], eb[halves][N], two flags.
 struct OzWs {
   __half* as;
   __half* bs;
   int* ea;
   int* eb;
+  int* flags;
 };
 static OzWs oz_layout(void* ws, int M, int N, int halves = 1) {
   const size_t kb = (size_t)kOzSlices * kOzK * 2 * halves;
@@ -686,14 +753,17 @@ static OzWs oz_layout(void* ws, int M, int N, int halves = 1) {
   w.bs = reinterpret_cast<__half*>(p);
   p += oz_round(kb * N);
   w.ea = reinterpret_cast<int*>(p);
-  p += oz_round((size_t)M * 4);
+  p += oz_round((size_t)M * halves * 4);
   w.eb = reinterpret_cast<int*>(p);
+  p += oz_round((size_t)N * halves * 4);
+  w.flags = reinterpret_cast<int*>(p);
   return w;
 }
 
 size_t ozaki_workspace_bytes(int m, int n) {
   const size_t kb = (size_t)kOzSlices * kOzK * 2 * kOzMaxHalves;
-  return oz_round(kb * m) + oz_round(kb * n) + oz_round((size_t)m * 4) + oz_round((size_t)n * 4);
+  return oz_round(kb * m) + oz_round(kb * n) + oz_round((size_t)m * kOzMaxHalves * 4) +
+         oz_round((size_t)n * kOzMaxHalves * 4) + oz_round(2 * sizeof(int));
 }
 
 bool ozaki_available(luhot_ctx* ctx) { return kOzSmem <= (size_t)ctx->max_smem_optin && encode_fn() != nullptr; }
@@ -727,7 +797,7 @@ static int oz_launch_gemm(luhot_ctx* ctx, const OzWs& w, int halves, double* c, 
   LUHOT_CUDA_TRY(ctx, allow_max_dynamic_smem(oz_gemm_kernel));
   const int cap = ctx->tc_grid_cap > 0 ? ctx->tc_grid_cap : ctx->num_sms;
   oz_gemm_kernel<<<std::min(tiles, cap), kOzThreads, kOzSmem, stream>>>(tmL, tmU, halves, c, ldc, M, N, w.ea, w.eb,
-                                                                                ctx->d_status);
+                                                                      w.flags, ctx->d_status);
   LUHOT_CUDA_TRY(ctx, cudaGetLastError());
   return LUHOT_OK;
 }
@@ -763,18 +833,25 @@ int ozaki_product(luhot_ctx* ctx, const double* l, int64_t ldl, const double* u,
   const int halves = w > kOzK ? 2 : 1;
   const OzWs lay = oz_layout(ws, M, N, halves);
   const double slice_bytes = (double)halves * kOzK * kOzSlices * 2;
+  if (halves == 2) LUHOT_CUDA_TRY(ctx, cudaMemsetAsync(lay.flags, 0, 2 * sizeof(int), stream));
   prof_begin(ctx, kProfOther);
   if (halves == 2)
-    oz_split_rows_kernel<2><<<(M + 7) / 8, 256, 0, stream>>>(l, ldl, 0, M, 0, w, lay.as, lay.ea);
+    oz_split_rows_kernel<2><<<(M + 7) / 8, 256, 0, stream>>>(l, ldl, M, w, lay.as, lay.ea, lay.flags);
   else
-    oz_split_rows_kernel<1><<<(M + 7) / 8, 256, 0, stream>>>(l, ldl, 0, M, 0, w, lay.as, lay.ea);
+    oz_split_rows_kernel<1><<<(M + 7) / 8, 256, 0, stream>>>(l, ldl, M, w, lay.as, lay.ea, nullptr);
   prof_end(ctx, kProfOther, 0.0, M * (w * 8.0 + slice_bytes));
   prof_begin(ctx, kProfOther);
   if (halves == 2)
-    oz_split_cols_kernel<2><<<(N + 31) / 32, 256, 0, stream>>>(u, ldu, 0, w, 0, N, lay.bs, lay.eb);
+    oz_split_cols_kernel<2><<<(N + 31) / 32, 256, 0, stream>>>(u, ldu, w, N, lay.bs, lay.eb, lay.flags);
   else
-    oz_split_cols_kernel<1><<<(N + 31) / 32, 256, 0, stream>>>(u, ldu, 0, w, 0, N, lay.bs, lay.eb);
+    oz_split_cols_kernel<1><<<(N + 31) / 32, 256, 0, stream>>>(u, ldu, w, N, lay.bs, lay.eb, nullptr);
   prof_end(ctx, kProfOther, 0.0, N * (w * 8.0 + slice_bytes));
+  if (halves == 2) {
+    prof_begin(ctx, kProfOther);
+    oz_resplit_kernel<<<ctx->num_sms, 256, 0, stream>>>(l, ldl, M, u, ldu, N, w, lay.as, lay.ea, lay.bs, lay.eb,
+                                                        lay.flags);
+    prof_end(ctx, kProfOther, 0.0, 0.0);
+  }
   LUHOT_CUDA_TRY(ctx, cudaGetLastError());
   prof_begin(ctx, kProfGemm);
   int rc = oz_launch_gemm(ctx, lay, halves, c, ldc, M, N, stream);
