@@ -22,14 +22,15 @@
 //                    CTA, partial sums per range (summed in a fixed order);
 //   qr_y_kernel      Y = T^T W: T^-1 is the upper triangle of V^T V with 1 / tau on
 //                    its diagonal, so y_j = tau_j (w_j - sum_{i<j} (V^T V)_ij y_i);
-//   A2 -= V Y        on the FP16 tensor cores (ozaki_product) for large blocks, else
-//                    by FP64 MMAs (qr_update_kernel).
+//   qr_update_kernel A2 -= V Y by FP64 MMAs.  (Slice products, ozaki.cu, on large blocks:
+//                    13.3 ms at 2000 x 1500 against 15.7, but they hold V and Y relative to the
+//                    largest of its row or column: where reflectors of rows of
+//                    different scale meet, 3e-9 of |V||Y| in place of 3e-16.)
 #include <algorithm>
 
 #include "cluster.cuh"
 #include "common.cuh"
 #include "luhot_internal.h"
-#include "ozaki.cuh"
 
 namespace luhot {
 
@@ -393,12 +394,6 @@ int geqrf_blocked(luhot_ctx* ctx, int m, int n, double* a, int64_t lda, double* 
   double* v = static_cast<double*>(ctx->work[2].ptr);
   double* y = v + v_elems;
   double* wp = y + y_elems;
-  void* oz = nullptr;
-  if (ctx->fp64_update != LUHOT_UPDATE_DMMA && ozaki_available(ctx)) {
-    rc = ensure_buf(ctx, ctx->oz_buf, ozaki_workspace_bytes(m, n));
-    if (rc) return rc;
-    oz = ctx->oz_buf.ptr;
-  }
   LUHOT_CUDA_TRY(ctx, allow_max_dynamic_smem(qr_panel_kernel));
   LUHOT_CUDA_TRY(ctx, allow_wide_clusters(reinterpret_cast<const void*>(qr_panel_kernel)));
   rc = reset_status(ctx);
@@ -432,17 +427,10 @@ int geqrf_blocked(luhot_ctx* ctx, int m, int n, double* a, int64_t lda, double* 
     qr_y_kernel<<<(n2 + 7) / 8, 128, 0, stream>>>(wp, ldw, ranges, tau + k0, w, n2, y, ldy);
     prof_end(ctx, kProfTrsm, (double)kQb * kQb * n2, 8.0 * kQb * n2 * (ranges + 1));
     LUHOT_CUDA_TRY(ctx, cudaGetLastError());
-    // A slice product takes 28 us for up to one 128 x 128 tile per SM and 13 us of
-    // splits, FP64 MMAs 8 us + 0.06 ns an element at K = 32.
-    if (oz && rows >= 128 && n2 >= 64 && (int64_t)rows * n2 > 500000) {
-      rc = ozaki_product(ctx, v, kQb, y, ldy, kQb, a2, lda, rows, n2, oz, stream);
-      if (rc) return rc;
-    } else {
-      prof_begin(ctx, kProfGemm);
-      qr_update_kernel<<<dim3((n2 + 31) / 32, (rows + 31) / 32), 128, 0, stream>>>(a2, lda, rows, n2, v, y, ldy);
-      prof_end(ctx, kProfGemm, 2.0 * rows * n2 * kQb, 16.0 * rows * n2);
-      LUHOT_CUDA_TRY(ctx, cudaGetLastError());
-    }
+    prof_begin(ctx, kProfGemm);
+    qr_update_kernel<<<dim3((n2 + 31) / 32, (rows + 31) / 32), 128, 0, stream>>>(a2, lda, rows, n2, v, y, ldy);
+    prof_end(ctx, kProfGemm, 2.0 * rows * n2 * kQb, 16.0 * rows * n2);
+    LUHOT_CUDA_TRY(ctx, cudaGetLastError());
   }
   // Its panels wait on one another: a wait that gave up is reported by this call, and
   // the status and workspace are free when it returns.
