@@ -181,15 +181,6 @@ __device__ __forceinline__ void batch_update(double* S, int ld, const int* act, 
   }
 }
 
-// y / d with the reciprocal r = 1/d and one correction where r and d are plain
-// numbers (`good`), else a division.
-template <typename T>
-__device__ __forceinline__ T batch_quot(T y, T d, T r, bool good) {
-  if (!good) return y / d;
-  const T q = y * r;
-  return isfinite(q) ? fma(fma(-q, d, y), r, q) : q;
-}
-
 // u[c] = P[ib][c] of lane src for c in [kC0, kCW) (ib and src uniform).
 template <typename T, int NI, int kC0, int kCW>
 __device__ __forceinline__ void batch_row(const T (&P)[NI][batch_nb<T>(NI)], int ib, int src, T (&u)[batch_nb<T>(NI)]) {
@@ -453,7 +444,7 @@ __device__ __forceinline__ void batch_back(T* S, int ld, int n, const int* prow,
     x[q] = on ? row[q][n] : T(0);
     d[q] = on ? row[q][i] : T(1);
     rc[q] = T(1) / d[q];
-    good = good && isfinite(rc[q]) && isfinite(d[q]) && fabs(rc[q]) > T(1e-30) && fabs(d[q]) > T(1e-30);
+    good = good && quot_plain(d[q], rc[q]);
   }
   good = __all_sync(kFull, good);
 #pragma unroll
@@ -461,7 +452,7 @@ __device__ __forceinline__ void batch_back(T* S, int ld, int n, const int* prow,
     if (32 * qb >= n) continue;
     for (int kk = min(31, n - 1 - 32 * qb); kk >= 0; --kk) {
       const int k = 32 * qb + kk;
-      if (lane == kk) x[qb] = batch_quot(x[qb], d[qb], rc[qb], good);
+      if (lane == kk) x[qb] = quot(x[qb], d[qb], rc[qb], good);
       const T xk = __shfl_sync(kFull, x[qb], kk);
 #pragma unroll
       for (int q = 0; q < NI; ++q)

@@ -95,6 +95,25 @@ __device__ __forceinline__ bool grid_barrier(DeviceStatus* st, unsigned int targ
   return s_ok != 0;
 }
 
+// y / d by the rounded reciprocal r = 1 / d: q = y r, then q + r (y - q d) with fused
+// multiply-adds, the correction step of P. Markstein, "Computation of elementary
+// functions on the IBM RISC System/6000 processor", IBM J. Res. Develop. 34 (1990).
+// `plain` (quot_plain of d and r): d and r are far from the ends of the range, so
+// that y - q d is exact and the result within one unit of the last place of y / d
+// rounded (y r alone: two), unless y is so small that y - q d underflows: then two.
+// A q that overflows (y r can where y / d does not) or is not a number takes the
+// division, as any y does where `plain` does not hold.
+template <typename T>
+__device__ __forceinline__ bool quot_plain(T d, T r) {
+  return isfinite(r) && isfinite(d) && fabs(r) > T(1e-30) && fabs(d) > T(1e-30);
+}
+template <typename T>
+__device__ __forceinline__ T quot(T y, T d, T r, bool plain) {
+  const T q = y * r;
+  if (!plain || !isfinite(q)) return y / d;
+  return fma(fma(-q, d, y), r, q);
+}
+
 // Loads that bypass L1 (data written by other CTAs during the same launch).
 template <typename T>
 __device__ __forceinline__ T ld_cg(const T* p) {

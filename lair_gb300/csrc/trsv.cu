@@ -385,13 +385,8 @@ cudaError_t launch_trsv_syncfree(cudaStream_t stream, const TA* a, int64_t lda, 
 // small n; this: 11 us for both, both in one launch.)
 constexpr int kInvCols = 4;
 
-// y / d for the warp's running quotient: by the reciprocal r = 1/d with one
-// correction step where r is a normal number (`good`), else by division.
-__device__ __forceinline__ double inv_quot(double y, double d, double r, bool good) {
-  if (!good) return y / d;
-  const double q = y * r;
-  return isfinite(q) ? fma(fma(-q, d, y), r, q) : q;
-}
+// y / d on the warp's chain: FP64 by the reciprocal (quot), FP32 by division.
+__device__ __forceinline__ double inv_quot(double y, double d, double r, bool good) { return quot(y, d, r, good); }
 __device__ __forceinline__ float inv_quot(float y, float d, float, bool) { return y / d; }
 
 template <typename T, typename TA>
@@ -424,9 +419,7 @@ __global__ void __launch_bounds__(32 * kInvCols) trsv_invert_diag_kernel(const T
       const bool on0 = lane < hi, on1 = lane + 32 < hi;
       const T d0 = on0 ? S[lane * kLds + lane] : T(1), d1 = on1 ? S[(lane + 32) * kLds + lane + 32] : T(1);
       const T r0 = T(1) / d0, r1 = T(1) / d1;
-      const bool good = __all_sync(0xffffffffu, isfinite(r0) && isfinite(r1) && isfinite(d0) && isfinite(d1) &&
-                                                    fabs(r0) > T(1e-30) && fabs(r1) > T(1e-30) &&
-                                                    fabs(d0) > T(1e-30) && fabs(d1) > T(1e-30));
+      const bool good = __all_sync(0xffffffffu, quot_plain(d0, r0) && quot_plain(d1, r1));
       for (int k = c; k >= 0; --k) {
         if (k >= 32) {
           if (lane + 32 == k) x1 = inv_quot(x1, d1, r1, good);
