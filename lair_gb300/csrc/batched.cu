@@ -724,10 +724,16 @@ static int upload_meta(luhot_batch* p) {
   int64_t* boff = aoff + c;
   int* sizes = reinterpret_cast<int*>(boff + c);
   int* order = sizes + c;
-  LUHOT_CUDA_TRY(ctx, cudaMemcpy(aoff, p->aoff.data(), c * sizeof(int64_t), cudaMemcpyHostToDevice));
-  LUHOT_CUDA_TRY(ctx, cudaMemcpy(boff, p->boff.data(), c * sizeof(int64_t), cudaMemcpyHostToDevice));
-  LUHOT_CUDA_TRY(ctx, cudaMemcpy(sizes, p->sizes.data(), c * sizeof(int), cudaMemcpyHostToDevice));
-  LUHOT_CUDA_TRY(ctx, cudaMemcpy(order, p->order.data(), c * sizeof(int), cudaMemcpyHostToDevice));
+  // On the context's stream and waited for: a copy on the default stream can return
+  // before its data has arrived, and orders nothing for streams that do not block on it.
+  auto up = [&](void* dst, const void* src, size_t bytes) {
+    return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx->stream);
+  };
+  LUHOT_CUDA_TRY(ctx, up(aoff, p->aoff.data(), c * sizeof(int64_t)));
+  LUHOT_CUDA_TRY(ctx, up(boff, p->boff.data(), c * sizeof(int64_t)));
+  LUHOT_CUDA_TRY(ctx, up(sizes, p->sizes.data(), c * sizeof(int)));
+  LUHOT_CUDA_TRY(ctx, up(order, p->order.data(), c * sizeof(int)));
+  LUHOT_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
   p->meta.sizes = sizes;
   p->meta.aoff = aoff;
   p->meta.boff = boff;
@@ -932,9 +938,9 @@ int luhot_batch_autotune(luhot_batch* p, const void* d_a, const void* d_b) {
   int* m_sizes = reinterpret_cast<int*>(m_boff + ns);
   int* m_order = m_sizes + ns;
   int* m_counter = m_order + ns;
-  cudaMemcpy(m_aoff, s_aoff.data(), ns * sizeof(int64_t), cudaMemcpyHostToDevice);
-  cudaMemcpy(m_boff, s_boff.data(), ns * sizeof(int64_t), cudaMemcpyHostToDevice);
-  cudaMemcpy(m_sizes, s_sizes.data(), ns * sizeof(int), cudaMemcpyHostToDevice);
+  cudaMemcpyAsync(m_aoff, s_aoff.data(), ns * sizeof(int64_t), cudaMemcpyHostToDevice, ctx->stream);
+  cudaMemcpyAsync(m_boff, s_boff.data(), ns * sizeof(int64_t), cudaMemcpyHostToDevice, ctx->stream);
+  cudaMemcpyAsync(m_sizes, s_sizes.data(), ns * sizeof(int), cudaMemcpyHostToDevice, ctx->stream);
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
@@ -958,7 +964,7 @@ int luhot_batch_autotune(luhot_batch* p, const void* d_a, const void* d_b) {
       for (auto& q : order) q += first;
       rc = ensure_buf(ctx, mat_buf, scratch_ctas(classes) * kScratchElems * es);
       if (rc) break;
-      cudaMemcpy(m_order, order.data(), cnt * sizeof(int), cudaMemcpyHostToDevice);
+      cudaMemcpyAsync(m_order, order.data(), cnt * sizeof(int), cudaMemcpyHostToDevice, ctx->stream);
       BatchMeta m{m_sizes, m_aoff, m_boff, m_order, cnt};
       float ms = 0.f;
       for (int rep = 0; rep < 2 && err == cudaSuccess; ++rep) {
