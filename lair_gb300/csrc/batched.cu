@@ -35,7 +35,6 @@
 #include <algorithm>
 #include <climits>
 #include <cstring>
-#include <numeric>
 #include <vector>
 
 #include "common.cuh"
@@ -619,7 +618,7 @@ static const void* batch_kernel(int dtype, int mode, int ni, bool scratch) {
 // matrices that fit in an SM's shared memory (or the scratch form).
 static void build_classes(luhot_ctx* ctx, int dtype, int mode, const int* tune, int smem_n,
                           const std::vector<int>& sizes, std::vector<int>& order, std::vector<BatchClass>& classes) {
-  auto key = [&](int n) {
+  auto key_of = [&](int n) {
     const int ni = n <= 32 ? 1 : n <= 64 ? 2 : n <= 128 ? 4 : 8;
     const bool scratch = n > smem_n || tune[batch_bucket(n)] != 0;
     const size_t bytes = smem_bytes(dtype, n);
@@ -631,17 +630,26 @@ static void build_classes(luhot_ctx* ctx, int dtype, int mode, const int* tune, 
         if (bytes + 3 * 1024 > kBatchSmem / f) fit = f == 6 ? 4 : f == 4 ? 3 : f == 3 ? 2 : 1;
     return (8 - ni) * 16 + fit;  // larger rows first, then fewer to an SM
   };
+  // Sizes by class and size, the systems of each in their order.
+  int key[kBatchMaxN + 1], by_class[kBatchMaxN], at[kBatchMaxN + 1], count[kBatchMaxN + 1] = {};
+  for (int n = 1; n <= kBatchMaxN; ++n) {
+    key[n] = key_of(n);
+    by_class[n - 1] = n;
+  }
+  std::sort(by_class, by_class + kBatchMaxN, [&](int x, int y) { return key[x] != key[y] ? key[x] < key[y] : x > y; });
+  for (int n : sizes) ++count[n];
+  int next = 0;
+  for (int n : by_class) {
+    at[n] = next;
+    next += count[n];
+  }
   order.resize(sizes.size());
-  std::iota(order.begin(), order.end(), 0);
-  std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
-    const int kx = key(sizes[x]), ky = key(sizes[y]);
-    return kx != ky ? kx < ky : sizes[x] > sizes[y];
-  });
+  for (size_t i = 0; i < sizes.size(); ++i) order[at[sizes[i]]++] = (int)i;
   classes.clear();
   for (size_t i = 0; i < order.size();) {
-    const int n = sizes[order[i]], k = key(n);
+    const int n = sizes[order[i]], k = key[n];
     size_t e = i;
-    while (e < order.size() && key(sizes[order[e]]) == k) ++e;
+    while (e < order.size() && key[sizes[order[e]]] == k) ++e;
     BatchClass c;
     c.first = (int)i;
     c.count = (int)(e - i);
@@ -663,13 +671,40 @@ static void build_classes(luhot_ctx* ctx, int dtype, int mode, const int* tune, 
   }
 }
 
+// Branches of a launch of `classes` classes (the first class's is the stream itself),
+// made when a plan first has so many: a plan of one class makes none.
+static int batch_branches(const std::vector<BatchClass>& classes) {
+  return std::max(0, std::min((int)classes.size(), kBatchStreams) - 1);
+}
+static int make_branches(luhot_batch* p, const std::vector<BatchClass>& classes) {
+  const int nb = batch_branches(classes);
+  if (nb > 0 && !p->fork) LUHOT_CUDA_TRY(p->ctx, cudaEventCreateWithFlags(&p->fork, cudaEventDisableTiming));
+  for (int q = 0; q < nb; ++q) {
+    if (!p->branch[q]) LUHOT_CUDA_TRY(p->ctx, cudaStreamCreateWithFlags(&p->branch[q], cudaStreamNonBlocking));
+    if (!p->joined[q]) LUHOT_CUDA_TRY(p->ctx, cudaEventCreateWithFlags(&p->joined[q], cudaEventDisableTiming));
+  }
+  return LUHOT_OK;
+}
+
+// The sample systems' matrices and right-hand sides, packed: sample q is system
+// sys[q] of the plan.  Words of the element's size.
+template <typename W>
+__global__ void gather_samples_kernel(const W* __restrict__ a, const W* __restrict__ b, const int* __restrict__ sys,
+                                      const int* __restrict__ sizes, const int64_t* __restrict__ aoff,
+                                      const int64_t* __restrict__ boff, const int64_t* __restrict__ s_aoff,
+                                      const int64_t* __restrict__ s_boff, W* __restrict__ pa, W* __restrict__ pb) {
+  const int q = blockIdx.x, i = sys[q], n = sizes[q];
+  for (int e = threadIdx.x; e < n * n; e += blockDim.x) pa[s_aoff[q] + e] = a[aoff[i] + e];
+  for (int e = threadIdx.x; e < n; e += blockDim.x) pb[s_boff[q] + e] = b[boff[i] + e];
+}
+
 // Clears the counters and launches every class, the branches' share on their
 // streams between a fork and a join (so a capture of `stream` holds them all).
 static cudaError_t launch_classes(luhot_batch* p, const std::vector<BatchClass>& classes, const BatchMeta& m,
                                   void* scratch, void* a, void* b, int* piv, int* info, int* counters,
                                   cudaStream_t stream) {
   cudaError_t e = cudaMemsetAsync(counters, 0, kMaxBatchClasses * sizeof(int), stream);
-  const int nb = std::min((int)classes.size(), kBatchStreams) - 1;
+  const int nb = batch_branches(classes);
   if (e == cudaSuccess && nb > 0) e = cudaEventRecord(p->fork, stream);
   for (int q = 0; q < nb && e == cudaSuccess; ++q) e = cudaStreamWaitEvent(p->branch[q], p->fork, 0);
   char* sp = static_cast<char*>(scratch);
@@ -706,6 +741,8 @@ static int upload_meta(luhot_batch* p) {
   const size_t c = (size_t)p->count;
   build_classes(ctx, p->dtype, p->mode, p->tune, p->smem_n, p->sizes, p->order, p->classes);
   if ((int)p->classes.size() > kMaxBatchClasses) return set_error(ctx, LUHOT_ERR_UNSUPPORTED, "batch: too many size classes");
+  int rc = make_branches(p, p->classes);
+  if (rc) return rc;
   const size_t need = scratch_ctas(p->classes);
   if (need > p->scratch_ctas) {
     if (p->d_scratch) cudaFree(p->d_scratch);
@@ -789,14 +826,6 @@ int luhot_batch_create(luhot_ctx* ctx, int64_t count, const int32_t* sizes, int 
   // Untuned: shared memory where it fits for FP32; FP64 up to 96, where three
   // CTAs or more share an SM (its pipe idles while one CTA's panel runs).
   for (int bk = 0; bk < kBuckets; ++bk) p->tune[bk] = dtype == 0 && bk > 3 ? batch_width(dtype) : 0;
-  bool ok = cudaEventCreateWithFlags(&p->fork, cudaEventDisableTiming) == cudaSuccess;
-  for (int q = 0; q < kBatchStreams - 1; ++q)
-    ok = ok && cudaStreamCreateWithFlags(&p->branch[q], cudaStreamNonBlocking) == cudaSuccess &&
-         cudaEventCreateWithFlags(&p->joined[q], cudaEventDisableTiming) == cudaSuccess;
-  if (!ok) {
-    luhot_batch_destroy(p);
-    return set_error(ctx, LUHOT_ERR_CUDA, std::string("batch: ") + cudaGetErrorString(cudaGetLastError()));
-  }
   int rc = count > 0 ? upload_meta(p) : LUHOT_OK;
   if (rc) {
     luhot_batch_destroy(p);
@@ -908,7 +937,7 @@ int luhot_batch_autotune(luhot_batch* p, const void* d_a, const void* d_b) {
   int* spiv = reinterpret_cast<int*>(pb + sb * es);
   int* sinfo = spiv + sb;
   // Per-bucket sample metadata in the plan's layout style.
-  std::vector<int> s_sizes, s_order;
+  std::vector<int> s_sizes, s_sys;
   std::vector<int64_t> s_aoff, s_boff;
   std::vector<int> bucket_first(kBuckets + 1, 0);
   int64_t ao = 0, bo = 0;
@@ -916,14 +945,10 @@ int luhot_batch_autotune(luhot_batch* p, const void* d_a, const void* d_b) {
     bucket_first[bk] = (int)s_sizes.size();
     for (int i : members[bk]) {
       const int n = p->sizes[i];
-      LUHOT_CUDA_TRY(ctx, cudaMemcpyAsync(pa + ao * es, static_cast<const char*>(d_a) + p->aoff[i] * es,
-                                          (size_t)n * n * es, cudaMemcpyDeviceToDevice, ctx->stream));
-      LUHOT_CUDA_TRY(ctx, cudaMemcpyAsync(pb + bo * es, static_cast<const char*>(d_b) + p->boff[i] * es, (size_t)n * es,
-                                          cudaMemcpyDeviceToDevice, ctx->stream));
       s_sizes.push_back(n);
+      s_sys.push_back(i);
       s_aoff.push_back(ao);
       s_boff.push_back(bo);
-      s_order.push_back((int)s_order.size());
       ao += (int64_t)n * n;
       bo += n;
     }
@@ -941,6 +966,21 @@ int luhot_batch_autotune(luhot_batch* p, const void* d_a, const void* d_b) {
   cudaMemcpyAsync(m_aoff, s_aoff.data(), ns * sizeof(int64_t), cudaMemcpyHostToDevice, ctx->stream);
   cudaMemcpyAsync(m_boff, s_boff.data(), ns * sizeof(int64_t), cudaMemcpyHostToDevice, ctx->stream);
   cudaMemcpyAsync(m_sizes, s_sizes.data(), ns * sizeof(int), cudaMemcpyHostToDevice, ctx->stream);
+  cudaMemcpyAsync(m_order, s_sys.data(), ns * sizeof(int), cudaMemcpyHostToDevice, ctx->stream);
+  if (es == 8)
+    gather_samples_kernel<unsigned long long><<<ns, 256, 0, ctx->stream>>>(
+        static_cast<const unsigned long long*>(d_a), static_cast<const unsigned long long*>(d_b), m_order, m_sizes,
+        p->meta.aoff, p->meta.boff, m_aoff, m_boff, reinterpret_cast<unsigned long long*>(pa),
+        reinterpret_cast<unsigned long long*>(pb));
+  else
+    gather_samples_kernel<unsigned><<<ns, 256, 0, ctx->stream>>>(
+        static_cast<const unsigned*>(d_a), static_cast<const unsigned*>(d_b), m_order, m_sizes, p->meta.aoff,
+        p->meta.boff, m_aoff, m_boff, reinterpret_cast<unsigned*>(pa), reinterpret_cast<unsigned*>(pb));
+  count_launch(ctx);
+  if (cudaError_t e = cudaGetLastError(); e != cudaSuccess || (e = cudaStreamSynchronize(ctx->stream)) != cudaSuccess) {
+    cudaFree(meta_buf.ptr);
+    return set_error(ctx, LUHOT_ERR_CUDA, std::string("batch autotune: ") + cudaGetErrorString(e));
+  }
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
@@ -961,6 +1001,8 @@ int luhot_batch_autotune(luhot_batch* p, const void* d_a, const void* d_b) {
       std::vector<int> order;
       std::vector<BatchClass> classes;
       build_classes(ctx, p->dtype, p->mode, tune_all, p->smem_n, b_sizes, order, classes);
+      rc = make_branches(p, classes);
+      if (rc) break;
       for (auto& q : order) q += first;
       rc = ensure_buf(ctx, mat_buf, scratch_ctas(classes) * kScratchElems * es);
       if (rc) break;
