@@ -254,6 +254,9 @@ int luhot_batch_autotune(luhot_batch* plan, const void* d_a, const void* d_b);
  * the panel width of the scratch form) and the largest n that fits in shared
  * memory. */
 int luhot_batch_tuning(const luhot_batch* plan, int32_t* nb_per_bucket, int32_t* smem_n);
+/* Self-test: every bucket in one form, 0 = shared memory where it fits, 1 = scratch
+ * (results do not depend on the form). */
+int luhot_selftest_batch_form(luhot_batch* plan, int form);
 /* Factor and solve every system in place on the device (one graph launch). */
 int luhot_batch_solve(luhot_batch* plan, void* d_a, void* d_b, int32_t* d_piv, int32_t* d_info);
 /* Same with packed host arrays (copied in and out). */

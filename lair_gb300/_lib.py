@@ -72,6 +72,7 @@ SIGNATURES = {
     "luhot_batch_layout": (_i32, [_vp, _vp, _vp]),
     "luhot_batch_autotune": (_i32, [_vp, _vp, _vp]),
     "luhot_batch_tuning": (_i32, [_vp, _vp, _vp]),
+    "luhot_selftest_batch_form": (_i32, [_vp, _i32]),
     "luhot_batch_solve": (_i32, [_vp, _vp, _vp, _vp, _vp]),
     "luhot_batch_solve_host": (_i32, [_vp, _vp, _vp, _vp, _vp]),
     "luhot_dfactor_create": (_i32, [_vp, _i64, _i64, _vp, _i64, _i64, _i32, _vp, ctypes.POINTER(_i64),

@@ -865,6 +865,14 @@ int luhot_batch_tuning(const luhot_batch* p, int32_t* nb_per_bucket, int32_t* sm
   return LUHOT_OK;
 }
 
+int luhot_selftest_batch_form(luhot_batch* p, int form) {
+  if (!p || form < 0 || form > 1) return LUHOT_ERR_INVALID_ARG;
+  CtxGuard g(p->ctx);
+  for (int& t : p->tune) t = form ? batch_width(p->dtype) : 0;
+  drop_graph(p);
+  return p->count > 0 ? upload_meta(p) : LUHOT_OK;
+}
+
 int luhot_batch_solve(luhot_batch* p, void* d_a, void* d_b, int32_t* d_piv, int32_t* d_info) {
   LUHOT_NVTX_FN();
   if (!p) return LUHOT_ERR_INVALID_ARG;

@@ -138,6 +138,7 @@ extern "C" {
     pub fn luhot_batch_layout(plan: *const luhot_batch, a_elems: *mut i64, b_elems: *mut i64) -> c_int;
     pub fn luhot_batch_autotune(plan: *mut luhot_batch, d_a: *const c_void, d_b: *const c_void) -> c_int;
     pub fn luhot_batch_tuning(plan: *const luhot_batch, nb_per_bucket: *mut i32, smem_n: *mut i32) -> c_int;
+    pub fn luhot_selftest_batch_form(plan: *mut luhot_batch, form: c_int) -> c_int;
     pub fn luhot_batch_solve(plan: *mut luhot_batch, d_a: *mut c_void, d_b: *mut c_void, d_piv: *mut i32,
                              d_info: *mut i32) -> c_int;
     pub fn luhot_batch_solve_host(plan: *mut luhot_batch, a: *mut c_void, b: *mut c_void, piv: *mut i32,
