@@ -17,7 +17,10 @@
 //                    every CTA derives the same beta, tau and row factors.  FP64:
 //                    a pass is two FMAs an element and fills the SMs' FP64 pipes
 //                    (2 us a column at 2000 rows); the exchange with its square
-//                    root and division takes about 1 us.
+//                    root and division takes about 1 us.  The products are of x itself,
+//                    not of v: columns whose products with others could leave the range
+//                    of FP64 (largest element outside 2^-450 .. 2^450) are held divided
+//                    by a power of two, on which V and tau do not depend.
 //   qr_w_kernel      W = V^T [V A2] by FP64 MMAs, 32 columns x a range of rows per
 //                    CTA, partial sums per range (summed in a fixed order);
 //   qr_y_kernel      Y = T^T W: T^-1 is the upper triangle of V^T V with 1 / tau on
@@ -42,6 +45,7 @@ constexpr int kQbMaxCtas = 16;
 constexpr int kQbThreads = 256;
 constexpr int kQbWarps = kQbThreads / 32;
 constexpr size_t kQbStatic = 16 * 1024;  // static shared memory of the panel kernel, rounded up
+constexpr int kQbRange = 450;
 
 struct QrPanelArgs {
   double* a;  // the matrix at (k0, k0)
@@ -59,6 +63,7 @@ __global__ void __launch_bounds__(kQbThreads, 1) qr_panel_kernel(QrPanelArgs p) 
   __shared__ __align__(16) double box[2][kQbMaxCtas][kQb];  // every CTA's sums
   __shared__ __align__(16) double arow[2][kQb];             // the diagonal's row
   __shared__ double part[kQbWarps][kQb], tot[kQb], scale_of[kQb];
+  __shared__ double s_unit[kQb];  // the power of two that a column is divided by
   __shared__ double s_tau, s_scale, s_beta;
   __shared__ __align__(8) unsigned long long bar[2];
   __shared__ int s_ok;
@@ -74,9 +79,42 @@ __global__ void __launch_bounds__(kQbThreads, 1) qr_panel_kernel(QrPanelArgs p) 
     asm volatile("fence.mbarrier_init.release.cluster;");
     s_ok = 1;
   }
-  for (int r = warp; r < nloc; r += kQbWarps)
-    S[r * kQbLd + lane] = lane < w ? p.a[(int64_t)(r_begin + r) * p.lda + lane] : 0.0;
-  cl_sync();
+  cl_sync();  // barriers initialised, every CTA there
+  {
+    // The columns' largest finite elements (bits of |x|), over the warps in `part`,
+    // over the CTAs in box[1], which step 1 is the first to use.
+    unsigned long long(*top)[kQb] = reinterpret_cast<unsigned long long(*)[kQb]>(part);
+    unsigned long long hi = 0;
+    for (int r = warp; r < nloc; r += kQbWarps) {
+      const double v = lane < w ? p.a[(int64_t)(r_begin + r) * p.lda + lane] : 0.0;
+      S[r * kQbLd + lane] = v;
+      const unsigned long long bits = (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
+      if (bits < 0x7ff0000000000000ull) hi = max(hi, bits);
+    }
+    top[warp][lane] = hi;
+    __syncthreads();
+    for (int idx = tid; idx < P * kQb; idx += kQbThreads) {
+      const int cta = idx / kQb, c = idx - cta * kQb;
+      unsigned long long t = 0;
+      for (int q = 0; q < kQbWarps; ++q) t = max(t, top[q][c]);
+      asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(cl_peer(cl_smem(&box[1][b][c]), cta)), "l"(t) : "memory");
+    }
+    cl_sync();
+    if (warp == 0) {
+      unsigned long long t = 0;
+      for (int q = 0; q < P; ++q) t = max(t, (unsigned long long)__double_as_longlong(box[1][q][lane]));
+      const int e = t != 0 ? ilogb(__longlong_as_double((long long)t)) : 0;
+      const int unit = e > kQbRange || e < -kQbRange ? max(-1000, min(1000, e)) : 0;
+      s_unit[lane] = __hiloint2double((unit + 1023) << 20, 0);
+    }
+    __syncthreads();
+    const double unit = s_unit[lane];
+    if (__any_sync(kFull, unit != 1.0)) {
+      const double down = __hiloint2double((2046 << 20) - __double2hiint(unit), 0);  // 1 / unit
+      for (int r = warp; r < nloc; r += kQbWarps) S[r * kQbLd + lane] *= down;
+    }
+    __syncthreads();
+  }
 
   bool ok = true;
   double g = 0.0;  // this lane's column: the factor of x in the pending update
@@ -149,7 +187,8 @@ __global__ void __launch_bounds__(kQbThreads, 1) qr_panel_kernel(QrPanelArgs p) 
         const double ss = __shfl_sync(kFull, t, (j & 3) * 8);
         const double alpha = ok ? arow[par][j] : 0.0;
         const double beta = -copysign(sqrt(fma(alpha, alpha, ss)), alpha);
-        const bool zero = ss == 0.0;
+        // lair's norm is zero where the squares underflow, in the column's own unit.
+        const bool zero = ss * s_unit[j] * s_unit[j] == 0.0;
         const double num = lane == 0 ? beta - alpha : 1.0, den = lane == 0 ? beta : alpha - beta;
         const double quot = zero ? 0.0 : num / den;
         if (lane == 0) {
@@ -158,7 +197,7 @@ __global__ void __launch_bounds__(kQbThreads, 1) qr_panel_kernel(QrPanelArgs p) 
         }
         if (lane == 1) {
           s_scale = quot;
-          scale_of[j] = zero ? 1.0 : quot;
+          scale_of[j] = zero ? s_unit[j] : quot;
         }
       }
       if (!ok && lane == 0) s_ok = 0;
@@ -188,7 +227,7 @@ __global__ void __launch_bounds__(kQbThreads, 1) qr_panel_kernel(QrPanelArgs p) 
     for (int r = warp; r < nloc; r += kQbWarps) {
       const int i = r_begin + r;
       double e = S[r * kQbLd + lane];
-      if (lane < w && i > lane) e *= scale_of[lane];
+      if (lane < w) e *= i > lane ? scale_of[lane] : s_unit[lane];
       if (lane < w) p.a[(int64_t)i * p.lda + lane] = e;
       p.v[(int64_t)i * kQb + lane] = lane >= w || i < lane ? 0.0 : i == lane ? 1.0 : e;
     }
