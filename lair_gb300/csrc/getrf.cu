@@ -101,9 +101,11 @@ __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src)
 // also gives the pivot value), the row id and the candidate's column j+1 value,
 // 96 (FP32) or 160 bits, in kHead words of 48 bits over a 16-bit tag (the step's
 // low bits; a header is rewritten at every second step, so that an old tag is
-// never 65536 steps old).  The headers of all CTAs are contiguous: a warp's poll of
-// 64 CTAs reads 16 lines of 128 bytes (FP32: 8) and has every load in flight
-// at once, an L2 latency (some 850 cycles across the dies) a poll.
+// never 65536 steps old).  The headers lie 64 bytes apart, ahead of all segments: a
+// warp's poll of 64 CTAs reads 32 lines of 128 bytes and has every load in flight at
+// once, an L2 latency (some 850 cycles across the dies) a poll.  (Packed, FP32 headers
+// share a line with seven others that are being written: 205 / 192 us a 64-column panel
+// of 20000 rows, 254 / 241 of 40000; FP64, two to a line or four, the same.)
 template <typename T>
 struct Tagged;
 template <>
@@ -295,9 +297,10 @@ __device__ __forceinline__ void panel_update(T* S, int lds, int r0, int nloc, in
 //               step's updates; barrier.
 // What bounds it is that chain: some 2200 of a column's 5000 cycles are the header's
 // way through L2 and its polls, 500 an FP64 division, 800 the scaling and search.
-// us a 64-column panel, with 40- or 64-byte slots polled one after the other / now:
-// FP64 191 / 196 at 4096 rows, 212 / 195 at 6144, 217 / 200 at 8192, 256 / 229 at 16384;
-// FP32 170 / 160 at 8192, 177 / 170 at 16384.
+// us a 64-column panel (a getrf call), with 40- or 64-byte slots polled one after the
+// other / now: FP64 218 / 230 at 4000 rows (polls of two headers a lane), 243 / 230 at 4500,
+// 242 / 230 at 6000, 287 / 258 at 16000; FP32 200 / 180 at 8000, 208 / 192 at 20000, 239 / 241
+// at 40000, 283 / 256 at 80000.
 // The arithmetic and its order per element are those of lair's
 // getrf_row_major (src/lapack/getrf.rs:56-89): 1/p rounded, l = a*(1/p)
 // rounded, a - l*u (separately rounded in exact mode), steps in order.
@@ -396,7 +399,7 @@ __global__ void __launch_bounds__(512, 1) panel_kernel(PanelArgs<T> p) {
         if (lane == 0) {
           unsigned long long h[Tagged<T>::kHead];
           Tagged<T>::pack(ck | sgn, ci, u1, tag, h);
-          st_head(const_cast<unsigned long long*>(heads) + b * Tagged<T>::kHead, h);
+          st_head(const_cast<unsigned long long*>(heads) + b * kPanelHeaderWords, h);
           if (cs >= 0 && j + 1 < w && dj >= 0) S[cs * lds + j + 1] = u1;
         }
       }
@@ -416,7 +419,7 @@ __global__ void __launch_bounds__(512, 1) panel_kernel(PanelArgs<T> p) {
           unsigned long long h[kB][Tagged<T>::kHead];
 #pragma unroll
           for (int e = 0; e < kB; ++e)
-            if (pending & (1u << (q0 + e))) ld_head(heads + (lane + 32 * (q0 + e)) * Tagged<T>::kHead, h[e]);
+            if (pending & (1u << (q0 + e))) ld_head(heads + (lane + 32 * (q0 + e)) * kPanelHeaderWords, h[e]);
 #pragma unroll
           for (int e = 0; e < kB; ++e) {
             if (!(pending & (1u << (q0 + e))) || !Tagged<T>::head_ok(h[e], tag)) continue;

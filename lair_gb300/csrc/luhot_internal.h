@@ -20,11 +20,10 @@ constexpr int kMaxPanelCtas = 256;     // >= SM count
 constexpr int kDefaultPanelWidth = 64; // FP64 / FP32 CUDA-core and DMMA paths
 constexpr int kTcPanelWidth = 128;     // tensor-core (tcgen05) Schur-update path
 constexpr int kMaxPanelWidth = 128;    // sizes the panel kernel's scratch
-// Panel exchange: per step parity and CTA a header of kPanelHeaderWords 8-byte
-// words (Tagged<T> in getrf.cu; all CTAs' headers are contiguous) and, behind all
-// headers, a slot with the candidate row's segment in 8-byte words of (payload,
+// Panel exchange: per step parity and CTA a header (Tagged<T> in getrf.cu) every
+// kPanelHeaderWords 8-byte words and, behind all headers, a slot with the candidate row's segment in 8-byte words of (payload,
 // step tag), two words per FP64 value.
-constexpr int kPanelHeaderWords = 4;
+constexpr int kPanelHeaderWords = 8;
 constexpr int kPanelSlotWords = 2 * kMaxPanelWidth;
 constexpr size_t kPanelSlotBytes =
     2 * (size_t)kMaxPanelCtas * (kPanelHeaderWords + kPanelSlotWords) * sizeof(unsigned long long);
