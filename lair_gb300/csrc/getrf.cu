@@ -1032,7 +1032,7 @@ static int launch_panel(luhot_ctx* ctx, T* a, int64_t lda, int m, int k0, int w,
                         int* moves = nullptr) {
   const int rows = m - k0;
   if (!moves) moves = live_moves(ctx);
-  if (panel_cluster_fits<T>(ctx, rows, w))
+  if (panel_cluster_fits<T, kExact>(ctx, rows, w))
     return launch_panel_cluster<T, kExact>(ctx, a, lda, m, k0, w, piv, moves, stream);
   auto kern = panel_kernel<T, kExact>;
   cudaFuncAttributes fa;
@@ -1274,7 +1274,7 @@ static bool la_pays(luhot_ctx* ctx, const void* oz_ws, int m, int n, int k0, int
   if (sizeof(T) == 4) return M * N >= 500000;
   if (M * N < 1000000) return false;
   const int rows = m - k0 - nb;
-  const bool cluster = panel_cluster_fits<T>(ctx, rows, nb);
+  const bool cluster = panel_cluster_fits<T, false>(ctx, rows, nb);
   const int P = cluster ? ctx->panel_cluster : panel_ctas<T>(ctx, rows);
   const bool slices = update_on_slices(oz_ws, ctx->fp64_update, rows, n - k0 - nb);
   const double rest = (double)M * N * (slices ? 5.0e-6 : 1.16e-4) * nb / 64;
@@ -1315,7 +1315,7 @@ static int la_loop(luhot_ctx* ctx, int m, int n, T* a, int64_t lda, int* piv, in
       OnStream on(ctx, ls);
       LUHOT_CUDA_TRY(ctx, cudaStreamWaitEvent(ls, ctx->la_ev[1], 0));
       ctx->tc_grid_cap =
-          std::max(1, ctx->num_sms - (panel_cluster_fits<T>(ctx, m - k1, nb) ? ctx->panel_cluster : panel_ctas<T>(ctx, m - k1)));
+          std::max(1, ctx->num_sms - (panel_cluster_fits<T, false>(ctx, m - k1, nb) ? ctx->panel_cluster : panel_ctas<T>(ctx, m - k1)));
       const int rc = columns(mv, k0, k0, e1, n, oz_ws, ls);
       ctx->tc_grid_cap = 0;
       if (rc) return rc;
@@ -1353,7 +1353,7 @@ static int getrf_impl(luhot_ctx* ctx, int m, int n, T* a, int64_t lda, int* piv,
   // Exchange words carry step tags; clear them so no word of an earlier
   // factorization carries a live tag.  Cluster panels exchange none, and once a panel
   // fits a cluster all that follow do.
-  if (!panel_cluster_fits<T>(ctx, m, nb))
+  if (!panel_cluster_fits<T, kExact>(ctx, m, nb))
     LUHOT_CUDA_TRY(ctx, cudaMemsetAsync(ctx->panel_scratch, 0, kPanelScratchBytes, stream));
   for (int k0 = 0; k0 < dim_min; k0 += nb) {
     if constexpr (std::is_same<T, double>::value && !kExact) {
@@ -1510,7 +1510,7 @@ int getrf_device(luhot_ctx* ctx, int m, int n, T* a, int64_t lda, int* piv, int 
   // in one cluster than outside (2048 x 128: FP64 0.48 ms as one panel, 0.32 as two;
   // FP32 0.20 either way).
   if (ctx->nb_override <= 0 && n <= kMaxPanelWidth && m >= n && m <= (sizeof(T) == 8 ? 512 : 2048) &&
-      panel_cluster_fits<T>(ctx, m, n))
+      (mode == LUHOT_MODE_EXACT ? panel_cluster_fits<T, true>(ctx, m, n) : panel_cluster_fits<T, false>(ctx, m, n)))
     nb = kMaxPanelWidth;
   void *oz_ws = nullptr, *oz_hi = nullptr;
   if (std::is_same<T, double>::value && mode != LUHOT_MODE_EXACT) {

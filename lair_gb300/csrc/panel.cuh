@@ -134,7 +134,7 @@ __device__ __forceinline__ int warp_best(unsigned long long k, int id) {
 
 // Cooperative form over one thread-block cluster (panel_cluster.cu): whether
 // it takes a panel of `rows` rows and width w, and its launch.
-template <typename T>
+template <typename T, bool kExact>
 bool panel_cluster_fits(luhot_ctx* ctx, int rows, int w);
 template <typename T, bool kExact>
 int launch_panel_cluster(luhot_ctx* ctx, T* a, int64_t lda, int m, int k0, int w, int* piv, int* moves,

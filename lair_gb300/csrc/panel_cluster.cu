@@ -646,7 +646,7 @@ static void cl_split(luhot_ctx* ctx, int rows, int* P, int* rows_per) {
 constexpr size_t kClStaticSmem = 8192;
 
 int panel_cluster_limit(luhot_ctx* ctx) {
-  auto kern = panel_cluster_kernel<double, false, 4>;
+  auto kern = panel_cluster_kernel<double, false, 2>;
   const size_t smem = (size_t)ctx->max_smem_optin - kClStaticSmem;
   if (allow_max_dynamic_smem(kern) != cudaSuccess ||
       allow_wide_clusters(reinterpret_cast<const void*>(kern)) != cudaSuccess) {
@@ -663,21 +663,24 @@ int panel_cluster_limit(luhot_ctx* ctx) {
   return 0;
 }
 
-// Rows of a CTA up to which the cluster is the faster form.  us per column of a
-// 64-column panel, cluster of 16 against the exchange through L2 on up to 96
-// (FP64) or 64 (FP32) CTAs: FP64 1.1 / 2.5 at 512 rows, 1.5 / 2.5 at 1024, 2.2 /
-// 2.6 at 2048, 2.7 / 2.9 at 2560, 3.0 / 3.0 at 3072, 3.6 / 3.0 at 4096 (the rank-1
-// updates of 256 rows fill one SM's FP64 pipes); FP32 1.1 / 2.3 at 1024, 1.4 / 2.3
-// at 2048, 1.7 / 2.4 at 4096, 2.5 / 2.4 at 8192.
-constexpr int kClRowsF64 = 160, kClRowsF32 = 384;
-static_assert(kClRowsF64 <= 4 * kClOwnRows && kClRowsF32 <= 4 * kClOwnRows, "an owner thread holds at most four rows");
+// Rows of a CTA up to which the cluster is the faster form.  us a 64-column panel (a
+// getrf call), cluster of 16 / exchange through L2 on up to 96 (FP64) or 64 (FP32)
+// CTAs: FP64 fast 166 / 235 at 2000 rows, 193 / 233 at 2500, 200 / 230 at 2600, 212 / 230
+// at 3000, 225 / 230 at 3200, 237 / 230 at 3500 (the rank-1 updates of 200 rows fill one
+// SM's FP64 pipes); exact, whose updates are two operations, 200 / 240 at 1500, 225 / 240 at
+// 1700, 239 / 241 at 2000, 286 / 242 at 2500; FP32, either mode, 116 / 180 at 2000, 150 / 181
+// at 5000, 165 / 180 at 6000.
+template <typename T, bool kExact>
+constexpr int cl_max_rows() {
+  return sizeof(T) == 4 ? 384 : kExact ? 125 : 192;
+}
 
-template <typename T>
+template <typename T, bool kExact>
 bool panel_cluster_fits(luhot_ctx* ctx, int rows, int w) {
   if (ctx->panel_cluster < 1 || w > kMaxPanelWidth || rows < 1) return false;
   int P, rows_per;
   cl_split<T>(ctx, rows, &P, &rows_per);
-  return rows_per <= (sizeof(T) == 8 ? kClRowsF64 : kClRowsF32) && cl_smem_bytes<T>(rows_per, w) + kClStaticSmem <= (size_t)ctx->max_smem_optin;
+  return rows_per <= cl_max_rows<T, kExact>() && cl_smem_bytes<T>(rows_per, w) + kClStaticSmem <= (size_t)ctx->max_smem_optin;
 }
 
 template <typename T, bool kExact>
@@ -686,9 +689,13 @@ int launch_panel_cluster(luhot_ctx* ctx, T* a, int64_t lda, int m, int k0, int w
   const int rows = m - k0;
   int P, rows_per;
   cl_split<T>(ctx, rows, &P, &rows_per);
-  auto kern = rows_per <= kClOwnRows       ? panel_cluster_kernel<T, kExact, 1>
-              : rows_per <= 2 * kClOwnRows ? panel_cluster_kernel<T, kExact, 2>
-                                           : panel_cluster_kernel<T, kExact, 4>;
+  constexpr int kMost = cl_max_rows<T, kExact>();  // owner threads hold kMost / kClOwnRows rows at most
+  static_assert(kMost <= 4 * kClOwnRows, "an owner thread holds at most four rows");
+  auto kern = panel_cluster_kernel<T, kExact, 1>;
+  if constexpr (kMost > kClOwnRows)
+    if (rows_per > kClOwnRows) kern = panel_cluster_kernel<T, kExact, 2>;
+  if constexpr (kMost > 2 * kClOwnRows)
+    if (rows_per > 2 * kClOwnRows) kern = panel_cluster_kernel<T, kExact, 4>;
   LUHOT_CUDA_TRY(ctx, allow_max_dynamic_smem(kern));
   LUHOT_CUDA_TRY(ctx, allow_wide_clusters(reinterpret_cast<const void*>(kern)));
   PanelArgs<T> args{};
@@ -713,8 +720,10 @@ int launch_panel_cluster(luhot_ctx* ctx, T* a, int64_t lda, int m, int k0, int w
   return LUHOT_OK;
 }
 
-template bool panel_cluster_fits<double>(luhot_ctx*, int, int);
-template bool panel_cluster_fits<float>(luhot_ctx*, int, int);
+template bool panel_cluster_fits<double, false>(luhot_ctx*, int, int);
+template bool panel_cluster_fits<double, true>(luhot_ctx*, int, int);
+template bool panel_cluster_fits<float, false>(luhot_ctx*, int, int);
+template bool panel_cluster_fits<float, true>(luhot_ctx*, int, int);
 template int launch_panel_cluster<double, false>(luhot_ctx*, double*, int64_t, int, int, int, int*, int*, cudaStream_t);
 template int launch_panel_cluster<double, true>(luhot_ctx*, double*, int64_t, int, int, int, int*, int*, cudaStream_t);
 template int launch_panel_cluster<float, false>(luhot_ctx*, float*, int64_t, int, int, int, int*, int*, cudaStream_t);
