@@ -222,6 +222,154 @@ __global__ void __launch_bounds__(tc_threads<kNR>())
   if (!ok) cl_drain();
 }
 
+// Wide chains of transposed FP32 sweeps (four right-hand sides).  A row of a tile is a
+// column of memory there, so that a load takes a line for every column of the tile
+// among its lanes; a thread has all four right-hand sides of its row, a quarter of the
+// loads: 16 rows x 16 parts of 4 columns, a warp on 16 rows and two columns (64 bytes
+// of two lines a load), sums over the parts by shuffle and over the warps in shared
+// memory.  Otherwise as above.  Two sweeps with 16 right-hand sides, us, one CTA a
+// block with flags / a sum a thread / so: n = 4097 535 / 388 / 260, 8000 1400 / 1343 / 581,
+// 16384 3413 / 4829 / 1700.
+template <bool kLower>
+__global__ void __launch_bounds__(256)
+    trsv_cluster_wide_kernel(const float* __restrict__ a, int64_t lda, float* x, int64_t ldx, int n, int nrhs,
+                             int nchain, const float* __restrict__ dinv, unsigned long long* xt, unsigned epoch,
+                             int* ticket, DeviceStatus* st) {
+  using Word = TcWord<float>;
+  constexpr int kNR = 4, kThreads = 256, kParts = kThreads / kTRows, kLen = kTB / kParts;
+  constexpr int kVals = kTB * kNR, kOut = kTRows * kNR;  // values of a block, of a CTA
+  static_assert(kVals == kThreads && kOut * kTCtas == kThreads, "a thread polls a value and sends one to a peer");
+  constexpr unsigned kFull = 0xffffffffu;
+  __shared__ __align__(16) float xs[2][kVals];                     // x(J), [k][c]
+  __shared__ __align__(16) float red[2][kThreads / 32][kOut];      // the warps' sums, of both products
+  __shared__ unsigned long long sums[kVals];                       // the block's sums, [row][c]
+  __shared__ __align__(8) unsigned long long bar;
+  __shared__ int s_ticket;
+  const int tid = threadIdx.x;
+  const int rank = blockIdx.x & (kTCtas - 1);
+  const int nblk = (n + kTB - 1) / kTB;
+  if (tid == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(cl_smem(&bar)));
+    asm volatile("fence.mbarrier_init.release.cluster;");
+    cl_expect(cl_smem(&bar), (unsigned)kVals * 8u);
+    if (rank == 0) {
+      const int t = atomicAdd(ticket, 1);
+      for (int r = 0; r < kTCtas; ++r)
+        asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cl_peer(cl_smem(&s_ticket), r)), "r"(t) : "memory");
+    }
+  }
+  cl_sync();
+  const int chain = s_ticket % nchain, t = s_ticket / nchain;
+  x += chain * kNR;
+  nrhs = min(kNR, nrhs - chain * kNR);
+  xt += (size_t)chain * nblk * kVals;
+  const int I = kLower ? t : nblk - 1 - t;
+  const int part = tid / kTRows, r = rank * kTRows + tid % kTRows;
+  const int row = I * kTB + r;
+  const int nupd = kLower ? I : nblk - 1 - I;  // blocks before I in sweep order
+  auto block = [&](int s) { return kLower ? s : nblk - 1 - s; };
+  auto load_tile = [&](int J, float(&v)[kLen]) {
+#pragma unroll
+    for (int e = 0; e < kLen; ++e) {
+      const int k = J * kTB + part + kParts * e;
+      v[e] = row < n && k < n ? a[(int64_t)k * lda + row] : 0.0f;
+    }
+  };
+  const bool polls = tid % kNR < nrhs;
+  auto word = [&](int J) { return xt + (size_t)J * kVals + tid; };
+  float d[kLen], v[kLen], acc[kNR];
+#pragma unroll
+  for (int e = 0; e < kLen; ++e) d[e] = dinv[(size_t)I * kTB * kTB + (part + kParts * e) * kTB + r];
+#pragma unroll
+  for (int c = 0; c < kNR; ++c) acc[c] = part == 0 && row < n && c < nrhs ? x[(int64_t)row * ldx + c] : 0.0f;
+  unsigned long long w[1];
+  bool ok = true;
+  if (nupd > 0) {
+    load_tile(block(0), v);
+    if (polls) Word::load(word(block(0)), w);
+  }
+  for (int s = 0; s < nupd; ++s) {
+    const int J = block(s);
+    float xv = 0.0f;
+    if (polls && J * kTB + tid / kNR < n) {
+      unsigned long long t0 = 0;
+      unsigned spins = 0;
+      while (!Word::ok(w, epoch)) {
+        Word::load(word(J), w);
+        if ((++spins & 31u) == 0) {
+          const unsigned long long now = global_timer_ns();
+          if (t0 == 0) t0 = now;
+          const bool late = now - t0 > st->timeout_ns;
+          if (late) {
+            atomicCAS(&st->error, kDevOk, kDevBarrierTimeout);
+            atomicExch(&st->timeout_where, (unsigned long long)J);
+            atomicExch(&st->abort, 1);
+          }
+          if (late || ld_relaxed_i32(&st->abort)) {
+            ok = false;
+            break;
+          }
+        }
+      }
+      xv = Word::value(w);
+    }
+    xs[s & 1][tid] = xv;
+    float nv[kLen];
+    if (s + 1 < nupd) {
+      load_tile(block(s + 1), nv);
+      if (polls) Word::load(word(block(s + 1)), w);
+    }
+    ok = __syncthreads_or(!ok) == 0;
+    if (!ok) break;
+#pragma unroll
+    for (int e = 0; e < kLen; ++e) {
+      const float4 xk = *reinterpret_cast<const float4*>(&xs[s & 1][(part + kParts * e) * kNR]);
+      acc[0] = fmaf(-v[e], xk.x, acc[0]);
+      acc[1] = fmaf(-v[e], xk.y, acc[1]);
+      acc[2] = fmaf(-v[e], xk.z, acc[2]);
+      acc[3] = fmaf(-v[e], xk.w, acc[3]);
+    }
+    if (s + 1 < nupd) {
+#pragma unroll
+      for (int e = 0; e < kLen; ++e) v[e] = nv[e];
+    }
+  }
+  if (ok) {
+    // Sums over the parts, to thread t for value t % kOut of the CTA and peer t / kOut.
+    auto over_parts = [&](float(&sum)[kNR], int buf) {
+#pragma unroll
+      for (int c = 0; c < kNR; ++c) sum[c] += __shfl_xor_sync(kFull, sum[c], kTRows);
+      if ((tid & 31) < kTRows)
+        *reinterpret_cast<float4*>(&red[buf][tid >> 5][(tid & 31) * kNR]) = make_float4(sum[0], sum[1], sum[2], sum[3]);
+      __syncthreads();
+      float total = 0.0f;
+#pragma unroll
+      for (int q = 0; q < kThreads / 32; ++q) total += red[buf][q][tid % kOut];
+      return total;
+    };
+    const int vr = rank * kTRows + tid % kOut / kNR, vc = tid % kNR, peer = tid / kOut, vrow = I * kTB + vr;
+    const bool on = vrow < n && vc < nrhs;
+    const float sum = over_parts(acc, 0);
+    cl_push8(cl_peer(cl_smem(&sums[vr * kNR + vc]), peer), cl_peer(cl_smem(&bar), peer), Word::bits(on ? sum : 0.0f));
+    // All warps alike: there is a barrier ahead.
+    ok = __syncthreads_and(cl_wait(cl_smem(&bar), 0u, st, I)) != 0;
+    if (ok) {
+      float y[kNR] = {};
+#pragma unroll
+      for (int e = 0; e < kLen; ++e)
+#pragma unroll
+        for (int c = 0; c < kNR; ++c) y[c] = fmaf(d[e], Word::from(sums[(part + kParts * e) * kNR + c]), y[c]);
+      const float out = over_parts(y, 1);
+      if (on && peer == 0) {
+        Word::store(xt + (size_t)I * kVals + vr * kNR + vc, out, epoch);
+        x[(int64_t)vrow * ldx + vc] = out;
+      }
+    }
+  }
+  cl_sync();  // as above
+  if (!ok) cl_drain();
+}
+
 // Right-hand sides of one chain (at most 16 chains run in a launch).  FP64 sweeps
 // run every right-hand side as a chain of its own: they are bound by the chain or,
 // with many, by the FP64 pipes, whatever the width.  FP32 sweeps of much work read
@@ -255,8 +403,18 @@ template <typename T, typename TA, bool LO, bool TR>
 static cudaError_t launch_dir(cudaStream_t stream, const TA* a, int64_t lda, T* x, int64_t ldx, int n, int nc,
                               const T* dinv, unsigned long long* xt, unsigned epoch, int* ticket, DeviceStatus* st) {
   if constexpr (sizeof(T) == 4) {
-    if (tc_width<T>(n, nc) == 4)
-      return launch_nr<T, TA, LO, TR, 4>(stream, a, lda, x, ldx, n, nc, dinv, xt, epoch, ticket, st);
+    if (tc_width<T>(n, nc) == 4) {
+      if constexpr (TR) {
+        const int nchain = (nc + 3) / 4;
+        cudaLaunchAttribute attr;
+        cudaLaunchConfig_t cfg = cl_config(kTCtas, 256, 0, stream, &attr);
+        cfg.gridDim = dim3(kTCtas * trsv_syncfree_blocks(n) * nchain);
+        return cudaLaunchKernelEx(&cfg, trsv_cluster_wide_kernel<LO>, a, lda, x, ldx, n, nc, nchain, dinv, xt, epoch,
+                                  ticket, st);
+      } else {
+        return launch_nr<T, TA, LO, TR, 4>(stream, a, lda, x, ldx, n, nc, dinv, xt, epoch, ticket, st);
+      }
+    }
   }
   return launch_nr<T, TA, LO, TR, 1>(stream, a, lda, x, ldx, n, nc, dinv, xt, epoch, ticket, st);
 }
