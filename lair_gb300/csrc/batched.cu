@@ -463,16 +463,21 @@ __device__ __forceinline__ void batch_back(T* S, int ld, int n, const int* prow,
     if (lane + 32 * q < n) xg[lane + 32 * q] = x[q];
 }
 
-// Threads of a CTA, and CTAs an SM's registers must hold.
+// Threads of a CTA, and CTAs an SM's registers must hold.  (kLone: in a plan of no more
+// systems than SMs each has an SM, and FP64 systems of more than 128 rows in scratch
+// take eight warps, and all its registers, to cover the latency of L2: one of 256 rows
+// 2996 -> 2125 us, 152 of them 3209 -> 2256.)
 __host__ __device__ constexpr int batch_max_threads(size_t elem, int ni) { return elem == 4 && ni == 8 ? 256 : 128; }
 __host__ __device__ constexpr int batch_min_ctas(size_t elem, int ni) {
   return ni <= 2 ? 5 : elem == 4 ? (ni == 4 ? 4 : 2) : (ni == 4 ? 3 : 2);
 }
 
 // kScratch: the matrix lives in this CTA's part of `scratch`.
-template <typename T, bool kExact, int NI, bool kScratch>
-__global__ void __launch_bounds__(batch_max_threads(sizeof(T), NI), batch_min_ctas(sizeof(T), NI)) batched_lu_kernel(BatchMeta m, T* a, T* b, int* piv, int* info, int* counter,
-                                                         T* scratch) {
+constexpr int kLoneThreads = 256;
+template <typename T, bool kExact, int NI, bool kScratch, bool kLone = false>
+__global__ void __launch_bounds__(kLone ? kLoneThreads : batch_max_threads(sizeof(T), NI),
+                                  kLone ? 1 : batch_min_ctas(sizeof(T), NI))
+    batched_lu_kernel(BatchMeta m, T* a, T* b, int* piv, int* info, int* counter, T* scratch) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int prow[kBatchMaxN], act[kBatchMaxN], slid[kBatchMaxN];
   __shared__ __align__(16) T pv[batch_nb<T>(NI) * batch_nb<T>(NI)];
@@ -545,6 +550,7 @@ struct BatchClass {
   int first = 0, count = 0;
   int ni = 1;            // rows of a panel lane
   bool scratch = false;
+  bool lone = false;     // an SM to each system (kLone)
   int threads = 0, grid = 0;
   size_t smem = 0;
 };
@@ -606,8 +612,11 @@ static const void* batch_kernel_of(int ni, bool scratch) {
          : ni == 4 ? (const void*)batched_lu_kernel<T, kExact, 4, false>
                    : (const void*)batched_lu_kernel<T, kExact, 8, false>;
 }
-static const void* batch_kernel(int dtype, int mode, int ni, bool scratch) {
+static const void* batch_kernel(int dtype, int mode, int ni, bool scratch, bool lone) {
   const bool ex = mode == LUHOT_MODE_EXACT;
+  if (lone)
+    return ex ? (const void*)batched_lu_kernel<double, true, 8, true, true>
+              : (const void*)batched_lu_kernel<double, false, 8, true, true>;
   if (dtype == 0)
     return ex ? batch_kernel_of<double, true>(ni, scratch) : batch_kernel_of<double, false>(ni, scratch);
   return ex ? batch_kernel_of<float, true>(ni, scratch) : batch_kernel_of<float, false>(ni, scratch);
@@ -615,8 +624,9 @@ static const void* batch_kernel(int dtype, int mode, int ni, bool scratch) {
 
 // Orders the systems (indices into sizes) by class, largest class and largest
 // system first.  A class is a panel form (NI) and the number of its largest
-// matrices that fit in an SM's shared memory (or the scratch form).
-static void build_classes(luhot_ctx* ctx, int dtype, int mode, const int* tune, int smem_n,
+// matrices that fit in an SM's shared memory (or the scratch form).  few: the plan
+// has no more systems than SMs.
+static void build_classes(luhot_ctx* ctx, int dtype, int mode, const int* tune, int smem_n, bool few,
                           const std::vector<int>& sizes, std::vector<int>& order, std::vector<BatchClass>& classes) {
   auto key_of = [&](int n) {
     const int ni = n <= 32 ? 1 : n <= 64 ? 2 : n <= 128 ? 4 : 8;
@@ -657,8 +667,9 @@ static void build_classes(luhot_ctx* ctx, int dtype, int mode, const int* tune, 
     c.scratch = k % 16 == 0;
     c.smem = c.scratch ? 0 : smem_bytes(dtype, n);  // the class's first system is its largest
     // Few matrices of more than 128 rows fit in an SM's shared memory: 8 warps each.
-    c.threads = c.scratch ? 128 : batch_max_threads(elem_size(dtype), c.ni);
-    const void* kern = batch_kernel(dtype, mode, c.ni, c.scratch);
+    c.lone = few && dtype == 0 && c.ni == 8 && c.scratch;
+    c.threads = c.lone ? kLoneThreads : c.scratch ? 128 : batch_max_threads(elem_size(dtype), c.ni);
+    const void* kern = batch_kernel(dtype, mode, c.ni, c.scratch, c.lone);
     allow_max_dynamic_smem(kern);
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, c.threads, c.smem) != cudaSuccess) {
@@ -718,7 +729,7 @@ static cudaError_t launch_classes(luhot_batch* p, const std::vector<BatchClass>&
     if (c.scratch) sp += (size_t)c.grid * kScratchElems * elem_size(p->dtype);
     void* args[] = {&cm, &a, &b, &piv, &info, &counter, &cs};
     const int q = (int)(i % kBatchStreams);
-    e = cudaLaunchKernel(batch_kernel(p->dtype, p->mode, c.ni, c.scratch), dim3(c.grid), dim3(c.threads), args, c.smem,
+    e = cudaLaunchKernel(batch_kernel(p->dtype, p->mode, c.ni, c.scratch, c.lone), dim3(c.grid), dim3(c.threads), args, c.smem,
                          q == 0 ? stream : p->branch[q - 1]);
   }
   for (int q = 0; q < nb; ++q) {  // the join, also after an error
@@ -739,7 +750,7 @@ static size_t scratch_ctas(const std::vector<BatchClass>& classes) {
 static int upload_meta(luhot_batch* p) {
   luhot_ctx* ctx = p->ctx;
   const size_t c = (size_t)p->count;
-  build_classes(ctx, p->dtype, p->mode, p->tune, p->smem_n, p->sizes, p->order, p->classes);
+  build_classes(ctx, p->dtype, p->mode, p->tune, p->smem_n, p->count <= ctx->num_sms, p->sizes, p->order, p->classes);
   if ((int)p->classes.size() > kMaxBatchClasses) return set_error(ctx, LUHOT_ERR_UNSUPPORTED, "batch: too many size classes");
   int rc = make_branches(p, p->classes);
   if (rc) return rc;
@@ -1008,7 +1019,7 @@ int luhot_batch_autotune(luhot_batch* p, const void* d_a, const void* d_b) {
       for (int q = 0; q < kBuckets; ++q) tune_all[q] = form;
       std::vector<int> order;
       std::vector<BatchClass> classes;
-      build_classes(ctx, p->dtype, p->mode, tune_all, p->smem_n, b_sizes, order, classes);
+      build_classes(ctx, p->dtype, p->mode, tune_all, p->smem_n, p->count <= ctx->num_sms, b_sizes, order, classes);
       rc = make_branches(p, classes);
       if (rc) break;
       for (auto& q : order) q += first;
