@@ -667,12 +667,12 @@ int panel_cluster_limit(luhot_ctx* ctx) {
 // getrf call), cluster of 16 / exchange through L2 on up to 96 (FP64) or 64 (FP32)
 // CTAs: FP64 fast 166 / 235 at 2000 rows, 193 / 233 at 2500, 200 / 230 at 2600, 212 / 230
 // at 3000, 225 / 230 at 3200, 237 / 230 at 3500 (the rank-1 updates of 200 rows fill one
-// SM's FP64 pipes); exact, whose updates are two operations, 200 / 240 at 1500, 225 / 240 at
-// 1700, 239 / 241 at 2000, 286 / 242 at 2500; FP32, either mode, 116 / 180 at 2000, 150 / 181
+// SM's FP64 pipes); exact, whose updates are two operations, 200 / 231 at 1500, 225 / 231 at
+// 1700, 239 / 231 at 2000, 286 / 230 at 2500; FP32, either mode, 116 / 180 at 2000, 150 / 181
 // at 5000, 165 / 180 at 6000.
 template <typename T, bool kExact>
 constexpr int cl_max_rows() {
-  return sizeof(T) == 4 ? 384 : kExact ? 125 : 192;
+  return sizeof(T) == 4 ? 384 : kExact ? 112 : 192;
 }
 
 template <typename T, bool kExact>

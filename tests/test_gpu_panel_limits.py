@@ -1,5 +1,5 @@
 """Around the rows up to which a panel runs in one cluster (panel_cluster.cu: FP64 3072
-rows in fast mode and 2000 in exact mode, FP32 6144): exact mode bit for bit against
+rows in fast mode and 1792 in exact mode, FP32 6144): exact mode bit for bit against
 the oracle, fast mode with one and two rows per owner thread against the
 definition and exact mode's pivots (lair's getrf, src/lapack/getrf.rs:46-120)."""
 import numpy as np
@@ -11,7 +11,7 @@ from lair_gb300 import lapack
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("m,n", [(1985, 64), (2000, 64), (2001, 64), (2000, 33), (2017, 70)])
+@pytest.mark.parametrize("m,n", [(1777, 64), (1792, 64), (1793, 64), (1792, 33), (1821, 70), (2000, 64), (3841, 64)])
 def test_exact_limit_bitwise(m, n):
     a = np.random.default_rng(m).uniform(-1, 1, (m, n))
     ref = a.copy()
