@@ -30,8 +30,10 @@
 //
 // 10 000 FP32 systems of n ~ U{8..256} 15.0 -> 8.0 ms, 1500 FP64 7.3 -> 6.0 ms,
 // against one 256-thread CTA per system with a block-wide search and four barriers
-// per column.  FP64 is within 1.5 of its pipe's 4.1 ms; FP32 is bound by the
-// panel warp (about 1100 cycles a step, instruction fetches among them).
+// per column.  FP64 is within 1.5 of its pipe's 4.1 ms.  FP32: the panel warps' steps (about
+// 1100 cycles each, instruction fetches among them) are some 3 of the 8 ms; updates,
+// U12 and copies run in turn with them in the same CTA, and systems of 164 to 235 rows
+// have an SM to themselves.
 #include <algorithm>
 #include <climits>
 #include <cstring>

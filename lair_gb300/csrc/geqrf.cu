@@ -17,9 +17,8 @@
 // the dot of each column of C with v summed in increasing row order, every
 // product and sum rounded apart (results are bit-identical to lair).  Fast
 // mode sums in trees and uses FMA.  This level-2 form reads the trailing
-// block twice and writes it once per column (~24 bytes per element); a
-// blocked (compact-WY) form would move the two updates onto the FP64 tensor
-// pipe.
+// block twice and writes it once per column (~24 bytes per element); fast FP64
+// factors whose panels fit a cluster go blocked (geqrf_blocked.cu).
 #include <algorithm>
 #include <cmath>
 #include <string>

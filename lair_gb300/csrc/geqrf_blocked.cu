@@ -233,11 +233,7 @@ __global__ void __launch_bounds__(kQbThreads, 1) qr_panel_kernel(QrPanelArgs p) 
     }
   }
   cl_sync();  // every push has been received, or its wait was given up
-  if (!s_ok) {
-    const unsigned long long t0 = global_timer_ns();
-    while (global_timer_ns() - t0 < 200000ull) __nanosleep(1000);
-    cl_sync();
-  }
+  if (!s_ok) cl_drain();
 }
 
 __device__ __forceinline__ void qr_dmma(double& d0, double& d1, double a, double b) {

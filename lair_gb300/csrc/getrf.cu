@@ -26,8 +26,9 @@
 //          increasing elimination-step order, which is exactly the sequence
 //          of lair's getrf_row_major (src/lapack/getrf.rs:76-89).  Blocking
 //          only moves data, so results are bit-identical to lair.
-//   fast:  the Schur update runs on the FP64 tensor cores (DMMA,
-//          mma.sync m8n8k4) and the other kernels use FMA.
+//   fast:  the FP64 Schur update runs as integer slice products on the FP16 tensor
+//          cores (ozaki.cu) for trailing blocks of at least 256 x 256, else on the
+//          FP64 tensor cores (DMMA, mma.sync m8n8k4); the other kernels use FMA.
 #include <cooperative_groups.h>
 
 #include <algorithm>

@@ -472,15 +472,14 @@ int getrs_apply(luhot_ctx* ctx, int n, int nrhs, const T* lu, int64_t lda, const
     // op(A) upper: U, or L^T (the kernel reads a given inverse transposed).
     const T* dinv = ex ? nullptr : ((lower != tr) ? dinv_l : dinv_u);
     cudaError_t e = cudaSuccess;
-    if (dinv) {
-      const int rc_ = cluster_sweep<T, T>(ctx, lu, lda, w, ldw, n, nrhs, lower, tr, dinv);
-      if (rc_) return rc_;
-    } else {
+    int rc_ = LUHOT_OK;
+    if (dinv)
+      rc_ = cluster_sweep<T, T>(ctx, lu, lda, w, ldw, n, nrhs, lower, tr, dinv);
+    else
       e = launch_trsv_syncfree<T>(stream, lu, lda, w, ldw, n, nrhs, lower, unit, tr, ex, flags, ticket, ctx->d_status);
-    }
     prof_end(ctx, kProfTrsv, (double)n * n * nrhs, ((double)n * n / 2 + 2.0 * total) * sizeof(T));
     if (e != cudaSuccess) return set_error(ctx, LUHOT_ERR_CUDA, std::string("getrs sweep: ") + cudaGetErrorString(e));
-    return LUHOT_OK;
+    return rc_;
   };
   if (!trans) {
     prof_begin(ctx, kProfPermute);
@@ -540,7 +539,7 @@ int getrs_device(luhot_ctx* ctx, int n, int nrhs, const T* lu, int64_t lda, cons
   rc = ensure_buf(ctx, ctx->work[3], (size_t)n * nrhs * sizeof(T));
   if (rc) return rc;
   // Fast solves use the inverses of the diagonal blocks (read transposed by
-  // the transposed sweeps); one small launch (64 threads per block) against
+  // the transposed sweeps); one small launch (a warp per column of a block) against
   // two n^2 sweeps.
   T* dinv_l = nullptr;
   T* dinv_u = nullptr;

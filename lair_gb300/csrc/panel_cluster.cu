@@ -23,7 +23,7 @@
 //   segment, the candidate's column j+2, then the push; the other rows' column
 //   j+2 while that is under way.
 // The divider (FP64) forms the candidates' reciprocals as soon as they are known
-// and adds them to their headers: a division is 340 cycles of dependent operations,
+// and adds them to their headers: a division is some 340 cycles of dependent operations,
 // which on the winner's side of the exchange would be the longest link.
 // The helper brings the candidates' rows up to date while their headers
 //   travel, arms the barriers, pushes the segment if this CTA won (its first 16
@@ -39,9 +39,9 @@
 // at one instruction every four cycles or so: no array of it is indexed by a
 // variable (such arrays live in local memory, whose lines the waits' acquire
 // discards), nor is there an integer division, and the waits' loops are out of line.
-// us a 64-column panel, before / now: FP64 75.6 / 61 at 64 rows, 77 / 64 at 256,
-// 82 / 71 at 512, 100 / 96 at 1024, 156 / 143 at 2048; FP32 61.4 / 59 at 64, 69 / 63
-// at 512, 73 / 68 at 1024, 91 / 92 at 2048.
+// us a 64-column panel (the launch alone), with the divider and without local arrays:
+// FP64 75.6 -> 61 at 64 rows, 77 -> 64 at 256, 82 -> 71 at 512, 100 -> 96 at 1024, 156 ->
+// 143 at 2048; FP32 61.4 -> 59 at 64, 69 -> 63 at 512, 73 -> 68 at 1024, 91 -> 92 at 2048.
 //
 // Reuse of the exchange buffers (two, by step parity): a warp pushes step j+2
 // only after it has every header of step j+1, and a warp sends that header only
@@ -563,7 +563,7 @@ __global__ void __launch_bounds__(cl_threads<T>(), 1) panel_cluster_kernel(Panel
   } else if (role == kDivide) {
     // ------------------------------------------------------------ divider
     // The candidates' reciprocals, while their headers are still being prepared.
-    // A division is some 430 cycles of dependent operations: on the winner's
+    // A division is some 340 cycles of dependent operations: on the winner's
     // side of the exchange it would be the longest link of the chain.
     if constexpr (kDivider) {
       // Lane (q, cta) pushes candidate q's (and q + 2's) to peer cta.
@@ -621,12 +621,7 @@ __global__ void __launch_bounds__(cl_threads<T>(), 1) panel_cluster_kernel(Panel
     }
   }
   cl_sync();  // every CTA's pushes have been received, or its waits were given up
-  if (!s_ok) {
-    // A push of a CTA that went on may still be under way: let it land.
-    const unsigned long long t0 = global_timer_ns();
-    while (global_timer_ns() - t0 < 200000ull) __nanosleep(1000);
-    cl_sync();
-  }
+  if (!s_ok) cl_drain();
 }
 
 // ---------------------------------------------------------------------------
