@@ -850,7 +850,7 @@ def run_qr(args, lib, ctx, torch):
     return {"workload": f"Householder QR (geqrf, fast mode) of an n x n N(0,1) matrix, n={n}", "n": n,
             "ms": ms, "gflops": 4.0 / 3.0 * n ** 3 / (ms * 1e-3) / 1e9,
             "residual_max_rel": resid, "orthogonality_max": orth,
-            "bound": "FP64 pipe (panels and W = V^T A of the blocked form; the updates run on the FP16 slices)"}
+            "bound": "FP64 pipe (panels, W = V^T A and updates of the blocked form)"}
 
 
 def run_batched(args, lib, ctx, torch):
