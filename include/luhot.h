@@ -318,7 +318,9 @@ void luhot_factor_destroy(luhot_factor* f);
  * strides) is overwritten by R on and above the diagonal and the reflectors
  * below it; tau receives min(m, n) scalars.  LUHOT_MODE_EXACT reproduces
  * lair's arithmetic (larfg's sequential nrm2, larf's increasing-row dots,
- * separately rounded products and sums) bit for bit. */
+ * separately rounded products and sums) bit for bit.  LUHOT_MODE_FAST takes a
+ * blocked form for FP64 with min(m, n) >= 32 and all elements finite; a NaN or an
+ * infinity reaches the same elements of R and tau as in lair. */
 int luhot_dgeqrf(luhot_ctx* ctx, int64_t m, int64_t n, double* a, int64_t rs, int64_t cs, double* tau, int mode);
 int luhot_sgeqrf(luhot_ctx* ctx, int64_t m, int64_t n, float* a, int64_t rs, int64_t cs, float* tau, int mode);
 /* Same on a row-major device matrix (leading dimension lda) and device tau.

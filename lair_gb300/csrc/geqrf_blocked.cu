@@ -394,6 +394,20 @@ __global__ void __launch_bounds__(128) qr_update_kernel(double* c, int64_t ldc, 
       }
 }
 
+// st->singular = 0 if an element of A is NaN or infinite: a warp a row, so that the
+// loads are whole lines whatever lda is.
+__global__ void __launch_bounds__(256) qr_finite_kernel(const double* __restrict__ a, int64_t lda, int m, int n,
+                                                        DeviceStatus* st) {
+  const int lane = threadIdx.x & 31;
+  bool bad = false;
+  for (int r = blockIdx.x * 8 + (threadIdx.x >> 5); r < m; r += gridDim.x * 8) {
+    const double* row = a + (int64_t)r * lda;
+#pragma unroll 4
+    for (int c = lane; c < n; c += 32) bad |= !isfinite(row[c]);
+  }
+  if (__any_sync(0xffffffffu, bad) && lane == 0) st->singular = 0;
+}
+
 size_t panel_smem(int rows_per) { return (size_t)rows_per * kQbLd * sizeof(double); }
 
 // CTAs: a power of two with at least 16 rows each.
@@ -417,6 +431,17 @@ bool geqrf_blocked_fits(luhot_ctx* ctx, int m, int n) {
   int P, rows_per;
   panel_split(ctx, m, &P, &rows_per);
   return panel_smem(rows_per) + kQbStatic <= (size_t)ctx->max_smem_optin;
+}
+
+int geqrf_all_finite(luhot_ctx* ctx, int m, int n, const double* a, int64_t lda, bool* finite) {
+  int rc = reset_status(ctx);
+  if (rc) return rc;
+  qr_finite_kernel<<<std::min((m + 7) / 8, 8 * ctx->num_sms), 256, 0, ctx->stream>>>(a, lda, m, n, ctx->d_status);
+  LUHOT_CUDA_TRY(ctx, cudaGetLastError());
+  int64_t first = -1;
+  rc = finish_status(ctx, &first);
+  *finite = first < 0;
+  return rc;
 }
 
 int geqrf_blocked(luhot_ctx* ctx, int m, int n, double* a, int64_t lda, double* tau) {

@@ -130,6 +130,8 @@ int copy_2d(luhot_ctx* ctx, void* dst, size_t dpitch, const void* src, size_t sp
 // for its result and reads the device status.
 bool geqrf_blocked_fits(luhot_ctx* ctx, int m, int n);
 int geqrf_blocked(luhot_ctx* ctx, int m, int n, double* a, int64_t lda, double* tau);
+// *finite: no element of the device matrix is NaN or infinite (waits for the answer).
+int geqrf_all_finite(luhot_ctx* ctx, int m, int n, const double* a, int64_t lda, bool* finite);
 
 // Largest power-of-two cluster in which the cluster form of the panel
 // (panel_cluster.cu) can run with its full shared memory, 0 if none.
